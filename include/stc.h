@@ -102,7 +102,8 @@ typedef struct stc_config {
    * depend on it: new meetings take their slots by priority, not by
    * arrival). */
   uint32_t job_chunk;            /* refinement jobs (32 rows against their candidate ranges) a warp
-                                    takes at a time; 0 = 8, at most 64 */
+                                    takes at a time, fewer when there are too few to go round;
+                                    0 = 8, at most 64 */
   uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 = 8, at most 32 */
   uint32_t hits_blocks_per_sm;   /* table-update blocks launched per SM; 0 = 16, at most 64 */
   uint32_t window_graphs;        /* stc_step_window replays each step from a captured CUDA graph:
@@ -118,8 +119,9 @@ typedef struct stc_config {
   uint32_t refine_chunk;         /* refinement tile length: a job tests 32 rows against this many
                                     positions of their candidate windows (launch shape, results do
                                     not depend on it); a multiple of 32 from 32 to 4096; 0 =
-                                    automatic, per step: 64 when the step before tested more than 16
-                                    candidates per checking unit (dense leaves), else 256 */
+                                    automatic, per step: 32 when there are too few rows to fill the
+                                    GPU several times over, 64 when the step before tested more than
+                                    16 candidates per checking unit (dense leaves), else 256 */
 } stc_config;
 
 /* Replay quadtree splits/merges on one device thread only (tests compare it

@@ -717,21 +717,27 @@ static void choose_hit_emission(stc_ctx *c) {
   }
 }
 
-// Tile length of the refinement's jobs when stc_config.refine_chunk is 0:
-// 64 candidates when the last step tested more than 16 candidates per
-// checking unit (dense leaves have long candidate windows, and 256-long
-// tiles left the tail of the pair tests to a few warps: hotspot-1M 8.46 ->
-// 6.18 ms a step; hotspot-3M, bound by the table update, within 0.3%), else
-// 256 (uniform-10M, 7.9 tests per unit: 64-long tiles cost 0.29 ms a step).
+// Tile length of the refinement's jobs when stc_config.refine_chunk is 0.
+// With fewer than FEW_ROW_BLOCKS row blocks of 32 checking units a warp, the
+// pair tests end with a few warps in the longest jobs, so the tiles are as
+// short as they go (32: hotspot window of 300k objects, 10k row blocks, 0.68
+// ms of pair tests and table update with 256, 0.47 with 64, 0.39 with 32; at
+// 24k row blocks all lengths are within 2%). Otherwise 64 candidates when the
+// last step tested more than 16 candidates per checking unit (dense leaves
+// have long candidate windows, and 256-long tiles left the tail of the pair
+// tests to a few warps: hotspot-1M 8.46 -> 6.18 ms a step), else 256
+// (uniform-10M, 7.9 tests per unit: 64-long tiles cost 0.29 ms a step).
 // Results do not depend on it.
 static constexpr unsigned long long SHORT_TILE_TESTS_PER_UNIT = 16;
+static constexpr unsigned long long FEW_ROW_BLOCKS = 4;
 static void choose_refine_chunk(stc_ctx *c) {
   PipeDev &p = c->p;
   uint32_t chunk = c->cfg.refine_chunk;
   if (!chunk) {
     const DevState &st = *c->st_host;  // the last step's counters
-    chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * ((unsigned long long)p.N + st.border_units) ? 64u
-                                                                                           : REFINE_CHUNK_DEFAULT;
+    const unsigned long long units = (unsigned long long)p.N + st.border_units;
+    if (units / 32 < FEW_ROW_BLOCKS * 32 * (unsigned long long)num_sms()) chunk = 32u;
+    else chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * units ? 64u : REFINE_CHUNK_DEFAULT;
   }
   if (chunk != p.refine_chunk) {
     p.refine_chunk = chunk;

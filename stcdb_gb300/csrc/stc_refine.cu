@@ -295,6 +295,7 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
   float4 rp = make_float4(0.f, 0.f, 0.f, 0.f);
   float2 fr = make_float2(0.f, 0.f);  // the row object's float position (fxy)
   uint32_t pid1 = 0, orig1 = 0, row_leaf = 0;
+  float ax0 = 0.f, ay0 = 0.f, ay1 = 0.f;  // a border row's own leaf, in float: low x, low y, high y
   uint32_t sa[3] = {0, 0, 0}, sl[3] = {0, 0, 0};  // candidate segments: start, length
   unsigned long long rank = 0;
   bool vr;
@@ -329,6 +330,10 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       // twice in this step iff the member also has a border unit targeting
       // pid1's leaf.
       row_leaf = p.leaf_gid[pid1];
+      const Node *ro = &p.sd.nodes[p.sd.gid_node[row_leaf]];
+      ax0 = __double2float_rn(ro->lo_x);
+      ay0 = __double2float_rn(ro->lo_y);
+      ay1 = __double2float_rn(ro->hi_y);
       // candidates: the members in the point's longitude window of the
       // strips beside its own (all of a strip too large to be ordered)
       const float4 ls = __ldg(&p.lstrip[g]);
@@ -432,10 +437,17 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
             h.order = ((unsigned long long)h.a << STC_ORDER_SHIFT) | (pid1 < cpid ? corig : orig1);
           } else {
             h.order = (rank << STC_ORDER_SHIFT) | corig;
-            const uint32_t cnb = p.bcount[cpid];
-            const uint32_t coff = cnb ? p.boff[cpid] : 0u;
-            for (uint32_t u2 = 0; u2 < cnb; u2++)
-              if (p.bu_gid[coff + u2] == row_leaf) h.order |= DUP_BIT;
+            // the member has a unit targeting the row's leaf only if it lies
+            // below that leaf, or left of it and below its top (the border
+            // lookup's rule); rounding to float keeps the order, so the test
+            // on floats passes every such member, and the three dependent
+            // loads of its units are left to the few that pass
+            if (fc.y <= ay0 || (fc.y <= ay1 && fc.x <= ax0)) {
+              const uint32_t cnb = p.bcount[cpid];
+              const uint32_t coff = cnb ? p.boff[cpid] : 0u;
+              for (uint32_t u2 = 0; u2 < cnb; u2++)
+                if (p.bu_gid[coff + u2] == row_leaf) h.order |= DUP_BIT;
+            }
           }
           if (!DIRECT) q[qn + __popc(hm & lt_mask)] = h;
         }
@@ -471,7 +483,11 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
   const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const unsigned long long J = p.st->jobs_total;
-  const unsigned long long jc = p.job_chunk;
+  // fewer jobs at a time when there are too few to go round: eight dense jobs
+  // of one leaf in one warp were the whole kernel's tail (20k objects in
+  // hotspots: 0.23 -> 0.06 ms a part)
+  const unsigned long long each = J / parts / nwarps;
+  const unsigned long long jc = each >= p.job_chunk ? p.job_chunk : (each ? each : 1ull);
   const unsigned long long nchunks = (J + jc - 1) / jc;
   const unsigned long long c0 = nchunks * part / parts, c1 = nchunks * (part + 1) / parts;
   Counters ct = {0, 0, 0, 0};
@@ -480,11 +496,16 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
     if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
     unsigned long long j0 = chunk * jc;
     unsigned long long j1 = j0 + jc < J ? j0 + jc : J;
-    // largest g with job_start[g] <= j0
-    uint32_t lo = 0, hi = p.G;
+    // largest g with job_start[g] <= j0, 32 probes a round (4 rounds of loads
+    // for 10^6 grid ids instead of 20)
+    uint32_t lo = 0, hi = p.G;  // job_start[lo] <= j0 < job_start[hi] (or hi = G)
     while (hi - lo > 1) {
-      uint32_t mid = (lo + hi) >> 1;
-      if (p.job_start[mid] <= j0) lo = mid; else hi = mid;
+      const uint32_t w32 = (hi - lo + 31) / 32;
+      const uint32_t at = lo + (lane_id() + 1) * w32;  // ascending over the lanes
+      const uint32_t below = __popc(__ballot_sync(0xffffffffu, at < hi && p.job_start[at] <= j0));
+      const uint32_t lo2 = lo + below * w32;
+      hi = min(hi, lo2 + w32);
+      lo = lo2;
     }
     uint32_t g = lo;
     for (unsigned long long job = j0; job < j1; job++) {
