@@ -619,32 +619,30 @@ def max_over_ranks(args, v):
     return float(t.item())
 
 
-# DRAM bytes (read + write) of the refinement phase (k_refine_a + k_hits)
-# per hit, from one ncu capture of each kernel on the 3M-object workload
-# (profiles/kernels_refine_hits_strips_uniform-3M.md): 388.5 MB (reads and
-# writes of both kernels) for one of the step's four parts, about a quarter
-# of its 6.086M hits. The traffic grows with the hits (32-byte records
-# written and read, one table slot per hit), so the 10M line scales it by
-# its own hit count.
-REFINE_DRAM_BYTES_PER_HIT = (54.36e6 + 33.70e6 + 264.20e6 + 36.23e6) / (6.086e6 / 4)
+# DRAM bytes (read + write) of the table update and sweep (k_table) per
+# algorithmic byte, from an ncu capture on the 3M-object workload
+# (profiles/kernels_table_uniform-3M.md): 2.348 GB read and 0.296 GB written
+# for 2.636 GB of table slots, hit records and changed slots.
+TABLE_DRAM_PER_BYTE = (2.348 + 0.296) / 2.636
 
 
 def kernel_bytes(s, N, B, prev_live=None):
     """Algorithmic bytes per launch of the step's kernels.
     partition: 36 N (read positions, write leaf-ordered points, id map)
-    refine:    16 N + 16 H + 8 Q plus the fused probe, 64 B per hit
-    sweep:     32 B per table slot read, 32 B per slot it writes (each new
-               meeting's claim finalised, each meeting not hit this step
-               cleared) + 64 B per emitted meeting. A meeting stays live only
-               when hit, so the cleared ones are the previous step's live
-               meetings less this step's extensions (hits - new);
-               `prev_live` defaults to this step's live count."""
+    refine:    16 N + 16 H + 32 per hit (its record, written)
+    sweep:     the table update and sweep: 32 B per hit record and per table
+               slot read, 32 B per slot it writes (each meeting extended or
+               started this step, each one not hit cleared) + 64 B per emitted
+               meeting. A meeting stays live only when hit, so the cleared
+               ones are the previous step's live meetings less this step's
+               extensions (hits - new); `prev_live` defaults to this step's
+               live count."""
     H, Q = s.border_units, s.hits
     new = s.new_candidates
     prev = s.taken_buckets if prev_live is None else prev_live
     cleared = max(prev - (Q - new), 0)
-    return {"partition": 36.0 * N, "refine": 16.0 * N + 16.0 * H + 72.0 * Q,
-            "sweep": 32.0 * B + 32.0 * (new + cleared) + 64.0 * s.emitted}
+    return {"partition": 36.0 * N, "refine": 16.0 * N + 16.0 * H + 32.0 * Q,
+            "sweep": 32.0 * B + 32.0 * (Q + s.taken_buckets + cleared) + 64.0 * s.emitted}
 
 
 FLUSH_STAGES = ("object_order", "key_sort", "ctf_limits", "encode", "store_and_index")
@@ -704,16 +702,13 @@ def sort_line(device, peak, n=100_000_000, reps=5):
             "achieved_gbs": b / (ms / 1e3) / 1e9, "frac_of_peak": b / (ms / 1e3) / 1e9 / peak, "sorted": ok}
 
 
-def random_access_line(device, buckets, hits, refine_ms):
-    """The meeting-table update's random-access ceiling: stc_measure_random_access
+def random_access_line(device, buckets, hits, update_ms):
+    """What HBM serves of random table accesses: stc_measure_random_access
     on a table of the workload's size (2^round(log2 B) 32-byte slots, at most
-    2^30) with as many accesses as the step has hits. Every hit reads its home
-    slot, a random 32-byte sector of the table, and writes it (its end time
-    or its claim); HBM serves such accesses at this rate, far below its copy
-    bandwidth.
-    `refine_frac` = the refine phase's hits per second (pair tests and table
-    update together) / the ceiling: how close the phase is to one random slot
-    access per hit at the measured rate."""
+    2^30) with as many accesses as the step has hits, each a read of a random
+    32-byte slot and a store to it. The table update applies the hits tile by
+    tile instead: `update_frac` = the step's hits per second of pair tests,
+    table update and sweep together / that rate."""
     import ctypes
     from stcdb_gb300._lib import load_library
     lib = load_library("libstc")
@@ -727,9 +722,9 @@ def random_access_line(device, buckets, hits, refine_ms):
         return {"error": lib.stc_last_error(None).decode(errors="replace")}
     ceiling = n / (ms.value / 1e3)
     line = {"table_bytes": 32 << log2, "accesses": n, "ms": ms.value, "accesses_per_s": ceiling}
-    if refine_ms > 0 and hits > 0:
-        line["refine_hits_per_s"] = hits / (refine_ms / 1e3)
-        line["refine_frac"] = line["refine_hits_per_s"] / ceiling
+    if update_ms > 0 and hits > 0:
+        line["update_hits_per_s"] = hits / (update_ms / 1e3)
+        line["update_frac"] = line["update_hits_per_s"] / ceiling
     return line
 
 
@@ -1006,7 +1001,7 @@ def main():
                     "leaf_capacity": w["grid_capacity"], "grid_amplify": w["amplify"],
                     "launch_shape": {"refine_blocks_per_sm": w.get("refine_bps", 8),
                                      "hits_blocks_per_sm": w.get("hits_bps", 16),
-                                     "refine_chunk": w.get("refine_chunk") or "by density (64 or 256)"},
+                                     "refine_chunk": w.get("refine_chunk") or "by density (32, 64 or 256)"},
                     "meeting_buckets": make_cfg(w).resolved().num_meeting_buckets,
                     "memtable": (f"on, flush past {w['kv_restriction']} directed keys, 100 CTFs, "
                                  f"{w.get('bitmap_edge', 256)}x{w.get('bitmap_edge', 256)} map bitmaps"
@@ -1061,9 +1056,8 @@ def main():
         "gpu_launches": launches,
         "roofline": {"bound": "hbm", "kernel": dom, "achieved": achieved, "peak": peak,
                      "peak_source": peak_kind, "unit": "GB/s", "frac": achieved / peak,
-                     "traffic": (REFINE_DRAM_BYTES_PER_HIT * sum(s.hits for s in r["stats"]) / K
-                                 if dom == "refine" else None),
-                     "traffic_source": "ncu capture of k_refine_a + k_hits at 3M objects, scaled by hits",
+                     "traffic": TABLE_DRAM_PER_BYTE * kb["sweep"] if dom == "sweep" else None,
+                     "traffic_source": "ncu capture of k_table at 3M objects, scaled by algorithmic bytes",
                      "algorithmic_bytes": kb[dom], "launch_ms": phase_ms[dom]},
         "phase_ms": phase_ms,
         "phase_gbs": {k: kb[k] / (phase_ms[k] / 1e3) / 1e9 for k in kb if phase_ms[k] > 0},
@@ -1075,7 +1069,7 @@ def main():
         "compaction": compaction_line(r["compaction"], peak),
         "sort": sort_line(local, peak),
         "table_random_access": random_access_line(local, B, sum(s.hits for s in r["stats"]) / K,
-                                                  phase_ms["refine"]),
+                                                  phase_ms["refine"] + phase_ms["insert"] + phase_ms["sweep"]),
         "batched": None if args.no_batched else batched_line(
             local, objects=(1e6, 2e7) if args.batched_full else (1e5, 2e6)),
         "autotune": None if args.no_batched else tune_line(local),

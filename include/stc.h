@@ -77,8 +77,10 @@ typedef struct stc_config {
   int32_t mbr_filter;            /* drop meetings whose MBR leaves the map box (cuda/geometry.cu:667-670) */
   uint64_t candidate_capacity;   /* new-meeting candidates per step; 0 = auto */
   uint64_t emit_capacity;        /* emitted meetings held between drains; 0 = auto */
-  uint64_t hit_capacity;         /* pairs buffered between refinement and table update; 0 = auto:
-                                    max(4M, 8 n), grown after a step (or window) that found more */
+  uint64_t hit_capacity;         /* pairs buffered between refinement and table update, spread over
+                                    bins of one table tile (up to 768 slots) each; 0 = auto:
+                                    max(4M, 8 n) and a quarter more, grown after a step (or window)
+                                    that found a fuller bin */
   uint32_t device;               /* CUDA device ordinal */
   uint32_t flags;                /* STC_FLAG_* (0 for normal operation) */
   /* Memtable and flush into a contact tracing block (CTB) of CTFs, the
@@ -105,7 +107,8 @@ typedef struct stc_config {
                                     takes at a time, fewer when there are too few to go round;
                                     0 = 8, at most 64 */
   uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 = 8, at most 32 */
-  uint32_t hits_blocks_per_sm;   /* table-update blocks launched per SM; 0 = 16, at most 64 */
+  uint32_t hits_blocks_per_sm;   /* blocks per SM of the general table update (a step whose table tiles
+                                    are too full for the tiled one); 0 = 16, at most 64 */
   uint32_t window_graphs;        /* stc_step_window replays each step from a captured CUDA graph:
                                     0 = automatic: when the context's last step took under 1.5 ms
                                     of device time (up to 2^21 objects), or, before any step, up to
@@ -127,9 +130,8 @@ typedef struct stc_config {
 /* Replay quadtree splits/merges on one device thread only (tests compare it
  * with the default parallel replay). */
 #define STC_FLAG_SERIAL_SCHEMA 1u
-/* How the pair tests hand over their hits (results do not depend on it; by
- * default the library picks by the last step's hits per checking unit):
- * straight to the hit buffer, or through a per-warp queue. Tests force each. */
+/* Former choices of how the pair tests hand over their hits; accepted, no
+ * effect (hits go to bins of the table tile they fall in). */
 #define STC_FLAG_DIRECT_HITS 2u
 #define STC_FLAG_QUEUED_HITS 4u
 /* stc_step_window copies page-locked host input with a copy engine instead
@@ -166,7 +168,9 @@ typedef struct stc_stats {
   uint32_t ambiguous_tests;      /* distance decisions within a few ulp of reach, where
                                     the last bit of sin() could matter */
   float step_ms;                 /* device time of the step */
-  float phase_ms[8];             /* partition, border+jobs, refine, insert, sweep, schema, copy-in, memtable append */
+  float phase_ms[8];             /* partition, border+jobs, refine (pair tests), insert (plan of the table
+                                    update: what is carried into its runs), sweep (table update, expiry and
+                                    emission), schema, copy-in, memtable append */
   uint64_t memtable_keys;        /* directed keys in the memtable after the step (and any flush) */
   uint32_t flushes;              /* blocks flushed so far */
   float flush_ms;                /* device time of the last flush */

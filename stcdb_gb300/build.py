@@ -30,6 +30,7 @@ CU_SOURCES = [
     "stc_partition.cu",
     "stc_refine.cu",
     "stc_meetings.cu",
+    "stc_table.cu",
     "stc_schema.cu",
     "stc_sort.cu",
     "stc_util.cu",

@@ -85,7 +85,7 @@ struct DevState {
   uint32_t error, error_info;
   unsigned long long border_units;
   unsigned long long jobs_total;
-  unsigned long long job_next;
+  unsigned long long tile_load;       // most (occupied slots + hits) of a table tile this step
   unsigned long long cand_count;
   unsigned long long emit_count;      // records in the emit buffer (pending drain)
   unsigned long long tests, exact_tests, hits, ambiguous;
@@ -99,7 +99,7 @@ struct DevState {
   uint32_t pad[2];
   unsigned long long border_points;   // points whose lookup starts above their leaf
   unsigned long long fast_claims;     // new meetings started this step (claims finalised by the sweep)
-  unsigned long long hit_count;       // hits appended to the hit buffer this step
+  unsigned long long hit_max;         // most hits of a table tile this step
   uint32_t schema_path;               // 1 parallel replay, 2 serial (cascade), 0 serial (other)
   uint32_t pad2;
   // memtable (stc_lsm.cu)

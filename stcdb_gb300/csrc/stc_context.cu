@@ -33,7 +33,6 @@ void set_thread_error(const std::string &msg) { g_create_error = msg; }
 }  // namespace stc
 
 static constexpr size_t DRAIN_CHUNK = (size_t)8 << 20;  // bytes per pinned staging chunk of a drain
-static constexpr uint32_t PAIR_PARTS = 4;                // parts of the pair tests (more while serving)
 // Input buffers of a pipelined window: the positions of step i + 3 are
 // copied in as soon as step i (that buffer's last reader) has run, two steps
 // before they are needed, so that a slow or uneven host link has slack.
@@ -55,10 +54,9 @@ struct stc_ctx {
   stc_config cfg;
   int device = 0;
   cudaStream_t stream = nullptr;
-  cudaStream_t side = nullptr;   // border units; the table update beside the pair tests
+  cudaStream_t side = nullptr;   // border units, beside the leaf order
   cudaStream_t side2 = nullptr;  // the schema update, beside the table update and sweep
-  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, fork2_ev = nullptr, join2_ev = nullptr, hits_ev = nullptr;
-  cudaEvent_t part_ev[STC_MAX_PARTS] = {};  // end of each part of the pair tests
+  cudaEvent_t fork_ev = nullptr, join_ev = nullptr, fork2_ev = nullptr, join2_ev = nullptr;
   cudaEvent_t ev[PH_COUNT] = {};
   std::string err;
   bool failed = false;
@@ -223,9 +221,6 @@ static void destroy_all(stc_ctx *c) {
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->fork2_ev) cudaEventDestroy(c->fork2_ev);
-  if (c->hits_ev) cudaEventDestroy(c->hits_ev);
-  for (cudaEvent_t ev : c->part_ev)
-    if (ev) cudaEventDestroy(ev);
   if (c->join2_ev) cudaEventDestroy(c->join2_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->side) cudaStreamDestroy(c->side);
@@ -261,6 +256,12 @@ static stc_status read_state(stc_ctx *c, const char *where) {
     return fail(c, status_of(c->st_host->error), buf);
   }
   return STC_OK;
+}
+
+// Records per bin when `total` are spread over nb bins, times num / den, plus
+// `more` (at least 1; a run of bins stays below 2^32 records).
+static uint32_t bin_share(uint64_t total, uint32_t nb, uint32_t num = 1, uint32_t den = 1, uint32_t more = 0) {
+  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>((total + nb - 1) / nb * num / den + more, 1), 1u << 24);
 }
 
 // Creates a context; builds the quadtree from xy0 unless xy0 is null (a
@@ -329,9 +330,6 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork2_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join2_ev, cudaEventDisableTiming);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->hits_ev, cudaEventDisableTiming);
-  for (uint32_t i = 0; i < STC_MAX_PARTS && e == cudaSuccess; i++)
-    e = cudaEventCreateWithFlags(&c->part_ev[i], cudaEventDisableTiming);
   for (int i = 0; i < PH_COUNT && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   if (e == cudaSuccess) e = cudaMallocHost(&c->st_host, sizeof(DevState));
   if (e == cudaSuccess) e = cudaMallocHost(&c->t_pinned, WIN_BUFS * sizeof(uint32_t));
@@ -344,6 +342,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->drain_stream, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->drained_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = schema_prepare();
+  if (e == cudaSuccess) e = table_prepare();
   for (int i = 0; i < 2 && e == cudaSuccess; i++) {
     e = cudaMallocHost(&c->drain_stage[i], DRAIN_CHUNK);
     if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->drain_ev[i], cudaEventDisableTiming);
@@ -370,8 +369,11 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   p.cand_cap = cand_cap;
   p.C = next_pow2(2 * cand_cap);
   p.E = k.emit_capacity ? k.emit_capacity : std::max<uint64_t>(1u << 20, 4ULL * n);
-  // hits beyond the buffer are applied inside the refinement instead
-  p.hit_cap = k.hit_capacity ? k.hit_capacity : std::max<uint64_t>(1u << 22, 8ULL * n);
+  // hits beyond a bin are applied inside the refinement instead; an automatic
+  // bin has room for a quarter more than its share
+  table_sizes(p);
+  p.bin_cap = k.hit_capacity ? bin_share(k.hit_capacity, p.nb)
+                             : bin_share(std::max<uint64_t>(1u << 22, 8ULL * n), p.nb, 5, 4, 64);
   p.U_cap = (uint64_t)k.refine_size * n - n;
   p.reach = k.reach_distance;
   p.x_buffer = k.reach_distance * stc_dpml_ref(mbr[1]);  // tracing/filter.cpp:30
@@ -410,7 +412,6 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
             dalloc(c, &p.sorted_pid, n) && dalloc(c, &p.sort_ktmp, nu) && dalloc(c, &p.sort_vtmp, nu) &&
             dalloc(c, &p.sort_hist, radix_hist_words(nu)) && dalloc(c, &p.grid_count, (size_t)p.G + 1) &&
             dalloc(c, &p.sort_ktmp2, nu) && dalloc(c, &p.sort_vtmp2, nu) &&
-            dalloc(c, &p.hit_bounds, STC_MAX_PARTS + 1) &&
             dalloc(c, &p.sort_hist2, radix_hist_words(nu)) && dalloc(c, &p.scan_tmp2, scan_words) &&
             dalloc(c, &p.grid_start, (size_t)p.G + 1) && dalloc(c, &p.pts, n) && dalloc(c, &p.fxy, n) &&
             dalloc(c, &p.gfxy, n) && dalloc(c, &p.sfxy, n) &&
@@ -421,7 +422,10 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
             dalloc(c, &p.bu_gid, p.U_cap) && dalloc(c, &p.bu_pid, p.U_cap) && dalloc(c, &p.bu_sorted_gid, p.U_cap) &&
             dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, (size_t)p.G + 1) &&
             dalloc(c, &p.bu_start, (size_t)p.G + 1) && dalloc(c, &p.job_cnt, (size_t)p.G + 1) &&
-            dalloc(c, &p.job_start, (size_t)p.G + 1) && dalloc(c, &p.slots, p.B) && dalloc(c, &p.hits, p.hit_cap) && dalloc(c, &p.cset, p.C) &&
+            dalloc(c, &p.job_start, (size_t)p.G + 1) && dalloc(c, &p.slots, p.B) && 
+            dalloc(c, &p.hits, (size_t)p.nb * p.bin_cap) && dalloc(c, &p.bin_cnt, p.nb) &&
+            dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
+            dalloc(c, &p.carry_cnt, p.runs) && dalloc(c, &p.cset, p.C) &&
             dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E) && dalloc(c, &p.scan_tmp, scan_words) &&
             dalloc(c, &p.n_dev, 1);
   if (ok && k.kv_restriction) {
@@ -487,6 +491,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   cudaStream_t s = c->stream;
   cudaMemsetAsync(p.st, 0, sizeof(DevState), s);
   cudaMemsetAsync(p.sw.queued, 0, p.S, s);
+  cudaMemsetAsync(p.tile_live, 0, (size_t)p.nb * sizeof(uint32_t), s);
   unsigned long long nn = n;
   cudaMemcpyAsync(p.n_dev, &nn, sizeof(nn), cudaMemcpyHostToDevice, s);
   iota_u32(p.iota, nu, s);
@@ -572,35 +577,29 @@ static void issue_step(stc_ctx *c, bool events, bool append, const uint32_t *two
   cudaStreamWaitEvent(s, c->join2_ev, 0);
   step_jobs(p, s);
   if (events) cudaEventRecord(c->ev[PH_BORDER], s);
-  // The pair tests run in parts; each part's hits are applied to the table
-  // on the side stream while the next part's pairs are tested (the two
-  // kernels are bound by different units; concurrent table updates are safe,
-  // new meetings take their slots by priority).
-  const uint32_t parts = std::min<uint32_t>(std::max<uint32_t>(p.slices, PAIR_PARTS), STC_MAX_PARTS);
-  for (uint32_t part = 0; part < parts; part++) {
-    step_pairs_part(p, part, parts, s);
-    cudaEventRecord(c->part_ev[part], s);
-    cudaStreamWaitEvent(c->side, c->part_ev[part], 0);
-    step_hits_part(p, part, parts, c->side);
-  }
-  cudaEventRecord(c->hits_ev, c->side);
+  step_pairs(p, s);
+  if (events) cudaEventRecord(c->ev[PH_REFINE], s);
   // The schema update reads this step's leaf counts and rewrites quadtree
   // nodes, which only the pair tests read: once they are done it runs on a
-  // third stream while the table update, insert, sweep and memtable append
-  // run (none of them touches the schema or its scan scratch), and the step
-  // ends when all have.
+  // third stream while the table update, sweep and memtable append run (none
+  // of them touches the schema or its scan scratch), and the step ends when
+  // all have.
   const bool schema = c->cfg.dynamic_schema != 0;
   if (schema) {
-    cudaStreamWaitEvent(c->side2, c->part_ev[parts - 1], 0);
+    cudaEventRecord(c->fork_ev, s);
+    cudaStreamWaitEvent(c->side2, c->fork_ev, 0);
     update_schema(p.sd, p.sw, p.grid_count, p.reach, p.grid_capacity, p.delay,
                   (c->cfg.flags & STC_FLAG_SERIAL_SCHEMA) != 0, p.st, c->side2);
     cudaEventRecord(c->join_ev, c->side2);
   }
-  cudaStreamWaitEvent(s, c->hits_ev, 0);
-  if (events) cudaEventRecord(c->ev[PH_REFINE], s);
-  if (c->gate_ev) cudaEventRecord(c->gate_ev, s);
-  step_insert(p, s);
+  step_table_plan(p, s);
   if (events) cudaEventRecord(c->ev[PH_INSERT], s);
+  if (c->gate_ev) cudaEventRecord(c->gate_ev, s);
+  step_table(p, s);
+  // the general path, for a step the tiled one cannot take (decided on the
+  // device; otherwise these return at once)
+  step_hits(p, s);
+  step_insert(p, s);
   step_sweep(p, s);
   if (events) cudaEventRecord(c->ev[PH_SWEEP], s);
   if (append && c->lsm_on) lsm_append(p, c->lsm, s);
@@ -672,17 +671,17 @@ static void fill_stats(stc_ctx *c, uint32_t t, const float *phase, float step_ms
 // (cuda/geometry.cu:1752).
 static bool flush_due(const stc_ctx *c) { return c->lsm_on && c->st_host->kv_count > c->cfg.kv_restriction; }
 
-// With the automatic hit capacity (stc_config.hit_capacity 0) the hit buffer
-// grows to the largest step seen: hits beyond it are applied inside the pair
-// tests, which is correct but slow (they hold the pair-test warps on random
-// table accesses). Called only with no step in flight; a failed allocation
-// keeps the old buffer.
+// With the automatic hit capacity (stc_config.hit_capacity 0) the bins grow to
+// the fullest bin seen: a hit beyond its bin is applied inside the pair tests,
+// which is correct but slow (random table accesses, and the general path for
+// that step). Called only with no step in flight; a failed allocation keeps
+// the old bins.
 static void grow_hits(stc_ctx *c, unsigned long long need) {
   PipeDev &p = c->p;
-  if (c->cfg.hit_capacity || need <= p.hit_cap) return;
-  const unsigned long long cap = next_pow2(need + need / 4);
+  if (c->cfg.hit_capacity || need <= p.bin_cap) return;
+  const uint32_t cap = bin_share(need, 1, 5, 4, 16);
   void *h = nullptr;
-  if (cudaMalloc(&h, cap * sizeof(HitRec)) != cudaSuccess) {
+  if (cudaMalloc(&h, (size_t)p.nb * cap * sizeof(HitRec)) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
@@ -692,29 +691,8 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
       a = h;
     }
   p.hits = (HitRec *)h;
-  p.hit_cap = cap;
+  p.bin_cap = cap;
   invalidate_graphs(c);  // the graphs hold the buffer by value
-}
-
-// How the pair tests hand over their hits: straight to the hit buffer when
-// the last step found many hits per checking unit (dense leaves: hotspot-1M
-// has about 17, its refinement 6.35 -> 5.94 ms a step that way), through a
-// per-warp shared-memory queue otherwise (uniform-10M has about 6; the direct
-// form's extra registers cost it 0.08 ms). Results do not depend on it.
-static constexpr unsigned long long DIRECT_HITS_PER_UNIT = 12;
-static void choose_hit_emission(stc_ctx *c) {
-  PipeDev &p = c->p;
-  uint32_t direct;
-  if (c->cfg.flags & STC_FLAG_DIRECT_HITS) direct = 1;
-  else if (c->cfg.flags & STC_FLAG_QUEUED_HITS) direct = 0;
-  else {
-    const DevState &st = *c->st_host;  // the last step's counters
-    direct = st.hits > DIRECT_HITS_PER_UNIT * ((unsigned long long)p.N + st.border_units) ? 1u : 0u;
-  }
-  if (direct != p.direct_hits) {
-    p.direct_hits = direct;
-    invalidate_graphs(c);  // the captured steps launch the other kernel
-  }
 }
 
 // Tile length of the refinement's jobs when stc_config.refine_chunk is 0.
@@ -747,7 +725,6 @@ static void choose_refine_chunk(stc_ctx *c) {
 
 static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copied) {
   PipeDev &p = c->p;
-  choose_hit_emission(c);
   choose_refine_chunk(c);
   cudaStream_t s = c->stream;
   p.xy = xy;
@@ -764,7 +741,7 @@ static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copie
   float tot = 0;
   cudaEventElapsedTime(&tot, c->ev[PH_START], c->ev[PH_SCHEMA]);
   fill_stats(c, t, phase, tot, (uint32_t)(tl_launches - launches0));
-  grow_hits(c, c->st_host->hit_count);
+  grow_hits(c, c->st_host->hit_max);
   if (flush_due(c)) return flush_now(c, t);
   return STC_OK;
 }
@@ -953,10 +930,8 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
   // copy event, time word and graph by i % WIN_BUFS)
   auto issue_core = [&](uint32_t i) -> stc_status {
     const int par = i & 1, b = (int)(i % WIN_BUFS);
-    // launch forms by the density of the latest step whose state has been
-    // taken (i - 2, or the step before the window): the hits' hand-over form
-    // and the pair tests' tile length
-    choose_hit_emission(c);
+    // the pair tests' tile length by the density of the latest step whose
+    // state has been taken (i - 2, or the step before the window)
     choose_refine_chunk(c);
     c->t_pinned[b] = t0 + i;  // step i - WIN_BUFS, the word's last reader, has been waited for
     const unsigned long long l0 = tl_launches;
@@ -1027,7 +1002,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
   const auto wall0 = std::chrono::steady_clock::now();
   double busy_ms = 0;  // device time of the window's steps
   size_t n = 0;
-  unsigned long long most_hits = 0;  // the window's largest step (hit buffer growth at its end)
+  unsigned long long most_hits = 0;  // the window's fullest bin (the bins grow at its end)
   unsigned long long dpos = 0;  // emit records [0, dpos) are on their way to out
   bool out_full = false;
   stc_status rs = STC_OK;
@@ -1059,7 +1034,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       ran = i + 1;
       busy_ms += c->stats.step_ms;
     }
-    if (rs == STC_OK) most_hits = std::max(most_hits, c->st_host->hit_count);
+    if (rs == STC_OK) most_hits = std::max(most_hits, c->st_host->hit_max);
     if (rs == STC_OK && out && !out_full) {
       const unsigned long long cnt = std::min<unsigned long long>(c->st_host->emit_count, p.E);
       const size_t k = (size_t)std::min<unsigned long long>(cnt - dpos, cap - n);
@@ -1100,8 +1075,8 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
     if (i + 1 < steps) {
       if (!ahead) {
         // held: nothing is in flight; every record emitted so far is drained
-        // or on its way out, so the emit buffer can be emptied, and the hit
-        // buffer can grow to the window's largest step
+        // or on its way out, so the emit buffer can be emptied, and the bins
+        // can grow to the window's fullest
         if (out) {
           e = emit_keep_tail(c, dpos, std::min<unsigned long long>(c->st_host->emit_count, p.E));
           if (e != cudaSuccess) return cuda_fail(c, e, "stc_step_window drain");
@@ -1127,9 +1102,9 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       // step i + 1 adds its meetings behind step i's; past half of the
       // emit buffer, step i + 2 waits until the buffer has been emptied
       if (out && c->st_host->emit_count > p.E / 2) hold = true;
-      // a step found more hits than the hit buffer holds (the rest were
-      // applied inside its pair tests): grow it at the next step boundary
-      if (!c->cfg.hit_capacity && most_hits > p.hit_cap) hold = true;
+      // a step found more hits than a bin holds (the rest were applied
+      // inside its pair tests): grow the bins at the next step boundary
+      if (!c->cfg.hit_capacity && most_hits > p.bin_cap) hold = true;
     }
   }
   cudaStreamSynchronize(c->copy_stream);
@@ -1647,6 +1622,13 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
   if (!bad.empty()) return bail(STC_ERR_INVALID_ARG, bad);
   fclose(f);
   e = cudaMemcpy(c->p.st, &h.st, sizeof(DevState), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);
+    stc_destroy(c);
+    return STC_ERR_CUDA;
+  }
+  count_tiles(c->p, c->stream);
+  e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);
     stc_destroy(c);

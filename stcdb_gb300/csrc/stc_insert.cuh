@@ -30,6 +30,28 @@
 
 namespace stc {
 
+#define DUP_BIT (1ULL << 63)  // HitRec::order: the pair may occur twice this step
+
+// Table tile (bin) of a slot: tile j covers [j * B / nb, (j + 1) * B / nb).
+__device__ __forceinline__ uint32_t tile_of(const PipeDev &p, unsigned long long slot) {
+  const unsigned long long x = (slot + 1) * p.nb - 1;  // tile = x / B
+  unsigned long long q = __umul64hi(x, p.B_magic);     // exact or one too large
+  if (q * p.B > x) q--;
+  return (uint32_t)q;
+}
+
+// Halo tiles the tiled table update (stc_table.cu) needs this step, or 0:
+// the step takes the general path (k_hits, k_insert_ordered, k_sweep).
+constexpr uint32_t MAX_HALO = 7;
+__device__ __forceinline__ uint32_t fuse_halo(const PipeDev &p) {
+  if (p.nb < 2 * MAX_HALO || p.st->hit_max > p.bin_cap) return 0;
+  const unsigned long long c = p.st->tile_load, T = p.B / p.nb;
+  if (c >= TILE_LOAD) return 0;  // the carry lists hold TILE_LOAD hits
+  for (uint32_t h = 1; h <= MAX_HALO; h++)
+    if (c * (h + 1) < T * h) return h;
+  return 0;
+}
+
 // (key, claim) pair of a slot in one 16-byte load at L2 (claims change during
 // the walk phase; a torn or stale value only makes a CAS fail and retry).
 __device__ __forceinline__ U128 load_slot_pair(const Slot *s) {

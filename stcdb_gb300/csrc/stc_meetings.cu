@@ -1,5 +1,6 @@
-// Step kernels (c): ordered insertion of new meetings and the expire/emit
-// sweep of the meeting table.
+// Step kernels (c), general path: ordered insertion of new meetings and the
+// expire/emit sweep of the meeting table, for a step that the tiled update
+// (stc_table.cu) does not take.
 //
 // The reference inserts hits one by one in its processing order with linear
 // probing from key % B and clears expired slots without tombstones
@@ -37,9 +38,9 @@ __global__ void k_step_begin(DevState *st) {
   st->border_units = 0;
   st->border_points = 0;
   st->fast_claims = 0;
-  st->hit_count = 0;
+  st->hit_max = 0;
   st->jobs_total = 0;
-  st->job_next = 0;
+  st->tile_load = 0;
   st->cand_count = 0;
   st->tests = st->exact_tests = st->hits = st->ambiguous = 0;
   st->taken = 0;
@@ -88,7 +89,10 @@ void init_tables(PipeDev &p, cudaStream_t s) {
 // Candidates that may occur twice in a step: walk with their minimum
 // priority once all instances are merged.
 __global__ void k_insert_ordered(PipeDev p) {
+  if (fuse_halo(p)) return;
   const uint32_t t = p.st->step_t;
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb; j += gridDim.x * blockDim.x)
+    p.tile_live[j] = 0;  // counted again by the sweep
   const unsigned long long nc = p.st->cand_count < p.cand_cap ? p.st->cand_count : p.cand_cap;
   for (unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; c < nc;
        c += (unsigned long long)gridDim.x * blockDim.x) {
@@ -181,6 +185,17 @@ __device__ __forceinline__ bool sweep_slot(const PipeDev &p, uint32_t t, unsigne
   return emit;
 }
 
+// Adds the warp's live slots (consecutive, one per lane) to their tiles' counts.
+__device__ __forceinline__ void count_live(const PipeDev &p, unsigned long long slot, bool live) {
+  const uint32_t ball = __ballot_sync(0xffffffffu, live);
+  if (!ball) return;
+  const uint32_t tile = live ? tile_of(p, slot) : STC_NONE;
+  const uint32_t first = __shfl_sync(0xffffffffu, tile, __ffs(ball) - 1);
+  const uint32_t same = __ballot_sync(0xffffffffu, tile == first);
+  if ((int)lane_id() == __ffs(ball) - 1) atomicAdd(&p.tile_live[first], (uint32_t)__popc(same));
+  if (live && tile != first) atomicAdd(&p.tile_live[tile], 1u);
+}
+
 static constexpr uint32_t SWEEP_THREADS = 256;
 static constexpr uint32_t SWEEP_BLOCKS_PER_SM = 5;
 static constexpr uint32_t SWEEP_WARPS = SWEEP_THREADS / 32;
@@ -212,6 +227,7 @@ __device__ __forceinline__ void flush_emits(const PipeDev &p, const stc_meeting 
 
 // Slice `part` of `parts` sweeps slots [B * part / parts, B * (part + 1) / parts).
 __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(PipeDev p, uint32_t part, uint32_t parts) {
+  if (fuse_halo(p)) return;
   const uint32_t t = p.st->step_t;
   __shared__ __align__(16) stc_meeting stage_all[SWEEP_WARPS][WARP_STAGE];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
@@ -237,7 +253,9 @@ __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(Pi
     for (uint32_t u = 0; u < SWEEP_UNROLL; u++) cp[u] = claim_positions(p, sl[u]);
 #pragma unroll
     for (uint32_t u = 0; u < SWEEP_UNROLL; u++) {
+      const unsigned long long before = active;
       bool emit = idx[u] < B && sweep_slot(p, t, idx[u], sl[u], cp[u], active, fresh);
+      count_live(p, idx[u], active != before);
       uint32_t ball = __ballot_sync(0xffffffffu, emit);
       if (emit) {
         stc_meeting m;

@@ -443,6 +443,7 @@ void step_strips(PipeDev &p, cudaStream_t s) {
 }
 
 void step_border(PipeDev &p, cudaStream_t s) {
+  cudaMemsetAsync(p.bin_cnt, 0, (size_t)p.nb * sizeof(uint32_t), s);  // hits of the step to come
   cudaMemsetAsync(p.bu_cnt, 0, (size_t)(p.G + 1) * sizeof(uint32_t), s);
   STC_KL k_border_count<<<num_sms() * 16, 128, 0, s>>>(p);
   exclusive_scan_u32(p.bcount, p.boff, p.N, &p.st->border_units, p.scan_tmp2, s);

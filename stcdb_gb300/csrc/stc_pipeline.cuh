@@ -29,7 +29,6 @@ struct PipeDev {
   int mbr_filter;
   uint32_t slices;                 // launches per long step kernel (stc_config.step_slices)
   uint32_t job_chunk;              // refinement jobs a warp takes at a time (stc_config.job_chunk)
-  uint32_t direct_hits;            // pair tests write hit records directly (dense steps), not via a queue
   uint32_t refine_chunk;               // candidate positions per refinement job (a multiple of 32)
   uint32_t refine_bps, hits_bps;   // blocks per SM of the pair tests and of the table update
   // state
@@ -69,9 +68,16 @@ struct PipeDev {
   uint32_t *job_cnt, *job_start;        // G+1
   // meetings
   Slot *slots;                          // B
-  HitRec *hits;                         // hit_cap: hits of the step, applied by k_hits
-  unsigned long long hit_cap;
-  unsigned long long *hit_bounds;       // [MAX_PARTS + 1]: hit buffer end after each part of the pair tests
+  // hits of the step, binned by table tile (tile_of): bin j holds records
+  // [j * bin_cap, j * bin_cap + min(bin_cnt[j], bin_cap)); a hit its bin has
+  // no room for is applied inside the pair tests
+  HitRec *hits;
+  uint32_t nb, bin_cap;                 // tiles of the table, records per bin
+  unsigned long long nb_magic;          // ceil(2^64 / nb)
+  uint32_t *bin_cnt;                    // nb
+  uint32_t *tile_live;                  // nb: occupied slots of each tile after the last step
+  uint32_t runs;                        // runs of tiles the tiled update is cut into
+  uint32_t *carry, *carry_cnt;          // runs x TILE_LOAD, runs: hits carried into each run
   Cand *cset;                           // C
   uint32_t *cand_list;                  // cand_cap
   stc_meeting *emit;                    // E
@@ -92,14 +98,20 @@ void step_strips(PipeDev &p, cudaStream_t s);
 void step_border(PipeDev &p, cudaStream_t s);
 void step_jobs(PipeDev &p, cudaStream_t s);
 // stc_refine.cu
-// refinement in two parts: the pair tests (which read the leaves' node
-// boxes) and the table update of their hits
-// Part `part` of `parts` of the pair tests, then the mark of its hit range;
-// the table update of that range (k_hits) may run beside the next part.
-constexpr uint32_t STC_MAX_PARTS = 64;
-void step_pairs_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s);
-void step_hits_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s);
-// stc_meetings.cu
+// the pair tests, which bin the step's hits by table tile, and the general
+// path's table update of them (nothing when the tiled path took the step)
+void step_pairs(PipeDev &p, cudaStream_t s);
+void step_hits(PipeDev &p, cudaStream_t s);
+// stc_table.cu: the tiled table update and sweep. plan decides whether the
+// step takes it and finds what is carried into each run of tiles.
+constexpr uint32_t TILE_SLOTS = 768;    // largest tile
+constexpr uint32_t TILE_LOAD = 576;     // (occupied slots + hits) of a tile stay below this on the tiled path
+cudaError_t table_prepare();
+void table_sizes(PipeDev &p);           // nb and runs of a table of p.B slots
+void count_tiles(PipeDev &p, cudaStream_t s);
+void step_table_plan(PipeDev &p, cudaStream_t s);
+void step_table(PipeDev &p, cudaStream_t s);
+// stc_meetings.cu: the general path's insert and sweep
 void step_insert(PipeDev &p, cudaStream_t s);
 void step_sweep(PipeDev &p, cudaStream_t s);
 void init_tables(PipeDev &p, cudaStream_t s);

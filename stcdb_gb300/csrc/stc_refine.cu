@@ -1,5 +1,4 @@
-// Step kernel (b): proximity refinement fused with the first pass of the
-// meeting-table insert.
+// Step kernel (b): proximity refinement, and the general path's table update.
 //
 // Work: every leaf's n kept members (the first leaf_cap in pid order,
 // tracing/filter.cpp:100-104) are ordered by horizontal strips at least
@@ -34,11 +33,12 @@
 //   d_f^2 >= (r + delta)^2 with delta = 4E + 64 u r + 1e-6 r, which leaves
 //   slack for the rounding of the squared thresholds themselves.
 //
-// Hits (tracing/refinement.cpp:34-55) probe the meeting table from
-// key % B. A key found before the first empty slot is extended in place
-// (end = t, MBR); every other key becomes a candidate for the ordered insert
-// of stc_meetings.cu, keyed with its first position in the reference's
-// sequential processing order: unit rank << 24 | member index.
+// Hits (tracing/refinement.cpp:34-55) go to the bin of the table tile their
+// home slot key % B lies in, with their position in the reference's
+// sequential processing order: unit rank << 24 | member index. stc_table.cu
+// applies them; the general path here (k_hits) does so for a step whose tiles
+// are too full: a key found before the first empty slot is extended in place
+// (end = t, MBR), every other key walks on for a slot by priority.
 #include "stc_insert.cuh"
 
 namespace stc {
@@ -53,7 +53,8 @@ __device__ __forceinline__ double dpml_fast_r(double lat) {
 }
 
 // Reference distance decision for p1 (whose latitude sets the scale) and p2.
-__device__ bool exact_within(const PipeDev &p, uint32_t pid1, uint32_t pid2, uint32_t &amb) {
+// (not inlined: about 1 in 180,000 tests comes here)
+__device__ __noinline__ bool exact_within(const PipeDev &p, uint32_t pid1, uint32_t pid2, uint32_t &amb) {
   double2 a = p.xy[pid1], b = p.xy[pid2];
   double d = stc_distance_ref(a.x, a.y, b.x, b.y, dpml_fast_r(a.y));
   if (fabs(d - p.reach) > 1e-12 * p.reach) return d <= p.reach;
@@ -94,9 +95,6 @@ __device__ void cand_insert(const PipeDev &p, unsigned long long key, unsigned l
 }
 
 
-static constexpr int QCAP = 64;  // per-warp queue; flushed 32 at a time
-#define DUP_BIT (1ULL << 63)
-
 // Applies one hit (key = cantor(h.a, h.b)) to the table. kv/mbr: the slot
 // at key % B, already loaded.
 __device__ void process_hit_at(const PipeDev &p, const HitRec &h, unsigned long long key, uint32_t t,
@@ -129,67 +127,34 @@ __device__ void process_hit_at(const PipeDev &p, const HitRec &h, unsigned long 
   stc_set_error(p.st, ERR_PROBE, (uint32_t)slot);
 }
 
-__device__ __forceinline__ void process_hit(const PipeDev &p, const HitRec &h, uint32_t t) {
+// (not inlined: it would cost the pair tests' loop its registers)
+__device__ __noinline__ void process_hit(const PipeDev &p, const HitRec &h, uint32_t t) {
   const unsigned long long key = stc_cantor(h.a, h.b);
   unsigned long long slot = fast_mod(key, p.B, p.B_magic);
   process_hit_at(p, h, key, t, slot, load_slot_pair(&p.slots[slot]), __ldcg((const float4 *)&p.slots[slot].lo_x));
 }
 
-// Per-warp window of the step's hit buffer, reserved HIT_CHUNK entries at a
-// time so that the shared counter sees one atomic per HIT_CHUNK hits.
-static constexpr uint32_t HIT_CHUNK = 256;
-struct HitWindow {
-  unsigned long long next, end;  // warp-uniform
-};
-
-// Moves the first `n` (<= 32) queued hits to the step's hit buffer, which
-// k_hits processes with one thread per hit; hits that do not fit are
-// processed here, one per lane.
-__device__ __forceinline__ void flush_queue(const PipeDev &p, HitRec *q, uint32_t n, uint32_t t, HitWindow &w) {
-  __syncwarp();
-  uint32_t lane = lane_id();
-  if (w.end - w.next < n) {
-    // pad the rest of the old window with empty records, then reserve a new one
-    for (unsigned long long i = w.next + lane; i < w.end; i += 32)
-      if (i < p.hit_cap) p.hits[i].a = STC_NONE;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&p.st->hit_count, (unsigned long long)HIT_CHUNK);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    w.next = base;
-    w.end = base + HIT_CHUNK;
-  }
-  if (lane < n) {
-    HitRec h = q[lane];
-    unsigned long long pos = w.next + lane;
-    if (pos < p.hit_cap) p.hits[pos] = h;
-    else process_hit(p, h, t);
-  }
-  w.next += n;
-  __syncwarp();
+// One 32-byte store: a whole sector per record (a plain assignment is split
+// into narrower stores, each a partial write of the sector in L2: 10M uniform
+// objects, 67.7M records a step, pair tests 5.8 ms with it).
+__device__ __forceinline__ void store_hit(HitRec *d, const HitRec &h) {
+  asm volatile("st.global.v8.b32 [%0], {%1, %2, %3, %4, %5, %6, %7, %8};" ::"l"(d), "r"(h.a), "r"(h.b),
+               "r"((uint32_t)h.order), "r"((uint32_t)(h.order >> 32)), "r"(__float_as_uint(h.lo_x)),
+               "r"(__float_as_uint(h.lo_y)), "r"(__float_as_uint(h.hi_x)), "r"(__float_as_uint(h.hi_y))
+               : "memory");
 }
 
-// Direct emission: the round's records (one per lane with has set; hm =
-// the ballot of has) go straight to the hit buffer at consecutive positions
-// of the warp's window, a new window of HIT_CHUNK reserved when the round
-// does not fit; records past the buffer are processed here.
-__device__ __forceinline__ void emit_round(const PipeDev &p, const HitRec &h, bool has, uint32_t hm, uint32_t t,
-                                           HitWindow &w) {
-  const uint32_t lane = lane_id(), cnt = __popc(hm);
-  if (w.end - w.next < cnt) {
-    for (unsigned long long i = w.next + lane; i < w.end; i += 32)
-      if (i < p.hit_cap) p.hits[i].a = STC_NONE;
-    unsigned long long base = 0;
-    if (lane == 0) base = atomicAdd(&p.st->hit_count, (unsigned long long)HIT_CHUNK);
-    base = __shfl_sync(0xffffffffu, base, 0);
-    w.next = base;
-    w.end = base + HIT_CHUNK;
-  }
-  if (has) {
-    const unsigned long long pos = w.next + __popc(hm & ((1u << lane) - 1u));
-    if (pos < p.hit_cap) p.hits[pos] = h;
-    else process_hit(p, h, t);
-  }
-  w.next += cnt;
+// Appends one hit to the bin of the table tile its home slot lies in, where
+// the table update finds the tile's hits together. The records are 32-byte
+// sectors whose bins' open ends stay in L2 (one 128-byte line a bin: 45 MB
+// for 2^28 slots), so they reach HBM as whole lines. A hit its bin has no
+// room for is applied here; the step then takes the general path.
+__device__ __forceinline__ void bin_hit(const PipeDev &p, const HitRec &h, uint32_t t) {
+  const unsigned long long key = stc_cantor(h.a, h.b);
+  const uint32_t bin = tile_of(p, fast_mod(key, p.B, p.B_magic));
+  const uint32_t pos = atomicAdd(&p.bin_cnt[bin], 1u);
+  if (pos < p.bin_cap) store_hit(&p.hits[(unsigned long long)bin * p.bin_cap + pos], h);
+  else process_hit(p, h, t);
 }
 
 __device__ __forceinline__ HitRec load_hit(const HitRec *r) {
@@ -207,37 +172,29 @@ __device__ __forceinline__ HitRec load_hit(const HitRec *r) {
   return h;
 }
 
-// One thread per hit, two hits in flight per thread: both records and both
-// home slots are requested before either is used.
-// Part `part` applies the hits the pair tests' part `part` appended:
-// [hit_bounds[part], hit_bounds[part + 1]).
-__global__ void __launch_bounds__(256) k_hits(PipeDev p, uint32_t part, uint32_t parts) {
+// The general path's table update: a warp takes 64 hits of a bin, one thread
+// per hit, two hits in flight per thread (both records and both home slots
+// are requested before either is used).
+__global__ void __launch_bounds__(256) k_hits(PipeDev p) {
+  if (fuse_halo(p)) return;
   const uint32_t t = p.st->step_t;
-  (void)parts;
-  const unsigned long long h0i = p.hit_bounds[part], nh = p.hit_bounds[part + 1];
-  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
-  for (unsigned long long i = h0i + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < nh;
-       i += 2 * stride) {
-    unsigned long long i2 = i + stride;
-    HitRec h0 = load_hit(&p.hits[i]);
-    HitRec h1;
-    h1.a = STC_NONE;
-    if (i2 < nh) h1 = load_hit(&p.hits[i2]);
-    const bool v0 = h0.a != STC_NONE, v1 = h1.a != STC_NONE;
-    const unsigned long long k0 = v0 ? stc_cantor(h0.a, h0.b) : 0, k1 = v1 ? stc_cantor(h1.a, h1.b) : 0;
-    unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
-    U128 kv0 = {0, 0}, kv1 = {0, 0};
-    float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
-    if (v0) {
-      kv0 = load_slot_pair(&p.slots[s0]);
-      m0 = __ldcg((const float4 *)&p.slots[s0].lo_x);
-    }
-    if (v1) {
-      kv1 = load_slot_pair(&p.slots[s1]);
-      m1 = __ldcg((const float4 *)&p.slots[s1].lo_x);
-    }
-    if (v0) process_hit_at(p, h0, k0, t, s0, kv0, m0);
-    if (v1) process_hit_at(p, h1, k1, t, s1, kv1, m1);
+  const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  const uint32_t parts = (min((uint32_t)p.st->hit_max, p.bin_cap) + 63) / 64;  // of the fullest bin
+  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+       w < (unsigned long long)p.nb * parts; w += warps) {
+    const uint32_t bin = (uint32_t)(w / parts), i = (uint32_t)(w % parts) * 64 + lane_id();
+    const uint32_t n = min(p.bin_cnt[bin], p.bin_cap);
+    if (i >= n) continue;
+    const HitRec *hits = p.hits + (unsigned long long)bin * p.bin_cap;
+    const bool two = i + 32 < n;
+    const HitRec h0 = load_hit(&hits[i]);
+    const HitRec h1 = load_hit(&hits[two ? i + 32 : i]);
+    const unsigned long long k0 = stc_cantor(h0.a, h0.b), k1 = stc_cantor(h1.a, h1.b);
+    const unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
+    const U128 kv0 = load_slot_pair(&p.slots[s0]), kv1 = load_slot_pair(&p.slots[s1]);
+    const float4 m0 = __ldcg((const float4 *)&p.slots[s0].lo_x), m1 = __ldcg((const float4 *)&p.slots[s1].lo_x);
+    process_hit_at(p, h0, k0, t, s0, kv0, m0);
+    if (two) process_hit_at(p, h1, k1, t, s1, kv1, m1);
   }
 }
 
@@ -273,64 +230,81 @@ __device__ __forceinline__ uint32_t strip_x_bound(const float4 *pts, uint32_t lo
   return lo;
 }
 
+// One row (an own member or a border unit) of the job a warp works on, in
+// shared memory: its point, its candidate segments and where its tests start
+// among the job's. 80 bytes apart, so that 16-byte reads of different rows
+// fall in different banks.
+struct __align__(16) Row {
+  float x, y, scale;         // leaf offsets, metres per degree of longitude
+  uint32_t pid;
+  float fx, fy;              // float position (fxy)
+  uint32_t off;              // first test of the row among the job's
+  uint32_t orig;             // own: place in pid order; border: place of the unit
+  uint32_t seg0, seg1, seg2; // segments: start | end (counted in the row's tests) << 16; start only in seg2
+  uint32_t leaf;             // border: the leaf of the row's point, and its low x, low y, high y in float
+  float ax0, ay0, ay1;
+  uint32_t pad[5];
+};
+
 // One job: 32 rows of leaf g, each against its candidate ranges of members
 // in (strip, longitude) order (stc_partition.cu, k_strip_order). Rows are
 // the leaf's own members (own = true; row i tests the members after it in
 // its strip up to its longitude window's end, and its window in the next
 // strip, so every pair of members within reach is tested once) or 32 border
 // units targeting the leaf (the members in the unit's longitude window in
-// the three strips beside its point). A lane's candidates come in up to
-// three contiguous segments, each read 32 at a time; hits are marked in a
-// bitmask and turned into records after each group.
-// DIRECT: records go straight to the hit buffer (emit_round) instead of
-// through the warp's shared-memory queue; it pays where rows have many hits
-// (dense leaves) and costs registers elsewhere.
-template <bool DIRECT>
+// the three strips beside its point). A row's candidates come in up to
+// three contiguous segments, of which the job takes one chunk of refine_chunk
+// positions. The job's tests are numbered through, row after row, and each
+// lane takes every 32nd, hit or miss: rows have 8 candidates on average but
+// the longest of 32 has several times that, and with a row per lane 17 of 32
+// lanes had work. The tests alone, without records: 1.15 ms of a 10M-object
+// step (93.6M tests, 67.7M hits); with the bins' counters 1.55, with the
+// records' stores 2.85: bound by L2's rate of scattered 32-byte stores (39 G/s
+// measured, 35 with an atomic each). A row per lane and a shared-memory queue
+// of records before it: 3.0 ms for the tests with sequential records.
 __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblock, uint32_t chunk, uint32_t n,
-                         uint32_t t, Counters &ct, HitRec *q, uint32_t &qn, HitWindow &w) {
+                         uint32_t t, Counters &ct, Row *rows) {
   const uint32_t lane = lane_id();
-  const uint32_t lt_mask = (1u << lane) - 1u;
   const uint32_t base = p.grid_start[g];
   const Node *o = &p.sd.nodes[p.sd.gid_node[g]];
-  float4 rp = make_float4(0.f, 0.f, 0.f, 0.f);
-  float2 fr = make_float2(0.f, 0.f);  // the row object's float position (fxy)
-  uint32_t pid1 = 0, orig1 = 0, row_leaf = 0;
-  float ax0 = 0.f, ay0 = 0.f, ay1 = 0.f;  // a border row's own leaf, in float: low x, low y, high y
-  uint32_t sa[3] = {0, 0, 0}, sl[3] = {0, 0, 0};  // candidate segments: start, length
-  unsigned long long rank = 0;
-  bool vr;
+  float x = 0.f, y = 0.f, scale = 0.f, ax0 = 0.f, ay0 = 0.f, ay1 = 0.f;
+  float2 fr = make_float2(0.f, 0.f);
+  uint32_t pid = 0, orig = 0, leaf = 0;
+  uint32_t sa0 = 0, sa1 = 0, sa2 = 0, sl0 = 0, sl1 = 0, sl2 = 0;  // candidate segments: start, length
   if (own) {
     const uint32_t i = rowblock * 32 + lane;
-    vr = i < n;
-    if (vr) {
-      rp = __ldg(&p.spts[base + i]);
+    if (i < n) {
+      const float4 rp = __ldg(&p.spts[base + i]);
       fr = __ldg(&p.sfxy[base + i]);
-      pid1 = __float_as_uint(rp.w);
-      orig1 = __ldg(&p.sorig[base + i]) & 0xFFFFu;
+      x = rp.x;
+      y = rp.y;
+      scale = rp.z;
+      pid = __float_as_uint(rp.w);
+      orig = __ldg(&p.sorig[base + i]) & 0xFFFFu;
       const uint2 c = __ldg(&p.scand[base + i]);
       const uint32_t e1 = c.x & 0xFFFFu, a2 = c.x >> 16;
-      sa[0] = i + 1;
-      sl[0] = e1 > i + 1 ? e1 - (i + 1) : 0u;
-      sa[1] = a2;
-      sl[1] = c.y > a2 ? c.y - a2 : 0u;
+      sa0 = i + 1;
+      sl0 = e1 > i + 1 ? e1 - (i + 1) : 0u;
+      sa1 = a2;
+      sl1 = c.y > a2 ? c.y - a2 : 0u;
     }
   } else {
     const uint32_t ub = p.bu_start[g], ue = p.bu_start[g + 1];
-    const uint32_t r = ub + rowblock * 32 + lane;
-    vr = r < ue;
-    if (vr) {
-      const uint32_t pos = p.bu_sorted_pos[r];
-      pid1 = p.bu_pid[pos];
-      rank = (unsigned long long)p.N + pos;  // border units follow the N own units
-      const double2 qq = p.xy[pid1];
+    const uint32_t u = ub + rowblock * 32 + lane;
+    if (u < ue) {
+      const uint32_t pos = p.bu_sorted_pos[u];
+      orig = pos;
+      pid = p.bu_pid[pos];
+      const double2 qq = p.xy[pid];
       fr = make_float2(__double2float_rn(qq.x), __double2float_rn(qq.y));
-      rp = make_float4(__double2float_rn(RN_SUB(qq.x, o->lo_x)), __double2float_rn(RN_SUB(qq.y, o->lo_y)),
-                       metres_per_deg_lon_f(qq.y), 0.f);
-      // A pair of a border row (pid1 outside leaf g) and a member occurs
-      // twice in this step iff the member also has a border unit targeting
-      // pid1's leaf.
-      row_leaf = p.leaf_gid[pid1];
-      const Node *ro = &p.sd.nodes[p.sd.gid_node[row_leaf]];
+      x = __double2float_rn(RN_SUB(qq.x, o->lo_x));
+      y = __double2float_rn(RN_SUB(qq.y, o->lo_y));
+      scale = metres_per_deg_lon_f(qq.y);
+      // A pair of a border row (outside leaf g) and a member occurs twice in
+      // this step iff the member also has a border unit targeting the row's
+      // leaf.
+      leaf = p.leaf_gid[pid];
+      const Node *ro = &p.sd.nodes[p.sd.gid_node[leaf]];
       ax0 = __double2float_rn(ro->lo_x);
       ay0 = __double2float_rn(ro->lo_y);
       ay1 = __double2float_rn(ro->hi_y);
@@ -338,148 +312,144 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       // strips beside its own (all of a strip too large to be ordered)
       const float4 ls = __ldg(&p.lstrip[g]);
       const int H = (int)ls.y;
-      const int c = (int)fminf(fmaxf(floorf(rp.y * ls.x), -4.0f), (float)H + 4.0f);
+      const int c = (int)fminf(fmaxf(floorf(y * ls.x), -4.0f), (float)H + 4.0f);
       const uint32_t *so = p.sorig + base;
       const float4 *sp = p.spts + base;
-      int k = 0;
-      for (int sidx = c - 1; sidx <= c + 1; sidx++, k++) {
-        if (sidx < 0 || sidx >= H) continue;
+      auto window = [&](int sidx, uint32_t &a, uint32_t &len) {
+        if (sidx < 0 || sidx >= H) return;
         const uint32_t st = strip_lower_bound(so, n, (uint32_t)sidx);
         const uint32_t en = strip_lower_bound(so, n, (uint32_t)sidx + 1);
-        if (st >= en) continue;
-        uint32_t a = st, b = en;
+        if (st >= en) return;
+        uint32_t lo = st, hi = en;
         if (__ldg(&so[st]) & STRIP_XSORTED) {
-          a = strip_x_bound(sp, st, en, rp.x - ls.z, false);
-          b = strip_x_bound(sp, a, en, rp.x + ls.z, true);
+          lo = strip_x_bound(sp, st, en, x - ls.z, false);
+          hi = strip_x_bound(sp, lo, en, x + ls.z, true);
         }
-        sa[k] = a;
-        sl[k] = b - a;
-      }
+        a = lo;
+        len = hi - lo;
+      };
+      window(c - 1, sa0, sl0);
+      window(c, sa1, sl1);
+      window(c + 1, sa2, sl2);
     }
   }
   // this job's chunk: positions [chunk * refine_chunk, (chunk + 1) *
-  // refine_chunk) of the lane's segments taken one after the other
+  // refine_chunk) of the row's segments taken one after the other
   {
     uint32_t skip = chunk * p.refine_chunk, take = p.refine_chunk;
-#pragma unroll
-    for (int seg = 0; seg < 3; seg++) {
-      const uint32_t d = min(skip, sl[seg]);
-      sa[seg] += d;
+    auto cut = [&](uint32_t &a, uint32_t &len) {
+      const uint32_t d = min(skip, len);
+      a += d;
       skip -= d;
-      const uint32_t tk = min(take, sl[seg] - d);
-      sl[seg] = tk;
-      take -= tk;
-    }
+      len = min(take, len - d);
+      take -= len;
+    };
+    cut(sa0, sl0);
+    cut(sa1, sl1);
+    cut(sa2, sl2);
   }
+  // the rows that have tests, with the number of their first one
+  const uint32_t len = sl0 + sl1 + sl2;
+  uint32_t incl = len;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+    if ((int)lane >= d) incl += up;
+  }
+  const uint32_t off = incl - len, total = __shfl_sync(0xffffffffu, incl, 31);
+  const uint32_t nz = __ballot_sync(0xffffffffu, len != 0);
   // error margin: offsets of the members are within the leaf's extent; a
   // border row's own offsets may exceed it
   const float wxl = (float)RN_SUB(o->hi_x, o->lo_x) * 1.000001f, wyl = (float)RN_SUB(o->hi_y, o->lo_y) * 1.000001f;
-  const float mx = fmaxf(wxl, warp_max(fabsf(rp.x))), my = fmaxf(wyl, warp_max(fabsf(rp.y)));
+  const float mx = fmaxf(wxl, warp_max(fabsf(x))), my = fmaxf(wyl, warp_max(fabsf(y)));
+  if (len) {
+    float4 *d = (float4 *)&rows[__popc(nz & ((1u << lane) - 1u))];
+    d[0] = make_float4(x, y, scale, __uint_as_float(pid));
+    d[1] = make_float4(fr.x, fr.y, __uint_as_float(off), __uint_as_float(orig));
+    *(uint4 *)&d[2] = make_uint4(sa0 | sl0 << 16, sa1 | (sl0 + sl1) << 16, sa2, leaf);
+    if (!own) d[3] = make_float4(ax0, ay0, ay1, 0.f);
+  }
+  __syncwarp();
   const float u = 5.9604645e-08f;
-  const float r = (float)p.reach;
+  const float reach = (float)p.reach;
   const float E = 2.1f * u * (2.0f * mx * STC_SMAX_F + 2.0f * my * STC_SLAT_F);
-  const float delta = 4.0f * E + 64.0f * u * r + 1e-6f * r;
-  const float lo = fmaxf(r - delta, 0.0f);
+  const float delta = 4.0f * E + 64.0f * u * reach + 1e-6f * reach;
+  const float lo = fmaxf(reach - delta, 0.0f);
   const float lo2 = lo * lo;
-  const float hi2 = (r + delta) * (r + delta);
-#pragma unroll 1
-  for (int seg = 0; seg < 3; seg++) {
-    const uint32_t a = sa[seg], len = sl[seg];
-    ct.tests += len;
-    const uint32_t maxlen = __reduce_max_sync(0xffffffffu, len);
-    const float4 *cand = p.spts + base + a;
-    for (uint32_t k0 = 0; k0 < maxlen; k0 += 32) {
-      const uint32_t kn = maxlen - k0 < 32u ? maxlen - k0 : 32u;
-      // the column loop only marks hits (one bit per candidate); records are
-      // made afterwards, one per lane per round, so that the loop carries no
-      // warp vote or branch for them
-      uint32_t hitmask = 0;
-#pragma unroll 4
-      for (uint32_t kk = 0; kk < kn; kk++) {
-        const bool valid = k0 + kk < len;
-        const float4 c = valid ? __ldg(&cand[k0 + kk]) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const uint32_t pid2 = __float_as_uint(c.w);
-        // the reference measures from the unit's point: an own pair from its
-        // lower pid (tracing/refinement.cpp:30), a border pair from the unit
-        const bool swap = own && pid2 < pid1;
-        const float dx = (rp.x - c.x) * (swap ? c.z : rp.z);
-        const float dy = (rp.y - c.y) * STC_SLAT_F;
-        const float d2 = dx * dx + dy * dy;
-        bool hit = valid && d2 <= lo2;
-        if (valid && !hit && d2 < hi2) {
-          ct.exact++;
-          hit = swap ? exact_within(p, pid2, pid1, ct.amb) : exact_within(p, pid1, pid2, ct.amb);
-        }
-        hitmask |= (uint32_t)hit << kk;
-      }
-      ct.hits += __popc(hitmask);
-      while (__any_sync(0xffffffffu, hitmask != 0)) {
-        const bool has = hitmask != 0;
-        const uint32_t kk = has ? (uint32_t)(__ffs(hitmask) - 1) : 0u;
-        hitmask &= hitmask - 1u;
-        const uint32_t hm = __ballot_sync(0xffffffffu, has);
-        HitRec h;
-        if (has) {
-          const uint32_t j = a + k0 + kk;
-          const uint32_t cpid = __float_as_uint(__ldg(&p.spts[base + j]).w);
-          const uint32_t corig = __ldg(&p.sorig[base + j]) & 0xFFFFu;
-          const float2 fc = __ldg(&p.sfxy[base + j]);
-          const float2 fa = pid1 < cpid ? fr : fc, fb = pid1 < cpid ? fc : fr;
-          h.a = pid1 < cpid ? pid1 : cpid;
-          h.b = pid1 < cpid ? cpid : pid1;
-          h.lo_x = fminf(fa.x, fb.x);
-          h.lo_y = fminf(fa.y, fb.y);
-          h.hi_x = fmaxf(fa.x, fb.x);
-          h.hi_y = fmaxf(fa.y, fb.y);
-          if (own) {
-            // the pair is found by the lower pid's own unit (rank = its pid)
-            // at the higher pid's place in the pid-ordered member list
-            h.order = ((unsigned long long)h.a << STC_ORDER_SHIFT) | (pid1 < cpid ? corig : orig1);
-          } else {
-            h.order = (rank << STC_ORDER_SHIFT) | corig;
-            // the member has a unit targeting the row's leaf only if it lies
-            // below that leaf, or left of it and below its top (the border
-            // lookup's rule); rounding to float keeps the order, so the test
-            // on floats passes every such member, and the three dependent
-            // loads of its units are left to the few that pass
-            if (fc.y <= ay0 || (fc.y <= ay1 && fc.x <= ax0)) {
-              const uint32_t cnb = p.bcount[cpid];
-              const uint32_t coff = cnb ? p.boff[cpid] : 0u;
-              for (uint32_t u2 = 0; u2 < cnb; u2++)
-                if (p.bu_gid[coff + u2] == row_leaf) h.order |= DUP_BIT;
-            }
-          }
-          if (!DIRECT) q[qn + __popc(hm & lt_mask)] = h;
-        }
-        if (DIRECT) {
-          emit_round(p, h, has, hm, t, w);
-        } else {
-          qn += __popc(hm);
-          if (qn >= 32) {
-            flush_queue(p, q, 32, t, w);
-            const uint32_t rest = qn - 32;
-            HitRec mv;
-            if (lane < rest) mv = q[32 + lane];
-            __syncwarp();
-            if (lane < rest) q[lane] = mv;
-            __syncwarp();
-            qn = rest;
-          }
-        }
+  const float hi2 = (reach + delta) * (reach + delta);
+  uint32_t before = 0;  // rows that started before this round
+  for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+    // one bit per test of the round that is its row's first
+    const uint32_t starts = __reduce_or_sync(0xffffffffu, len != 0 && off - f0 < 32u ? 1u << (off - f0) : 0u);
+    const uint32_t ri = before + __popc(starts & (0xffffffffu >> (31u - lane))) - 1u;
+    before += __popc(starts);
+    if (f0 + lane >= total) continue;
+    const Row *w = &rows[ri];
+    const float4 rp = *(const float4 *)w;
+    const float4 r1 = *((const float4 *)w + 1);
+    const uint4 r2 = *((const uint4 *)w + 2);
+    const uint32_t k = f0 + lane - __float_as_uint(r1.z);
+    const uint32_t e0 = r2.x >> 16, e1 = r2.y >> 16;
+    const uint32_t j = base + (k < e0 ? (r2.x & 0xFFFFu) + k : k < e1 ? (r2.y & 0xFFFFu) + k - e0 : r2.z + k - e1);
+    const float4 c = __ldg(&p.spts[j]);
+    const float2 fc = __ldg(&p.sfxy[j]);
+    const uint32_t corig = __ldg(&p.sorig[j]) & 0xFFFFu;
+    const uint32_t pid1 = __float_as_uint(rp.w), pid2 = __float_as_uint(c.w);
+    const bool less = pid1 < pid2;
+    // the reference measures from the unit's point: an own pair from its
+    // lower pid (tracing/refinement.cpp:30), a border pair from the unit
+    const bool swap = own && !less;
+    const float dx = (rp.x - c.x) * (swap ? c.z : rp.z);
+    const float dy = (rp.y - c.y) * STC_SLAT_F;
+    const float d2 = dx * dx + dy * dy;
+    ct.tests++;
+    bool hit = d2 <= lo2;
+    if (!hit && d2 < hi2) {
+      ct.exact++;
+      hit = swap ? exact_within(p, pid2, pid1, ct.amb) : exact_within(p, pid1, pid2, ct.amb);
+    }
+    if (!hit) continue;
+    ct.hits++;
+    HitRec h;
+    h.a = less ? pid1 : pid2;
+    h.b = less ? pid2 : pid1;
+    const float2 f1 = make_float2(r1.x, r1.y), fa = less ? f1 : fc, fb = less ? fc : f1;
+    h.lo_x = fminf(fa.x, fb.x);
+    h.lo_y = fminf(fa.y, fb.y);
+    h.hi_x = fmaxf(fa.x, fb.x);
+    h.hi_y = fmaxf(fa.y, fb.y);
+    const uint32_t orig1 = __float_as_uint(r1.w);
+    if (own) {
+      // the pair is found by the lower pid's own unit (rank = its pid) at
+      // the higher pid's place in the pid-ordered member list
+      h.order = ((unsigned long long)h.a << STC_ORDER_SHIFT) | (less ? corig : orig1);
+    } else {
+      // border units follow the N own units
+      h.order = (((unsigned long long)p.N + orig1) << STC_ORDER_SHIFT) | corig;
+      // the member has a unit targeting the row's leaf only if it lies below
+      // that leaf, or left of it and below its top (the border lookup's
+      // rule); rounding to float keeps the order, so the test on floats
+      // passes every such member, and the three dependent loads of its units
+      // are left to the few that pass
+      const float4 r3 = *((const float4 *)w + 3);
+      if (fc.y <= r3.y || (fc.y <= r3.z && fc.x <= r3.x)) {
+        const uint32_t cnb = p.bcount[pid2];
+        const uint32_t coff = cnb ? p.boff[pid2] : 0u;
+        for (uint32_t u2 = 0; u2 < cnb; u2++)
+          if (p.bu_gid[coff + u2] == r2.w) h.order |= DUP_BIT;
       }
     }
+    bin_hit(p, h, t);
   }
+  __syncwarp();
 }
 
 // Slice `part` of `parts` runs job chunks [C * part / parts, C * (part + 1) / parts)
 // of the C = ceil(jobs / p.job_chunk) chunks.
-template <bool DIRECT>
 __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint32_t part, uint32_t parts) {
+  __shared__ Row rows_all[REFINE_THREADS / 32][32];
+  Row *rows = rows_all[threadIdx.x >> 5];
   const uint32_t t = p.st->step_t;
-  __shared__ HitRec queues[DIRECT ? 1 : REFINE_THREADS / 32][QCAP];
-  HitRec *q = queues[DIRECT ? 0 : threadIdx.x >> 5];
-  uint32_t qn = 0;  // warp-uniform queue length
-  HitWindow w = {0, 0};
   const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const unsigned long long J = p.st->jobs_total;
@@ -515,16 +485,13 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
       const uint32_t n = cnt < p.leaf_cap ? cnt : p.leaf_cap;
       const uint32_t R = (n + 31) / 32, cc = p.cchunks[g], own_jobs = R * cc;
       if (local < own_jobs) {
-        run_rows<DIRECT>(p, g, true, local / cc, local % cc, n, t, ct, q, qn, w);
+        run_rows(p, g, true, local / cc, local % cc, n, t, ct, rows);
       } else {
         const uint32_t ccb = (n + p.refine_chunk - 1) / p.refine_chunk, b = local - own_jobs;
-        run_rows<DIRECT>(p, g, false, b / ccb, b % ccb, n, t, ct, q, qn, w);
+        run_rows(p, g, false, b / ccb, b % ccb, n, t, ct, rows);
       }
     }
   }
-  if (!DIRECT && qn) flush_queue(p, q, qn, t, w);
-  for (unsigned long long i = w.next + lane_id(); i < w.end; i += 32)
-    if (i < p.hit_cap) p.hits[i].a = STC_NONE;
   // reduce counters per warp (64-bit sums)
   unsigned long long tests = ct.tests, exact = ct.exact, hits = ct.hits, amb = ct.amb;
 #pragma unroll
@@ -542,24 +509,11 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
   }
 }
 
-// hit_bounds[part + 1] = the hit buffer's end after part `part` (its hits
-// are [hit_bounds[part], hit_bounds[part + 1]): parts run in stream order)
-__global__ void k_hit_mark(PipeDev p, uint32_t part) {
-  const unsigned long long n = p.st->hit_count;
-  p.hit_bounds[part + 1] = n < p.hit_cap ? n : p.hit_cap;
-  if (part == 0) p.hit_bounds[0] = 0;
+void step_pairs(PipeDev &p, cudaStream_t s) {
+  for (uint32_t part = 0; part < p.slices; part++)
+    STC_KL k_refine_a<<<num_sms() * p.refine_bps, REFINE_THREADS, 0, s>>>(p, part, p.slices);
 }
 
-void step_pairs_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s) {
-  if (p.direct_hits)
-    STC_KL k_refine_a<true><<<num_sms() * p.refine_bps, REFINE_THREADS, 0, s>>>(p, part, parts);
-  else
-    STC_KL k_refine_a<false><<<num_sms() * p.refine_bps, REFINE_THREADS, 0, s>>>(p, part, parts);
-  STC_KL k_hit_mark<<<1, 1, 0, s>>>(p, part);
-}
-
-void step_hits_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s) {
-  STC_KL k_hits<<<num_sms() * p.hits_bps, 256, 0, s>>>(p, part, parts);
-}
+void step_hits(PipeDev &p, cudaStream_t s) { STC_KL k_hits<<<num_sms() * p.hits_bps, 256, 0, s>>>(p); }
 
 }  // namespace stc
