@@ -375,61 +375,71 @@ __device__ uint32_t heap_pop(uint32_t *h, uint32_t &n) {
 // PAR_MAX_EVENTS events and no merge whose parent has a higher index (the
 // only source of a cascade). Without cascades every event's decision is fixed
 // by phase 1, and the sequential replay's only coupling is through the two
-// free stacks: a split pushes its own grid id, then pops 4 node slots and 4
-// grid ids; a merge pushes its 4 children and their grid ids and pops the last
-// one back. The events touch at most 4 stack positions each side of where the
-// step starts, so one thread replays just the stack operations, in event
-// order, on windows of both stacks held in shared memory; all node and grid
-// bookkeeping is then written in parallel, merges before splits (a node or
-// grid id freed by a merge can only be reused by a later split). The per-step
-// grid counts are not reset: nothing reads them before the next step
-// recounts. Sets *done; k_schema_phase2 then does nothing.
+// free stacks, whose operations have a closed form. A split takes 4 node
+// slots off the schema stack and, its own grid id first, 3 more grid ids off
+// the grid stack; a merge puts its 4 children's slots and 3 of their grid ids
+// back and keeps the fourth. So both stacks move by one group at a time, and
+// at level k (splits less merges so far) a split takes group k: what the
+// latest earlier merge that ended at level k put there, or the stack's
+// content from before the step. Every split looks for its merge among the
+// events' levels in shared memory (one thread replaying the stacks took 0.86
+// ms of a 10M-object step, which the table update no longer hides; this
+// takes 0.03). Node and grid bookkeeping is then written in parallel, merges
+// before splits (a node or grid id freed by a merge can only be reused by a
+// later split). The per-step grid counts are not reset: nothing reads them
+// before the next step recounts. Sets *done; k_schema_phase2 then does
+// nothing.
 static constexpr uint32_t PAR_MAX_EVENTS = 4096;
-static constexpr uint32_t PAR_WIN = 4 * PAR_MAX_EVENTS + 8;  // stack positions one step can touch
-static constexpr size_t PAR_SMEM = (size_t)PAR_MAX_EVENTS * 5 + (size_t)2 * PAR_WIN * 4;  // 148 KB
 
-// Per-event scratch in global memory: popped / pushed values.
+// Per-event scratch in global memory: split -> 4 children, 4 grid ids taken;
+// merge -> its 4 children, their 4 grid ids.
 struct ParScratch {
-  uint32_t *node;
-  uint32_t *val;  // 8 per event: split -> 4 children, 4 grid ids; merge -> 4 children, 4 grid ids
+  uint32_t *val;  // 8 per event
 };
 
-__device__ __forceinline__ ParScratch par_scratch(uint32_t *base, uint32_t cap) {
-  ParScratch ps;
-  ps.node = base;
-  ps.val = base + cap;
-  return ps;
+// Largest j < e with v[j] == want, or -1 (v 16-byte aligned).
+__device__ __forceinline__ int last_equal(const int *v, int e, int want) {
+  int j = e - 1;
+  for (; j >= 0 && (j & 3) != 3; j--)
+    if (v[j] == want) return j;
+  for (; j >= 0; j -= 4) {
+    const int4 q = *(const int4 *)&v[j - 3];
+    if (q.w == want) return j;
+    if (q.z == want) return j - 1;
+    if (q.y == want) return j - 2;
+    if (q.x == want) return j - 3;
+  }
+  return -1;
 }
 
 __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const uint32_t *ev_list,
                                                             const unsigned long long *ev_total, unsigned int *done,
                                                             int serial_only, uint32_t *scratch, DevState *st) {
-  extern __shared__ __align__(16) unsigned char smem[];
-  uint32_t *sh_node = (uint32_t *)smem;                              // PAR_MAX_EVENTS
-  uint32_t *swin = sh_node + PAR_MAX_EVENTS;                          // PAR_WIN: schema stack window
-  uint32_t *gwin = swin + PAR_WIN;                                    // PAR_WIN: grid stack window
-  uint8_t *sh_kind = (uint8_t *)(gwin + PAR_WIN);                    // PAR_MAX_EVENTS
-  __shared__ int cascade;
-  __shared__ uint32_t n_merges;
-  const uint32_t tid = threadIdx.x;
+  __shared__ uint32_t sh_node[PAR_MAX_EVENTS];
+  __shared__ __align__(16) int sh_lev[PAR_MAX_EVENTS];  // 4 * (level before the event) + kind
+  __shared__ int warp_sum[32];
+  __shared__ int cascade, bad;
+  const uint32_t tid = threadIdx.x, lane = tid & 31u;
   uint32_t nev = (uint32_t)*ev_total;
   if (tid == 0) {
     *done = 0;
     cascade = 0;
-    n_merges = 0;
+    bad = 0;
     st->schema_path = 0;
   }
   if (nev > PAR_MAX_EVENTS || serial_only) return;
-  ParScratch ps = par_scratch(scratch, PAR_MAX_EVENTS);
+  ParScratch ps{scratch};
   const int ssi0 = (int)st->schema_stack_index, gsi0 = (int)st->grids_stack_index;
   __syncthreads();
-  for (uint32_t e = tid; e < nev; e += blockDim.x) {
-    uint32_t v = ev_list[e];
-    uint32_t node = v >> 2, kind = v & 3u;
+  // thread t owns events [t * per, (t + 1) * per)
+  const uint32_t per = (nev + blockDim.x - 1) / blockDim.x, e0 = min(tid * per, nev), e1 = min(e0 + per, nev);
+  int sum = 0;
+  for (uint32_t e = e0; e < e1; e++) {
+    const uint32_t v = ev_list[e], node = v >> 2, kind = v & 3u;
     sh_node[e] = node;
-    sh_kind[e] = (uint8_t)kind;
+    sh_lev[e] = (int)kind;
+    sum += kind == EV_SPLIT ? 1 : -1;
     if (kind == EV_MERGE) {
-      atomicAdd(&n_merges, 1u);
       uint32_t par = sd.meta[node].parent;
       if (node != 0 && par != STC_NONE && par > node) cascade = 1;
       Node q = sd.nodes[node];
@@ -438,61 +448,77 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
         ps.val[8 * e + 4 + i] = sd.meta[q.child[i]].grid_id;
       }
     } else {
-      ps.val[8 * e + 4] = sd.meta[node].grid_id;  // the split pushes this first
+      ps.val[8 * e + 4] = sd.meta[node].grid_id;  // the split's own grid id goes to its first child
     }
   }
-  __syncthreads();
-  // merges move the stack indices down by 4 each, splits up by 4 (schema) and
-  // at most 4 (grid): the window [idx0 - 4 merges - 4, +PAR_WIN) holds every
-  // position the step touches
-  const int sbase = ssi0 - 4 * (int)n_merges - 4, gbase = gsi0 - 4 * (int)n_merges - 4;
-  for (uint32_t k = tid; k < PAR_WIN; k += blockDim.x) {
-    int qs = sbase + (int)k, qg = gbase + (int)k;
-    swin[k] = (qs >= 0 && qs < (int)sd.S) ? sd.schema_stack[qs] : STC_NONE;
-    gwin[k] = (qg >= 0 && qg < (int)sd.G) ? sd.grids_stack[qg] : STC_NONE;
+  int incl = sum;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+    if ((int)lane >= d) incl += up;
   }
+  if (lane == 31) warp_sum[tid >> 5] = incl;
   __syncthreads();
   if (cascade) {
     if (tid == 0) st->schema_path = 2;
     return;
   }
-  if (tid == 0) {
-    // the stack operations of tracing/filter.cpp:316-375, in event order
-    int si = ssi0 - sbase, gi = gsi0 - gbase;
-    bool bad = false;
-    for (uint32_t e = 0; e < nev && !bad; e++) {
-      uint32_t *v = ps.val + 8 * e;
-      if (sh_kind[e] == EV_SPLIT) {
-        if (si + 4 + sbase > (int)sd.S || gi - 1 + gbase < 0 || gi + 3 + gbase > (int)sd.G) { bad = true; break; }
-        gwin[--gi] = v[4];
-        for (int i = 0; i < 4; i++) {
-          v[i] = swin[si++];
-          v[4 + i] = gwin[gi++];
-        }
-      } else {
-        if (si - 4 + sbase < 0 || gi - 4 + gbase < 0) { bad = true; break; }
-        for (int i = 0; i < 4; i++) {
-          swin[--si] = v[i];
-          gwin[--gi] = v[4 + i];
-        }
-        gi++;  // pops the last pushed grid id back for the merged node (v[7])
-      }
+  int level = incl - sum, total = 0;
+  for (uint32_t w = 0; w < 32; w++) {
+    if (w < (tid >> 5)) level += warp_sum[w];
+    total += warp_sum[w];
+  }
+  for (uint32_t e = e0; e < e1; e++) {
+    const int kind = sh_lev[e], si = ssi0 + 4 * level, gi = gsi0 + 3 * level;
+    sh_lev[e] = level * 4 + kind;
+    if (kind == EV_SPLIT) {
+      if (si + 4 > (int)sd.S || gi - 1 < 0 || gi + 3 > (int)sd.G) bad = 1;
+      level++;
+    } else {
+      if (si - 4 < 0 || gi - 4 < 0) bad = 1;
+      level--;
     }
-    if (bad) stc_set_error(st, ERR_SCHEMA, 0u);
-    st->schema_stack_index = (uint32_t)(si + sbase);
-    st->grids_stack_index = (uint32_t)(gi + gbase);
   }
   __syncthreads();
-  if (st->error) return;
-  // stack windows back to global memory
-  for (uint32_t k = tid; k < PAR_WIN; k += blockDim.x) {
-    int qs = sbase + (int)k, qg = gbase + (int)k;
-    if (qs >= 0 && qs < (int)sd.S) sd.schema_stack[qs] = swin[k];
-    if (qg >= 0 && qg < (int)sd.G) sd.grids_stack[qg] = gwin[k];
+  if (bad) {
+    if (tid == 0) stc_set_error(st, ERR_SCHEMA, 0u);
+    return;
+  }
+  for (uint32_t e = tid; e < nev; e += blockDim.x) {
+    const int lk = sh_lev[e], k = lk >> 2;
+    uint32_t *v = ps.val + 8 * e;
+    if ((lk & 3) == EV_SPLIT) {
+      // the latest earlier merge from level k + 1
+      const int j = last_equal(sh_lev, (int)e, (k + 1) * 4 + EV_MERGE);
+      if (j >= 0) {
+        const uint32_t *m = ps.val + 8 * j;
+        for (int i = 0; i < 4; i++) v[i] = m[3 - i];
+        for (int i = 1; i < 4; i++) v[4 + i] = m[4 + 3 - i];
+      } else {
+        for (int i = 0; i < 4; i++) v[i] = sd.schema_stack[ssi0 + 4 * k + i];
+        for (int i = 1; i < 4; i++) v[4 + i] = sd.grids_stack[gsi0 + 3 * k + i - 1];
+      }
+    }
+  }
+  __syncthreads();
+  // what the step leaves on the stacks: each free group's last merge
+  for (uint32_t e = tid; e < nev; e += blockDim.x) {
+    const int lk = sh_lev[e], k = (lk >> 2) - 1;  // the group a merge fills
+    if ((lk & 3) != EV_MERGE || k < total) continue;
+    uint32_t j = e + 1;
+    while (j < nev && sh_lev[j] != lk) j++;
+    if (j < nev) continue;  // filled again later
+    const uint32_t *m = ps.val + 8 * e;
+    for (int i = 0; i < 4; i++) sd.schema_stack[ssi0 + 4 * k + 3 - i] = m[i];
+    for (int i = 0; i < 3; i++) sd.grids_stack[gsi0 + 3 * k + 2 - i] = m[4 + i];
+  }
+  if (tid == 0) {
+    st->schema_stack_index = (uint32_t)(ssi0 + 4 * total);
+    st->grids_stack_index = (uint32_t)(gsi0 + 3 * total);
   }
   // merges (tracing/filter.cpp:316-336)
   for (uint32_t e = tid; e < nev; e += blockDim.x) {
-    if (sh_kind[e] != EV_MERGE) continue;
+    if ((sh_lev[e] & 3) != EV_MERGE) continue;
     uint32_t cur = sh_node[e];
     const uint32_t *v = ps.val + 8 * e;
     for (int i = 0; i < 4; i++) sd.meta[v[i]].type = NODE_INVALID;
@@ -506,7 +532,7 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
   __syncthreads();
   // splits (tracing/filter.cpp:338-375)
   for (uint32_t e = tid; e < nev; e += blockDim.x) {
-    if (sh_kind[e] != EV_SPLIT) continue;
+    if ((sh_lev[e] & 3) != EV_SPLIT) continue;
     uint32_t cur = sh_node[e];
     const uint32_t *v = ps.val + 8 * e;
     Node q = sd.nodes[cur];
@@ -540,10 +566,8 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
   }
   __syncthreads();
   if (tid == 0) {
-    uint32_t splits = 0, merges = 0;
-    for (uint32_t e = 0; e < nev; e++) (sh_kind[e] == EV_SPLIT ? splits : merges)++;
-    st->splits = splits;
-    st->merges = merges;
+    st->splits = (uint32_t)((int)nev + total) / 2;
+    st->merges = (uint32_t)((int)nev - total) / 2;
     st->events = nev;
     st->schema_path = 1;
     *done = 1;
@@ -610,10 +634,6 @@ __global__ void k_schema_phase2(SchemaDev sd, uint32_t *grid_count, const uint32
   st->events = nev;
 }
 
-cudaError_t schema_prepare() {
-  return cudaFuncSetAttribute(k_schema_phase2_par, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)PAR_SMEM);
-}
-
 void update_schema(SchemaDev sd, SchemaWork w, uint32_t *grid_count, double reach, uint32_t grid_capacity,
                    uint32_t delay, int serial_only, DevState *st, cudaStream_t s) {
   STC_KL k_schema_phase1<<<nblk(sd.S), 256, 0, s>>>(sd, grid_count, reach, grid_capacity, delay, w.ev_flag, w.old_under);
@@ -622,7 +642,7 @@ void update_schema(SchemaDev sd, SchemaWork w, uint32_t *grid_count, double reac
   exclusive_scan_u32(w.ev_pos, w.ev_pos, sd.S, w.ev_total, w.scan_tmp, s);
   STC_KL k_schema_compact<<<nblk(sd.S), 256, 0, s>>>(w.ev_flag, w.ev_pos, sd.S, w.ev_list);
   unsigned int *done = (unsigned int *)(w.ev_total + 1);
-  STC_KL k_schema_phase2_par<<<1, 1024, PAR_SMEM, s>>>(sd, w.ev_list, w.ev_total, done, serial_only, w.par_scratch,
+  STC_KL k_schema_phase2_par<<<1, 1024, 0, s>>>(sd, w.ev_list, w.ev_total, done, serial_only, w.par_scratch,
                                                       st);
   STC_KL k_schema_phase2<<<1, 32, 0, s>>>(sd, grid_count, w.ev_list, w.ev_total, w.old_under, w.heap, w.queued,
                                    grid_capacity, delay, done, st);
