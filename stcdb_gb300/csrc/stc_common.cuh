@@ -11,7 +11,6 @@
 #define STC_INIT_LO 100000.0f
 #define STC_INIT_HI -100000.0f
 #define STC_NONE 0xFFFFFFFFu
-#define STC_ORDER_SHIFT 24          // order = unit_rank << 24 | member index
 #define STC_MAX_LEAF_CAP (1u << 16)    // leaf list capacity bound (tile counts fit in 32 bits)
 #define STC_MAX_DEPTH 96            // descent / lookup depth bound
 #define STC_PROBE_LIMIT (1ULL << 16)  // longest probe walk before the table counts as full
@@ -66,9 +65,9 @@ struct NodeMeta {
 // One pair within reach found by the refinement, waiting to be applied to
 // the meeting table: the pair (a < b; a = STC_NONE marks an unused record),
 // its priority and its MBR contribution, the box of the two objects' float
-// positions of the step (fxy; lo = fminf(a's, b's), hi = fmaxf(a's, b's)).
+// positions of the step (lo = fminf(a's, b's), hi = fmaxf(a's, b's)).
 // The key cantor(a, b) is rebuilt when applied. Carrying the box saves the
-// table update two dependent random reads of fxy per extended meeting.
+// table update two dependent random reads of positions per extended meeting.
 struct __align__(32) HitRec {
   uint32_t a, b;
   unsigned long long order;  // bit 63: the pair may occur twice this step
@@ -183,12 +182,17 @@ __device__ __forceinline__ void cantor_decode(unsigned long long z, uint32_t *a,
   *a = (uint32_t)(w - (z - t));
 }
 
-// metres per degree of longitude at latitude y (1/dpml), single precision;
-// used only by the conservative pre-filter, never for a decision by itself.
-__device__ __forceinline__ float metres_per_deg_lon_f(double y) {
-  float absla = (float)fabs(y);
-  float arg = (90.0f - absla) * (3.14159265f / 180.0f);
+// metres per degree of longitude at float latitude y (1/dpml), single
+// precision; used only by the conservative pre-filter, never for a decision
+// by itself.
+__device__ __forceinline__ float metres_per_deg_lon_f(float y) {
+  float arg = (90.0f - fabsf(y)) * (3.14159265f / 180.0f);
   return sinf(arg) * 111322.2222222f;
+}
+
+// An object's float position (the MBR's coordinates).
+__device__ __forceinline__ float2 float_pos(double2 q) {
+  return make_float2(__double2float_rn(q.x), __double2float_rn(q.y));
 }
 
 #define STC_SLAT_F 111322.2222222f   // metres per degree of latitude (1/dpm_lat)
@@ -220,6 +224,9 @@ namespace stc {
 size_t scan_tmp_words(size_t n);
 void exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, unsigned long long *total, uint32_t *tmp,
                         cudaStream_t s);
+
+// In-place exclusive scan of nb block sums by one block; total as above.
+void scan_sums_u32(uint32_t *sums, size_t nb, unsigned long long *total, cudaStream_t s);
 
 // Stable LSD radix sort of (key, value) uint32 pairs on the low `bits` key
 // bits. n_dev (device) holds the item count, n_max bounds it. Result lands

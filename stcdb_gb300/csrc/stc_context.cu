@@ -382,8 +382,11 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
                              : bin_share(std::max<uint64_t>(1u << 22, 8ULL * n), p.nb, 5, 4, 64);
   p.U_cap = (uint64_t)k.refine_size * n - n;
   p.reach = k.reach_distance;
+  p.reach_f = (float)k.reach_distance;
   p.x_buffer = k.reach_distance * stc_dpml_ref(mbr[1]);  // tracing/filter.cpp:30
   p.y_buffer = k.reach_distance * stc_dpm_lat();          // tracing/filter.cpp:31
+  p.x_buffer_f = (float)p.x_buffer;
+  p.y_buffer_f = (float)p.y_buffer;
   p.map_lo_x = mbr[0]; p.map_lo_y = mbr[1]; p.map_hi_x = mbr[2]; p.map_hi_y = mbr[3];
   {
     // for a float f and double D: f >= D <=> f >= (smallest float >= D), and
@@ -403,37 +406,53 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   p.refine_bps = k.refine_blocks_per_sm ? std::min<uint32_t>(k.refine_blocks_per_sm, 32u) : 8u;
   p.hits_bps = k.hits_blocks_per_sm ? std::min<uint32_t>(k.hits_blocks_per_sm, 64u) : 16u;
 
-  size_t nu = std::max<size_t>(n, p.U_cap);
-  size_t scan_words = scan_tmp_words(std::max<size_t>({(size_t)n, (size_t)p.G + 1, (size_t)p.S,
-                                                      radix_hist_words(nu)}));
+  p.leaves_max = std::min(p.G, n);
+  // refinement jobs: one per row block of 32 members or units, and room to
+  // cut those with long candidate windows into chunks
+  p.jobs_extra = std::min<uint64_t>(1ull << 22, (1ull << 16) + 16ull * n);
+  const uint64_t jobs_cap = (n + p.U_cap) / 32 + 2ull * p.leaves_max + p.jobs_extra + 64;
+  // blocks of the border lookup: large ones pack the border points of 1024
+  // pids together (10M objects), small ones spread few objects over the GPU
+  p.border_tile = n >= (1u << 19) ? 1024 : 256;
+  const uint32_t border_tiles = (uint32_t)(((uint64_t)n + p.border_tile - 1) / p.border_tile);
+  p.order_shift = 1;
+  while ((1ull << p.order_shift) < n) p.order_shift++;
+  if (((n + p.U_cap) >> (63 - p.order_shift)) != 0) {
+    // (unit ranks and pids that need more than 63 bits together; the units
+    // alone would not fit any device)
+    g_create_error = "stc_create: refine_size * num_objects is too large";
+    destroy_all(c);
+    delete c;
+    return STC_ERR_CAPACITY;
+  }
+  // descents start from a grid of about one cell per 50 objects
+  p.sd.start_edge = 64;
+  while (p.sd.start_edge < 1024 && (double)p.sd.start_edge * p.sd.start_edge * 50.0 < (double)n) p.sd.start_edge *= 2;
+  p.sd.start_sx = (float)(p.sd.start_edge / (mbr[2] - mbr[0]));
+  p.sd.start_sy = (float)(p.sd.start_edge / (mbr[3] - mbr[1]));
   bool ok = dalloc(c, &p.st, 1) && dalloc(c, &c->xy_own, n) && dalloc(c, &p.sd.nodes, p.S) &&
+            dalloc(c, &p.sd.walk, p.S) && dalloc(c, &p.sd.wbox, p.S) && dalloc(c, &p.sd.start, (size_t)p.sd.start_edge * p.sd.start_edge + 1) &&
             dalloc(c, &p.sd.meta, p.S) && dalloc(c, &p.sd.schema_stack, p.S) && dalloc(c, &p.sd.grids_stack, p.G) &&
             dalloc(c, &p.sd.gid_node, p.G) && dalloc(c, &p.sw.bnodes, p.S) && dalloc(c, &p.sw.bmeta, p.S) &&
             dalloc(c, &p.sw.bcount, p.S) && dalloc(c, &p.sw.bsub_nodes, p.S) &&
             dalloc(c, &p.sw.bsub_leaves, p.S) && dalloc(c, &p.sw.bpre, p.S) && dalloc(c, &p.sw.bleafbase, p.S) &&
-            dalloc(c, &p.sw.node_of, n) && dalloc(c, &p.sw.ev_flag, p.S) && dalloc(c, &p.sw.ev_pos, p.S) &&
+            dalloc(c, &p.sw.node_of, n) && dalloc(c, &p.sw.ev_flag, (size_t)p.S + 16) && dalloc(c, &p.sd.high, 2) &&
             dalloc(c, &p.sw.ev_list, p.S) && dalloc(c, &p.sw.old_under, p.S) && dalloc(c, &p.sw.heap, p.S) &&
-            dalloc(c, &p.sw.ev_total, 2) && dalloc(c, &p.sw.par_scratch, 8 * 4096) && dalloc(c, &p.sw.queued, p.S) && dalloc(c, &p.leaf_gid, n) &&
-            dalloc(c, &p.lastvalid, n) && dalloc(c, &p.iota, nu) && dalloc(c, &p.sorted_gid, n) &&
-            dalloc(c, &p.sorted_pid, n) && dalloc(c, &p.sort_ktmp, nu) && dalloc(c, &p.sort_vtmp, nu) &&
-            dalloc(c, &p.sort_hist, radix_hist_words(nu)) && dalloc(c, &p.grid_count, (size_t)p.G + 1) &&
-            dalloc(c, &p.sort_ktmp2, nu) && dalloc(c, &p.sort_vtmp2, nu) &&
-            dalloc(c, &p.sort_hist2, radix_hist_words(nu)) && dalloc(c, &p.scan_tmp2, scan_words) &&
-            dalloc(c, &p.grid_start, (size_t)p.G + 1) && dalloc(c, &p.pts, n) && dalloc(c, &p.fxy, n) &&
-            dalloc(c, &p.gfxy, n) && dalloc(c, &p.sfxy, n) &&
-            dalloc(c, &p.spts, n) && dalloc(c, &p.sorig, n) && dalloc(c, &p.scand, n) &&
-            dalloc(c, &p.lstrip, p.G) && dalloc(c, &p.cchunks, p.G) &&
-            dalloc(c, &p.bcount, (size_t)n + 1) && dalloc(c, &p.boff, (size_t)n + 1) &&
-            dalloc(c, &p.blist, n) && dalloc(c, &p.bres, 4 * (size_t)n) && dalloc(c, &p.sd.fbox, p.S) &&
-            dalloc(c, &p.bu_gid, p.U_cap) && dalloc(c, &p.bu_pid, p.U_cap) && dalloc(c, &p.bu_sorted_gid, p.U_cap) &&
-            dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, (size_t)p.G + 1) &&
-            dalloc(c, &p.bu_start, (size_t)p.G + 1) && dalloc(c, &p.job_cnt, (size_t)p.G + 1) &&
-            dalloc(c, &p.job_start, (size_t)p.G + 1) && dalloc(c, &p.slots, p.B) && 
+            dalloc(c, &p.sw.par_scratch, 8 * 4096) && dalloc(c, &p.sw.queued, p.S) && dalloc(c, &p.leaf_gid, n) &&
+            dalloc(c, &p.ctr, CTR_COUNT) && dalloc(c, &p.lastvalid, n) && dalloc(c, &p.rank, n) &&
+            dalloc(c, &p.lpid, n) && dalloc(c, &p.lpid2, n) && dalloc(c, &p.grid_count, p.G) &&
+            dalloc(c, &p.grid_start, p.G) && dalloc(c, &p.leaf_list, p.leaves_max) && dalloc(c, &p.pts, n) &&
+            dalloc(c, &p.sfxy, n) && dalloc(c, &p.spts, n) && dalloc(c, &p.scand, n) &&
+            dalloc(c, &p.sstart, (size_t)p.G * STRIP_STRIDE) && dalloc(c, &p.lgeo, p.G) &&
+            dalloc(c, &p.jobs, jobs_cap) && dalloc(c, &p.bcount, n) && dalloc(c, &p.boff, n) &&
+            dalloc(c, &p.bsum, border_tiles) && dalloc(c, &p.bres, 4 * (size_t)n) && dalloc(c, &p.sd.fbox, p.S) &&
+            dalloc(c, &p.bu_gid, p.U_cap) && dalloc(c, &p.bu_pid, p.U_cap) && dalloc(c, &p.bu_rank, p.U_cap) &&
+            dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, p.G) && dalloc(c, &p.bu_start, p.G) &&
+            dalloc(c, &p.slots, p.B) &&
             dalloc(c, &p.hits, (size_t)p.nb * p.bin_cap) && dalloc(c, &p.bin_cnt, p.nb) &&
             dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
             dalloc(c, &p.carry_cnt, p.runs) && dalloc(c, &p.cset, p.C) &&
-            dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E) && dalloc(c, &p.scan_tmp, scan_words) &&
-            dalloc(c, &p.n_dev, 1);
+            dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E);
   if (ok && k.kv_restriction) {
     LsmDev &L = c->lsm;
     memset(&L, 0, sizeof(L));
@@ -491,16 +510,20 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
     // the degree distance adds <= u W, scaled to metres by <= 111.4 km/deg.
     const double u = 5.9604644775390625e-08;
     double ext_m = (mbr[2] - mbr[0]) * 111322.3 + (mbr[3] - mbr[1]) * 111322.3;
+    // float comparisons of box corners and points: offsets from the map corner
+    // round by u times the extent, the buffers by u times themselves, sums and
+    // differences by u times both
+    p.border_eps = (float)(u * (16.0 * std::max(mbr[2] - mbr[0], mbr[3] - mbr[1]) +
+                                8.0 * std::max(p.x_buffer, p.y_buffer)));
     p.border_delta = (float)(32.0 * u * ext_m + 64.0 * u * k.reach_distance + 1e-6 * k.reach_distance);
   }
-  p.sw.scan_tmp = p.scan_tmp;
   cudaStream_t s = c->stream;
   cudaMemsetAsync(p.st, 0, sizeof(DevState), s);
   cudaMemsetAsync(p.sw.queued, 0, p.S, s);
+  cudaMemsetAsync(p.sw.ev_flag, 0, (size_t)p.S + 16, s);
+  cudaMemsetAsync(p.grid_count, 0, (size_t)p.G * sizeof(uint32_t), s);
+  cudaMemsetAsync(p.bu_cnt, 0, (size_t)p.G * sizeof(uint32_t), s);
   cudaMemsetAsync(p.tile_live, 0, (size_t)p.nb * sizeof(uint32_t), s);
-  unsigned long long nn = n;
-  cudaMemcpyAsync(p.n_dev, &nn, sizeof(nn), cudaMemcpyHostToDevice, s);
-  iota_u32(p.iota, nu, s);
   init_tables(p, s);
   if (c->lsm_on) lsm_init(c->lsm, s);
   e = cudaSuccess;
@@ -570,18 +593,15 @@ static void issue_step(stc_ctx *c, bool events, bool append, const uint32_t *two
   step_begin(p, tword, s);
   if (events) cudaEventRecord(c->ev[PH_COPY], s);
   step_descend(p, s);
-  // the border units (lookups, scan, sort by leaf) need the descent only:
-  // they run on the side stream, with their own scratch, beside the
-  // leaf-order sort and gather
+  // the border units need the descent only: they run on the side stream
+  // beside the leaves' members
   cudaEventRecord(c->fork2_ev, s);
   cudaStreamWaitEvent(c->side, c->fork2_ev, 0);
   step_border(p, c->side);
   cudaEventRecord(c->join2_ev, c->side);
-  step_leaf_order(p, s);
-  step_strips(p, s);
+  step_leaves(p, s);
   if (events) cudaEventRecord(c->ev[PH_PART], s);
   cudaStreamWaitEvent(s, c->join2_ev, 0);
-  step_jobs(p, s);
   if (events) cudaEventRecord(c->ev[PH_BORDER], s);
   step_pairs(p, s);
   if (events) cudaEventRecord(c->ev[PH_REFINE], s);
@@ -1633,7 +1653,16 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
     stc_destroy(c);
     return STC_ERR_CUDA;
   }
+  // the ids in use and on the free stacks are not searched for the highest
+  const uint32_t high[2] = {c->p.S, c->p.G};
+  e = cudaMemcpy(c->p.sd.high, high, sizeof(high), cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);
+    stc_destroy(c);
+    return STC_ERR_CUDA;
+  }
   count_tiles(c->p, c->stream);
+  schema_walk(c->p.sd, c->stream);
   e = cudaStreamSynchronize(c->stream);
   if (e != cudaSuccess) {
     g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);

@@ -67,7 +67,7 @@ __device__ __forceinline__ U128 load_slot_pair(const Slot *s) {
 __device__ __forceinline__ void extend_found(const PipeDev &p, Slot *s, unsigned long long key, uint32_t t) {
   uint32_t a, b;
   cantor_decode(key, &a, &b);
-  float2 fa = p.fxy[a], fb = p.fxy[b];
+  const float2 fa = float_pos(p.xy[a]), fb = float_pos(p.xy[b]);
   s->end = t;
   float lx = fminf(fa.x, fb.x), ly = fminf(fa.y, fb.y), hx = fmaxf(fa.x, fb.x), hy = fmaxf(fa.y, fb.y);
   if (lx < s->lo_x) atomic_min_f(&s->lo_x, lx);

@@ -28,11 +28,25 @@
 // only), keeps active meetings, emits finished ones whose duration reaches
 // min_meet_time (tracing/meeting.cpp:59, plus the map-box filter of
 // cuda/geometry.cu:667) and clears the rest.
+#include <algorithm>
+
 #include "stc_insert.cuh"
 
 namespace stc {
 
-__global__ void k_step_begin(DevState *st) {
+// The step's counters and counts, and its time: a page-locked word that the
+// host sets before the step is issued (also when the step is replayed from a
+// captured graph), read here over the host link; the step's kernels read it
+// from DevState::step_t.
+__global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t_pinned) {
+  const uint32_t first = blockIdx.x * blockDim.x + threadIdx.x, stride = gridDim.x * blockDim.x;
+  const uint32_t leaves = p.sd.high[1];
+  for (uint32_t i = first; i < leaves; i += stride) p.grid_count[i] = p.bu_cnt[i] = 0;
+  for (uint32_t i = first; i < p.nb; i += stride) p.bin_cnt[i] = 0;
+  if (first < CTR_COUNT) p.ctr[first] = 0;
+  if (first) return;
+  DevState *st = p.st;
+  st->step_t = *(const volatile uint32_t *)t_pinned;
   st->error = 0;
   st->error_info = 0;
   st->border_units = 0;
@@ -50,12 +64,8 @@ __global__ void k_step_begin(DevState *st) {
   st->overflow_objects = 0;
 }
 
-// The step's time goes to the device from a page-locked word that the host
-// sets before the step is issued (also when the step is replayed from a
-// captured graph); the step's kernels read it from DevState::step_t.
 void step_begin(PipeDev &p, const uint32_t *t_pinned, cudaStream_t s) {
-  cudaMemcpyAsync(&p.st->step_t, t_pinned, sizeof(uint32_t), cudaMemcpyHostToDevice, s);
-  STC_KL k_step_begin<<<1, 1, 0, s>>>(p.st);
+  STC_KL k_step_begin<<<num_sms() * 2, 256, 0, s>>>(p, t_pinned);
 }
 
 __global__ void k_init_slots(Slot *slots, unsigned long long B) {
@@ -140,8 +150,8 @@ __device__ __forceinline__ ClaimPos claim_positions(const PipeDev &p, const Slot
   if (s.key != STC_EMPTY_KEY && (s.key & STC_CLAIM_BIT)) {
     uint32_t a, b;
     cantor_decode(s.key & ~STC_CLAIM_BIT, &a, &b);
-    c.fa = __ldg(&p.fxy[a]);
-    c.fb = __ldg(&p.fxy[b]);
+    c.fa = float_pos(p.xy[a]);
+    c.fb = float_pos(p.xy[b]);
   }
   return c;
 }
@@ -298,8 +308,13 @@ __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(Pi
 static constexpr uint32_t SWEEP_WAVES = 8;
 
 void step_sweep(PipeDev &p, cudaStream_t s) {
+  // (a small table takes fewer: a step that does not need the sweep leaves it
+  // at once, block by block)
+  const unsigned blocks = (unsigned)std::min<unsigned long long>(
+      (unsigned long long)num_sms() * SWEEP_BLOCKS_PER_SM * SWEEP_WAVES,
+      p.B / (4 * SWEEP_WARPS * WARP_TILE) + 1);
   for (uint32_t part = 0; part < p.slices; part++)
-    STC_KL k_sweep<<<num_sms() * SWEEP_BLOCKS_PER_SM * SWEEP_WAVES, SWEEP_THREADS, 0, s>>>(p, part, p.slices);
+    STC_KL k_sweep<<<blocks, SWEEP_THREADS, 0, s>>>(p, part, p.slices);
 }
 
 }  // namespace stc

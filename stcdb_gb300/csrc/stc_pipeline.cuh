@@ -5,8 +5,25 @@
 
 namespace stc {
 
-// sorig flag: the member's strip is ordered by longitude offset
-#define STRIP_XSORTED (1u << 22)
+constexpr uint32_t STRIPS_MAX = 64;     // horizontal strips of a leaf
+constexpr uint32_t STRIP_STRIDE = 68;   // words of a leaf's strip starts (STRIPS_MAX + 1, padded)
+constexpr uint32_t XSORT_MAX = 128;     // strips of at most this many members are in longitude order
+constexpr uint32_t LEAF_SMALL = 256;    // kept members of the leaves k_leaf_small takes
+constexpr uint32_t JOB_OWN = 1u << 31;
+
+// A leaf as the refinement sees it.
+struct __align__(16) LeafGeo {
+  double lo_x, lo_y;       // low corner
+  float inv, wx;           // strips per degree of latitude from the low edge; longitude window in degrees
+  uint32_t strips;
+  float ext_x, ext_y;      // extent in degrees
+  uint32_t base, n;        // its members: spts[base .. base + n)
+  uint32_t pad;
+};
+
+// counters of a step (PipeDev::ctr)
+enum { CTR_MEMBERS = 0, CTR_SMALL, CTR_BIG, CTR_EXTRA, CTR_UNITS, CTR_POOL, CTR_COUNT };
+
 // Candidate positions per refinement job and lane: a row block's candidate
 // ranges are cut into chunks of this many, so that the n^2 / 2 pair tests of
 // a dense leaf spread over many warps.
@@ -23,6 +40,7 @@ struct PipeDev {
   unsigned long long U_cap;        // border units (refine_size*N - N - 1)
   // parameters
   double reach, x_buffer, y_buffer;
+  float reach_f, x_buffer_f, y_buffer_f;
   double map_lo_x, map_lo_y, map_hi_x, map_hi_y;
   float fmap_lo_x, fmap_lo_y, fmap_hi_x, fmap_hi_y;  // float f: f >= map_lo <=> f >= fmap_lo, etc.
   uint32_t min_meet_time, grid_capacity, delay;
@@ -39,33 +57,39 @@ struct PipeDev {
   const double2 *xy_in = nullptr;  // when set: page-locked host positions the descent reads and
                                    // copies to xy (a buffer of the context's own)
   // partition
-  uint32_t *leaf_gid, *lastvalid, *iota, *sorted_gid, *sorted_pid, *sort_ktmp, *sort_vtmp, *sort_hist;
-  uint32_t *grid_count, *grid_start;   // G, G+1
-  float4 *pts;                          // N sorted: lx, ly, metres/deg lon, pid bits
-  float2 *fxy;                          // N by pid: float lon, lat (MBR of new meetings)
-  float2 *gfxy;                         // N in leaf order (pid order within a leaf): fxy of each member
-  float2 *sfxy;                         // N in strip order (as spts): fxy of each member
-  // each leaf's kept members again, ordered by horizontal strip (strips at
-  // least reach tall) and, within a small strip, by longitude: spts as pts;
-  // sorig = member index in pid order | strip << 16 | STRIP_XSORTED;
-  // scand = the member's candidate ranges within the leaf: [i + 1, x & 0xFFFF)
-  // in its strip and [x >> 16, y) in the next; lstrip[g] = (strips per degree
-  // of latitude from the leaf's low corner, strip count, longitude window wx
-  // in degrees, 0)
+  unsigned long long *ctr;              // CTR_COUNT
+  uint32_t *leaf_gid, *lastvalid;       // N
+  uint32_t *rank;                       // N: the object's number within its leaf (any order)
+  uint32_t *lpid, *lpid2;               // N: leaf member lists; the kept members of overfull leaves
+  uint32_t *grid_count, *grid_start;    // G: members of each leaf, start of its list
+  uint32_t *leaf_list;                  // leaves with members: small ones from the front, big from the end
+  uint32_t leaves_max;                  // its length
+  float4 *pts;                          // N: big leaves' members before the strip order
+  float2 *sfxy;                         // N in strip order (as spts): float lon, lat of each member
+  // each leaf's kept members, ordered by horizontal strip (strips at least
+  // reach tall) and, within a small strip, by longitude: spts = leaf offsets
+  // lx, ly, metres per degree of longitude, pid bits; scand = the member's
+  // candidate ranges within the leaf: [i + 1, x & 0xFFFF) in its strip and
+  // [x >> 16, y) in the next; sstart[g * STRIP_STRIDE + s] = first member of
+  // strip s
   float4 *spts;
-  uint32_t *sorig;
   uint2 *scand;
-  float4 *lstrip;
-  uint32_t *cchunks;                    // G: candidate chunks of refine_chunk per own row block
+  uint16_t *sstart;
+  LeafGeo *lgeo;                        // G
+  // refinement jobs: (leaf, row block | JOB_OWN, first chunk, chunks)
+  uint4 *jobs;
+  unsigned long long jobs_extra;        // jobs beyond one per row block the list has room for
+  uint32_t order_shift;                 // a hit's priority: unit rank << order_shift | member pid
   // border units
-  uint32_t *bcount, *boff;              // N+1 (border units per pid, exclusive offsets)
-  uint32_t *blist;                      // N: pids of border points (any order)
+  uint32_t *bcount, *boff;              // N (border units per pid, their place in rank order)
+  uint32_t *bsum;                       // units before each block of border_tile pids
+  uint32_t border_tile;                 // 256 or 1024 pids per block of the border lookup
   uint32_t *bres;                       // 4N: first four lookup results per border point
   float border_delta;                   // fp32 band (metres) of the border lookup pre-filter
+  float border_eps;                     // fp32 band (degrees) of its leaf test
   uint32_t *bu_gid, *bu_pid;            // U_cap (rank order)
-  uint32_t *bu_sorted_gid, *bu_sorted_pos;  // U_cap grouped by leaf
-  uint32_t *bu_cnt, *bu_start;          // G+1
-  uint32_t *job_cnt, *job_start;        // G+1
+  uint32_t *bu_rank, *bu_sorted_pos;    // U_cap: number within the leaf; places grouped by leaf
+  uint32_t *bu_cnt, *bu_start;          // G
   // meetings
   Slot *slots;                          // B
   // hits of the step, binned by table tile (tile_of): bin j holds records
@@ -81,22 +105,14 @@ struct PipeDev {
   Cand *cset;                           // C
   uint32_t *cand_list;                  // cand_cap
   stc_meeting *emit;                    // E
-  uint32_t *scan_tmp;
-  // scratch of the border units' scan and sort, which run on the side
-  // stream beside the leaf-order sort
-  uint32_t *scan_tmp2, *sort_ktmp2, *sort_vtmp2, *sort_hist2;
-  unsigned long long *n_dev;            // device copy of N (for radix sort)
 };
 
 // stc_partition.cu
-// partition in two parts: the descent (leaf of every object, border
-// candidates), then the leaf-order sort, leaf starts and gathered points
+// the descent (leaf of every object), the leaves' members in strip order with
+// their jobs, and beside those the border units with theirs
 void step_descend(PipeDev &p, cudaStream_t s);
-void step_leaf_order(PipeDev &p, cudaStream_t s);
-// each leaf's members in strip order (after step_leaf_order)
-void step_strips(PipeDev &p, cudaStream_t s);
+void step_leaves(PipeDev &p, cudaStream_t s);
 void step_border(PipeDev &p, cudaStream_t s);
-void step_jobs(PipeDev &p, cudaStream_t s);
 // stc_refine.cu
 // the pair tests, which bin the step's hits by table tile, and the general
 // path's table update of them (nothing when the tiled path took the step)

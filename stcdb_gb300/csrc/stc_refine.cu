@@ -13,8 +13,9 @@
 // point -- can hit, and only those are tested. A job is 32 rows (members or
 // border units) of one leaf, one per lane, each over one chunk of
 // refine_chunk positions of its own contiguous segments (a dense leaf's
-// n^2 / 2 pair tests spread over many jobs). Each hit keeps the reference's priority: the finding unit's
-// rank and the member's index in pid order.
+// n^2 / 2 pair tests spread over many jobs). Each hit keeps the reference's
+// priority: the finding unit's rank, then the member's pid, which orders a
+// leaf's members as their place in the reference's pid-ordered list does.
 //
 // Distance decisions equal the reference's fp64 test
 // `p1->distance(p2, true) <= reach` (tracing/refinement.cpp:30-33,
@@ -35,10 +36,12 @@
 //
 // Hits (tracing/refinement.cpp:34-55) go to the bin of the table tile their
 // home slot key % B lies in, with their position in the reference's
-// sequential processing order: unit rank << 24 | member index. stc_table.cu
+// sequential processing order: unit rank << order_shift | pid. stc_table.cu
 // applies them; the general path here (k_hits) does so for a step whose tiles
 // are too full: a key found before the first empty slot is extended in place
 // (end = t, MBR), every other key walks on for a slot by priority.
+#include <algorithm>
+
 #include "stc_insert.cuh"
 
 namespace stc {
@@ -208,17 +211,6 @@ struct Counters {
   uint32_t tests, exact, hits, amb;  // per thread; summed into 64-bit totals per warp
 };
 
-// Lower bound of strip value v among the strip ids ((sorig >> 16) & 63,
-// ascending) of a leaf's n members in strip order.
-__device__ __forceinline__ uint32_t strip_lower_bound(const uint32_t *sorig, uint32_t n, uint32_t v) {
-  uint32_t lo = 0, hi = n;
-  while (lo < hi) {
-    const uint32_t mid = (lo + hi) >> 1;
-    if (((__ldg(&sorig[mid]) >> 16) & 63u) < v) lo = mid + 1; else hi = mid;
-  }
-  return lo;
-}
-
 // First index in [lo, hi) of a longitude-ordered strip whose offset is
 // greater than x (upper) or not below x (!upper).
 __device__ __forceinline__ uint32_t strip_x_bound(const float4 *pts, uint32_t lo, uint32_t hi, float x, bool upper) {
@@ -237,9 +229,9 @@ __device__ __forceinline__ uint32_t strip_x_bound(const float4 *pts, uint32_t lo
 struct __align__(16) Row {
   float x, y, scale;         // leaf offsets, metres per degree of longitude
   uint32_t pid;
-  float fx, fy;              // float position (fxy)
+  float fx, fy;              // float position
   uint32_t off;              // first test of the row among the job's
-  uint32_t orig;             // own: place in pid order; border: place of the unit
+  uint32_t unit;             // border: place of the unit
   uint32_t seg0, seg1, seg2; // segments: start | end (counted in the row's tests) << 16; start only in seg2
   uint32_t leaf;             // border: the leaf of the row's point, and its low x, low y, high y in float
   float ax0, ay0, ay1;
@@ -262,14 +254,15 @@ struct __align__(16) Row {
 // records' stores 2.85: bound by L2's rate of scattered 32-byte stores (39 G/s
 // measured, 35 with an atomic each). A row per lane and a shared-memory queue
 // of records before it: 3.0 ms for the tests with sequential records.
-__device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblock, uint32_t chunk, uint32_t n,
-                         uint32_t t, Counters &ct, Row *rows) {
+__device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblock, uint32_t chunk, uint32_t t,
+                         Counters &ct, Row *rows) {
   const uint32_t lane = lane_id();
-  const uint32_t base = p.grid_start[g];
-  const Node *o = &p.sd.nodes[p.sd.gid_node[g]];
+  const LeafGeo *lg = &p.lgeo[g];
+  const uint32_t base = lg->base, n = lg->n;
+  const float ext_x = lg->ext_x, ext_y = lg->ext_y;
   float x = 0.f, y = 0.f, scale = 0.f, ax0 = 0.f, ay0 = 0.f, ay1 = 0.f;
   float2 fr = make_float2(0.f, 0.f);
-  uint32_t pid = 0, orig = 0, leaf = 0;
+  uint32_t pid = 0, unit = 0, leaf = 0;
   uint32_t sa0 = 0, sa1 = 0, sa2 = 0, sl0 = 0, sl1 = 0, sl2 = 0;  // candidate segments: start, length
   if (own) {
     const uint32_t i = rowblock * 32 + lane;
@@ -280,7 +273,6 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       y = rp.y;
       scale = rp.z;
       pid = __float_as_uint(rp.w);
-      orig = __ldg(&p.sorig[base + i]) & 0xFFFFu;
       const uint2 c = __ldg(&p.scand[base + i]);
       const uint32_t e1 = c.x & 0xFFFFu, a2 = c.x >> 16;
       sa0 = i + 1;
@@ -289,17 +281,15 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       sl1 = c.y > a2 ? c.y - a2 : 0u;
     }
   } else {
-    const uint32_t ub = p.bu_start[g], ue = p.bu_start[g + 1];
-    const uint32_t u = ub + rowblock * 32 + lane;
-    if (u < ue) {
-      const uint32_t pos = p.bu_sorted_pos[u];
-      orig = pos;
-      pid = p.bu_pid[pos];
+    const uint32_t i = rowblock * 32 + lane;
+    if (i < p.bu_cnt[g]) {
+      unit = p.bu_sorted_pos[p.bu_start[g] + i];
+      pid = p.bu_pid[unit];
       const double2 qq = p.xy[pid];
-      fr = make_float2(__double2float_rn(qq.x), __double2float_rn(qq.y));
-      x = __double2float_rn(RN_SUB(qq.x, o->lo_x));
-      y = __double2float_rn(RN_SUB(qq.y, o->lo_y));
-      scale = metres_per_deg_lon_f(qq.y);
+      fr = float_pos(qq);
+      x = __double2float_rn(RN_SUB(qq.x, lg->lo_x));
+      y = __double2float_rn(RN_SUB(qq.y, lg->lo_y));
+      scale = metres_per_deg_lon_f(fr.y);
       // A pair of a border row (outside leaf g) and a member occurs twice in
       // this step iff the member also has a border unit targeting the row's
       // leaf.
@@ -310,20 +300,18 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       ay1 = __double2float_rn(ro->hi_y);
       // candidates: the members in the point's longitude window of the
       // strips beside its own (all of a strip too large to be ordered)
-      const float4 ls = __ldg(&p.lstrip[g]);
-      const int H = (int)ls.y;
-      const int c = (int)fminf(fmaxf(floorf(y * ls.x), -4.0f), (float)H + 4.0f);
-      const uint32_t *so = p.sorig + base;
+      const int H = (int)lg->strips;
+      const float wx = lg->wx;
+      const int c = (int)fminf(fmaxf(floorf(y * lg->inv), -4.0f), (float)H + 4.0f);
+      const uint16_t *ss = p.sstart + (size_t)g * STRIP_STRIDE;
       const float4 *sp = p.spts + base;
       auto window = [&](int sidx, uint32_t &a, uint32_t &len) {
         if (sidx < 0 || sidx >= H) return;
-        const uint32_t st = strip_lower_bound(so, n, (uint32_t)sidx);
-        const uint32_t en = strip_lower_bound(so, n, (uint32_t)sidx + 1);
-        if (st >= en) return;
+        const uint32_t st = ss[sidx], en = ss[sidx + 1];
         uint32_t lo = st, hi = en;
-        if (__ldg(&so[st]) & STRIP_XSORTED) {
-          lo = strip_x_bound(sp, st, en, x - ls.z, false);
-          hi = strip_x_bound(sp, lo, en, x + ls.z, true);
+        if (en - st >= 2 && en - st <= XSORT_MAX) {
+          lo = strip_x_bound(sp, st, en, x - wx, false);
+          hi = strip_x_bound(sp, lo, en, x + wx, true);
         }
         a = lo;
         len = hi - lo;
@@ -360,18 +348,18 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
   const uint32_t nz = __ballot_sync(0xffffffffu, len != 0);
   // error margin: offsets of the members are within the leaf's extent; a
   // border row's own offsets may exceed it
-  const float wxl = (float)RN_SUB(o->hi_x, o->lo_x) * 1.000001f, wyl = (float)RN_SUB(o->hi_y, o->lo_y) * 1.000001f;
+  const float wxl = ext_x * 1.000001f, wyl = ext_y * 1.000001f;
   const float mx = fmaxf(wxl, warp_max(fabsf(x))), my = fmaxf(wyl, warp_max(fabsf(y)));
   if (len) {
     float4 *d = (float4 *)&rows[__popc(nz & ((1u << lane) - 1u))];
     d[0] = make_float4(x, y, scale, __uint_as_float(pid));
-    d[1] = make_float4(fr.x, fr.y, __uint_as_float(off), __uint_as_float(orig));
+    d[1] = make_float4(fr.x, fr.y, __uint_as_float(off), __uint_as_float(unit));
     *(uint4 *)&d[2] = make_uint4(sa0 | sl0 << 16, sa1 | (sl0 + sl1) << 16, sa2, leaf);
     if (!own) d[3] = make_float4(ax0, ay0, ay1, 0.f);
   }
   __syncwarp();
   const float u = 5.9604645e-08f;
-  const float reach = (float)p.reach;
+  const float reach = p.reach_f;
   const float E = 2.1f * u * (2.0f * mx * STC_SMAX_F + 2.0f * my * STC_SLAT_F);
   const float delta = 4.0f * E + 64.0f * u * reach + 1e-6f * reach;
   const float lo = fmaxf(reach - delta, 0.0f);
@@ -393,7 +381,6 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
     const uint32_t j = base + (k < e0 ? (r2.x & 0xFFFFu) + k : k < e1 ? (r2.y & 0xFFFFu) + k - e0 : r2.z + k - e1);
     const float4 c = __ldg(&p.spts[j]);
     const float2 fc = __ldg(&p.sfxy[j]);
-    const uint32_t corig = __ldg(&p.sorig[j]) & 0xFFFFu;
     const uint32_t pid1 = __float_as_uint(rp.w), pid2 = __float_as_uint(c.w);
     const bool less = pid1 < pid2;
     // the reference measures from the unit's point: an own pair from its
@@ -418,14 +405,13 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
     h.lo_y = fminf(fa.y, fb.y);
     h.hi_x = fmaxf(fa.x, fb.x);
     h.hi_y = fmaxf(fa.y, fb.y);
-    const uint32_t orig1 = __float_as_uint(r1.w);
     if (own) {
       // the pair is found by the lower pid's own unit (rank = its pid) at
       // the higher pid's place in the pid-ordered member list
-      h.order = ((unsigned long long)h.a << STC_ORDER_SHIFT) | (less ? corig : orig1);
+      h.order = ((unsigned long long)h.a << p.order_shift) | h.b;
     } else {
       // border units follow the N own units
-      h.order = (((unsigned long long)p.N + orig1) << STC_ORDER_SHIFT) | corig;
+      h.order = (((unsigned long long)p.N + __float_as_uint(r1.w)) << p.order_shift) | pid2;
       // the member has a unit targeting the row's leaf only if it lies below
       // that leaf, or left of it and below its top (the border lookup's
       // rule); rounding to float keeps the order, so the test on floats
@@ -444,8 +430,10 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
   __syncwarp();
 }
 
-// Slice `part` of `parts` runs job chunks [C * part / parts, C * (part + 1) / parts)
-// of the C = ceil(jobs / p.job_chunk) chunks.
+// Slice `part` of `parts` runs jobs [J * part / parts, J * (part + 1) / parts),
+// up to p.job_chunk at a time; fewer when there are too few to go round: eight
+// dense jobs of one leaf in one warp were the whole kernel's tail (20k objects
+// in hotspots: 0.23 -> 0.06 ms a quarter).
 __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint32_t part, uint32_t parts) {
   __shared__ Row rows_all[REFINE_THREADS / 32][32];
   Row *rows = rows_all[threadIdx.x >> 5];
@@ -453,43 +441,18 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
   const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const unsigned long long J = p.st->jobs_total;
-  // fewer jobs at a time when there are too few to go round: eight dense jobs
-  // of one leaf in one warp were the whole kernel's tail (20k objects in
-  // hotspots: 0.23 -> 0.06 ms a part)
-  const unsigned long long each = J / parts / nwarps;
+  const unsigned long long J0 = J * part / parts, J1 = J * (part + 1) / parts;
+  const unsigned long long each = (J1 - J0) / nwarps;
   const unsigned long long jc = each >= p.job_chunk ? p.job_chunk : (each ? each : 1ull);
-  const unsigned long long nchunks = (J + jc - 1) / jc;
-  const unsigned long long c0 = nchunks * part / parts, c1 = nchunks * (part + 1) / parts;
   Counters ct = {0, 0, 0, 0};
-  for (unsigned long long chunk = c0 + warp; chunk < c1; chunk += nwarps) {
+  for (unsigned long long j0 = J0 + warp * jc; j0 < J1; j0 += nwarps * jc) {
     // one lane reads the flag so that the whole warp leaves together
     if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
-    unsigned long long j0 = chunk * jc;
-    unsigned long long j1 = j0 + jc < J ? j0 + jc : J;
-    // largest g with job_start[g] <= j0, 32 probes a round (4 rounds of loads
-    // for 10^6 grid ids instead of 20)
-    uint32_t lo = 0, hi = p.G;  // job_start[lo] <= j0 < job_start[hi] (or hi = G)
-    while (hi - lo > 1) {
-      const uint32_t w32 = (hi - lo + 31) / 32;
-      const uint32_t at = lo + (lane_id() + 1) * w32;  // ascending over the lanes
-      const uint32_t below = __popc(__ballot_sync(0xffffffffu, at < hi && p.job_start[at] <= j0));
-      const uint32_t lo2 = lo + below * w32;
-      hi = min(hi, lo2 + w32);
-      lo = lo2;
-    }
-    uint32_t g = lo;
+    const unsigned long long j1 = j0 + jc < J1 ? j0 + jc : J1;
     for (unsigned long long job = j0; job < j1; job++) {
-      while (p.job_start[g + 1] <= job) g++;
-      const uint32_t local = (uint32_t)(job - p.job_start[g]);
-      const uint32_t cnt = p.grid_count[g];
-      const uint32_t n = cnt < p.leaf_cap ? cnt : p.leaf_cap;
-      const uint32_t R = (n + 31) / 32, cc = p.cchunks[g], own_jobs = R * cc;
-      if (local < own_jobs) {
-        run_rows(p, g, true, local / cc, local % cc, n, t, ct, rows);
-      } else {
-        const uint32_t ccb = (n + p.refine_chunk - 1) / p.refine_chunk, b = local - own_jobs;
-        run_rows(p, g, false, b / ccb, b % ccb, n, t, ct, rows);
-      }
+      const uint4 w = p.jobs[job];
+      for (uint32_t c = 0; c < w.w; c++)
+        run_rows(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
     }
   }
   // reduce counters per warp (64-bit sums)
@@ -514,6 +477,9 @@ void step_pairs(PipeDev &p, cudaStream_t s) {
     STC_KL k_refine_a<<<num_sms() * p.refine_bps, REFINE_THREADS, 0, s>>>(p, part, p.slices);
 }
 
-void step_hits(PipeDev &p, cudaStream_t s) { STC_KL k_hits<<<num_sms() * p.hits_bps, 256, 0, s>>>(p); }
+void step_hits(PipeDev &p, cudaStream_t s) {
+  const unsigned most = std::max<unsigned>(p.nb, 4 * num_sms());
+  STC_KL k_hits<<<std::min<unsigned>(num_sms() * p.hits_bps, most), 256, 0, s>>>(p);
+}
 
 }  // namespace stc

@@ -17,6 +17,7 @@
 // visited, so phase 2 replays the flagged events in index order on one
 // thread, with those parents queued for re-evaluation at their own index.
 // Stack pops and pushes happen in exactly the reference's order.
+#include <algorithm>
 #include <vector>
 
 #include "stc_schema.cuh"
@@ -181,12 +182,14 @@ __global__ void k_build_write(const Node *bn, const NodeMeta *bm, uint32_t total
 }
 
 __global__ void k_build_finish(const uint32_t *sub_nodes, const uint32_t *sub_leaves, uint32_t S, uint32_t G,
-                               DevState *st) {
+                               uint32_t *high, DevState *st) {
   uint32_t nodes = sub_nodes[0], leaves = sub_leaves[0];
   // tracing/filter.cpp:82-85 asserts strict inequality
   if (nodes >= S || leaves >= G) stc_set_error(st, ERR_BUILD, nodes);
   st->schema_stack_index = nodes;
   st->grids_stack_index = leaves;
+  high[0] = min(nodes, S);
+  high[1] = min(leaves, G);
 }
 
 static inline unsigned nblk(size_t n, unsigned t = 256) { return (unsigned)((n + t - 1) / t); }
@@ -228,7 +231,8 @@ cudaError_t build_schema(const double2 *xy, uint32_t n, const double mbr[4], dou
                                                      w.bleafbase);
   }
   STC_KL k_build_write<<<nblk(total), 256, 0, s>>>(w.bnodes, w.bmeta, total, w.bpre, w.bleafbase, sd);
-  STC_KL k_build_finish<<<1, 1, 0, s>>>(w.bsub_nodes, w.bsub_leaves, sd.S, sd.G, st);
+  STC_KL k_build_finish<<<1, 1, 0, s>>>(w.bsub_nodes, w.bsub_leaves, sd.S, sd.G, sd.high, st);
+  schema_walk(sd, s);
   return cudaGetLastError();
 }
 
@@ -237,51 +241,41 @@ cudaError_t build_schema(const double2 *xy, uint32_t n, const double mbr[4], dou
 
 enum { EV_NONE = 0, EV_SPLIT = 1, EV_MERGE = 2 };
 
-__global__ void k_flags_to_bits(const uint32_t *flag, uint32_t *bits, uint32_t n) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i < n) bits[i] = flag[i] ? 1u : 0u;
-}
-
 __global__ void k_schema_phase1(SchemaDev sd, const uint32_t *grid_count, double reach, uint32_t cap, uint32_t delay,
-                                uint32_t *ev_flag, int16_t *old_under) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= sd.S) return;
-  NodeMeta m = sd.meta[i];
-  uint32_t flag = EV_NONE;
-  old_under[i] = m.underflow;
-  if (m.type == NODE_LEAF) {
-    bool cond = false;
-    if (grid_count[m.grid_id] > cap) {
-      const Node &q = sd.nodes[i];
-      double thr = RN_MUL(reach, 2.0);
-      cond = width_geo(q.lo_x, q.lo_y, q.hi_x, thr) > thr;
-    }
-    int16_t nv = cond ? (int16_t)(m.overflow + 1) : (int16_t)0;
-    if (cond && (uint32_t)nv >= delay) flag = EV_SPLIT;
-    else sd.meta[i].overflow = nv;
-  } else if (m.type == NODE_BRANCH) {
-    const Node &q = sd.nodes[i];
-    int leafchild = 0;
-    int ncounter = 0;
-    for (int k = 0; k < 4; k++) {
-      NodeMeta cm = sd.meta[q.child[k]];
-      if (cm.type == NODE_LEAF) {
-        leafchild++;
-        ncounter += (int)grid_count[cm.grid_id];
+                                uint8_t *ev_flag, int16_t *old_under) {
+  const uint32_t high = sd.high[0];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < high; i += gridDim.x * blockDim.x) {
+    NodeMeta m = sd.meta[i];
+    uint32_t flag = EV_NONE;
+    old_under[i] = m.underflow;
+    if (m.type == NODE_LEAF) {
+      bool cond = false;
+      if (grid_count[m.grid_id] > cap) {
+        const Node &q = sd.nodes[i];
+        double thr = RN_MUL(reach, 2.0);
+        cond = width_geo(q.lo_x, q.lo_y, q.hi_x, thr) > thr;
       }
+      int16_t nv = cond ? (int16_t)(m.overflow + 1) : (int16_t)0;
+      if (cond && (uint32_t)nv >= delay) flag = EV_SPLIT;
+      else sd.meta[i].overflow = nv;
+    } else if (m.type == NODE_BRANCH) {
+      const Node &q = sd.nodes[i];
+      int leafchild = 0;
+      int ncounter = 0;
+      for (int k = 0; k < 4; k++) {
+        NodeMeta cm = sd.meta[q.child[k]];
+        if (cm.type == NODE_LEAF) {
+          leafchild++;
+          ncounter += (int)grid_count[cm.grid_id];
+        }
+      }
+      bool cond = leafchild == 4 && (uint32_t)ncounter < cap;
+      int16_t nv = cond ? (int16_t)(m.underflow + 1) : (int16_t)0;
+      if (cond && (uint32_t)nv >= delay) flag = EV_MERGE;
+      else sd.meta[i].underflow = nv;
     }
-    bool cond = leafchild == 4 && (uint32_t)ncounter < cap;
-    int16_t nv = cond ? (int16_t)(m.underflow + 1) : (int16_t)0;
-    if (cond && (uint32_t)nv >= delay) flag = EV_MERGE;
-    else sd.meta[i].underflow = nv;
+    ev_flag[i] = (uint8_t)flag;
   }
-  ev_flag[i] = flag;
-}
-
-__global__ void k_schema_compact(const uint32_t *ev_flag, const uint32_t *ev_pos, uint32_t S, uint32_t *ev_list) {
-  uint32_t i = blockIdx.x * blockDim.x + threadIdx.x;
-  if (i >= S) return;
-  if (ev_flag[i]) ev_list[ev_pos[i]] = (i << 2) | ev_flag[i];
 }
 
 __device__ bool split_node(SchemaDev sd, uint32_t cur, uint32_t *grid_count, DevState *st) {
@@ -387,8 +381,7 @@ __device__ uint32_t heap_pop(uint32_t *h, uint32_t &n) {
 // takes 0.03). Node and grid bookkeeping is then written in parallel, merges
 // before splits (a node or grid id freed by a merge can only be reused by a
 // later split). The per-step grid counts are not reset: nothing reads them
-// before the next step recounts. Sets *done; k_schema_phase2 then does
-// nothing.
+// before the next step recounts.
 static constexpr uint32_t PAR_MAX_EVENTS = 4096;
 
 // Per-event scratch in global memory: split -> 4 children, 4 grid ids taken;
@@ -412,22 +405,37 @@ __device__ __forceinline__ int last_equal(const int *v, int e, int want) {
   return -1;
 }
 
-__global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const uint32_t *ev_list,
-                                                            const unsigned long long *ev_total, unsigned int *done,
-                                                            int serial_only, uint32_t *scratch, DevState *st) {
+// Block-wide exclusive scan of one value per thread of a 1024-thread block;
+// total receives the sum. warp_sum: 32 words of shared memory.
+__device__ __forceinline__ int block_scan(int v, int *warp_sum, int &total) {
+  const uint32_t lane = threadIdx.x & 31u;
+  int incl = v;
+#pragma unroll
+  for (int d = 1; d < 32; d <<= 1) {
+    const int up = __shfl_up_sync(0xffffffffu, incl, d);
+    if ((int)lane >= d) incl += up;
+  }
+  __syncthreads();  // the last use of warp_sum is over
+  if (lane == 31) warp_sum[threadIdx.x >> 5] = incl;
+  __syncthreads();
+  int before = incl - v;
+  total = 0;
+  for (uint32_t w = 0; w < 32; w++) {
+    if (w < (threadIdx.x >> 5)) before += warp_sum[w];
+    total += warp_sum[w];
+  }
+  return before;
+}
+
+// The whole block; false when the events need the one-thread replay.
+__device__ __forceinline__ bool replay_block(const SchemaDev &sd, const uint32_t *ev_list, uint32_t nev,
+                                             uint32_t *scratch, DevState *st, int *warp_sum) {
   __shared__ uint32_t sh_node[PAR_MAX_EVENTS];
   __shared__ __align__(16) int sh_lev[PAR_MAX_EVENTS];  // 4 * (level before the event) + kind
-  __shared__ int warp_sum[32];
   __shared__ int cascade, bad;
-  const uint32_t tid = threadIdx.x, lane = tid & 31u;
-  uint32_t nev = (uint32_t)*ev_total;
-  if (tid == 0) {
-    *done = 0;
-    cascade = 0;
-    bad = 0;
-    st->schema_path = 0;
-  }
-  if (nev > PAR_MAX_EVENTS || serial_only) return;
+  const uint32_t tid = threadIdx.x;
+  if (tid == 0) cascade = bad = 0;
+  if (nev > PAR_MAX_EVENTS) return false;
   ParScratch ps{scratch};
   const int ssi0 = (int)st->schema_stack_index, gsi0 = (int)st->grids_stack_index;
   __syncthreads();
@@ -451,23 +459,9 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
       ps.val[8 * e + 4] = sd.meta[node].grid_id;  // the split's own grid id goes to its first child
     }
   }
-  int incl = sum;
-#pragma unroll
-  for (int d = 1; d < 32; d <<= 1) {
-    const int up = __shfl_up_sync(0xffffffffu, incl, d);
-    if ((int)lane >= d) incl += up;
-  }
-  if (lane == 31) warp_sum[tid >> 5] = incl;
-  __syncthreads();
-  if (cascade) {
-    if (tid == 0) st->schema_path = 2;
-    return;
-  }
-  int level = incl - sum, total = 0;
-  for (uint32_t w = 0; w < 32; w++) {
-    if (w < (tid >> 5)) level += warp_sum[w];
-    total += warp_sum[w];
-  }
+  int total = 0;
+  int level = block_scan(sum, warp_sum, total);
+  if (cascade) return false;
   for (uint32_t e = e0; e < e1; e++) {
     const int kind = sh_lev[e], si = ssi0 + 4 * level, gi = gsi0 + 3 * level;
     sh_lev[e] = level * 4 + kind;
@@ -482,7 +476,7 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
   __syncthreads();
   if (bad) {
     if (tid == 0) stc_set_error(st, ERR_SCHEMA, 0u);
-    return;
+    return true;
   }
   for (uint32_t e = tid; e < nev; e += blockDim.x) {
     const int lk = sh_lev[e], k = lk >> 2;
@@ -569,18 +563,14 @@ __global__ void __launch_bounds__(1024) k_schema_phase2_par(SchemaDev sd, const 
     st->splits = (uint32_t)((int)nev + total) / 2;
     st->merges = (uint32_t)((int)nev - total) / 2;
     st->events = nev;
-    st->schema_path = 1;
-    *done = 1;
   }
+  return true;
 }
 
-__global__ void k_schema_phase2(SchemaDev sd, uint32_t *grid_count, const uint32_t *ev_list,
-                                const unsigned long long *ev_total, const int16_t *old_under, uint32_t *heap,
-                                uint8_t *queued, uint32_t cap, uint32_t delay, const unsigned int *done,
-                                DevState *st) {
-  if (threadIdx.x != 0 || blockIdx.x != 0) return;
-  if (*done) return;  // handled by k_schema_phase2_par
-  uint32_t nev = (uint32_t)*ev_total;
+// One thread, in the reference's order, with cascades.
+__device__ void replay_serial(const SchemaDev &sd, uint32_t *grid_count, const uint32_t *ev_list, uint32_t nev,
+                              const int16_t *old_under, uint32_t *heap, uint8_t *queued, uint32_t cap, uint32_t delay,
+                              DevState *st) {
   uint32_t hn = 0, ei = 0;
   uint32_t splits = 0, merges = 0;
   while (ei < nev || hn > 0) {
@@ -634,18 +624,100 @@ __global__ void k_schema_phase2(SchemaDev sd, uint32_t *grid_count, const uint32
   st->events = nev;
 }
 
+// The flagged nodes in index order, then their replay. One block: thread t
+// collects the flags of nodes [t * per, (t + 1) * per).
+__global__ void __launch_bounds__(1024) k_schema_phase2(SchemaDev sd, SchemaWork w, uint32_t *grid_count, uint32_t cap,
+                                                        uint32_t delay, int serial_only, DevState *st) {
+  __shared__ int warp_sum[32];
+  const uint32_t tid = threadIdx.x, high = sd.high[0];
+  const uint32_t per = ((high + 1023) / 1024 + 15) / 16 * 16;
+  const uint32_t n0 = min(tid * per, high), n1 = min(n0 + per, high);
+  int count = 0;
+  for (uint32_t i = n0; i < n1; i += 16) {
+    const uint4 f = *(const uint4 *)&w.ev_flag[i];  // flags past the last node are 0
+    const uint32_t v[4] = {f.x, f.y, f.z, f.w};
+    for (int k = 0; k < 4; k++) count += __popc((v[k] | v[k] >> 1) & 0x01010101u);
+  }
+  int total = 0;
+  int at = block_scan(count, warp_sum, total);
+  if (count)
+    for (uint32_t i = n0; i < n1; i++) {
+      const uint32_t f = w.ev_flag[i];
+      if (f) w.ev_list[at++] = i << 2 | f;
+    }
+  __syncthreads();
+  const uint32_t ssi0 = st->schema_stack_index, gsi0 = st->grids_stack_index;
+  __syncthreads();
+  uint32_t path = 0;
+  if (!serial_only) path = replay_block(sd, w.ev_list, (uint32_t)total, w.par_scratch, st, warp_sum) ? 1u : 2u;
+  if (tid) return;
+  if (path != 1) replay_serial(sd, grid_count, w.ev_list, (uint32_t)total, w.old_under, w.heap, w.queued, cap, delay, st);
+  st->schema_path = path;
+  // ids ever handed out: a split takes at most 4 node and 3 more grid ids
+  sd.high[0] = min(max(high, ssi0 + 4 * st->splits), sd.S);
+  sd.high[1] = min(max(sd.high[1], gsi0 + 3 * st->splits), sd.G);
+}
+
+__global__ void __launch_bounds__(256) k_schema_walk(SchemaDev sd) {
+  const uint32_t high = sd.high[0];
+  for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < high; i += gridDim.x * blockDim.x) {
+    const NodeMeta m = sd.meta[i];
+    if (i == 0) sd.start[sd.start_edge * sd.start_edge] = m.type == NODE_LEAF ? (m.grid_id | WALK_LEAF) : 0u;
+    if (m.type != NODE_BRANCH) continue;
+    const Node *n = &sd.nodes[i];
+    const uint4 c = *(const uint4 *)n->child;
+    uint32_t ch[4] = {c.x, c.y, c.z, c.w};
+#pragma unroll
+    for (int k = 0; k < 4; k++) {
+      const NodeMeta cm = sd.meta[ch[k]];
+      // (an invalid child stands for no node: the descent reports it)
+      if (cm.type == NODE_LEAF) ch[k] = cm.grid_id | WALK_LEAF;
+      else if (cm.type != NODE_BRANCH) ch[k] = STC_NONE;
+    }
+    Walk w;
+    w.mid_x = order_key(__double_as_longlong(n->mid_x));
+    w.mid_y = order_key(__double_as_longlong(n->mid_y));
+    for (int k = 0; k < 4; k++) w.child[k] = ch[k];
+    sd.walk[i] = w;
+    const float4 b = sd.fbox[i];
+    sd.wbox[i] = WalkBox{b.x, b.y, b.z, b.w, __double2float_rn(RN_SUB(n->mid_x, sd.ox)),
+                         __double2float_rn(RN_SUB(n->mid_y, sd.oy)), {0.f, 0.f}};
+  }
+}
+
+// A cell's corners, widened by 2e-3 of it and dozens of the coordinates' last
+// places (several times the rounding of a point's float cell number, at most
+// 1024 cells times a few 2^-24), walk down together while they take the same
+// child: the descent compares each coordinate with the split points alone, so
+// every point between them takes it too.
+__global__ void __launch_bounds__(256) k_schema_start(SchemaDev sd) {
+  const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, E = sd.start_edge;
+  if (i >= E * E) return;
+  const double cx = 1.0 / (double)sd.start_sx, cy = 1.0 / (double)sd.start_sy;
+  const double ix = (double)(i % E), iy = (double)(i / E);
+  const double wx = 2e-3 * cx + 1e-14 * (fabs(sd.ox) + E * cx), wy = 2e-3 * cy + 1e-14 * (fabs(sd.oy) + E * cy);
+  const double x0 = sd.ox + ix * cx - wx, x1 = sd.ox + (ix + 1.0) * cx + wx;
+  const double y0 = sd.oy + iy * cy - wy, y1 = sd.oy + (iy + 1.0) * cy + wy;
+  uint32_t cur = sd.start[E * E];
+  for (int d = 0; !(cur & WALK_LEAF) && d < STC_MAX_DEPTH; d++) {
+    const double mx = sd.nodes[cur].mid_x, my = sd.nodes[cur].mid_y;
+    if ((x0 > mx) != (x1 > mx) || (y0 > my) != (y1 > my)) break;
+    cur = sd.walk[cur].child[(y0 > my) * 2 + (x0 > mx)];
+  }
+  sd.start[i] = cur;
+}
+
+void schema_walk(SchemaDev sd, cudaStream_t s) {
+  STC_KL k_schema_walk<<<std::min<unsigned>(nblk(sd.S), num_sms() * 4), 256, 0, s>>>(sd);
+  STC_KL k_schema_start<<<nblk((size_t)sd.start_edge * sd.start_edge), 256, 0, s>>>(sd);
+}
+
 void update_schema(SchemaDev sd, SchemaWork w, uint32_t *grid_count, double reach, uint32_t grid_capacity,
                    uint32_t delay, int serial_only, DevState *st, cudaStream_t s) {
-  STC_KL k_schema_phase1<<<nblk(sd.S), 256, 0, s>>>(sd, grid_count, reach, grid_capacity, delay, w.ev_flag, w.old_under);
-  // ordered compaction of the flagged node indices: ev_pos = exclusive scan of (flag != 0)
-  STC_KL k_flags_to_bits<<<nblk(sd.S), 256, 0, s>>>(w.ev_flag, w.ev_pos, sd.S);
-  exclusive_scan_u32(w.ev_pos, w.ev_pos, sd.S, w.ev_total, w.scan_tmp, s);
-  STC_KL k_schema_compact<<<nblk(sd.S), 256, 0, s>>>(w.ev_flag, w.ev_pos, sd.S, w.ev_list);
-  unsigned int *done = (unsigned int *)(w.ev_total + 1);
-  STC_KL k_schema_phase2_par<<<1, 1024, 0, s>>>(sd, w.ev_list, w.ev_total, done, serial_only, w.par_scratch,
-                                                      st);
-  STC_KL k_schema_phase2<<<1, 32, 0, s>>>(sd, grid_count, w.ev_list, w.ev_total, w.old_under, w.heap, w.queued,
-                                   grid_capacity, delay, done, st);
+  STC_KL k_schema_phase1<<<std::min<unsigned>(nblk(sd.S), num_sms() * 4), 256, 0, s>>>(
+      sd, grid_count, reach, grid_capacity, delay, w.ev_flag, w.old_under);
+  STC_KL k_schema_phase2<<<1, 1024, 0, s>>>(sd, w, grid_count, grid_capacity, delay, serial_only, st);
+  schema_walk(sd, s);
 }
 
 }  // namespace stc

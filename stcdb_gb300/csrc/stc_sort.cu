@@ -127,6 +127,10 @@ void exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, unsigned lo
   STC_KL k_scan_down<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, tmp);
 }
 
+void scan_sums_u32(uint32_t *sums, size_t nb, unsigned long long *total, cudaStream_t s) {
+  STC_KL k_scan_sums<<<1, 1024, 0, s>>>(sums, nb, total);
+}
+
 // ---------------------------------------------------------------------------
 // Radix sort: 8-bit digits, tiles of 256 threads x 16 items.
 
