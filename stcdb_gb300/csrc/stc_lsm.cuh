@@ -90,6 +90,7 @@ struct CtbBlock {
   uint32_t *cbase = nullptr;       // [F + 1] first dense cell id of each CTF
   uint4 *ixg = nullptr;            // [F] (g, levels, 0, 0) of each CTF's index
   double2 *ixs = nullptr;          // [F] level-0 cells per degree in x and y (g / CTF box side)
+  double2 *ixq = nullptr;          // [F] widening of box queries in x and y (index_slack)
   float4 *ixf = nullptr;           // [2F] float filing of keys: per axis (cells per low unit, cells per
                                    // edge unit, error margin, 1 if usable)
   uint16_t *pend = nullptr;       // [keys] end offset of the key at each perm position, saturated at
@@ -110,6 +111,7 @@ struct QBlock {
   const uint32_t *cbase;
   const uint4 *ixg;
   const double2 *ixs;
+  const double2 *ixq;
   const uint16_t *pend;
   unsigned long long n_over;
   uint32_t F, index, o_end_time_min, edge;  // edge: of the map bitmap
@@ -120,6 +122,21 @@ struct QueryRec {
   stc_contact c;
   uint32_t q, pad;
 };
+
+// A (query, block, CTF) pair of a box query as its rows see it (k_box_plan).
+struct __align__(16) BoxPlan {
+  uint32_t q, block, ctf, rows;    // rows of all index levels and the wide list; of an oversize buffer: chunks
+  int16_t i0, i1, j0, j1;          // query window in level-0 cells
+  int16_t ii0, ii1, jj0, jj1;      // interior level-0 cells
+  uint32_t ts, flags;              // end offsets above ts pass; PLAN_*
+  uint16_t g, levels;              // the CTF's index
+  float d;                         // band of the float box test
+  float f[4];                      // query edges from the CTF's low corner, degrees
+  float ax, ay, ae, pad;           // degrees per unit of the low x, low y and edge fields
+};
+
+// Counters of a batch: matches, box plans, work items, pieces.
+constexpr size_t QUERY_COUNTERS = 4;
 
 // The device and pinned buffers and the stream of one query batch in
 // flight. A context keeps QUERY_LANES of them, so that that many batches
@@ -134,13 +151,14 @@ struct QueryLane {
   size_t q_cap = 0;
   QueryRec *d_out = nullptr;
   size_t out_cap = 0;
-  unsigned long long *d_count = nullptr;
+  unsigned long long *d_count = nullptr;    // [QUERY_COUNTERS]
   unsigned long long *d_qcounts = nullptr;  // per-query match counts
   size_t qc_cap = 0;
-  uint32_t *d_items = nullptr;     // box-query plan: work items per (query, block, CTF), then their scan
+  BoxPlan *d_plans = nullptr;      // box queries: (query, block, CTF) pairs with keys to look at
+  size_t plans_cap = 0;
+  uint2 *d_items = nullptr;        // their work items: (plan, first row)
+  uint4 *d_pieces = nullptr;       // ranges of keys left by crowded items
   size_t items_cap = 0;
-  uint32_t *d_iscan = nullptr;     // scan scratch
-  size_t iscan_cap = 0;
   // Mapped pinned host buffers of a batch's inputs and results. Kernels on
   // the lane's stream read and write them over the host link directly, so a
   // batch never queues on a copy engine behind a step's position copy (tens
@@ -148,7 +166,7 @@ struct QueryLane {
   QBlock *h_qb = nullptr, *m_qb = nullptr;                // [retain]
   stc_query *h_q = nullptr, *m_q = nullptr;
   size_t hq_cap = 0;
-  unsigned long long *h_counts = nullptr, *m_counts = nullptr;  // [hq_cap + 1]: per-query counts, then the total
+  unsigned long long *h_counts = nullptr, *m_counts = nullptr;  // [hq_cap + QUERY_COUNTERS]: per-query counts, then the counters
   QueryRec *h_recs = nullptr, *m_recs = nullptr;
   size_t hrecs_cap = 0;
 };

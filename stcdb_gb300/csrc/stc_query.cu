@@ -5,7 +5,7 @@
 // oversize buffer or a CTF, one thread runs the reference's binary search for
 // the first key of the pid and the CTA scans on while the pid matches. Box
 // queries are planned per (query, block, CTF) and run as rows of the blocks'
-// cell indexes, one warp per row (k_box_plan, k_box_rows). Matches are
+// cell indexes, up to 32 rows a warp (k_box_plan, k_box_rows). Matches are
 // appended to one device buffer tagged with their query; the host groups
 // them by query.
 #include <algorithm>
@@ -80,46 +80,6 @@ __device__ __forceinline__ unsigned long long key_fields(unsigned __int128 k, co
   k >>= c.duration_bit;
   o.target = (uint32_t)(k & mask64(c.id_bit));
   return vm;
-}
-
-// Screening of the box test without decode_key's four correctly rounded
-// divisions: the decoded corners computed with reciprocals differ from the
-// exact ones by a few ulp of coordinates below 2^8 degrees (< 1e-12), so a
-// key whose approximate box clears every query edge by BOX_EPS is decided;
-// box_screen returns 1 (meets the query), 0 (misses it) or -1 (decode it).
-constexpr double BOX_EPS = 1e-10;
-struct BoxRecip {
-  double m0, m1, wx, wy, le, rx, ry, re;
-};
-
-__device__ __forceinline__ BoxRecip box_recip(const stc_ctf &c) {
-  BoxRecip r;
-  const float wx = __fsub_rn(c.mbr[2], c.mbr[0]), wy = __fsub_rn(c.mbr[3], c.mbr[1]);
-  r.m0 = c.mbr[0];
-  r.m1 = c.mbr[1];
-  r.wx = wx;
-  r.wy = wy;
-  r.le = (double)fmaxf(wx, wy);
-  r.rx = 1.0 / (double)mask64(c.low_x_bit);
-  r.ry = 1.0 / (double)mask64(c.low_y_bit);
-  r.re = 1.0 / (double)mask64(c.edge_bit);
-  return r;
-}
-
-__device__ __forceinline__ int box_screen(unsigned long long vm, const stc_ctf &c, const BoxRecip &r, const double *q) {
-  const unsigned long long y = vm & mask64(c.edge_bit);
-  vm >>= c.edge_bit;
-  const unsigned long long x = vm & mask64(c.edge_bit);
-  vm >>= c.edge_bit;
-  const unsigned long long low1 = vm & mask64(c.low_y_bit);
-  vm >>= c.low_y_bit;
-  const unsigned long long low0 = vm & mask64(c.low_x_bit);
-  const double b0 = r.m0 + (double)low0 * r.rx * r.wx, b1 = r.m1 + (double)low1 * r.ry * r.wy;
-  const double b2 = b0 + (double)x * r.re * r.le, b3 = b1 + (double)y * r.re * r.le;
-  // box::intersect (geometry/geometry.h:128-133) on closed intervals
-  if (b0 > q[2] + BOX_EPS || b2 < q[0] - BOX_EPS || b1 > q[3] + BOX_EPS || b3 < q[1] - BOX_EPS) return 0;
-  if (b0 < q[2] - BOX_EPS && b2 > q[0] + BOX_EPS && b1 < q[3] - BOX_EPS && b3 > q[1] + BOX_EPS) return 1;
-  return -1;
 }
 
 __device__ void decode_key(unsigned __int128 k, const stc_ctf &c, Key &o) {
@@ -471,14 +431,19 @@ __global__ void k_set_one(unsigned long long *p, unsigned long long v) { *p = v;
 
 // ---- box queries: plan, then rows --------------------------------------------
 //
-// A batch's box queries run in three launches. k_box_plan gives every
-// (query, block, CTF or oversize buffer) pair one thread: it prunes by the CTF
-// box and bitmap (widened so that no key whose decoded box meets the query is
-// lost), counts whole CTFs a counting query holds, and writes how many work
-// items the pair needs: one per row of every index level plus the wide list
-// (CTFs), or one per OV_CHUNK oversize keys. An exclusive scan turns the
-// counts into the items' first numbers, and k_box_rows gives each work item
-// one warp, so that big and small queries alike spread over the whole GPU.
+// A batch's box queries run in three launches. k_box_plan gives every (query,
+// block, CTF or oversize buffer) pair one thread: it prunes by the CTF box and
+// bitmap (widened so that no key whose decoded box meets the query is lost),
+// counts whole CTFs a counting query holds, and leaves a plan of every other
+// pair -- all that its rows need, so that they do no double arithmetic -- and
+// work items: `rpi` of its rows each, which are those of every index level and
+// the wide list (CTFs), or OV_CHUNK keys (oversize buffers). k_box_rows gives each item one
+// warp: a lane a row looks up its cells' key ranges, then the keys to decode
+// of all rows are numbered through and dealt to the lanes; the ranges of an item
+// over a crowd go to k_box_pieces, a warp a piece. (A warp a row, each
+// finding its pair by binary search and computing the pair's ranges in double,
+// took 2.35 ms for 2048 queries, 0.8k of them boxes, over four blocks of 0.6M
+// keys; now plan 59 us, rows 153, pieces 66.)
 
 constexpr uint32_t OV_CHUNK = 2048;       // oversize keys per work item
 constexpr uint32_t SEQ_BITMAP_CELLS = 1024;  // larger windows skip the per-thread bitmap test
@@ -490,18 +455,21 @@ __device__ bool any_bit_seq(const uint32_t *bm, int i0, int i1, int j0, int j1, 
   long long ni = (long long)i1 - i0 + 1, nj = (long long)j1 - j0 + 1;
   if (ni <= 0 || nj <= 0) return false;
   if (ni * nj > SEQ_BITMAP_CELLS) return true;
-  for (long long j = j0; j <= j1; j++)
-    for (long long i = i0; i <= i1; i++) {
-      long long bit = i + j * (long long)xg;
-      if (bit >= 0 && bit < nbits && ((__ldg(&bm[bit >> 5]) >> (bit & 31)) & 1u)) return true;
+  for (long long j = j0; j <= j1; j++) {  // a row's bits lie side by side
+    const long long lo = max(i0 + j * (long long)xg, 0ll), hi = min(i1 + j * (long long)xg, nbits - 1);
+    for (long long w = lo >> 5; w <= hi >> 5 && lo <= hi; w++) {
+      uint32_t m = 0xffffffffu;
+      if (w == lo >> 5) m &= 0xffffffffu << (lo & 31);
+      if (w == hi >> 5) m &= 0xffffffffu >> (31 - (hi & 31));
+      if (__ldg(&bm[w]) & m) return true;
     }
+  }
   return false;
 }
 
 // What a box query needs to know about one CTF.
 struct BoxCtx {
   double wide[4];
-  double qx, qy;
   bool all_starts, all_ends;
   uint32_t ts;                 // end offsets above ts pass t_start < end
   uint32_t g, levels;          // the CTF's index
@@ -509,21 +477,15 @@ struct BoxCtx {
   int ii0, ii1, jj0, jj1;      // interior level-0 cells (counting queries), empty if ii0 > ii1
 };
 
-// Fills x for CTF t and query q; false when the CTF box misses the widened query.
-__device__ bool box_ctx(const stc_ctf &t, const uint4 &ix, const double2 &sc, const stc_query &q, BoxCtx &x) {
-  // A decoded box differs from the key's exact box (which set the CTF box
-  // and the bitmap) by less than one corner quantum plus one edge quantum on
-  // either side (float conversions truncate, and may round up first): widen
-  // the query by that much for the box and bitmap tests.
+// Fills x for CTF t and query q; false when the CTF box misses the widened
+// query. slack: the CTF's widening in x and y (index_slack).
+__device__ bool box_ctx(const stc_ctf &t, const uint4 &ix, const double2 &sc, const double2 &slack, const stc_query &q,
+                        BoxCtx &x) {
   const double *qbox = q.box;
-  const float fwx = __fsub_rn(t.mbr[2], t.mbr[0]), fwy = __fsub_rn(t.mbr[3], t.mbr[1]);
-  const double le = (double)fmaxf(fwx, fwy), me = (double)mask64(t.edge_bit);
-  x.qx = (double)fwx / (double)mask64(t.low_x_bit) + le / me + 1e-9;
-  x.qy = (double)fwy / (double)mask64(t.low_y_bit) + le / me + 1e-9;
-  x.wide[0] = qbox[0] - x.qx;
-  x.wide[1] = qbox[1] - x.qy;
-  x.wide[2] = qbox[2] + x.qx;
-  x.wide[3] = qbox[3] + x.qy;
+  x.wide[0] = qbox[0] - slack.x;
+  x.wide[1] = qbox[1] - slack.y;
+  x.wide[2] = qbox[2] + slack.x;
+  x.wide[3] = qbox[3] + slack.y;
   const double ctfb[4] = {t.mbr[0], t.mbr[1], t.mbr[2], t.mbr[3]};
   if (!box_hits(ctfb, x.wide)) return false;
   // Time conditions that hold for every key of the CTF: no time field can
@@ -562,171 +524,322 @@ __device__ bool box_ctx(const stc_ctf &t, const uint4 &ix, const double2 &sc, co
   return true;
 }
 
-// Rows of level lv in the window: a key filed at level lv under cell
-// (cx, cy) whose box meets the widened query has cy in
+// Rows of level lv in the window [j0, j1] of level-0 cells: a key filed at
+// level lv under cell (cx, cy) whose box meets the widened query has cy in
 // [(j0 >> lv) - 1, j1 >> lv] (its box ends at most one cell above cy), and
 // likewise cx.
-__device__ __forceinline__ int level_rows(const BoxCtx &x, uint32_t lv, int &cj0) {
-  const int side = (int)index_level_side(x.g, lv);
-  cj0 = max((x.j0 >> lv) - 1, 0);
-  return max(min(x.j1 >> lv, side - 1) - cj0 + 1, 0);
+__device__ __forceinline__ int level_rows(int j0, int j1, uint32_t g, uint32_t lv, int &cj0) {
+  const int side = (int)index_level_side(g, lv);
+  cj0 = max((j0 >> lv) - 1, 0);
+  return max(min(j1 >> lv, side - 1) - cj0 + 1, 0);
 }
 
-__global__ void k_box_plan(const QBlock *qb, uint32_t nb, const stc_query *qs, uint32_t nq, uint32_t F1,
-                           double m0x, double m0y, double m1x, double m1y, uint32_t *items,
-                           unsigned long long *qcounts) {
+// Most keys to decode, and most end offsets to compare, that one item keeps
+// (up to 32 rows of fewer than 32 or 256 each come on top), and the pieces that
+// the ranges of a fuller one are cut into.
+constexpr uint32_t ITEM_KEYS = 1024, PIECE_KEYS = 512, ITEM_ENDS = 8192, PIECE_ENDS = 4096;
+constexpr size_t PIECE_CAP = 1 << 18;
+constexpr uint32_t PLAN_COUNT_ONLY = 1u, PLAN_ALL_ENDS = 2u;
+
+__global__ void __launch_bounds__(256) k_box_plan(const QBlock *qb, uint32_t nb, const stc_query *qs, uint32_t nq,
+                                                  uint32_t F1, double m0x, double m0y, double m1x, double m1y,
+                                                  uint32_t rpi, BoxPlan *plans, uint32_t plan_cap, uint2 *items,
+                                                  uint32_t item_cap, unsigned long long *counts,
+                                                  unsigned long long *qcounts) {
   const uint32_t P = nq * nb * F1;
   for (uint32_t p = blockIdx.x * blockDim.x + threadIdx.x; p < P; p += gridDim.x * blockDim.x) {
     const uint32_t c = p % F1, bi = (p / F1) % nb, qi = p / F1 / nb;
     const stc_query &q = qs[qi];
     const QBlock &b = qb[bi];
-    uint32_t n = 0;
-    if ((q.kind & 0xFFu) == STC_QUERY_BOX && c <= b.F) {
-      if (c == b.F) {  // oversize buffer: the map bitmap prunes
-        if (b.n_over) {
-          int i0, i1, j0, j1;
-          cell_range(q.box[0], q.box[2], m0x, m1x, b.edge, i0, i1);
-          cell_range(q.box[1], q.box[3], m0y, m1y, b.edge, j0, j1);
-          if (any_bit_seq(b.obitmap, i0, i1, j0, j1, b.edge, (long long)b.edge * b.edge))
-            n = (uint32_t)((b.n_over + OV_CHUNK - 1) / OV_CHUNK);
-        }
-      } else {
-        const stc_ctf &t = b.ctfs[c];
-        BoxCtx x;
-        if (t.kv_count && box_ctx(t, b.ixg[c], b.ixs[c], q, x)) {
-          const double *qbox = q.box;
-          const bool count_only = (q.kind & STC_QUERY_COUNT_ONLY) != 0;
-          if (count_only && x.all_starts && x.all_ends && qbox[0] <= t.mbr[0] - x.qx && qbox[1] <= t.mbr[1] - x.qy &&
-              qbox[2] >= t.mbr[2] + x.qx && qbox[3] >= t.mbr[3] + x.qy) {
-            // Every key matches -- count the CTF without decoding it, as the
-            // reference's box search does (workbench.cpp:525-528).
-            atomicAdd(&qcounts[qi], (unsigned long long)t.kv_count);
-          } else {
-            int bi0, bi1, bj0, bj1;  // the bitmap's cells
-            cell_range(x.wide[0], x.wide[2], t.mbr[0], t.mbr[2], t.x_grid, bi0, bi1);
-            cell_range(x.wide[1], x.wide[3], t.mbr[1], t.mbr[3], t.y_grid, bj0, bj1);
-            if (any_bit_seq(b.bitmaps + (size_t)c * (STC_BITMAP_BYTES / 4), bi0, bi1, bj0, bj1, t.x_grid,
-                            8ll * STC_BITMAP_BYTES)) {
-              n = 1;  // the wide list
-              for (uint32_t lv = 0; lv < x.levels; lv++) {
-                int cj0;
-                n += (uint32_t)level_rows(x, lv, cj0);
-              }
-            }
-          }
-        }
-      }
-    }
-    items[p] = n;
-  }
-}
-
-// One warp per work item; item numbers come from the exclusive scan of the
-// plan's counts (items[P] = all items).
-__global__ void __launch_bounds__(QBOX_THREADS) k_box_rows(const QBlock *qb, uint32_t nb, const stc_query *qs,
-                                                          uint32_t nq, uint32_t F1, const uint32_t *first,
-                                                          QueryRec *out, unsigned long long cap,
-                                                          unsigned long long *count, unsigned long long *qcounts) {
-  const uint32_t P = nq * nb * F1;
-  const uint32_t total = first[P];
-  const uint32_t lane = threadIdx.x & 31u;
-  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
-  for (uint32_t item = gw; item < total; item += nw) {
-    uint32_t lo = 0, hi = P - 1;  // the pair: largest p with first[p] <= item
-    while (lo < hi) {
-      uint32_t mid = (lo + hi + 1) >> 1;
-      if (__ldg(&first[mid]) <= item) lo = mid;
-      else hi = mid - 1;
-    }
-    const uint32_t p = lo, r = item - first[p];
-    const uint32_t c = p % F1, bi = (p / F1) % nb, qi = p / F1 / nb;
-    const stc_query q = qs[qi];
-    const QBlock &b = qb[bi];
+    if ((q.kind & 0xFFu) != STC_QUERY_BOX || c > b.F) continue;
     const bool count_only = (q.kind & STC_QUERY_COUNT_ONLY) != 0;
-    const double *qbox = q.box;
-    uint32_t mine = 0;
-    if (c == b.F) {  // oversize keys [r * OV_CHUNK, ...): float boxes decide
-      const unsigned long long k1 = min((unsigned long long)(r + 1) * OV_CHUNK, b.n_over);
-      for (unsigned long long i = (unsigned long long)r * OV_CHUNK + lane; i < k1; i += 32) {
-        float4 fb = b.obox[i];
-        double box[4] = {fb.x, fb.y, fb.z, fb.w};
-        uint32_t pid, target, start, end;
-        oversize_key(b, i, pid, target, start, end);
-        if (time_ok(start, end, q.t_start, q.t_end) && box_hits(box, qbox)) {
-          mine++;
-          if (!count_only) emit(out, cap, count, qi, pid, target, start, end, box, b.index, c);
-        }
+    BoxPlan w;
+    w.rows = 0;
+    w.flags = count_only ? PLAN_COUNT_ONLY : 0u;
+    if (c == b.F) {  // oversize buffer: the map bitmap prunes
+      if (b.n_over) {
+        int i0, i1, j0, j1;
+        cell_range(q.box[0], q.box[2], m0x, m1x, b.edge, i0, i1);
+        cell_range(q.box[1], q.box[3], m0y, m1y, b.edge, j0, j1);
+        if (any_bit_seq(b.obitmap, i0, i1, j0, j1, b.edge, (long long)b.edge * b.edge))
+          w.rows = (uint32_t)((b.n_over + OV_CHUNK - 1) / OV_CHUNK);
       }
     } else {
       const stc_ctf &t = b.ctfs[c];
       BoxCtx x;
-      box_ctx(t, b.ixg[c], b.ixs[c], q, x);  // the plan saw it pass
-      const uint32_t cb = b.cbase[c], wide_slot = b.cbase[c + 1] - 1u;
-      uint32_t a, e, ma, me2;  // scan [a, ma) and [me2, e); [ma, me2) is counted
-      int clo = 1, chi = 0;    // counted cells of this row
-      uint32_t row_base = 0;
-      uint32_t rr = r, lv = 0, off = 0;
-      int cj0 = 0, n = 0;
-      for (; lv < x.levels; lv++) {
-        n = level_rows(x, lv, cj0);
-        if (rr < (uint32_t)n) break;
-        rr -= (uint32_t)n;
-        const uint32_t side = index_level_side(x.g, lv);
-        off += side * side;
-      }
-      if (lv < x.levels) {  // row cj0 + rr of level lv
-        const int side = (int)index_level_side(x.g, lv);
-        const int jr = cj0 + (int)rr;
-        const int ci0 = max((x.i0 >> lv) - 1, 0), ci1 = min(x.i1 >> lv, side - 1);
-        row_base = cb + off + (uint32_t)(jr * side);
-        a = b.cstart[row_base + (uint32_t)ci0];
-        e = ci1 >= ci0 ? b.cstart[row_base + (uint32_t)ci1 + 1] : a;
-        ma = me2 = a;
-        // interior at this level: cell C covers level-0 cells [C 2^lv, (C + 1) 2^lv - 1]
-        const int s2 = 1 << lv;
-        const bool row_in = x.ii0 <= x.ii1 && x.jj0 <= x.jj1 && jr * s2 >= x.jj0 && (jr + 1) * s2 - 1 <= x.jj1;
-        if (row_in) {
-          clo = max((x.ii0 + s2 - 1) >> lv, ci0);
-          chi = min(((x.ii1 + 1) >> lv) - 1, ci1);
-        }
-        if (clo <= chi) {
-          ma = b.cstart[row_base + (uint32_t)clo];
-          me2 = b.cstart[row_base + (uint32_t)chi + 1];
-          if (x.all_ends) {
-            if (lane == 0) mine += me2 - ma;
-          } else {
-            // the counted cells' end offsets lie side by side: one coalesced pass
-            for (uint32_t pp = ma + lane; pp < me2; pp += 32) mine += __ldg(&b.pend[pp]) > x.ts;
-          }
-        }
-      } else {  // the wide list
-        a = b.cstart[wide_slot];
-        e = b.cstart[wide_slot + 1];
-        ma = me2 = a;
-      }
-      const uint32_t kb = t.key_bit / 8u;
-      const uint8_t *base = b.keys + t.key_offset;
-      const BoxRecip rc = box_recip(t);
-      for (int seg = 0; seg < 2; seg++) {
-        for (uint32_t pp = (seg ? me2 : a) + lane, pe = seg ? e : ma; pp < pe; pp += 32) {
-          const unsigned long long local = (unsigned long long)b.perm[pp] - t.first_key;
-          Key k;
-          const unsigned long long vm = key_fields(load_key(base + local * kb, kb), t, k);
-          uint32_t end = k.end + t.end_time_min, start = end - k.duration;
-          if (!time_ok(start, end, q.t_start, q.t_end)) continue;
-          const int sc = box_screen(vm, t, rc, qbox);
-          if (sc == 0) continue;
-          if (sc < 0 || !count_only) exact_box(vm, t, k.box);
-          if (sc > 0 || box_hits(k.box, qbox)) {
-            mine++;
-            if (!count_only) emit(out, cap, count, qi, k.oid, k.target, start, end, k.box, b.index, c);
+      const double2 slack = b.ixq[c];
+      if (t.kv_count && box_ctx(t, b.ixg[c], b.ixs[c], slack, q, x)) {
+        const double *qbox = q.box;
+        if (count_only && x.all_starts && x.all_ends && qbox[0] <= t.mbr[0] - slack.x &&
+            qbox[1] <= t.mbr[1] - slack.y && qbox[2] >= t.mbr[2] + slack.x && qbox[3] >= t.mbr[3] + slack.y) {
+          // Every key matches -- count the CTF without decoding it, as the
+          // reference's box search does (workbench.cpp:525-528).
+          atomicAdd(&qcounts[qi], (unsigned long long)t.kv_count);
+        } else {
+          int bi0, bi1, bj0, bj1;  // the bitmap's cells
+          cell_range(x.wide[0], x.wide[2], t.mbr[0], t.mbr[2], t.x_grid, bi0, bi1);
+          cell_range(x.wide[1], x.wide[3], t.mbr[1], t.mbr[3], t.y_grid, bj0, bj1);
+          if (any_bit_seq(b.bitmaps + (size_t)c * (STC_BITMAP_BYTES / 4), bi0, bi1, bj0, bj1, t.x_grid,
+                          8ll * STC_BITMAP_BYTES)) {
+            w.rows = 1;  // the wide list
+            for (uint32_t lv = 0; lv < x.levels; lv++) {
+              int cj0;
+              w.rows += (uint32_t)level_rows(x.j0, x.j1, x.g, lv, cj0);
+            }
+            w.i0 = (int16_t)x.i0; w.i1 = (int16_t)x.i1; w.j0 = (int16_t)x.j0; w.j1 = (int16_t)x.j1;
+            w.ii0 = (int16_t)x.ii0; w.ii1 = (int16_t)x.ii1; w.jj0 = (int16_t)x.jj0; w.jj1 = (int16_t)x.jj1;
+            w.g = (uint16_t)x.g;
+            w.levels = (uint16_t)x.levels;
+            w.ts = x.ts;
+            if (x.all_ends) w.flags |= PLAN_ALL_ENDS;
+            // The box test on floats: the query's edges from the CTF's low
+            // corner against low and low + edge fields in degrees, decided
+            // when clear of the band d. The float corners are off by at most
+            // 4 * 2^-24 of the CTF box and its longer side, the edges by 2^-24
+            // of themselves, the double sums of the exact test by 2^-53 of the
+            // coordinates; d is some eight times that. (Edges beyond four boxes are pulled in; with NaN
+            // every key takes the exact test.)
+            const float wx = __fsub_rn(t.mbr[2], t.mbr[0]), wy = __fsub_rn(t.mbr[3], t.mbr[1]), le = fmaxf(wx, wy);
+            const float L = 4.0f * (wx + wy + le) + 1.0f;
+            float big = 0.0f, far = 0.0f;
+            bool nan = false;
+#pragma unroll
+            for (int k = 0; k < 4; k++) {
+              const double f = qbox[k] - (double)t.mbr[k & 1];
+              nan |= f != f;
+              w.f[k] = fminf(fmaxf(__double2float_rn(f), -L), L);
+              big = fmaxf(big, fabsf(w.f[k]));
+              far = fmaxf(far, fabsf(t.mbr[k]));
+            }
+            w.ax = wx / __ull2float_rn(mask64(t.low_x_bit));
+            w.ay = wy / __ull2float_rn(mask64(t.low_y_bit));
+            w.ae = le / __ull2float_rn(mask64(t.edge_bit));
+            w.d = nan ? INFINITY : 2e-6f * (wx + wy + le) + 5e-7f * big + 1e-15f * far + 1e-9f;
           }
         }
       }
     }
+    if (!w.rows) continue;
+    w.q = qi;
+    w.block = bi;
+    w.ctf = c;
+    const uint32_t step = c == b.F ? 1u : rpi, n = (w.rows + step - 1) / step;
+    const unsigned long long at = agg_inc(&counts[1]), first = atomicAdd(&counts[2], (unsigned long long)n);
+    if (at < plan_cap) plans[at] = w;
+    for (uint32_t k = 0; k < n && first + k < item_cap && at < plan_cap; k++)
+      items[first + k] = make_uint2((uint32_t)at, k * step);
+  }
+}
+
+// The keys one lane's row asks for: positions [a, a + la) and [b, ...) of
+// perm, numbered from off on among the item's.
+struct __align__(16) RowKeys {
+  uint32_t off, a, la, b;
+};
+
+// Deals the lanes' len items to the warp one by one: do_item(slot, k) for item
+// k of the lane whose RowKeys was put at slot (the lanes with len > 0 in
+// order). Called by the whole warp.
+template <typename Put, typename Do>
+__device__ __forceinline__ void deal(uint32_t len, Put put, Do do_item) {
+  const uint32_t lane = lane_id();
+  uint32_t incl = len;
 #pragma unroll
-    for (int o = 16; o > 0; o >>= 1) mine += __shfl_xor_sync(0xffffffffu, mine, o);
+  for (int d = 1; d < 32; d <<= 1) {
+    const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
+    if ((int)lane >= d) incl += up;
+  }
+  const uint32_t off = incl - len, total = __shfl_sync(0xffffffffu, incl, 31);
+  if (!total) return;
+  const uint32_t nz = __ballot_sync(0xffffffffu, len != 0);
+  if (len) put(__popc(nz & ((1u << lane) - 1u)), off);
+  __syncwarp();
+  uint32_t before = 0;
+  for (uint32_t f0 = 0; f0 < total; f0 += 32) {
+    const uint32_t starts = __reduce_or_sync(0xffffffffu, len != 0 && off - f0 < 32u ? 1u << (off - f0) : 0u);
+    const uint32_t slot = before + __popc(starts & (0xffffffffu >> (31u - lane))) - 1u;
+    before += __popc(starts);
+    if (f0 + lane < total) do_item(slot, f0 + lane);
+  }
+  __syncwarp();
+}
+
+// Tests the key at position pp of a planned CTF; 1 when it matches (then
+// emitted, unless the query counts).
+__device__ __forceinline__ uint32_t box_key(const QBlock &b, const stc_ctf &t, const BoxPlan &w, const stc_query &q,
+                                            uint32_t pp, QueryRec *out, unsigned long long cap,
+                                            unsigned long long *counts) {
+  const uint32_t kb = t.key_bit / 8u;
+  const unsigned long long local = (unsigned long long)b.perm[pp] - t.first_key;
+  Key o;
+  const unsigned long long vm = key_fields(load_key(b.keys + t.key_offset + local * kb, kb), t, o);
+  const uint32_t end = o.end + t.end_time_min, start = end - o.duration;
+  if (!time_ok(start, end, q.t_start, q.t_end)) return 0;
+  unsigned long long m = vm;
+  const float ey = __ull2float_rn(m & mask64(t.edge_bit)) * w.ae;
+  m >>= t.edge_bit;
+  const float ex = __ull2float_rn(m & mask64(t.edge_bit)) * w.ae;
+  m >>= t.edge_bit;
+  const float y0 = __ull2float_rn(m & mask64(t.low_y_bit)) * w.ay;
+  m >>= t.low_y_bit;
+  const float x0 = __ull2float_rn(m & mask64(t.low_x_bit)) * w.ax;
+  const float x1 = x0 + ex, y1 = y0 + ey, d = w.d;
+  // box::intersect (geometry/geometry.h:128-133) on closed intervals
+  if (x0 > w.f[2] + d || x1 < w.f[0] - d || y0 > w.f[3] + d || y1 < w.f[1] - d) return 0;
+  const bool sure = x0 < w.f[2] - d && x1 > w.f[0] + d && y0 < w.f[3] - d && y1 > w.f[1] + d;
+  const bool count_only = (w.flags & PLAN_COUNT_ONLY) != 0;
+  if (!sure || !count_only) {
+    exact_box(vm, t, o.box);
+    if (!box_hits(o.box, q.box)) return 0;
+  }
+  if (!count_only) emit(out, cap, &counts[0], w.q, o.oid, o.target, start, end, o.box, b.index, w.ctf);
+  return 1;
+}
+
+// Leaves positions [first, first + n) of a plan's keys to k_box_pieces, cut
+// into pieces of `size`; false when the list has no room for them.
+__device__ __forceinline__ bool leave_pieces(uint4 *pieces, uint32_t piece_cap, unsigned long long *counts,
+                                             uint32_t plan, uint32_t first, uint32_t n, uint32_t size,
+                                             uint32_t kind) {
+  const uint32_t k = (n + size - 1) / size;
+  const unsigned long long at = atomicAdd(&counts[3], (unsigned long long)k);
+  const bool room = at + k <= piece_cap;
+  for (uint32_t i = 0; i < k && at + i < piece_cap; i++)
+    pieces[at + i] = make_uint4(plan, first + i * size, room ? min(size, n - i * size) : 0u, kind);
+  return room;
+}
+
+__global__ void __launch_bounds__(QBOX_THREADS) k_box_rows(const QBlock *qb, const stc_query *qs, uint32_t rpi,
+                                                          const BoxPlan *plans, uint32_t plan_cap,
+                                                          const uint2 *items, uint32_t item_cap, uint4 *pieces,
+                                                          uint32_t piece_cap,
+                                                          QueryRec *out, unsigned long long cap,
+                                                          unsigned long long *counts, unsigned long long *qcounts) {
+  __shared__ RowKeys keys_all[QBOX_THREADS / 32][32];
+  RowKeys *keys = keys_all[threadIdx.x >> 5];
+  // a plan without room for all is run again by the host; its items are not all written
+  const uint32_t total = counts[1] <= plan_cap && counts[2] <= item_cap ? (uint32_t)counts[2] : 0u;
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t item = gw; item < total; item += nw) {
+    const uint2 it = items[item];
+    const BoxPlan &w = plans[it.x];
+    const uint32_t c = w.ctf, qi = w.q;
+    const stc_query &q = qs[qi];
+    const QBlock &b = qb[w.block];
+    const uint32_t t_start = q.t_start, t_end = q.t_end;
+    const bool count_only = (w.flags & PLAN_COUNT_ONLY) != 0;
+    uint32_t mine = 0;
+    if (c == b.F) {  // a chunk of oversize keys: float boxes decide
+      const unsigned long long k0 = (unsigned long long)it.y * OV_CHUNK;
+      const unsigned long long k1 = min(k0 + OV_CHUNK, b.n_over);
+      for (unsigned long long i = k0 + lane; i < k1; i += 32) {
+        float4 fb = b.obox[i];
+        double box[4] = {fb.x, fb.y, fb.z, fb.w};
+        uint32_t pid, target, start, end;
+        oversize_key(b, i, pid, target, start, end);
+        if (time_ok(start, end, t_start, t_end) && box_hits(box, q.box)) {
+          mine++;
+          if (!count_only) emit(out, cap, &counts[0], qi, pid, target, start, end, box, b.index, c);
+        }
+      }
+    } else {
+      const stc_ctf &t = b.ctfs[c];
+      const uint32_t g = w.g, levels = w.levels, ts = w.ts;
+      const bool all_ends = (w.flags & PLAN_ALL_ENDS) != 0;
+      // this lane's row: scan [a, ma) and [me2, e); [ma, me2) is counted
+      uint32_t a = 0, e = 0, ma = 0, me2 = 0;
+      if (lane < rpi && it.y + lane < w.rows) {
+        uint32_t rr = it.y + lane, lv = 0, off = 0;
+        int cj0 = 0;
+        for (; lv < levels; lv++) {
+          const uint32_t n = (uint32_t)level_rows(w.j0, w.j1, g, lv, cj0);
+          if (rr < n) break;
+          rr -= n;
+          const uint32_t side = index_level_side(g, lv);
+          off += side * side;
+        }
+        const uint32_t cb = b.cbase[c];
+        if (lv < levels) {  // row cj0 + rr of level lv
+          const int side = (int)index_level_side(g, lv);
+          const int jr = cj0 + (int)rr;
+          const int ci0 = max((w.i0 >> lv) - 1, 0), ci1 = min(w.i1 >> lv, side - 1);
+          const uint32_t row_base = cb + off + (uint32_t)(jr * side);
+          a = b.cstart[row_base + (uint32_t)ci0];
+          e = ci1 >= ci0 ? b.cstart[row_base + (uint32_t)ci1 + 1] : a;
+          ma = me2 = a;
+          // interior at this level: cell C covers level-0 cells [C 2^lv, (C + 1) 2^lv - 1]
+          const int s2 = 1 << lv;
+          if (w.ii0 <= w.ii1 && w.jj0 <= w.jj1 && jr * s2 >= w.jj0 && (jr + 1) * s2 - 1 <= w.jj1) {
+            const int clo = max((w.ii0 + s2 - 1) >> lv, ci0), chi = min(((w.ii1 + 1) >> lv) - 1, ci1);
+            if (clo <= chi) {
+              ma = b.cstart[row_base + (uint32_t)clo];
+              me2 = b.cstart[row_base + (uint32_t)chi + 1];
+            }
+          }
+        } else {  // the wide list
+          const uint32_t wide_slot = b.cbase[c + 1] - 1u;
+          a = b.cstart[wide_slot];
+          e = b.cstart[wide_slot + 1];
+          ma = me2 = a;
+        }
+      }
+      if (all_ends) mine += me2 - ma;
+      // An item over a crowd goes to other warps: a few such held k_box_rows
+      // for 1.78 ms with the SMs 28% active (2048 queries over four blocks of
+      // 0.6M keys).
+      const uint32_t scan = __reduce_add_sync(0xffffffffu, (ma - a) + (e - me2));
+      const uint32_t ends = __reduce_add_sync(0xffffffffu, all_ends ? 0u : me2 - ma);
+      if (scan > ITEM_KEYS) {
+        if (ma - a >= 32u && leave_pieces(pieces, piece_cap, counts, it.x, a, ma - a, PIECE_KEYS, 0u)) a = ma;
+        if (e - me2 >= 32u && leave_pieces(pieces, piece_cap, counts, it.x, me2, e - me2, PIECE_KEYS, 0u)) e = me2;
+      }
+      uint32_t cnt = all_ends ? 0u : me2 - ma;
+      if (ends > ITEM_ENDS && cnt >= 256u && leave_pieces(pieces, piece_cap, counts, it.x, ma, cnt, PIECE_ENDS, 1u))
+        cnt = 0;
+      if (!all_ends) {
+        // the counted cells' end offsets lie side by side
+        deal(cnt, [&](uint32_t slot, uint32_t off) { keys[slot] = RowKeys{off, ma, 0u, 0u}; },
+             [&](uint32_t slot, uint32_t k) { mine += __ldg(&b.pend[keys[slot].a + (k - keys[slot].off)]) > ts; });
+      }
+      deal((ma - a) + (e - me2), [&](uint32_t slot, uint32_t off) { keys[slot] = RowKeys{off, a, ma - a, me2}; },
+           [&](uint32_t slot, uint32_t at) {
+             const RowKeys r = keys[slot];
+             const uint32_t k = at - r.off;
+             mine += box_key(b, t, w, q, k < r.la ? r.a + k : r.b + (k - r.la), out, cap, counts);
+           });
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
     if (lane == 0 && mine) atomicAdd(&qcounts[qi], (unsigned long long)mine);
+  }
+}
+
+// The ranges that crowded items left (leave_pieces), one warp each.
+__global__ void __launch_bounds__(QBOX_THREADS) k_box_pieces(const QBlock *qb, const stc_query *qs,
+                                                            const BoxPlan *plans, const uint4 *pieces,
+                                                            uint32_t piece_cap, QueryRec *out, unsigned long long cap,
+                                                            unsigned long long *counts,
+                                                            unsigned long long *qcounts) {
+  const uint32_t total = (uint32_t)min(counts[3], (unsigned long long)piece_cap);
+  const uint32_t lane = threadIdx.x & 31u;
+  const uint32_t gw = (blockIdx.x * blockDim.x + threadIdx.x) >> 5, nw = (gridDim.x * blockDim.x) >> 5;
+  for (uint32_t k = gw; k < total; k += nw) {
+    const uint4 it = pieces[k];
+    const BoxPlan &w = plans[it.x];
+    const QBlock &b = qb[w.block];
+    const uint32_t end = it.y + it.z;
+    uint32_t mine = 0;
+    if (it.w) {
+      const uint32_t ts = w.ts;
+#pragma unroll 4
+      for (uint32_t pp = it.y + lane; pp < end; pp += 32) mine += __ldg(&b.pend[pp]) > ts;
+    } else {
+      const stc_ctf &t = b.ctfs[w.ctf];
+      const stc_query &q = qs[w.q];
+      for (uint32_t pp = it.y + lane; pp < end; pp += 32) mine += box_key(b, t, w, q, pp, out, cap, counts);
+    }
+    mine = __reduce_add_sync(0xffffffffu, mine);
+    if (lane == 0 && mine) atomicAdd(&qcounts[w.q], (unsigned long long)mine);
   }
 }
 
@@ -757,11 +870,13 @@ __global__ void k_link_copy(unsigned long long *__restrict__ dst, const unsigned
     dst[i] = src[i];
 }
 
-// A batch's per-query match counts, then its total, into mapped host memory.
+// A batch's per-query match counts, then its counters (matches, box plans,
+// work items), into mapped host memory.
 __global__ void k_counts_out(unsigned long long *__restrict__ dst, const unsigned long long *__restrict__ qcounts,
-                             size_t nq, const unsigned long long *__restrict__ total) {
-  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i <= nq; i += (size_t)gridDim.x * blockDim.x)
-    dst[i] = i < nq ? qcounts[i] : *total;
+                             size_t nq, const unsigned long long *__restrict__ counts) {
+  for (size_t i = blockIdx.x * (size_t)blockDim.x + threadIdx.x; i < nq + QUERY_COUNTERS;
+       i += (size_t)gridDim.x * blockDim.x)
+    dst[i] = i < nq ? qcounts[i] : counts[i - nq];
 }
 
 constexpr unsigned LINK_THREADS = 256;
@@ -799,11 +914,12 @@ cudaError_t grow(T **p, size_t *cap, size_t need) {
 void free_block(CtbBlock &B) {
   for (void *v : {(void *)B.keys, (void *)B.d_ctfs, (void *)B.bitmaps, (void *)B.sids, (void *)B.orec,
                   (void *)B.obox, (void *)B.obitmap, (void *)B.perm, (void *)B.cstart, (void *)B.cbase,
-                  (void *)B.ixg, (void *)B.ixs, (void *)B.ixf, (void *)B.pend})
+                  (void *)B.ixg, (void *)B.ixs, (void *)B.ixq, (void *)B.ixf, (void *)B.pend})
     if (v) cudaFree(v);
   B.ixf = nullptr;
   B.ixg = nullptr;
   B.ixs = nullptr;
+  B.ixq = nullptr;
   B.pend = nullptr;
   B.keys = nullptr;
   B.d_ctfs = nullptr;
@@ -838,11 +954,22 @@ static float4 index_file_coeffs(const stc_ctf &t, double scale, bool x_axis) {
   return ok ? make_float4((float)a, (float)b, (float)d + 1e-9f, 1.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
 }
 
+// How far a box query is widened for the CTF box, bitmap and index tests. A
+// decoded box differs from the key's exact box (which set the CTF box and the
+// bitmap) by less than one corner quantum plus one edge quantum on either
+// side (float conversions truncate, and may round up first).
+static double2 index_slack(const stc_ctf &t) {
+  const float fwx = t.mbr[2] - t.mbr[0], fwy = t.mbr[3] - t.mbr[1];
+  const double le = (double)std::max(fwx, fwy), me = (double)mask64(t.edge_bit);
+  return make_double2((double)fwx / (double)mask64(t.low_x_bit) + le / me + 1e-9,
+                      (double)fwy / (double)mask64(t.low_y_bit) + le / me + 1e-9);
+}
+
 cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
   const uint32_t F = (uint32_t)B.ctfs.size();
   std::vector<uint32_t> cbase(F + 1, 0);
   std::vector<uint4> ixg(F);
-  std::vector<double2> ixs(F);
+  std::vector<double2> ixs(F), ixq(F);
   std::vector<float4> ixf(2 * (size_t)F);
   unsigned long long total = 0;
   for (uint32_t c = 0; c < F; c++) {
@@ -856,6 +983,7 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
     const double wx = (double)t.mbr[2] - (double)t.mbr[0], wy = (double)t.mbr[3] - (double)t.mbr[1];
     ixs[c] = make_double2(t.mbr[2] > t.mbr[0] && t.mbr[3] > t.mbr[1] ? (double)g / wx : 0.0,
                           t.mbr[2] > t.mbr[0] && t.mbr[3] > t.mbr[1] ? (double)g / wy : 0.0);
+    ixq[c] = index_slack(t);
     ixf[2 * c] = index_file_coeffs(t, ixs[c].x, true);
     ixf[2 * c + 1] = index_file_coeffs(t, ixs[c].y, false);
     cbase[c + 1] = cbase[c] + cells;
@@ -868,8 +996,10 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
   if (e == cudaSuccess) e = cudaMalloc(&B.cbase, (F + 1) * sizeof(uint32_t));
   if (e == cudaSuccess) e = cudaMalloc(&B.ixg, std::max<size_t>(F, 1) * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&B.ixs, std::max<size_t>(F, 1) * sizeof(double2));
+  if (e == cudaSuccess) e = cudaMalloc(&B.ixq, std::max<size_t>(F, 1) * sizeof(double2));
   if (e == cudaSuccess) e = cudaMalloc(&B.ixf, std::max<size_t>(2 * (size_t)F, 1) * sizeof(float4));
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixs, ixs.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixq, ixq.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixf, ixf.data(), 2 * (size_t)F * sizeof(float4), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.cbase, cbase.data(), (F + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixg, ixg.data(), F * sizeof(uint4), cudaMemcpyHostToDevice, s);
@@ -910,7 +1040,7 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
     }
   }
   STC_KL k_cell_starts<<<num_sms() * 8, 256, 0, s>>>(sk[2], shift, total, ncells, B.cstart);
-  e = cudaStreamSynchronize(s);  // the copies of cbase, ixg and ixs read this stack frame
+  e = cudaStreamSynchronize(s);  // the copies of cbase, ixg, ixs and ixq read this stack frame
   return e == cudaSuccess ? cudaGetLastError() : e;
 }
 
@@ -966,7 +1096,7 @@ void lsm_release(LsmHost &H) {
     std::lock_guard<std::mutex> ql(Q.mu);
     if (Q.stream) cudaStreamSynchronize(Q.stream);
     for (void *v : {(void *)Q.d_qb, (void *)Q.d_q, (void *)Q.d_out, (void *)Q.d_count, (void *)Q.d_qcounts,
-                    (void *)Q.d_items, (void *)Q.d_iscan})
+                    (void *)Q.d_items, (void *)Q.d_plans, (void *)Q.d_pieces})
       if (v) cudaFree(v);
     for (void *v : {(void *)Q.h_qb, (void *)Q.h_q, (void *)Q.h_counts, (void *)Q.h_recs})
       if (v) cudaFreeHost(v);
@@ -978,13 +1108,15 @@ void lsm_release(LsmHost &H) {
     Q.d_q = nullptr;
     Q.d_out = nullptr;
     Q.d_count = Q.d_qcounts = nullptr;
-    Q.d_items = Q.d_iscan = nullptr;
+    Q.d_items = nullptr;
+    Q.d_plans = nullptr;
+    Q.d_pieces = nullptr;
     Q.h_qb = Q.m_qb = nullptr;
     Q.h_q = Q.m_q = nullptr;
     Q.h_counts = Q.m_counts = nullptr;
     Q.h_recs = Q.m_recs = nullptr;
     Q.stream = nullptr;
-    Q.q_cap = Q.out_cap = Q.qc_cap = Q.items_cap = Q.iscan_cap = Q.hq_cap = Q.hrecs_cap = 0;
+    Q.q_cap = Q.out_cap = Q.qc_cap = Q.items_cap = Q.plans_cap = Q.hq_cap = Q.hrecs_cap = 0;
   }
 }
 
@@ -998,19 +1130,21 @@ static cudaError_t query_buffers(const LsmHost &H, QueryLane &Q, size_t nq, uint
   if (!Q.d_qb) e = cudaMalloc(&Q.d_qb, nb * sizeof(QBlock));
   size_t cap_qb = Q.h_qb ? nb : 0;
   if (e == cudaSuccess) e = grow_mapped(&Q.h_qb, &Q.m_qb, &cap_qb, nb);
-  if (e == cudaSuccess && !Q.d_count) e = cudaMalloc(&Q.d_count, sizeof(unsigned long long));
+  if (e == cudaSuccess && !Q.d_count) e = cudaMalloc(&Q.d_count, QUERY_COUNTERS * sizeof(unsigned long long));
   if (e == cudaSuccess && Q.hq_cap < nq) {
     size_t cap_q = Q.hq_cap;
     e = grow_mapped(&Q.h_q, &Q.m_q, &Q.hq_cap, nq);
-    if (e == cudaSuccess) e = grow_mapped(&Q.h_counts, &Q.m_counts, &cap_q, Q.hq_cap + 1);
+    if (e == cudaSuccess) e = grow_mapped(&Q.h_counts, &Q.m_counts, &cap_q, Q.hq_cap + QUERY_COUNTERS);
   }
   if (e == cudaSuccess) e = grow(&Q.d_q, &Q.q_cap, nq);
   if (e == cudaSuccess) e = grow(&Q.d_qcounts, &Q.qc_cap, nq);
   if (e == cudaSuccess) e = grow(&Q.d_out, &Q.out_cap, std::max<size_t>(1 << 16, Q.out_cap));
-  // size the plan for the retained-block limit, not today's count
-  const size_t npairs = nq * nb * ((size_t)F + 1) + 1;
-  if (e == cudaSuccess) e = grow(&Q.d_items, &Q.items_cap, npairs);
-  if (e == cudaSuccess) e = grow(&Q.d_iscan, &Q.iscan_cap, scan_tmp_words(npairs));
+  // box plans and work items: room for the batches that are served in
+  // earnest; one that needs more grows them and runs again
+  const size_t npairs = nq * nb * ((size_t)F + 1);
+  if (e == cudaSuccess) e = grow(&Q.d_plans, &Q.plans_cap, std::min<size_t>(npairs, 1 << 19));
+  if (e == cudaSuccess && !Q.d_pieces) e = cudaMalloc(&Q.d_pieces, PIECE_CAP * sizeof(uint4));
+  if (e == cudaSuccess) e = grow(&Q.d_items, &Q.items_cap, std::min<size_t>(8 * npairs, 1 << 21));
   if (e == cudaSuccess) e = grow_mapped(&Q.h_recs, &Q.m_recs, &Q.hrecs_cap, 1 << 16);
   return e;
 }
@@ -1028,7 +1162,7 @@ stc_status lsm_query_reserve(LsmHost &H, size_t nq, uint32_t F, int priority, st
   // would load them then, which waits for a step in flight
   cudaFuncAttributes fa;
   for (const void *k : {(const void *)k_query_object, (const void *)k_box_plan, (const void *)k_box_rows,
-                        (const void *)k_link_copy, (const void *)k_counts_out})
+                        (const void *)k_box_pieces, (const void *)k_link_copy, (const void *)k_counts_out})
     if (e == cudaSuccess) e = cudaFuncGetAttributes(&fa, k);
   if (e != cudaSuccess) {
     err = std::string("query buffers: ") + cudaGetErrorString(e);
@@ -1075,7 +1209,7 @@ stc_status lsm_query(LsmHost &H, int lane, const stc_query *qs, size_t nq, stc_c
   cudaStream_t s = Q.stream;
   uint32_t maxF = 0;
   for (uint32_t i = 0; i < nb; i++) maxF = std::max(maxF, H.blocks[i].info.ctf_count);
-  // box-query plan: one count per (query, block, CTF or oversize buffer), then their exclusive scan
+  // the box plan's threads: one per (query, block, CTF or oversize buffer)
   if (nq * nb * ((size_t)maxF + 1) + 1 > 0xFFFFFFFFull) {
     err = "query batch too large for the box-query plan";
     return STC_ERR_INVALID_ARG;
@@ -1089,7 +1223,7 @@ stc_status lsm_query(LsmHost &H, int lane, const stc_query *qs, size_t nq, stc_c
   for (uint32_t i = 0; i < nb; i++) {
     const CtbBlock &B = H.blocks[i];
     qb[i] = QBlock{B.keys, B.d_ctfs, B.sids, B.orec, B.obox, B.bitmaps, B.obitmap, B.perm, B.cstart, B.cbase, B.ixg,
-                   B.ixs, B.pend,
+                   B.ixs, B.ixq, B.pend,
                    (unsigned long long)B.info.oversize_kv_count, B.info.ctf_count, B.info.index,
                    B.info.o_end_time_min, B.info.bitmap_edge ? B.info.bitmap_edge : 256u};
   }
@@ -1101,8 +1235,8 @@ stc_status lsm_query(LsmHost &H, int lane, const stc_query *qs, size_t nq, stc_c
   if (e == cudaSuccess) e = link_copy(Q.d_q, Q.m_q, nq * sizeof(stc_query), s);
   unsigned long long total = 0;
   bool over = false;  // more matches than device_limit: counted only
-  for (int attempt = 0; attempt < 2 && e == cudaSuccess; attempt++) {
-    e = cudaMemsetAsync(Q.d_count, 0, sizeof(unsigned long long), s);
+  for (int attempt = 0; attempt < 4 && e == cudaSuccess; attempt++) {
+    e = cudaMemsetAsync(Q.d_count, 0, QUERY_COUNTERS * sizeof(unsigned long long), s);
     if (e == cudaSuccess) e = cudaMemsetAsync(Q.d_qcounts, 0, nq * sizeof(unsigned long long), s);
     if (e != cudaSuccess) break;
     if (has_obj)
@@ -1110,21 +1244,36 @@ stc_status lsm_query(LsmHost &H, int lane, const stc_query *qs, size_t nq, stc_c
                                                                            Q.d_count, Q.d_qcounts);
     if (has_box) {
       const uint32_t F1 = maxF + 1, P = (uint32_t)nq * nb * F1;
+      // fewer rows an item for a few queries, so that they spread over more warps
+      const uint32_t rpi = nq >= 64 ? 32u : 8u;
+      const uint32_t pc = (uint32_t)std::min<size_t>(Q.plans_cap, 0xFFFFFFFFu);
+      const uint32_t ic = (uint32_t)std::min<size_t>(Q.items_cap, 0xFFFFFFFFu);
       STC_KL k_box_plan<<<(P + 255) / 256, 256, 0, s>>>(Q.d_qb, nb, Q.d_q, (uint32_t)nq, F1, H.map[0], H.map[1],
-                                                        H.map[2], H.map[3], Q.d_items, Q.d_qcounts);
-      exclusive_scan_u32(Q.d_items, Q.d_items, (size_t)P + 1, nullptr, Q.d_iscan, s);
-      STC_KL k_box_rows<<<num_sms() * 16, QBOX_THREADS, 0, s>>>(Q.d_qb, nb, Q.d_q, (uint32_t)nq, F1, Q.d_items,
-                                                                Q.d_out, Q.out_cap, Q.d_count, Q.d_qcounts);
+                                                        H.map[2], H.map[3], rpi, Q.d_plans, pc, Q.d_items, ic,
+                                                        Q.d_count, Q.d_qcounts);
+      STC_KL k_box_rows<<<num_sms() * 16, QBOX_THREADS, 0, s>>>(Q.d_qb, Q.d_q, rpi, Q.d_plans, pc, Q.d_items, ic,
+                                                                Q.d_pieces, (uint32_t)PIECE_CAP, Q.d_out, Q.out_cap,
+                                                                Q.d_count, Q.d_qcounts);
+      STC_KL k_box_pieces<<<num_sms() * 8, QBOX_THREADS, 0, s>>>(Q.d_qb, Q.d_q, Q.d_plans, Q.d_pieces,
+                                                                 (uint32_t)PIECE_CAP, Q.d_out, Q.out_cap, Q.d_count,
+                                                                 Q.d_qcounts);
     }
     e = cudaGetLastError();
     if (e == cudaSuccess) {
-      k_counts_out<<<link_blocks(nq + 1), LINK_THREADS, 0, s>>>(Q.m_counts, Q.d_qcounts, nq, Q.d_count);
+      k_counts_out<<<link_blocks(nq + QUERY_COUNTERS), LINK_THREADS, 0, s>>>(Q.m_counts, Q.d_qcounts, nq, Q.d_count);
       e = cudaGetLastError();
     }
     if (e == cudaSuccess) e = cudaStreamSynchronize(s);
     total = Q.h_counts[nq];
     if (e == cudaSuccess && counts) memcpy(counts, Q.h_counts, nq * sizeof(unsigned long long));
-    if (e != cudaSuccess || total <= Q.out_cap) break;
+    if (e != cudaSuccess) break;
+    const size_t np = (size_t)Q.h_counts[nq + 1], ni = (size_t)Q.h_counts[nq + 2];
+    if (np > Q.plans_cap || ni > Q.items_cap) {  // once more with room for the plan
+      e = grow(&Q.d_plans, &Q.plans_cap, np);
+      if (e == cudaSuccess) e = grow(&Q.d_items, &Q.items_cap, ni);
+      continue;
+    }
+    if (total <= Q.out_cap) break;
     if (device_limit && total > device_limit) {
       over = true;
       break;

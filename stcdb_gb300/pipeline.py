@@ -503,7 +503,13 @@ class Pipeline:
         """Match counts only (STC_QUERY_COUNT_ONLY on every query)."""
         q = np.array(queries, dtype=QUERY_DTYPE, copy=True)
         q["kind"] |= QUERY_COUNT_ONLY
-        return self.query_batch(q, with_counts=True)[1]
+        q = np.ascontiguousarray(q)
+        offs = np.zeros(len(q) + 1, np.uint64)
+        counts = np.zeros(max(len(q), 1), np.uint64)
+        st = self._lib.stc_query_batch(self._h, q.ctypes.data, len(q), None, 0, offs.ctypes.data, counts.ctypes.data)
+        if st != 0:
+            raise StcError(st, self._lib.stc_last_error(None).decode())
+        return counts[:len(q)]
 
     def server(self, max_batch: int = 0, result_cap: int = 0, hbm_budget: int = 0) -> "Server":
         """A request loop answering queries by continuous batching (stc_server_start)."""
