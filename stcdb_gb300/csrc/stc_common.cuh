@@ -78,6 +78,11 @@ struct __align__(16) U128 {
   unsigned long long lo, hi;
 };
 
+// Where a tile of the meeting table keeps its meetings: each in its slot, or
+// packed in slot order at the front or the back of the tile, the slots being
+// the marks of PipeDev::occ (stc_table.cu).
+enum TableLayout : uint32_t { TABLE_SLOTS = 0, TABLE_FRONT = 1, TABLE_BACK = 2 };
+
 // Small device-resident control block.
 struct DevState {
   uint32_t schema_stack_index, grids_stack_index;
@@ -95,12 +100,13 @@ struct DevState {
   uint32_t build_nodes, build_leaves, build_active, build_level;
   uint32_t work_next;                 // generic persistent-kernel work counter
   uint32_t step_t;                    // time of the step in flight (set at its start)
-  uint32_t pad[2];
+  uint32_t packed;                    // layout of the meeting table's tiles (TableLayout)
+  uint32_t redo;                      // a bin overflowed while the tiles were packed (stc_refine.cu, bin_hit)
   unsigned long long border_points;   // points whose lookup starts above their leaf
   unsigned long long fast_claims;     // new meetings started this step (claims finalised by the sweep)
   unsigned long long hit_max;         // most hits of a table tile this step
   uint32_t schema_path;               // 1 parallel replay, 2 serial (cascade), 0 serial (other)
-  uint32_t pad2;
+  uint32_t same_t;                    // the step's time is the last step's
   // memtable (stc_lsm.cu)
   unsigned long long kv_count;        // directed keys in the memtable
   unsigned long long lsm_over_keys;   // keys partitioned to the oversize buffer (flush)

@@ -450,7 +450,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
             dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, p.G) && dalloc(c, &p.bu_start, p.G) &&
             dalloc(c, &p.slots, p.B) &&
             dalloc(c, &p.hits, (size_t)p.nb * p.bin_cap) && dalloc(c, &p.bin_cnt, p.nb) &&
-            dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
+            dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.occ, (size_t)p.nb * OCC_WORDS) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
             dalloc(c, &p.carry_cnt, p.runs) && dalloc(c, &p.cset, p.C) &&
             dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E);
   if (ok && k.kv_restriction) {
@@ -524,6 +524,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   cudaMemsetAsync(p.grid_count, 0, (size_t)p.G * sizeof(uint32_t), s);
   cudaMemsetAsync(p.bu_cnt, 0, (size_t)p.G * sizeof(uint32_t), s);
   cudaMemsetAsync(p.tile_live, 0, (size_t)p.nb * sizeof(uint32_t), s);
+  cudaMemsetAsync(p.occ, 0, (size_t)p.nb * OCC_WORDS * sizeof(uint32_t), s);
   init_tables(p, s);
   if (c->lsm_on) lsm_init(c->lsm, s);
   e = cudaSuccess;
@@ -1532,6 +1533,11 @@ extern "C" stc_status stc_checkpoint(stc_ctx *c, const char *path) {
   cudaSetDevice(c->device);
   stc_status rs = read_state(c, "stc_checkpoint");
   if (rs != STC_OK) return rs;
+  if (c->st_host->packed != TABLE_SLOTS) {  // the file holds the meetings in their slots
+    unpack_tiles(c->p, c->st_host->packed, c->stream);
+    rs = read_state(c, "stc_checkpoint");
+    if (rs != STC_OK) return rs;
+  }
   CkptHeader h;
   memset(&h, 0, sizeof(h));
   memcpy(h.magic, CKPT_MAGIC, 8);

@@ -40,6 +40,14 @@ __device__ __forceinline__ uint32_t tile_of(const PipeDev &p, unsigned long long
   return (uint32_t)q;
 }
 
+// First slot of tile j.
+__device__ __forceinline__ unsigned long long tile_start(const PipeDev &p, uint32_t j) {
+  const unsigned long long x = (unsigned long long)j * p.B;
+  unsigned long long q = __umul64hi(x, p.nb_magic);  // x / nb: exact or one too large
+  if (q * p.nb > x) q--;
+  return q;
+}
+
 // Halo tiles the tiled table update (stc_table.cu) needs this step, or 0:
 // the step takes the general path (k_hits, k_insert_ordered, k_sweep).
 constexpr uint32_t MAX_HALO = 7;

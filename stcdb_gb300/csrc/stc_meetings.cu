@@ -46,7 +46,10 @@ __global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t
   if (first < CTR_COUNT) p.ctr[first] = 0;
   if (first) return;
   DevState *st = p.st;
-  st->step_t = *(const volatile uint32_t *)t_pinned;
+  const uint32_t t = *(const volatile uint32_t *)t_pinned;
+  st->same_t = t == st->step_t;
+  st->step_t = t;
+  st->redo = 0;
   st->error = 0;
   st->error_info = 0;
   st->border_units = 0;
@@ -99,10 +102,16 @@ void init_tables(PipeDev &p, cudaStream_t s) {
 // Candidates that may occur twice in a step: walk with their minimum
 // priority once all instances are merged.
 __global__ void k_insert_ordered(PipeDev p) {
-  if (fuse_halo(p)) return;
+  const bool fused = fuse_halo(p) != 0;
+  if (blockIdx.x == 0 && threadIdx.x == 0)  // what the tiled update, or the general path, leaves
+    p.st->packed = !fused ? TABLE_SLOTS : p.st->packed == TABLE_FRONT ? TABLE_BACK : TABLE_FRONT;
+  if (fused) return;
   const uint32_t t = p.st->step_t;
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb; j += gridDim.x * blockDim.x)
-    p.tile_live[j] = 0;  // counted again by the sweep
+  // counted and marked again by the sweep
+  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb * OCC_WORDS; j += gridDim.x * blockDim.x) {
+    p.occ[j] = 0;
+    if (j < p.nb) p.tile_live[j] = 0;
+  }
   const unsigned long long nc = p.st->cand_count < p.cand_cap ? p.st->cand_count : p.cand_cap;
   for (unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; c < nc;
        c += (unsigned long long)gridDim.x * blockDim.x) {
@@ -195,7 +204,8 @@ __device__ __forceinline__ bool sweep_slot(const PipeDev &p, uint32_t t, unsigne
   return emit;
 }
 
-// Adds the warp's live slots (consecutive, one per lane) to their tiles' counts.
+// Adds the warp's live slots (consecutive, one per lane) to their tiles'
+// counts and marks.
 __device__ __forceinline__ void count_live(const PipeDev &p, unsigned long long slot, bool live) {
   const uint32_t ball = __ballot_sync(0xffffffffu, live);
   if (!ball) return;
@@ -204,6 +214,14 @@ __device__ __forceinline__ void count_live(const PipeDev &p, unsigned long long 
   const uint32_t same = __ballot_sync(0xffffffffu, tile == first);
   if ((int)lane_id() == __ffs(ball) - 1) atomicAdd(&p.tile_live[first], (uint32_t)__popc(same));
   if (live && tile != first) atomicAdd(&p.tile_live[tile], 1u);
+  const uint32_t at = live ? (uint32_t)(slot - tile_start(p, tile)) : 0u;
+  const uint32_t word = live ? tile * OCC_WORDS + (at >> 5) : STC_NONE;
+  for (uint32_t todo = ball; todo;) {  // two or three words
+    const uint32_t w = __shfl_sync(0xffffffffu, word, __ffs(todo) - 1);
+    const uint32_t bits = __reduce_or_sync(0xffffffffu, word == w ? 1u << (at & 31u) : 0u);
+    if ((int)lane_id() == __ffs(todo) - 1) atomicOr(&p.occ[w], bits);
+    todo &= ~__ballot_sync(0xffffffffu, word == w);
+  }
 }
 
 static constexpr uint32_t SWEEP_THREADS = 256;

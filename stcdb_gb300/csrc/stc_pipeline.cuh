@@ -100,6 +100,7 @@ struct PipeDev {
   unsigned long long nb_magic;          // ceil(2^64 / nb)
   uint32_t *bin_cnt;                    // nb
   uint32_t *tile_live;                  // nb: occupied slots of each tile after the last step
+  uint32_t *occ;                        // nb x OCC_WORDS: which ones, a bit a slot of the tile
   uint32_t runs;                        // runs of tiles the tiled update is cut into
   uint32_t *carry, *carry_cnt;          // runs x TILE_LOAD, runs: hits carried into each run
   Cand *cset;                           // C
@@ -121,10 +122,12 @@ void step_hits(PipeDev &p, cudaStream_t s);
 // stc_table.cu: the tiled table update and sweep. plan decides whether the
 // step takes it and finds what is carried into each run of tiles.
 constexpr uint32_t TILE_SLOTS = 768;    // largest tile
+constexpr uint32_t OCC_WORDS = TILE_SLOTS / 32;
 constexpr uint32_t TILE_LOAD = 576;     // (occupied slots + hits) of a tile stay below this on the tiled path
 cudaError_t table_prepare();
 void table_sizes(PipeDev &p);           // nb and runs of a table of p.B slots
 void count_tiles(PipeDev &p, cudaStream_t s);
+void unpack_tiles(PipeDev &p, uint32_t layout, cudaStream_t s);  // every meeting into its slot
 void step_table_plan(PipeDev &p, cudaStream_t s);
 void step_table(PipeDev &p, cudaStream_t s);
 // stc_meetings.cu: the general path's insert and sweep

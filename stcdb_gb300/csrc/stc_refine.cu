@@ -151,13 +151,16 @@ __device__ __forceinline__ void store_hit(HitRec *d, const HitRec &h) {
 // the table update finds the tile's hits together. The records are 32-byte
 // sectors whose bins' open ends stay in L2 (one 128-byte line a bin: 45 MB
 // for 2^28 slots), so they reach HBM as whole lines. A hit its bin has no
-// room for is applied here; the step then takes the general path.
+// room for is applied here, and the step then takes the general path; while
+// the tiles are packed that has to wait until they are unpacked, and the pair
+// tests are done once more (k_hits).
 __device__ __forceinline__ void bin_hit(const PipeDev &p, const HitRec &h, uint32_t t) {
   const unsigned long long key = stc_cantor(h.a, h.b);
   const uint32_t bin = tile_of(p, fast_mod(key, p.B, p.B_magic));
   const uint32_t pos = atomicAdd(&p.bin_cnt[bin], 1u);
   if (pos < p.bin_cap) store_hit(&p.hits[(unsigned long long)bin * p.bin_cap + pos], h);
-  else process_hit(p, h, t);
+  else if (p.st->packed == TABLE_SLOTS) process_hit(p, h, t);
+  else p.st->redo = 1;
 }
 
 __device__ __forceinline__ HitRec load_hit(const HitRec *r) {
@@ -173,32 +176,6 @@ __device__ __forceinline__ HitRec load_hit(const HitRec *r) {
   h.hi_x = m.z;
   h.hi_y = m.w;
   return h;
-}
-
-// The general path's table update: a warp takes 64 hits of a bin, one thread
-// per hit, two hits in flight per thread (both records and both home slots
-// are requested before either is used).
-__global__ void __launch_bounds__(256) k_hits(PipeDev p) {
-  if (fuse_halo(p)) return;
-  const uint32_t t = p.st->step_t;
-  const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  const uint32_t parts = (min((uint32_t)p.st->hit_max, p.bin_cap) + 63) / 64;  // of the fullest bin
-  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
-       w < (unsigned long long)p.nb * parts; w += warps) {
-    const uint32_t bin = (uint32_t)(w / parts), i = (uint32_t)(w % parts) * 64 + lane_id();
-    const uint32_t n = min(p.bin_cnt[bin], p.bin_cap);
-    if (i >= n) continue;
-    const HitRec *hits = p.hits + (unsigned long long)bin * p.bin_cap;
-    const bool two = i + 32 < n;
-    const HitRec h0 = load_hit(&hits[i]);
-    const HitRec h1 = load_hit(&hits[two ? i + 32 : i]);
-    const unsigned long long k0 = stc_cantor(h0.a, h0.b), k1 = stc_cantor(h1.a, h1.b);
-    const unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
-    const U128 kv0 = load_slot_pair(&p.slots[s0]), kv1 = load_slot_pair(&p.slots[s1]);
-    const float4 m0 = __ldcg((const float4 *)&p.slots[s0].lo_x), m1 = __ldcg((const float4 *)&p.slots[s1].lo_x);
-    process_hit_at(p, h0, k0, t, s0, kv0, m0);
-    if (two) process_hit_at(p, h1, k1, t, s1, kv1, m1);
-  }
 }
 
 __device__ __forceinline__ float warp_max(float v) {
@@ -254,6 +231,9 @@ struct __align__(16) Row {
 // records' stores 2.85: bound by L2's rate of scattered 32-byte stores (39 G/s
 // measured, 35 with an atomic each). A row per lane and a shared-memory queue
 // of records before it: 3.0 ms for the tests with sequential records.
+// REDO: every hit is applied to the table at once, nothing is binned; the
+// schema is not read, which its update may be rewriting.
+template <bool REDO>
 __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblock, uint32_t chunk, uint32_t t,
                          Counters &ct, Row *rows) {
   const uint32_t lane = lane_id();
@@ -294,10 +274,12 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       // this step iff the member also has a border unit targeting the row's
       // leaf.
       leaf = p.leaf_gid[pid];
-      const Node *ro = &p.sd.nodes[p.sd.gid_node[leaf]];
-      ax0 = __double2float_rn(ro->lo_x);
-      ay0 = __double2float_rn(ro->lo_y);
-      ay1 = __double2float_rn(ro->hi_y);
+      if (!REDO) {
+        const Node *ro = &p.sd.nodes[p.sd.gid_node[leaf]];
+        ax0 = __double2float_rn(ro->lo_x);
+        ay0 = __double2float_rn(ro->lo_y);
+        ay1 = __double2float_rn(ro->hi_y);
+      }
       // candidates: the members in the point's longitude window of the
       // strips beside its own (all of a strip too large to be ordered)
       const int H = (int)lg->strips;
@@ -418,16 +400,63 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       // passes every such member, and the three dependent loads of its units
       // are left to the few that pass
       const float4 r3 = *((const float4 *)w + 3);
-      if (fc.y <= r3.y || (fc.y <= r3.z && fc.x <= r3.x)) {
+      if (REDO || fc.y <= r3.y || (fc.y <= r3.z && fc.x <= r3.x)) {
         const uint32_t cnb = p.bcount[pid2];
         const uint32_t coff = cnb ? p.boff[pid2] : 0u;
         for (uint32_t u2 = 0; u2 < cnb; u2++)
           if (p.bu_gid[coff + u2] == r2.w) h.order |= DUP_BIT;
       }
     }
-    bin_hit(p, h, t);
+    if (REDO) process_hit(p, h, t);
+    else bin_hit(p, h, t);
   }
   __syncwarp();
+}
+
+// The pair tests of a step whose bins overflowed while the table's tiles were
+// packed, once more, by the whole grid.
+__device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows) {
+  const uint32_t t = p.st->step_t;
+  const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+  const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  Counters ct = {0, 0, 0, 0};  // counted the first time
+  for (unsigned long long job = warp; job < p.st->jobs_total; job += nwarps) {
+    if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
+    const uint4 w = p.jobs[job];
+    for (uint32_t c = 0; c < w.w; c++)
+      run_rows<true>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
+  }
+}
+
+// The general path's table update: a warp takes 64 hits of a bin, one thread
+// per hit, two hits in flight per thread (both records and both home slots
+// are requested before either is used).
+__global__ void __launch_bounds__(256) k_hits(PipeDev p) {
+  if (fuse_halo(p)) return;
+  __shared__ Row rows_all[256 / 32][32];
+  if (p.st->redo) {
+    redo_pairs(p, rows_all[threadIdx.x >> 5]);
+    return;
+  }
+  const uint32_t t = p.st->step_t;
+  const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  const uint32_t parts = (min((uint32_t)p.st->hit_max, p.bin_cap) + 63) / 64;  // of the fullest bin
+  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
+       w < (unsigned long long)p.nb * parts; w += warps) {
+    const uint32_t bin = (uint32_t)(w / parts), i = (uint32_t)(w % parts) * 64 + lane_id();
+    const uint32_t n = min(p.bin_cnt[bin], p.bin_cap);
+    if (i >= n) continue;
+    const HitRec *hits = p.hits + (unsigned long long)bin * p.bin_cap;
+    const bool two = i + 32 < n;
+    const HitRec h0 = load_hit(&hits[i]);
+    const HitRec h1 = load_hit(&hits[two ? i + 32 : i]);
+    const unsigned long long k0 = stc_cantor(h0.a, h0.b), k1 = stc_cantor(h1.a, h1.b);
+    const unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
+    const U128 kv0 = load_slot_pair(&p.slots[s0]), kv1 = load_slot_pair(&p.slots[s1]);
+    const float4 m0 = __ldcg((const float4 *)&p.slots[s0].lo_x), m1 = __ldcg((const float4 *)&p.slots[s1].lo_x);
+    process_hit_at(p, h0, k0, t, s0, kv0, m0);
+    if (two) process_hit_at(p, h1, k1, t, s1, kv1, m1);
+  }
 }
 
 // Slice `part` of `parts` runs jobs [J * part / parts, J * (part + 1) / parts),
@@ -452,7 +481,7 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
     for (unsigned long long job = j0; job < j1; job++) {
       const uint4 w = p.jobs[job];
       for (uint32_t c = 0; c < w.w; c++)
-        run_rows(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
+        run_rows<false>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
     }
   }
   // reduce counters per warp (64-bit sums)
