@@ -37,6 +37,7 @@
 #include <cstring>
 #include <vector>
 
+#include "stc_fixed.cuh"
 #include "stc_lsm_kernels.cuh"
 
 namespace stc {
@@ -50,22 +51,27 @@ struct InCtf {
   unsigned long long first;  // first key of this CTF among all decoded CTF keys
   const uint8_t *keys;       // its packed keys (block buffer padded by 32 bytes)
   stc_ctf ctf;
-  double rx, ry, re;         // 1 / the largest low-x, low-y and edge field
-  double dx, dy, de;         // bounds on the reciprocal decode's error (parse_coord)
+  FixedBox fixed;            // decode of its boxes in fixed point
 };
 
-// One box coordinate as CTF::new_parse_mbr_f_box computes it: the float
-// nearest to base + (q / qmax) * w evaluated in double. The correctly rounded
-// division costs many FP64 instructions, so q * (1 / qmax) is tried first: it
-// differs from the exact double by at most d, and when both ends of
-// [v - d, v + d] round to the same float that float is the result.
-__device__ __forceinline__ float parse_coord(double base, unsigned long long q, unsigned long long qmax, double rq,
-                                            double w, double d) {
-  const double qd = __ull2double_rn(q);
-  const double v = base + qd * rq * w;
-  const float lo = __double2float_rn(v - d), hi = __double2float_rn(v + d);
-  if (lo == hi) return lo;
-  return __double2float_rn(__dadd_rn(base, __dmul_rn(__ddiv_rn(qd, __ull2double_rn(qmax)), w)));
+// A box as CTF::new_parse_mbr_f_box computes it: each coordinate the float
+// nearest to base + (field / fieldmax) * width evaluated in double, the high
+// corner's base being the low corner's float. Fixed point decides it for all
+// but a few in a million (stc_fixed.cuh); those take the double arithmetic.
+__device__ __noinline__ float4 parse_box_exact(const stc_ctf &t, unsigned long long low0, unsigned long long low1,
+                                               unsigned long long ex, unsigned long long ey, unsigned long long mx,
+                                               unsigned long long my, unsigned long long me) {
+  const float wx = __fsub_rn(t.mbr[2], t.mbr[0]), wy = __fsub_rn(t.mbr[3], t.mbr[1]), le = fmaxf(wx, wy);
+  auto coord = [](double base, unsigned long long q, unsigned long long qmax, double w) {
+    return __double2float_rn(
+        __dadd_rn(base, __dmul_rn(__ddiv_rn(__ull2double_rn(q), __ull2double_rn(qmax)), w)));
+  };
+  float4 b;
+  b.x = coord((double)t.mbr[0], low0, mx, (double)wx);
+  b.y = coord((double)t.mbr[1], low1, my, (double)wy);
+  b.z = coord((double)b.x, ex, me, (double)le);
+  b.w = coord((double)b.y, ey, me, (double)le);
+  return b;
 }
 
 __host__ __device__ __forceinline__ unsigned long long mask64(uint32_t bits) {
@@ -86,6 +92,15 @@ __device__ __forceinline__ unsigned __int128 load_packed(const uint8_t *p, uint3
 __device__ __forceinline__ uint32_t ordered(float f) {
   uint32_t u = __float_as_uint(f == 0.0f ? 0.0f : f);
   return (u & 0x80000000u) ? ~u : (u | 0x80000000u);
+}
+
+// The order of floats (no NaN) as that of unsigned integers, and back.
+__device__ __forceinline__ uint32_t float_rank(float f) {
+  const uint32_t u = __float_as_uint(f);
+  return u ^ ((uint32_t)((int32_t)u >> 31) | 0x80000000u);
+}
+__device__ __forceinline__ float rank_float(uint32_t r) {
+  return __uint_as_float(r ^ ((uint32_t)((int32_t)~r >> 31) | 0x80000000u));
 }
 
 struct Objs {
@@ -112,67 +127,102 @@ __global__ void k_cmp_init(const uint16_t *const *in_sids, uint32_t m, uint32_t 
 // kid` gets (oid, target, duration, end offset) and the float box; keys of
 // oversize objects go to the oversize buffer (end relative to o_etm), the
 // others mark their object (sid 2), count and box it (end relative to etm).
-__global__ void k_cmp_decode(const InCtf *ic, uint32_t nc, unsigned long long nk, unsigned long long base,
-                             uint32_t N, uint32_t etm, uint32_t o_etm, Objs o, uint4 *rec, float4 *box,
-                             uint8_t *over, DevState *st) {
+// Bound by its FP64 instructions before (35 a warp of keys, 16 cycles each;
+// five atomics a key behind them): 87.4M keys 6.2 ms, now 2.3. Each block
+// takes a contiguous run of keys; a CTF's keys are in object order, so a warp
+// has few objects and adds each one's count and box at once.
+__global__ void __launch_bounds__(256) k_cmp_decode(const InCtf *ic, uint32_t nc, unsigned long long nk,
+                                                    unsigned long long base, uint32_t N, uint32_t etm, uint32_t o_etm,
+                                                    Objs o, uint4 *rec, float4 *box, uint8_t *over, DevState *st) {
   uint32_t md = 0, me = 0;
-  for (unsigned long long kid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; kid < nk;
-       kid += (unsigned long long)gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = nc - 1;  // largest c with first <= kid
-    while (lo < hi) {
-      uint32_t mid = (lo + hi + 1) >> 1;
-      if (ic[mid].first <= kid) lo = mid;
-      else hi = mid - 1;
+  const uint32_t lane = lane_id();
+  const unsigned long long per = (nk + gridDim.x - 1) / gridDim.x;
+  const unsigned long long k0 = min(nk, per * blockIdx.x), k1 = min(nk, k0 + per);
+  uint32_t lo = 0;  // largest c with first <= kid
+  for (uint32_t hi = nc - 1; lo < hi;) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (ic[mid].first <= k0) lo = mid;
+    else hi = mid - 1;
+  }
+  for (unsigned long long kb0 = k0 + (threadIdx.x & ~31u); kb0 < k1; kb0 += blockDim.x) {
+    const unsigned long long kid = kb0 + lane;
+    bool part = kid < k1;
+    uint32_t oid = 0;
+    float4 b = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (part) {
+      while (lo + 1 < nc && ic[lo + 1].first <= kid) lo++;
+      const stc_ctf &t = ic[lo].ctf;
+      const uint32_t kb = t.key_bit / 8u;
+      uint32_t target = 0;
+      part = kid - ic[lo].first < t.kv_count;  // outside every CTF: never read past its keys
+      if (!part) {
+        stc_set_error(st, ERR_COMPACT, lo);
+      } else {
+        unsigned __int128 k = load_packed(ic[lo].keys + (kid - ic[lo].first) * kb, kb);
+        unsigned long long vm = (unsigned long long)(k & (unsigned __int128)mask64(t.mbr_bit));
+        k >>= t.mbr_bit;
+        const uint32_t end = (uint32_t)(k & mask64(t.end_bit));
+        k >>= t.end_bit;
+        const uint32_t dur = (uint32_t)(k & mask64(t.duration_bit));
+        k >>= t.duration_bit;
+        target = (uint32_t)(k & mask64(t.id_bit));
+        k >>= t.id_bit;
+        oid = (uint32_t)(k & mask64(t.id_bit));
+        part = oid < N && target < N;
+        if (!part) {
+          stc_set_error(st, ERR_COMPACT, oid);
+        } else {
+          const uint32_t real_end = end + t.end_time_min;
+          const unsigned long long mm = mask64(t.edge_bit), my = mask64(t.low_y_bit), mx = mask64(t.low_x_bit);
+          const unsigned long long ey = vm & mm;
+          vm >>= t.edge_bit;
+          const unsigned long long ex = vm & mm;
+          vm >>= t.edge_bit;
+          const unsigned long long low1 = vm & my;
+          vm >>= t.low_y_bit;
+          const unsigned long long low0 = vm & mx;
+          const FixedBox &f = ic[lo].fixed;
+          long long ux = 0, uy = 0, none;
+          const bool sure = fixed_to_float(f.x0 + (long long)(low0 * f.kx), f.e, f.q, b.x, ux) &&
+                            fixed_to_float(f.y0 + (long long)(low1 * f.ky), f.e, f.q, b.y, uy) &&
+                            fixed_to_float(ux + (long long)(ex * f.ke), f.e, f.q, b.z, none) &&
+                            fixed_to_float(uy + (long long)(ey * f.ke), f.e, f.q, b.w, none);
+          if (!sure) b = parse_box_exact(t, low0, low1, ex, ey, mx, my, mm);
+          const bool ov = o.csid[oid] == 1;
+          const uint32_t off = real_end - (ov ? o_etm : etm);
+          rec[base + kid] = make_uint4(oid, target, dur, off);
+          box[base + kid] = b;
+          over[base + kid] = ov;
+          md = max(md, dur);
+          me = max(me, off);
+          if (ov) agg_inc(&st->lsm_over_keys);
+          part = !ov;
+        }
+      }
     }
-    const stc_ctf &t = ic[lo].ctf;
-    const uint32_t kb = t.key_bit / 8u;
-    if (kid - ic[lo].first >= t.kv_count) {  // outside every CTF: never read past its keys
-      stc_set_error(st, ERR_COMPACT, lo);
-      continue;
+    // counts and boxes of the warp's objects, a group of lanes at a time
+    uint32_t todo = __ballot_sync(0xffffffffu, part);
+    for (int round = 0; round < 4 && todo; round++) {
+      const int first = __ffs(todo) - 1;
+      const uint32_t obj = __shfl_sync(0xffffffffu, oid, first);
+      const bool mine = part && oid == obj;
+      const uint32_t group = __ballot_sync(0xffffffffu, mine);
+      const uint32_t x0 = __reduce_min_sync(0xffffffffu, mine ? float_rank(b.x) : 0xffffffffu);
+      const uint32_t y0 = __reduce_min_sync(0xffffffffu, mine ? float_rank(b.y) : 0xffffffffu);
+      const uint32_t x1 = __reduce_max_sync(0xffffffffu, mine ? float_rank(b.z) : 0u);
+      const uint32_t y1 = __reduce_max_sync(0xffffffffu, mine ? float_rank(b.w) : 0u);
+      if ((int)lane == first) {
+        o.csid[obj] = 2;  // every writer stores the same value
+        atomicAdd(&o.cnt[obj], (uint32_t)__popc(group));
+        atomic_min_f(&o.box[obj].x, rank_float(x0));
+        atomic_min_f(&o.box[obj].y, rank_float(y0));
+        atomic_max_f(&o.box[obj].z, rank_float(x1));
+        atomic_max_f(&o.box[obj].w, rank_float(y1));
+      }
+      todo &= ~group;
     }
-    unsigned __int128 k = load_packed(ic[lo].keys + (kid - ic[lo].first) * kb, kb);
-    unsigned long long vm = (unsigned long long)(k & (unsigned __int128)mask64(t.mbr_bit));
-    k >>= t.mbr_bit;
-    uint32_t end = (uint32_t)(k & mask64(t.end_bit));
-    k >>= t.end_bit;
-    uint32_t dur = (uint32_t)(k & mask64(t.duration_bit));
-    k >>= t.duration_bit;
-    uint32_t target = (uint32_t)(k & mask64(t.id_bit));
-    k >>= t.id_bit;
-    uint32_t oid = (uint32_t)(k & mask64(t.id_bit));
-    if (oid >= N || target >= N) {
-      stc_set_error(st, ERR_COMPACT, oid);
-      continue;
-    }
-    const uint32_t real_end = end + t.end_time_min;
-    // CTF::new_parse_mbr_f_box: double arithmetic, stored as float
-    const InCtf &x = ic[lo];
-    unsigned long long me_ = mask64(t.edge_bit), my = mask64(t.low_y_bit), mx = mask64(t.low_x_bit);
-    unsigned long long ey = vm & me_;
-    vm >>= t.edge_bit;
-    unsigned long long ex = vm & me_;
-    vm >>= t.edge_bit;
-    unsigned long long low1 = vm & my;
-    vm >>= t.low_y_bit;
-    unsigned long long low0 = vm & mx;
-    float wx = __fsub_rn(t.mbr[2], t.mbr[0]), wy = __fsub_rn(t.mbr[3], t.mbr[1]);
-    float le = fmaxf(wx, wy);
-    float4 b;
-    b.x = parse_coord((double)t.mbr[0], low0, mx, x.rx, (double)wx, x.dx);
-    b.y = parse_coord((double)t.mbr[1], low1, my, x.ry, (double)wy, x.dy);
-    b.z = parse_coord((double)b.x, ex, me_, x.re, (double)le, x.de);
-    b.w = parse_coord((double)b.y, ey, me_, x.re, (double)le, x.de);
-    const bool ov = o.csid[oid] == 1;
-    const uint32_t off = real_end - (ov ? o_etm : etm);
-    rec[base + kid] = make_uint4(oid, target, dur, off);
-    box[base + kid] = b;
-    over[base + kid] = ov;
-    md = max(md, dur);
-    me = max(me, off);
-    if (ov) {
-      agg_inc(&st->lsm_over_keys);
-    } else {
-      o.csid[oid] = 2;  // every writer stores the same value
+    if ((todo >> lane) & 1u) {  // more objects than rounds
+      o.csid[oid] = 2;
       atomicAdd(&o.cnt[oid], 1u);
       atomic_min_f(&o.box[oid].x, b.x);
       atomic_min_f(&o.box[oid].y, b.y);
@@ -182,7 +232,7 @@ __global__ void k_cmp_decode(const InCtf *ic, uint32_t nc, unsigned long long nk
   }
   md = warp_max_u32(md);
   me = warp_max_u32(me);
-  if ((threadIdx.x & 31u) == 0) {
+  if (lane == 0) {
     atomicMax(&st->lsm_max_dur, md);
     atomicMax(&st->lsm_max_end, me);
   }
@@ -373,21 +423,9 @@ stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32
       x.first = first;
       x.keys = b->keys + t.key_offset;
       x.ctf = t;
-      // each of the exact decode's five roundings (and the reciprocal
-      // decode's) is within 2^-53 of a value below |base| + 2|w| in size; the
-      // bound used is 2^7 times their sum
-      const double mx = (double)mask64(t.low_x_bit), my = (double)mask64(t.low_y_bit), me = (double)mask64(t.edge_bit);
-      const float wx = t.mbr[2] - t.mbr[0], wy = t.mbr[3] - t.mbr[1], le = std::max(wx, wy);
-      double m = 0.0;
-      for (int i = 0; i < 4; i++) m = std::max(m, std::fabs((double)t.mbr[i]));
-      const bool ok = mx > 0 && my > 0 && me > 0 && std::isfinite(m) && std::isfinite((double)le);
-      x.rx = ok ? 1.0 / mx : 0.0;
-      x.ry = ok ? 1.0 / my : 0.0;
-      x.re = ok ? 1.0 / me : 0.0;
-      const double u = std::ldexp(1.0, -46);
-      x.dx = ok ? (std::fabs((double)t.mbr[0]) + 2.0 * std::fabs((double)wx) + 1.0) * u : INFINITY;
-      x.dy = ok ? (std::fabs((double)t.mbr[1]) + 2.0 * std::fabs((double)wy) + 1.0) * u : INFINITY;
-      x.de = ok ? (m + std::fabs((double)wx) + std::fabs((double)wy) + 2.0 * std::fabs((double)le) + 1.0) * u : INFINITY;
+      const float wx = t.mbr[2] - t.mbr[0], wy = t.mbr[3] - t.mbr[1];
+      x.fixed = fixed_box(t.mbr, wx, wy, std::max(wx, wy), (double)mask64(t.low_x_bit), (double)mask64(t.low_y_bit),
+                          (double)mask64(t.edge_bit));
       ic.push_back(x);
       first += t.kv_count;
     }

@@ -73,6 +73,7 @@ constexpr uint32_t LSM_INDEX_MAX_GRID = 256;
 __host__ __device__ inline uint32_t index_level_side(uint32_t g, uint32_t k) { return (g >> k) + 1u; }
 
 // Device copy of one flushed block, kept for queries.
+struct FixedAxis;  // stc_fixed.cuh
 struct CtbBlock {
   stc_ctb_info info{};
   std::vector<stc_ctf> ctfs;       // host copy
@@ -91,8 +92,7 @@ struct CtbBlock {
   uint4 *ixg = nullptr;            // [F] (g, levels, 0, 0) of each CTF's index
   double2 *ixs = nullptr;          // [F] level-0 cells per degree in x and y (g / CTF box side)
   double2 *ixq = nullptr;          // [F] widening of box queries in x and y (index_slack)
-  float4 *ixf = nullptr;           // [2F] float filing of keys: per axis (cells per low unit, cells per
-                                   // edge unit, error margin, 1 if usable)
+  FixedAxis *ixf = nullptr;        // [2F] filing of keys in fixed point, per axis
   uint16_t *pend = nullptr;       // [keys] end offset of the key at each perm position, saturated at
                                    // 65535; within a cell the keys go by increasing end
 };

@@ -14,6 +14,7 @@
 #include <string>
 #include <vector>
 
+#include "stc_fixed.cuh"
 #include "stc_lsm.cuh"
 
 namespace stc {
@@ -272,18 +273,17 @@ __device__ __forceinline__ void index_range(double a, double b, double m0, doubl
 
 // ---- cell index of a block ------------------------------------------------------
 
-constexpr uint32_t MAX_CTF = 3969;
-
 // Dense cell id of each CTF key in its CTF's loose grid (stc_lsm.cuh): the
 // level whose cells cover the extent of its decoded box, the cell of the box's
 // low corner there; or the CTF's wide slot.
 //
 // The cell depends on the decoded box only through floor() of its four corner
-// coordinates in level-0 cells. These are first computed in float from the
-// key's integer fields (cells per field unit, ixf); a corner whose float value
-// lies within its error margin of an integer could floor the other way, and
-// only keys with such a corner take the exact decode (four correctly rounded
-// FP64 divisions, which the key's filing must agree with).
+// coordinates in level-0 cells, which are computed in fixed point from the
+// key's integer fields (stc_fixed.cuh); only keys with a corner at a cell edge
+// take the exact decode (four correctly rounded FP64 divisions, which the
+// key's filing must agree with). In float the margin was wide enough, and the
+// corners at the CTF box's edge (field 0) many enough, that most warps had a
+// lane in the double path: 87.4M keys 7.7 ms, now 3.7.
 struct IndexFile {
   uint32_t l0, l1;  // floor of the low corner, level-0 cells
   float ext;        // extent in level-0 cells: max over x, y of floor(high) - floor(low)
@@ -302,15 +302,8 @@ __device__ __forceinline__ uint32_t index_cell_of(const IndexFile &f, uint32_t g
   return off + (f.l1 >> lv) * index_level_side(g, lv) + (f.l0 >> lv);
 }
 
-// floor(v) when every value within d of v has the same floor; else false.
-__device__ __forceinline__ bool sure_floor(float v, float d, float &fl) {
-  fl = floorf(v - d);
-  return fl == floorf(v + d);
-}
-
-__device__ __forceinline__ bool index_file_fast(unsigned long long vm, const stc_ctf &c, const float4 &ax,
-                                                const float4 &ay, uint32_t g, IndexFile &f) {
-  if (ax.w == 0.0f || ay.w == 0.0f) return false;
+__device__ __forceinline__ bool index_file_fast(unsigned long long vm, const stc_ctf &c, const FixedAxis &ax,
+                                                const FixedAxis &ay, uint32_t g, IndexFile &f) {
   const unsigned long long y = vm & mask64(c.edge_bit);
   vm >>= c.edge_bit;
   const unsigned long long x = vm & mask64(c.edge_bit);
@@ -318,16 +311,20 @@ __device__ __forceinline__ bool index_file_fast(unsigned long long vm, const stc
   const unsigned long long low1 = vm & mask64(c.low_y_bit);
   vm >>= c.low_y_bit;
   const unsigned long long low0 = vm & mask64(c.low_x_bit);
-  const float fx0 = __ull2float_rn(low0) * ax.x, fy0 = __ull2float_rn(low1) * ay.x;
-  const float fx1 = fx0 + __ull2float_rn(x) * ax.y, fy1 = fy0 + __ull2float_rn(y) * ay.y;
-  float a, b, p, q;
-  if (!sure_floor(fx0, fmaf(fx0, 1e-6f, ax.z), a) || !sure_floor(fy0, fmaf(fy0, 1e-6f, ay.z), b) ||
-      !sure_floor(fx1, fmaf(fx1, 1e-6f, ax.z), p) || !sure_floor(fy1, fmaf(fy1, 1e-6f, ay.z), q))
-    return false;
-  f.inside = a >= 0.0f && b >= 0.0f && a <= (float)g && b <= (float)g;
-  f.l0 = f.inside ? (uint32_t)a : 0u;
-  f.l1 = f.inside ? (uint32_t)b : 0u;
-  f.ext = fmaxf(p - a, q - b);
+  // Field 0 decodes to the CTF box's edge, cell 0, exactly, and an edge field
+  // of 0 to the low corner again.
+  uint32_t a = 0, b = 0, p, q;
+  const unsigned long long px = low0 * ax.kl, py = low1 * ay.kl;
+  bool sure = ax.e != ~0ull && ay.e != ~0ull;
+  sure &= fixed_cell(px, ax.e, a) || low0 == 0;
+  sure &= fixed_cell(py, ay.e, b) || low1 == 0;
+  sure &= fixed_cell(px + x * ax.ke, ax.e, p) || x == 0;
+  sure &= fixed_cell(py + y * ay.ke, ay.e, q) || y == 0;
+  if (!sure) return false;
+  f.inside = a <= g && b <= g;
+  f.l0 = a;
+  f.l1 = b;
+  f.ext = (float)max(p - a, q - b);
   return true;
 }
 
@@ -343,27 +340,27 @@ __device__ __forceinline__ void index_file_exact(unsigned long long vm, const st
   f.ext = f.inside ? (float)fmax(floor(fx1) - f.l0, floor(fy1) - f.l1) : 0.0f;
 }
 
-__global__ void k_index_cells(const uint8_t *keys, const stc_ctf *ctfs, uint32_t F, const uint32_t *cbase,
-                              const uint4 *ixg, const double2 *ixs, const float4 *ixf, unsigned long long total,
-                              uint32_t *cells, uint32_t *pos, uint32_t *endo, unsigned long long *max_end) {
-  __shared__ unsigned long long s_first[MAX_CTF + 1];
-  __shared__ uint32_t s_max;
-  if (threadIdx.x == 0) s_max = 0;
+// Each block takes a contiguous run of keys, so that the search for a key's
+// CTF is a step or none.
+__global__ void __launch_bounds__(256) k_index_cells(const uint8_t *keys, const stc_ctf *ctfs, uint32_t F,
+                                                     const uint32_t *cbase, const uint4 *ixg, const double2 *ixs,
+                                                     const FixedAxis *ixf, unsigned long long total, uint32_t *cells,
+                                                     uint32_t *pos, uint32_t *endo, unsigned long long *max_end) {
   uint32_t my_max = 0;
-  for (uint32_t c = threadIdx.x; c < F; c += blockDim.x) s_first[c] = ctfs[c].first_key;
-  __syncthreads();
-  for (unsigned long long kid = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; kid < total;
-       kid += (unsigned long long)gridDim.x * blockDim.x) {
-    uint32_t lo = 0, hi = F - 1;
-    while (lo < hi) {
-      uint32_t mid = (lo + hi + 1) >> 1;
-      if (s_first[mid] <= kid) lo = mid;
-      else hi = mid - 1;
-    }
+  const unsigned long long per = (total + gridDim.x - 1) / gridDim.x;
+  const unsigned long long k0 = min(total, per * blockIdx.x), k1 = min(total, k0 + per);
+  uint32_t lo = 0;  // the last CTF that starts at or before the key (empty ones share their start)
+  for (uint32_t hi = F - 1; lo < hi;) {
+    const uint32_t mid = (lo + hi + 1) >> 1;
+    if (ctfs[mid].first_key <= k0) lo = mid;
+    else hi = mid - 1;
+  }
+  for (unsigned long long kid = k0 + threadIdx.x; kid < k1; kid += blockDim.x) {
+    while (lo + 1 < F && ctfs[lo + 1].first_key <= kid) lo++;
     const stc_ctf &t = ctfs[lo];
     const uint32_t kb = t.key_bit / 8u;
     Key k;
-    const unsigned long long vm = key_fields(load_key(keys + t.key_offset + (kid - s_first[lo]) * kb, kb), t, k);
+    const unsigned long long vm = key_fields(load_key(keys + t.key_offset + (kid - t.first_key) * kb, kb), t, k);
     const uint32_t g = ixg[lo].x, levels = ixg[lo].y;
     const double2 sc = ixs[lo];
     uint32_t cell = 0xFFFFFFFFu;  // the wide slot, after every level
@@ -378,10 +375,8 @@ __global__ void k_index_cells(const uint8_t *keys, const stc_ctf *ctfs, uint32_t
     endo[kid] = min(k.end, 65535u);
     my_max = max(my_max, min(k.end, 65535u));
   }
-  __syncthreads();
-  atomicMax(&s_max, my_max);
-  __syncthreads();
-  if (threadIdx.x == 0 && s_max) atomicMax(max_end, (unsigned long long)s_max);
+  my_max = __reduce_max_sync(0xffffffffu, my_max);
+  if (lane_id() == 0 && my_max) atomicMax(max_end, (unsigned long long)my_max);
 }
 
 // Sort keys of the one-pass index order: cell above the end offset.
@@ -935,23 +930,20 @@ void free_block(CtbBlock &B) {
 
 static void retain_block(LsmHost &H, CtbBlock &&B);
 
-// Float filing coefficients of one axis of CTF t (k_index_cells): level-0
-// cells per unit of the low field and of the edge field, the absolute error
-// margin of the exact filing in cells, and 1 when the float filing applies.
-// The exact corner differs from its real value by a few units of 2^-52 of the
-// largest coordinate (one division, one product, two sums and a difference,
-// each correctly rounded); the margin is 2^6 times that.
-static float4 index_file_coeffs(const stc_ctf &t, double scale, bool x_axis) {
+// Filing of CTF t's keys on one axis (k_index_cells): level-0 cells per unit of
+// the low field and of the edge field, and the error of the exact filing in
+// cells. The exact corner differs from its real value by a few units of 2^-52
+// of the largest coordinate (one division, one product, two sums and a
+// difference, each correctly rounded); the bound used is 2^6 times that.
+static FixedAxis index_file_axis(const stc_ctf &t, double scale, bool x_axis) {
   const float wx = t.mbr[2] - t.mbr[0], wy = t.mbr[3] - t.mbr[1];
   const double w = x_axis ? wx : wy, le = std::max(wx, wy);
   const double lowmax = (double)mask64(x_axis ? t.low_x_bit : t.low_y_bit), edgemax = (double)mask64(t.edge_bit);
   double m = 0.0;
   for (int i = 0; i < 4; i++) m = std::max(m, std::fabs((double)t.mbr[i]));
   m += le + 1.0;
-  const double a = scale * w / lowmax, b = scale * le / edgemax, d = scale * m * std::ldexp(1.0, -46);
-  const bool ok = scale > 0.0 && w > 0.0 && le > 0.0 && lowmax > 0.0 && edgemax > 0.0 && std::isfinite(a) &&
-                  std::isfinite(b) && std::isfinite(d) && a < 1e30 && b < 1e30 && d < 1e30;
-  return ok ? make_float4((float)a, (float)b, (float)d + 1e-9f, 1.0f) : make_float4(0.f, 0.f, 0.f, 0.f);
+  if (!(scale > 0.0 && w > 0.0 && le > 0.0 && lowmax > 0.0 && edgemax > 0.0)) return FixedAxis{0, 0, ~0ull, 0};
+  return fixed_axis(scale * w / lowmax, scale * le / edgemax, scale * m * std::ldexp(1.0, -46), lowmax, edgemax);
 }
 
 // How far a box query is widened for the CTF box, bitmap and index tests. A
@@ -970,7 +962,7 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
   std::vector<uint32_t> cbase(F + 1, 0);
   std::vector<uint4> ixg(F);
   std::vector<double2> ixs(F), ixq(F);
-  std::vector<float4> ixf(2 * (size_t)F);
+  std::vector<FixedAxis> ixf(2 * (size_t)F);
   unsigned long long total = 0;
   for (uint32_t c = 0; c < F; c++) {
     const stc_ctf &t = B.ctfs[c];
@@ -984,8 +976,8 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
     ixs[c] = make_double2(t.mbr[2] > t.mbr[0] && t.mbr[3] > t.mbr[1] ? (double)g / wx : 0.0,
                           t.mbr[2] > t.mbr[0] && t.mbr[3] > t.mbr[1] ? (double)g / wy : 0.0);
     ixq[c] = index_slack(t);
-    ixf[2 * c] = index_file_coeffs(t, ixs[c].x, true);
-    ixf[2 * c + 1] = index_file_coeffs(t, ixs[c].y, false);
+    ixf[2 * c] = index_file_axis(t, ixs[c].x, true);
+    ixf[2 * c + 1] = index_file_axis(t, ixs[c].y, false);
     cbase[c + 1] = cbase[c] + cells;
     total = std::max<unsigned long long>(total, t.first_key + t.kv_count);
   }
@@ -997,10 +989,10 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
   if (e == cudaSuccess) e = cudaMalloc(&B.ixg, std::max<size_t>(F, 1) * sizeof(uint4));
   if (e == cudaSuccess) e = cudaMalloc(&B.ixs, std::max<size_t>(F, 1) * sizeof(double2));
   if (e == cudaSuccess) e = cudaMalloc(&B.ixq, std::max<size_t>(F, 1) * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc(&B.ixf, std::max<size_t>(2 * (size_t)F, 1) * sizeof(float4));
+  if (e == cudaSuccess) e = cudaMalloc(&B.ixf, std::max<size_t>(2 * (size_t)F, 1) * sizeof(FixedAxis));
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixs, ixs.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixq, ixq.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
-  if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixf, ixf.data(), 2 * (size_t)F * sizeof(float4), cudaMemcpyHostToDevice, s);
+  if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixf, ixf.data(), 2 * (size_t)F * sizeof(FixedAxis), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.cbase, cbase.data(), (F + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixg, ixg.data(), F * sizeof(uint4), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
