@@ -245,4 +245,59 @@ void radix_sort_u32(const uint32_t *k_in, const uint32_t *v_in, uint32_t *k_out,
 
 void iota_u32(uint32_t *out, size_t n, cudaStream_t s);
 
+// Device memory (stc_util.cu). pool_alloc takes it from a pool of the current
+// device, in stream order: cudaMalloc and cudaFree of a call's scratch cost
+// 0.3 ms each for 300 MB, and stop the device. The pool keeps at most
+// POOL_KEEP_BYTES of freed memory and gives it back when an allocation of the
+// library fails and when a context is destroyed (pool_trim). dev_malloc is
+// cudaMalloc with that second attempt. What the pool would not keep is taken
+// plainly: a pool maps new gigabytes at a quarter of cudaMalloc's rate (8 GB
+// of compaction scratch: 7.3 against 1.1 ms).
+constexpr unsigned long long POOL_KEEP_BYTES = 512ull << 20;
+constexpr size_t POOL_LARGEST_KEPT = 64u << 20;  // largest single array of a block that is kept for queries
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
+void pool_free(void *p, cudaStream_t s);
+void pool_trim();
+cudaError_t dev_malloc(void **p, size_t bytes);
+
+// Device scratch of one call on stream s, `total` bytes in all, freed when it
+// ends.
+class CallScratch {
+ public:
+  CallScratch(cudaStream_t s, unsigned long long total) : s_(s), pooled_(total <= POOL_KEEP_BYTES) {}
+  CallScratch(const CallScratch &) = delete;
+  CallScratch &operator=(const CallScratch &) = delete;
+  ~CallScratch() {
+    for (int i = 0; i < n_; i++) {
+      if (pooled_) pool_free(ptr_[i], s_);
+      else cudaFree(ptr_[i]);
+    }
+  }
+  template <typename T>
+  T *get(size_t count) {
+    void *p = nullptr;
+    const size_t bytes = (count ? count : 1) * sizeof(T);
+    if (error_ == cudaSuccess && n_ == MOST) error_ = cudaErrorMemoryAllocation;
+    if (error_ == cudaSuccess) error_ = pooled_ ? pool_alloc(&p, bytes, s_) : dev_malloc(&p, bytes);
+    if (error_ != cudaSuccess) return nullptr;
+    ptr_[n_++] = p;
+    return (T *)p;
+  }
+  cudaError_t error() const { return error_; }
+
+ private:
+  static constexpr int MOST = 40;
+  cudaStream_t s_;
+  bool pooled_;
+  int n_ = 0;
+  void *ptr_[MOST];
+  cudaError_t error_ = cudaSuccess;
+};
+
+// An array of a block kept for queries: cudaFree frees it.
+template <typename T>
+inline cudaError_t block_alloc(T **p, size_t bytes, cudaStream_t s) {
+  return bytes <= POOL_LARGEST_KEPT ? pool_alloc((void **)p, bytes, s) : dev_malloc((void **)p, bytes);
+}
+
 }  // namespace stc

@@ -301,25 +301,6 @@ __global__ void k_cmp_state_init(DevState *st) {
   st->lsm_os_max = 0;
 }
 
-// Device scratch of one compaction, freed when it ends.
-struct Scratch {
-  std::vector<void *> ptrs;
-  bool ok = true;
-  template <typename T>
-  T *get(size_t n) {
-    void *p = nullptr;
-    if (ok && cudaMalloc(&p, std::max<size_t>(n, 1) * sizeof(T)) != cudaSuccess) {
-      ok = false;
-      p = nullptr;
-    }
-    if (p) ptrs.push_back(p);
-    return (T *)p;
-  }
-  ~Scratch() {
-    for (void *p : ptrs) cudaFree(p);
-  }
-};
-
 }  // namespace
 
 stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32_t count, uint32_t split,
@@ -379,7 +360,7 @@ stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32
     }
   } marks;
   auto mark = [&](int i) { cudaEventRecord(marks.ev[i], s); };
-  Scratch sc;
+  CallScratch sc(s, T * (2 * sizeof(uint4) + 2 * sizeof(float4) + 1) + 7 * W * sizeof(uint32_t) + 64ull * N);
   LsmDev C = L;  // configuration; every array below is the compaction's own
   C.F = F2;
   C.split = S;
@@ -407,7 +388,7 @@ stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32
   float4 *objbox = sc.get<float4>(N);
   InCtf *d_ic = sc.get<InCtf>(nc);
   const uint16_t **d_sids = sc.get<const uint16_t *>(count);
-  if (!sc.ok) {
+  if (sc.error() != cudaSuccess) {
     err = "compact: device memory for the merge scratch";
     return STC_ERR_CAPACITY;
   }
@@ -501,7 +482,7 @@ stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32
   CtbBlock B;
   const size_t no_out = (size_t)n_over;
   const size_t obm_bytes = STC_MAP_BITMAP_BYTES(L.edge);
-  e = cudaMalloc(&B.obitmap, obm_bytes);
+  e = block_alloc(&B.obitmap, obm_bytes, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(B.obitmap, 0, obm_bytes, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(C.ctf_first, cfirst.data(), (F2 + 1) * sizeof(unsigned long long),
                                             cudaMemcpyHostToDevice, s);
@@ -578,12 +559,12 @@ stc_status lsm_compact(const LsmDev &L, LsmHost &H, uint32_t first_index, uint32
   B.info.o_end_time_min = o_etm;
   B.info.o_end_time_max = o_etmax;
   B.info.bitmap_edge = L.edge;
-  e = cudaMalloc(&B.keys, off + 32);
-  if (e == cudaSuccess) e = cudaMalloc(&B.d_ctfs, F2 * sizeof(stc_ctf));
-  if (e == cudaSuccess) e = cudaMalloc(&B.bitmaps, (size_t)F2 * STC_BITMAP_BYTES);
-  if (e == cudaSuccess) e = cudaMalloc(&B.sids, (size_t)N * sizeof(uint16_t));
-  if (e == cudaSuccess) e = cudaMalloc(&B.orec, std::max<size_t>(no_out, 1) * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&B.obox, std::max<size_t>(no_out, 1) * sizeof(float4));
+  e = block_alloc(&B.keys, off + 32, s);
+  if (e == cudaSuccess) e = block_alloc(&B.d_ctfs, F2 * sizeof(stc_ctf), s);
+  if (e == cudaSuccess) e = block_alloc(&B.bitmaps, (size_t)F2 * STC_BITMAP_BYTES, s);
+  if (e == cudaSuccess) e = block_alloc(&B.sids, (size_t)N * sizeof(uint16_t), s);
+  if (e == cudaSuccess) e = block_alloc(&B.orec, std::max<size_t>(no_out, 1) * sizeof(uint4), s);
+  if (e == cudaSuccess) e = block_alloc(&B.obox, std::max<size_t>(no_out, 1) * sizeof(float4), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(B.keys, 0, off + 32, s);
   if (e == cudaSuccess) e = cudaMemsetAsync(B.bitmaps, 0, (size_t)F2 * STC_BITMAP_BYTES, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.d_ctfs, B.ctfs.data(), F2 * sizeof(stc_ctf), cudaMemcpyHostToDevice, s);

@@ -137,7 +137,7 @@ template <typename T>
 static bool dalloc(stc_ctx *c, T **ptr, size_t count) {
   size_t bytes = std::max<size_t>(count, 1) * sizeof(T);
   void *v = nullptr;
-  cudaError_t e = cudaMalloc(&v, bytes);
+  cudaError_t e = dev_malloc(&v, bytes);
   if (e != cudaSuccess) {
     char buf[256];
     snprintf(buf, sizeof(buf), "cudaMalloc(%zu bytes) failed: %s", bytes, cudaGetErrorString(e));
@@ -234,6 +234,7 @@ extern "C" void stc_destroy(stc_ctx *c) {
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   destroy_all(c);
+  pool_trim();
   cudaSetDevice(prev);
   delete c;
 }
@@ -708,7 +709,7 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
   if (c->cfg.hit_capacity || need <= p.bin_cap) return;
   const uint32_t cap = bin_share(need, 1, 5, 4, 16);
   void *h = nullptr;
-  if (cudaMalloc(&h, (size_t)p.nb * cap * sizeof(HitRec)) != cudaSuccess) {
+  if (dev_malloc(&h, (size_t)p.nb * cap * sizeof(HitRec)) != cudaSuccess) {
     cudaGetLastError();
     return;
   }
@@ -875,7 +876,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
     cudaError_t e = cudaSuccess;
     for (int b = 0; b < WIN_BUFS - 1 && e == cudaSuccess; b++)
       if (!c->xy_win[b]) {
-        e = cudaMalloc(&c->xy_win[b], step_bytes);
+        e = dev_malloc((void **)&c->xy_win[b], step_bytes);
         if (e == cudaSuccess) c->allocs.push_back(c->xy_win[b]);
       }
     if (e == cudaSuccess && !c->copy_stream) e = cudaStreamCreateWithFlags(&c->copy_stream, cudaStreamNonBlocking);

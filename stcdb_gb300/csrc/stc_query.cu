@@ -899,7 +899,7 @@ cudaError_t grow(T **p, size_t *cap, size_t need) {
   size_t n = std::max<size_t>(need, 2 * *cap);
   if (*p) cudaFree(*p);
   *p = nullptr;
-  cudaError_t e = cudaMalloc(p, n * sizeof(T));
+  cudaError_t e = dev_malloc((void **)p, n * sizeof(T));
   *cap = e == cudaSuccess ? n : 0;
   return e;
 }
@@ -907,6 +907,9 @@ cudaError_t grow(T **p, size_t *cap, size_t need) {
 }  // namespace
 
 void free_block(CtbBlock &B) {
+  // cudaFree waits for nothing where the memory came from the pool: whatever
+  // still uses the block (a build that failed half-way) ends first
+  if (B.keys || B.obitmap) cudaDeviceSynchronize();
   for (void *v : {(void *)B.keys, (void *)B.d_ctfs, (void *)B.bitmaps, (void *)B.sids, (void *)B.orec,
                   (void *)B.obox, (void *)B.obitmap, (void *)B.perm, (void *)B.cstart, (void *)B.cbase,
                   (void *)B.ixg, (void *)B.ixs, (void *)B.ixq, (void *)B.ixf, (void *)B.pend})
@@ -983,20 +986,20 @@ cudaError_t build_index(const LsmDev &L, CtbBlock &B, cudaStream_t s) {
   }
   const uint32_t ncells = cbase[F];
   if (total > lsm_sort_words(L)) return cudaErrorInvalidValue;  // more keys than the sort scratch holds
-  cudaError_t e = cudaMalloc(&B.perm, std::max<unsigned long long>(total, 1) * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&B.cstart, ((size_t)ncells + 1) * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&B.cbase, (F + 1) * sizeof(uint32_t));
-  if (e == cudaSuccess) e = cudaMalloc(&B.ixg, std::max<size_t>(F, 1) * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&B.ixs, std::max<size_t>(F, 1) * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc(&B.ixq, std::max<size_t>(F, 1) * sizeof(double2));
-  if (e == cudaSuccess) e = cudaMalloc(&B.ixf, std::max<size_t>(2 * (size_t)F, 1) * sizeof(FixedAxis));
+  cudaError_t e = block_alloc(&B.perm, std::max<unsigned long long>(total, 1) * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = block_alloc(&B.cstart, ((size_t)ncells + 1) * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = block_alloc(&B.cbase, (F + 1) * sizeof(uint32_t), s);
+  if (e == cudaSuccess) e = block_alloc(&B.ixg, std::max<size_t>(F, 1) * sizeof(uint4), s);
+  if (e == cudaSuccess) e = block_alloc(&B.ixs, std::max<size_t>(F, 1) * sizeof(double2), s);
+  if (e == cudaSuccess) e = block_alloc(&B.ixq, std::max<size_t>(F, 1) * sizeof(double2), s);
+  if (e == cudaSuccess) e = block_alloc(&B.ixf, std::max<size_t>(2 * (size_t)F, 1) * sizeof(FixedAxis), s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixs, ixs.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixq, ixq.data(), F * sizeof(double2), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixf, ixf.data(), 2 * (size_t)F * sizeof(FixedAxis), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.cbase, cbase.data(), (F + 1) * sizeof(uint32_t), cudaMemcpyHostToDevice, s);
   if (e == cudaSuccess) e = cudaMemcpyAsync(B.ixg, ixg.data(), F * sizeof(uint4), cudaMemcpyHostToDevice, s);
   if (e != cudaSuccess) return e;
-  if (e == cudaSuccess) e = cudaMalloc(&B.pend, std::max<unsigned long long>(total, 1) * sizeof(uint16_t));
+  if (e == cudaSuccess) e = block_alloc(&B.pend, std::max<unsigned long long>(total, 1) * sizeof(uint16_t), s);
   if (e != cudaSuccess) return e;
   uint32_t *const *sk = L.sk;
   uint32_t shift = 0;  // of the cell ids in the sorted keys (sk[2])
@@ -1041,13 +1044,13 @@ stc_status lsm_store_block(const LsmDev &L, LsmHost &H, cudaStream_t s, std::str
   B.info = H.info;
   B.ctfs = H.ctfs;
   const size_t F = L.F, no = (size_t)H.info.oversize_kv_count;
-  cudaError_t e = cudaMalloc(&B.keys, H.info.key_bytes + 32);
-  if (e == cudaSuccess) e = cudaMalloc(&B.d_ctfs, F * sizeof(stc_ctf));
-  if (e == cudaSuccess) e = cudaMalloc(&B.bitmaps, F * STC_BITMAP_BYTES);
-  if (e == cudaSuccess) e = cudaMalloc(&B.sids, (size_t)L.N * sizeof(uint16_t));
-  if (e == cudaSuccess) e = cudaMalloc(&B.orec, std::max<size_t>(no, 1) * sizeof(uint4));
-  if (e == cudaSuccess) e = cudaMalloc(&B.obox, std::max<size_t>(no, 1) * sizeof(float4));
-  if (e == cudaSuccess) e = cudaMalloc(&B.obitmap, STC_MAP_BITMAP_BYTES(L.edge));
+  cudaError_t e = block_alloc(&B.keys, H.info.key_bytes + 32, s);
+  if (e == cudaSuccess) e = block_alloc(&B.d_ctfs, F * sizeof(stc_ctf), s);
+  if (e == cudaSuccess) e = block_alloc(&B.bitmaps, F * STC_BITMAP_BYTES, s);
+  if (e == cudaSuccess) e = block_alloc(&B.sids, (size_t)L.N * sizeof(uint16_t), s);
+  if (e == cudaSuccess) e = block_alloc(&B.orec, std::max<size_t>(no, 1) * sizeof(uint4), s);
+  if (e == cudaSuccess) e = block_alloc(&B.obox, std::max<size_t>(no, 1) * sizeof(float4), s);
+  if (e == cudaSuccess) e = block_alloc(&B.obitmap, STC_MAP_BITMAP_BYTES(L.edge), s);
   if (e == cudaSuccess) e = cudaMemsetAsync(B.keys + H.info.key_bytes, 0, 32, s);
   if (e == cudaSuccess && H.info.key_bytes)
     e = cudaMemcpyAsync(B.keys, L.kbytes, H.info.key_bytes, cudaMemcpyDeviceToDevice, s);

@@ -113,12 +113,41 @@ __global__ void k_scan_down(const uint32_t *in, uint32_t *out, size_t n, const u
   }
 }
 
+// The whole scan by one block, for up to SCAN_ONE words: a radix pass of a
+// few tens of thousands of items has a few thousand, and the three launches
+// above take 8 us whatever their number (60k objects in a flush: 40 passes).
+static constexpr size_t SCAN_ONE = 16 * 1024;
+__global__ void __launch_bounds__(1024) k_scan_one(const uint32_t *in, uint32_t *out, uint32_t n,
+                                                   unsigned long long *total) {
+  constexpr int PER = SCAN_ONE / 1024;
+  const uint32_t per = (n + 1023) / 1024, base = threadIdx.x * per;
+  uint32_t v[PER];
+  uint32_t s = 0;
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
+    v[i] = i < per && base + i < n ? in[base + i] : 0u;
+    s += v[i];
+  }
+  uint32_t tot;
+  uint32_t off = block_excl_scan(s, &tot);
+#pragma unroll
+  for (int i = 0; i < PER; i++) {
+    if (i < per && base + i < n) out[base + i] = off;
+    off += v[i];
+  }
+  if (threadIdx.x == 0 && total) *total = tot;
+}
+
 size_t scan_tmp_words(size_t n) { return (n + SCAN_TILE - 1) / SCAN_TILE + 1; }
 
 void exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, unsigned long long *total, uint32_t *tmp,
                         cudaStream_t s) {
   if (n == 0) {
     if (total) cudaMemsetAsync(total, 0, sizeof(unsigned long long), s);
+    return;
+  }
+  if (n <= SCAN_ONE) {
+    STC_KL k_scan_one<<<1, 1024, 0, s>>>(in, out, (uint32_t)n, total);
     return;
   }
   size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;

@@ -6,7 +6,70 @@
 
 namespace stc {
 void set_thread_error(const std::string &msg);
+
+static constexpr int POOL_DEVICES = 64;
+static std::mutex g_pool_mutex;
+static cudaMemPool_t g_pool[POOL_DEVICES] = {};
+
+// The current device's pool, made by the first call that asks; null without
+// one (allocations are then plain).
+static cudaMemPool_t device_pool(bool make) {
+  int dev = 0;
+  if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= POOL_DEVICES) return nullptr;
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (!g_pool[dev] && make) {
+    cudaMemPoolProps props = {};
+    props.allocType = cudaMemAllocationTypePinned;
+    props.location.type = cudaMemLocationTypeDevice;
+    props.location.id = dev;
+    unsigned long long keep = POOL_KEEP_BYTES;
+    cudaMemPool_t pool = nullptr;
+    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
+        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
+      g_pool[dev] = pool;
+    else
+      cudaGetLastError();
+  }
+  return g_pool[dev];
 }
+
+cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
+  *p = nullptr;
+  cudaMemPool_t pool = device_pool(true);
+  if (!pool) return dev_malloc(p, bytes);
+  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pool_trim();
+    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  }
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    *p = nullptr;
+  }
+  return e;
+}
+
+void pool_free(void *p, cudaStream_t s) {
+  if (!p) return;
+  if (device_pool(false)) cudaFreeAsync(p, s);
+  else cudaFree(p);
+}
+
+void pool_trim() {
+  if (cudaMemPool_t pool = device_pool(false)) cudaMemPoolTrimTo(pool, 0);
+}
+
+cudaError_t dev_malloc(void **p, size_t bytes) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e == cudaErrorMemoryAllocation) {
+    cudaGetLastError();
+    pool_trim();
+    e = cudaMalloc(p, bytes);
+  }
+  return e;
+}
+}  // namespace stc
 
 using namespace stc;
 
@@ -53,14 +116,18 @@ extern "C" stc_status stc_sort_pairs_u32(const uint32_t *keys, const uint32_t *v
   stc_status st = sort_args_ok(keys, values, keys_out, values_out, n, key_bits, "stc_sort_pairs_u32");
   if (st != STC_OK || n == 0) return st;
   cudaError_t e = cudaSetDevice((int)device);
+  const size_t hw = radix_hist_words(n), sw = scan_tmp_words(hw);
+  CallScratch sc(0, 4ull * (2 * n + hw + sw));
   uint32_t *ktmp = nullptr, *vtmp = nullptr, *hist = nullptr, *scan = nullptr;
   unsigned long long *n_dev = nullptr;
-  size_t hw = radix_hist_words(n);
-  if (e == cudaSuccess) e = cudaMalloc(&ktmp, n * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&vtmp, n * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&hist, hw * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&scan, scan_tmp_words(hw) * 4);
-  if (e == cudaSuccess) e = cudaMalloc(&n_dev, sizeof(unsigned long long));
+  if (e == cudaSuccess) {
+    ktmp = sc.get<uint32_t>(n);
+    vtmp = sc.get<uint32_t>(n);
+    hist = sc.get<uint32_t>(hw);
+    scan = sc.get<uint32_t>(sw);
+    n_dev = sc.get<unsigned long long>(1);
+    e = sc.error();
+  }
   if (e == cudaSuccess) {
     SortTimer tm;
     STC_KL k_set_count<<<1, 1, 0, 0>>>(n_dev, (unsigned long long)n);
@@ -71,11 +138,6 @@ extern "C" stc_status stc_sort_pairs_u32(const uint32_t *keys, const uint32_t *v
     if (e == cudaSuccess) e = cudaStreamSynchronize(0);
     if (e == cudaSuccess) tm.read();
   }
-  cudaFree(ktmp);
-  cudaFree(vtmp);
-  cudaFree(hist);
-  cudaFree(scan);
-  cudaFree(n_dev);
   if (e != cudaSuccess) {
     set_thread_error(std::string("stc_sort_pairs_u32: ") + cudaGetErrorString(e));
     return STC_ERR_CUDA;
