@@ -450,7 +450,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
             dalloc(c, &p.bu_gid, p.U_cap) && dalloc(c, &p.bu_pid, p.U_cap) && dalloc(c, &p.bu_rank, p.U_cap) &&
             dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, p.G) && dalloc(c, &p.bu_start, p.G) &&
             dalloc(c, &p.slots, p.B) &&
-            dalloc(c, &p.hits, (size_t)p.nb * p.bin_cap) && dalloc(c, &p.bin_cnt, p.nb) &&
+            dalloc(c, &p.hits, hit_records(p.nb, p.bin_cap)) && dalloc(c, &p.bin_cnt, p.nb) &&
             dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.occ, (size_t)p.nb * OCC_WORDS) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
             dalloc(c, &p.carry_cnt, p.runs) && dalloc(c, &p.cset, p.C) &&
             dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E);
@@ -709,7 +709,7 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
   if (c->cfg.hit_capacity || need <= p.bin_cap) return;
   const uint32_t cap = bin_share(need, 1, 5, 4, 16);
   void *h = nullptr;
-  if (dev_malloc(&h, (size_t)p.nb * cap * sizeof(HitRec)) != cudaSuccess) {
+  if (dev_malloc(&h, hit_records(p.nb, cap) * sizeof(HitRec)) != cudaSuccess) {
     cudaGetLastError();
     return;
   }

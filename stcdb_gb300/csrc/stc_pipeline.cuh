@@ -92,10 +92,10 @@ struct PipeDev {
   uint32_t *bu_cnt, *bu_start;          // G
   // meetings
   Slot *slots;                          // B
-  // hits of the step, binned by table tile (tile_of): bin j holds records
-  // [j * bin_cap, j * bin_cap + min(bin_cnt[j], bin_cap)); a hit its bin has
-  // no room for is applied inside the pair tests
-  HitRec *hits;
+  // hits of the step, binned by table tile (tile_of): bin j holds
+  // min(bin_cnt[j], bin_cap) records, at hit_place; a hit its bin has no room
+  // for is applied inside the pair tests
+  HitRec *hits;                         // hit_records(nb, bin_cap)
   uint32_t nb, bin_cap;                 // tiles of the table, records per bin
   unsigned long long nb_magic;          // ceil(2^64 / nb)
   uint32_t *bin_cnt;                    // nb
@@ -107,6 +107,20 @@ struct PipeDev {
   uint32_t *cand_list;                  // cand_cap
   stc_meeting *emit;                    // E
 };
+
+// Place of record i of bin j: bins are cut into chunks of HIT_CHUNK records, the
+// first chunks of all bins come first, then the second ones. The bins fill at
+// much the same pace, so the step writes to a few hundred MB at a time and not
+// to all of the buffer: scattered stores are bound by the reach of the address
+// translation (67.7M records into 349526 bins, with their counters: 36 G/s bin
+// after bin, 2.8 GB; 52 with chunks of 16; 80 if all went to 180 MB).
+constexpr uint32_t HIT_CHUNK = 16;
+__host__ __device__ __forceinline__ unsigned long long hit_place(const PipeDev &p, uint32_t j, uint32_t i) {
+  return ((unsigned long long)(i / HIT_CHUNK) * p.nb + j) * HIT_CHUNK + i % HIT_CHUNK;
+}
+inline size_t hit_records(uint32_t nb, uint32_t bin_cap) {
+  return (size_t)nb * ((bin_cap + HIT_CHUNK - 1) / HIT_CHUNK * HIT_CHUNK);
+}
 
 // stc_partition.cu
 // the descent (leaf of every object), the leaves' members in strip order with

@@ -158,7 +158,7 @@ __device__ __forceinline__ void bin_hit(const PipeDev &p, const HitRec &h, uint3
   const unsigned long long key = stc_cantor(h.a, h.b);
   const uint32_t bin = tile_of(p, fast_mod(key, p.B, p.B_magic));
   const uint32_t pos = atomicAdd(&p.bin_cnt[bin], 1u);
-  if (pos < p.bin_cap) store_hit(&p.hits[(unsigned long long)bin * p.bin_cap + pos], h);
+  if (pos < p.bin_cap) store_hit(&p.hits[hit_place(p, bin, pos)], h);
   else if (p.st->packed == TABLE_SLOTS) process_hit(p, h, t);
   else p.st->redo = 1;
 }
@@ -228,8 +228,8 @@ struct __align__(16) Row {
 // the longest of 32 has several times that, and with a row per lane 17 of 32
 // lanes had work. The tests alone, without records: 1.15 ms of a 10M-object
 // step (93.6M tests, 67.7M hits); with the bins' counters 1.55, with the
-// records' stores 2.85: bound by L2's rate of scattered 32-byte stores (39 G/s
-// measured, 35 with an atomic each). A row per lane and a shared-memory queue
+// records' stores 2.85, or 2.4 in chunks (hit_place): bound by the rate of
+// scattered stores over that many pages (52 G/s measured). A row per lane and a shared-memory queue
 // of records before it: 3.0 ms for the tests with sequential records.
 // REDO: every hit is applied to the table at once, nothing is binned; the
 // schema is not read, which its update may be rewriting.
@@ -446,10 +446,9 @@ __global__ void __launch_bounds__(256) k_hits(PipeDev p) {
     const uint32_t bin = (uint32_t)(w / parts), i = (uint32_t)(w % parts) * 64 + lane_id();
     const uint32_t n = min(p.bin_cnt[bin], p.bin_cap);
     if (i >= n) continue;
-    const HitRec *hits = p.hits + (unsigned long long)bin * p.bin_cap;
     const bool two = i + 32 < n;
-    const HitRec h0 = load_hit(&hits[i]);
-    const HitRec h1 = load_hit(&hits[two ? i + 32 : i]);
+    const HitRec h0 = load_hit(&p.hits[hit_place(p, bin, i)]);
+    const HitRec h1 = load_hit(&p.hits[hit_place(p, bin, two ? i + 32 : i)]);
     const unsigned long long k0 = stc_cantor(h0.a, h0.b), k1 = stc_cantor(h1.a, h1.b);
     const unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
     const U128 kv0 = load_slot_pair(&p.slots[s0]), kv1 = load_slot_pair(&p.slots[s1]);

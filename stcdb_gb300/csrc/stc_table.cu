@@ -95,7 +95,7 @@ __device__ __forceinline__ const HitRec *run_record(const PipeDev &p, uint32_t r
   const uint32_t seq = id / p.bin_cap;
   uint32_t tile = r0 + seq;
   if (tile >= p.nb) tile -= p.nb;
-  return p.hits + (unsigned long long)tile * p.bin_cap + (id - seq * p.bin_cap);
+  return p.hits + hit_place(p, tile, id - seq * p.bin_cap);
 }
 
 __device__ __forceinline__ uint32_t smem_addr(const void *p) { return (uint32_t)__cvta_generic_to_shared(p); }
@@ -112,9 +112,8 @@ __device__ __forceinline__ uint32_t packed_at(uint32_t layout, uint32_t len, uin
 __device__ __forceinline__ uint32_t tile_fetch(const PipeDev &p, Tile &s, uint32_t tile, unsigned long long start,
                                                uint32_t len, uint32_t n, uint32_t turn, uint32_t layout) {
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
-  const HitRec *bin = p.hits + (unsigned long long)tile * p.bin_cap;
   for (uint32_t i = threadIdx.x; i < min(n, TB_RECS); i += TB_THREADS)
-    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(&s.rec[i])), "l"(bin + i) : "memory");
+    asm volatile("cp.async.cg.shared.global [%0], [%1], 16;" ::"r"(smem_addr(&s.rec[i])), "l"(p.hits + hit_place(p, tile, i)) : "memory");
   const uint32_t w = lane < OCC_WORDS ? s.bits[lane] : 0u;
   uint32_t incl = __popc(w);
 #pragma unroll
@@ -151,8 +150,8 @@ __device__ __forceinline__ uint32_t bin_hits(const PipeDev &p, uint32_t tile) {
 
 // The tile being worked on, as every thread sees it.
 struct TileView {
-  const HitRec *bin;         // the tile's bin
   unsigned long long start;  // its first slot
+  uint32_t tile;
   uint32_t n, nc;            // its hits, hits carried in
   uint32_t r0, id0;          // the run's first bin, the place of this bin's first hit
   uint32_t len, turn;        // slots, the tile's number in its run
@@ -160,7 +159,7 @@ struct TileView {
 
 // Record of hit i of the tile (i < n: its own, then the ones carried in).
 __device__ __forceinline__ const HitRec *tile_rec(const PipeDev &p, const Tile &s, const TileView &v, uint32_t i) {
-  return i < v.n ? v.bin + i : run_record(p, v.r0, s.carry[v.turn & 1u][i - v.n]);
+  return i < v.n ? p.hits + hit_place(p, v.tile, i) : run_record(p, v.r0, s.carry[v.turn & 1u][i - v.n]);
 }
 
 // Its pair (a | b << 32) and order.
@@ -404,7 +403,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_BLOCKS_PER_SM) k_table_halo(Pip
     v.n = bin_hits(p, tile);
     v.nc = min(s.ncarry[q % 3], TILE_LOAD);
     v.id0 = q * p.bin_cap;
-    v.bin = p.hits + (unsigned long long)tile * p.bin_cap;
+    v.tile = tile;
     if (tid < OCC_WORDS) s.bits[tid] = p.occ[(size_t)tile * OCC_WORDS + tid];
     __syncthreads();
     tile_fetch(p, s, tile, v.start, v.len, v.n, q, layout);
@@ -457,7 +456,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_BLOCKS_PER_SM) k_table(PipeDev 
   for (uint32_t tile = first; tile < last; tile++) {
     v.turn = tile - first;
     v.id0 = (halo + v.turn) * p.bin_cap;
-    v.bin = p.hits + (unsigned long long)tile * p.bin_cap;
+    v.tile = tile;
     v.nc = min(s.ncarry[v.turn % 3], TILE_LOAD);
     // the next tile's count and occupied slots, on their way beside the hits
     const uint32_t next_n = tile + 1 < last ? bin_hits(p, tile + 1) : 0u;
