@@ -105,8 +105,9 @@ typedef struct stc_config {
    * arrival). */
   uint32_t job_chunk;            /* refinement jobs (32 rows against their candidate ranges) a warp
                                     takes at a time, fewer when there are too few to go round;
-                                    0 = 8, at most 64 */
-  uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 = 8, at most 32 */
+                                    0 = 8, or one at a time by demand where that is faster;
+                                    at most 64 */
+  uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 = 8 or 12, at most 32 */
   uint32_t hits_blocks_per_sm;   /* blocks per SM of the general table update (a step whose table tiles
                                     are too full for the tiled one); 0 = 16, at most 64 */
   uint32_t window_graphs;        /* stc_step_window replays each step from a captured CUDA graph:

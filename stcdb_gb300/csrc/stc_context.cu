@@ -401,10 +401,11 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   p.grid_capacity = k.grid_capacity;
   p.delay = k.schema_update_delay;
   p.mbr_filter = k.mbr_filter;
-  p.slices = std::min<uint32_t>(std::max<uint32_t>(k.step_slices, 1u), 64u);
+  p.slices = std::min<uint32_t>(std::max<uint32_t>(k.step_slices, 1u), MAX_SLICES);
   p.job_chunk = k.job_chunk ? std::min<uint32_t>(k.job_chunk, 64u) : 8u;
+  p.job_share = 0;
   p.refine_chunk = k.refine_chunk ? k.refine_chunk : REFINE_CHUNK_DEFAULT;
-  p.refine_bps = k.refine_blocks_per_sm ? std::min<uint32_t>(k.refine_blocks_per_sm, 32u) : 8u;
+  p.refine_bps = k.refine_blocks_per_sm ? std::min<uint32_t>(k.refine_blocks_per_sm, 32u) : 0u;
   p.hits_bps = k.hits_blocks_per_sm ? std::min<uint32_t>(k.hits_blocks_per_sm, 64u) : 16u;
 
   p.leaves_max = std::min(p.G, n);
@@ -728,7 +729,11 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
 // pair tests end with a few warps in the longest jobs, so the tiles are as
 // short as they go (32: hotspot window of 300k objects, 10k row blocks, 0.68
 // ms of pair tests and table update with 256, 0.47 with 64, 0.39 with 32; at
-// 24k row blocks all lengths are within 2%). Otherwise 64 candidates when the
+// 24k row blocks all lengths are within 2%), half that where some
+// units have several tests (four on average) but all tests fewer than FEW_TESTS, seven
+// rounds a resident warp (20k objects in hotspots, 0.28M tests, 0.046 -> 0.035
+// ms; 60k, 2.9M tests: the same; 100k uniform, 0.015M: 0.024 -> 0.027).
+// Otherwise 64 candidates when the
 // last step tested more than 16 candidates per checking unit (dense leaves
 // have long candidate windows, and 256-long tiles left the tail of the pair
 // tests to a few warps: hotspot-1M 8.46 -> 6.18 ms a step), else 256
@@ -736,19 +741,25 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
 // Results do not depend on it.
 static constexpr unsigned long long SHORT_TILE_TESTS_PER_UNIT = 16;
 static constexpr unsigned long long FEW_ROW_BLOCKS = 4;
+static constexpr unsigned long long FEW_TESTS = 1ull << 20;
 static void choose_refine_chunk(stc_ctx *c) {
   PipeDev &p = c->p;
   uint32_t chunk = c->cfg.refine_chunk;
   if (!chunk) {
     const DevState &st = *c->st_host;  // the last step's counters
     const unsigned long long units = (unsigned long long)p.N + st.border_units;
-    if (units / 32 < FEW_ROW_BLOCKS * 32 * (unsigned long long)num_sms()) chunk = 32u;
-    else chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * units ? 64u : REFINE_CHUNK_DEFAULT;
+    if (units / 32 < FEW_ROW_BLOCKS * 32 * (unsigned long long)num_sms())
+      chunk = st.tests > 4 * units && st.tests < FEW_TESTS ? REFINE_CHUNK_FEW / 2 : REFINE_CHUNK_FEW;
+    else
+      chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * units ? REFINE_CHUNK_DENSE : REFINE_CHUNK_DEFAULT;
   }
-  if (chunk != p.refine_chunk) {
-    p.refine_chunk = chunk;
-    invalidate_graphs(c);  // the captured steps carry the tile length
-  }
+  const uint32_t chunk0 = p.refine_chunk, share0 = p.job_share;
+  p.refine_chunk = chunk;
+  // by the last step's jobs; a quarter fewer before it changes back
+  const unsigned long long jobs = c->st_host->jobs_total;
+  const unsigned long long warps = (unsigned long long)num_sms() * refine_blocks(p) * (REFINE_THREADS / 32);
+  p.job_share = !c->cfg.job_chunk && job_shares(share0 ? jobs + jobs / 4 : jobs, warps, chunk);
+  if (chunk != chunk0 || p.job_share != share0) invalidate_graphs(c);  // the captured steps carry both
 }
 
 static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copied) {
@@ -1418,7 +1429,7 @@ extern "C" stc_status stc_read_block(stc_ctx *c, uint32_t index, stc_ctf *ctfs, 
 extern "C" stc_status stc_set_step_slices(stc_ctx *c, uint32_t slices) {
   if (!c) return STC_ERR_INVALID_ARG;
   c->cfg.step_slices = slices;
-  c->p.slices = std::min<uint32_t>(std::max<uint32_t>(slices, 1u), 64u);
+  c->p.slices = std::min<uint32_t>(std::max<uint32_t>(slices, 1u), MAX_SLICES);
   invalidate_graphs(c);
   return STC_OK;
 }

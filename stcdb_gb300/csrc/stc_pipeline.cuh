@@ -22,12 +22,14 @@ struct __align__(16) LeafGeo {
 };
 
 // counters of a step (PipeDev::ctr)
-enum { CTR_MEMBERS = 0, CTR_SMALL, CTR_BIG, CTR_EXTRA, CTR_UNITS, CTR_POOL, CTR_COUNT };
+constexpr uint32_t MAX_SLICES = 64;  // of a long step kernel (stc_config.step_slices)
+enum { CTR_MEMBERS = 0, CTR_SMALL, CTR_BIG, CTR_EXTRA, CTR_UNITS, CTR_POOL, CTR_JOBS, CTR_COUNT = CTR_JOBS + MAX_SLICES };
 
 // Candidate positions per refinement job and lane: a row block's candidate
 // ranges are cut into chunks of this many, so that the n^2 / 2 pair tests of
 // a dense leaf spread over many warps.
 constexpr uint32_t REFINE_CHUNK_DEFAULT = 256;  // tile length before the first step's density is known
+constexpr uint32_t REFINE_CHUNK_DENSE = 64, REFINE_CHUNK_FEW = 32;  // of dense leaves, of few rows (choose_refine_chunk)
 
 struct PipeDev {
   // sizes
@@ -47,8 +49,9 @@ struct PipeDev {
   int mbr_filter;
   uint32_t slices;                 // launches per long step kernel (stc_config.step_slices)
   uint32_t job_chunk;              // refinement jobs a warp takes at a time (stc_config.job_chunk)
+  uint32_t job_share;              // 1: or one at a time from a common counter (job_shares)
   uint32_t refine_chunk;               // candidate positions per refinement job (a multiple of 32)
-  uint32_t refine_bps, hits_bps;   // blocks per SM of the pair tests and of the table update
+  uint32_t refine_bps, hits_bps;   // blocks per SM of the pair tests (0: step_pairs chooses) and of the table update
   // state
   DevState *st;
   SchemaDev sd;
@@ -120,6 +123,26 @@ __host__ __device__ __forceinline__ unsigned long long hit_place(const PipeDev &
 }
 inline size_t hit_records(uint32_t nb, uint32_t bin_cap) {
   return (size_t)nb * ((bin_cap + HIT_CHUNK - 1) / HIT_CHUNK * HIT_CHUNK);
+}
+
+// Blocks an SM of the pair tests: three for each that it holds at once where
+// the last warps are a larger part of the time (few rows, short tiles: 300k
+// objects, half of them in hotspots, 0.46 -> 0.43 ms a step), else two.
+constexpr uint32_t REFINE_THREADS = 256;
+inline uint32_t refine_blocks(const PipeDev &p) {
+  return p.refine_bps ? p.refine_bps : p.refine_chunk <= REFINE_CHUNK_FEW ? 12u : 8u;
+}
+
+// Whether warps take their jobs one by one from a common counter: `jobs` to
+// take by `warps`. Dense leaves lie together, and with all jobs dealt out
+// beforehand a fifth of the SMs' time was the wait for the last warps; asking
+// costs more than that where a warp has few jobs, or a dozen short ones (long
+// tiles: few candidates a job). ms of pair tests, dealt out and by demand: 10M
+// uniform (47 jobs a warp) 2.38, 2.13; hotspot-1M (short tiles) 1.40, 1.22; the
+// stress model 1.89, 1.66; 3M uniform (14 jobs a warp) 0.28, 0.31; 60k in
+// hotspots 0.119, 0.126.
+inline bool job_shares(unsigned long long jobs, unsigned long long warps, uint32_t chunk) {
+  return jobs >= (chunk <= REFINE_CHUNK_DENSE ? 8ull : 24ull) * warps;
 }
 
 // stc_partition.cu

@@ -46,7 +46,6 @@
 
 namespace stc {
 
-static constexpr int REFINE_THREADS = 256;
 
 __device__ __forceinline__ double dpml_fast_r(double lat) {
   double absla = fabs(lat);
@@ -459,9 +458,13 @@ __global__ void __launch_bounds__(256) k_hits(PipeDev p) {
 }
 
 // Slice `part` of `parts` runs jobs [J * part / parts, J * (part + 1) / parts),
-// up to p.job_chunk at a time; fewer when there are too few to go round: eight
-// dense jobs of one leaf in one warp were the whole kernel's tail (20k objects
-// in hotspots: 0.23 -> 0.06 ms a quarter).
+// dealt out beforehand, up to p.job_chunk at a time; fewer when there are too
+// few to go round: eight dense jobs of one leaf in one warp were the whole
+// kernel's tail (20k objects in hotspots: 0.23 -> 0.06 ms a quarter). SHARE
+// (job_share): a warp takes its next job from a common counter instead, and a
+// quarter more than its share at most, so that blocks still end, and let query
+// batches in, during the kernel.
+template <bool SHARE>
 __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint32_t part, uint32_t parts) {
   __shared__ Row rows_all[REFINE_THREADS / 32][32];
   Row *rows = rows_all[threadIdx.x >> 5];
@@ -471,17 +474,25 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
   const unsigned long long J = p.st->jobs_total;
   const unsigned long long J0 = J * part / parts, J1 = J * (part + 1) / parts;
   const unsigned long long each = (J1 - J0) / nwarps;
-  const unsigned long long jc = each >= p.job_chunk ? p.job_chunk : (each ? each : 1ull);
+  const unsigned long long jc = SHARE || !each ? 1ull : each >= p.job_chunk ? p.job_chunk : each;
+  const unsigned long long quota = each + each / 4 + 2;
   Counters ct = {0, 0, 0, 0};
-  for (unsigned long long j0 = J0 + warp * jc; j0 < J1; j0 += nwarps * jc) {
+  unsigned long long taken = 0;
+  for (unsigned long long j0 = J0 + warp * jc; j0 < J1;) {
     // one lane reads the flag so that the whole warp leaves together
     if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
+    unsigned long long next = j0 + nwarps * jc;
+    if (SHARE) {  // asked for ahead of the job at hand
+      next = J1;
+      if (++taken < quota && lane_id() == 0) next = J0 + nwarps + atomicAdd(&p.ctr[CTR_JOBS + part], 1ull);
+    }
     const unsigned long long j1 = j0 + jc < J1 ? j0 + jc : J1;
     for (unsigned long long job = j0; job < j1; job++) {
       const uint4 w = p.jobs[job];
       for (uint32_t c = 0; c < w.w; c++)
         run_rows<false>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
     }
+    j0 = SHARE ? __shfl_sync(0xffffffffu, next, 0) : next;
   }
   // reduce counters per warp (64-bit sums)
   unsigned long long tests = ct.tests, exact = ct.exact, hits = ct.hits, amb = ct.amb;
@@ -501,8 +512,11 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
 }
 
 void step_pairs(PipeDev &p, cudaStream_t s) {
-  for (uint32_t part = 0; part < p.slices; part++)
-    STC_KL k_refine_a<<<num_sms() * p.refine_bps, REFINE_THREADS, 0, s>>>(p, part, p.slices);
+  for (uint32_t part = 0; part < p.slices; part++) {
+    const unsigned blocks = num_sms() * refine_blocks(p);
+    if (p.job_share) STC_KL k_refine_a<true><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
+    else STC_KL k_refine_a<false><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
+  }
 }
 
 void step_hits(PipeDev &p, cudaStream_t s) {
