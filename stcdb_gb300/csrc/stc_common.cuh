@@ -220,6 +220,29 @@ int num_sms();
 // Prefix for every kernel launch statement: `STC_KL k<<<g, b, 0, s>>>(...);`
 #define STC_KL ::stc::tl_launches++,
 
+// Launches a kernel behind the one before it in the stream, without the gap
+// between them: its blocks are set up as that one's last blocks end, and wait
+// for all of it in after_previous(), which every kernel launched this way
+// calls first. A step of 20k objects is 21 short launches: 0.204 -> 0.186 ms;
+// 100k 0.142 -> 0.122, 700k 0.291 -> 0.279. (Letting the next kernel's blocks in
+// from this one's start holds up its side streams: 700k 0.293, 10M 6.3 -> 6.6.)
+template <typename... K, typename... A>
+inline void launch_behind(void (*kernel)(K...), unsigned grid, unsigned block, size_t smem, cudaStream_t s, A... args) {
+  cudaLaunchAttribute at[1];
+  at[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  at[0].val.programmaticStreamSerializationAllowed = 1;
+  cudaLaunchConfig_t c = {};
+  c.gridDim = dim3(grid);
+  c.blockDim = dim3(block);
+  c.dynamicSmemBytes = smem;
+  c.stream = s;
+  c.attrs = at;
+  c.numAttrs = 1;
+  ::stc::tl_launches++;
+  cudaLaunchKernelEx(&c, kernel, K(args)...);
+}
+__device__ __forceinline__ void after_previous() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+
 // Primitives implemented in stc_sort.cu.
 #define STC_SCAN_TILE 2048  // items per scan block
 #define STC_RS_TILE 4096    // items per radix-sort block

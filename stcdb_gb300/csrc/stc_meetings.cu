@@ -102,6 +102,7 @@ void init_tables(PipeDev &p, cudaStream_t s) {
 // Candidates that may occur twice in a step: walk with their minimum
 // priority once all instances are merged.
 __global__ void k_insert_ordered(PipeDev p) {
+  after_previous();
   const bool fused = fuse_halo(p) != 0;
   if (blockIdx.x == 0 && threadIdx.x == 0)  // what the tiled update, or the general path, leaves
     p.st->packed = !fused ? TABLE_SLOTS : p.st->packed == TABLE_FRONT ? TABLE_BACK : TABLE_FRONT;
@@ -128,7 +129,7 @@ __global__ void k_insert_ordered(PipeDev p) {
   }
 }
 
-void step_insert(PipeDev &p, cudaStream_t s) { STC_KL k_insert_ordered<<<num_sms() * 4, 256, 0, s>>>(p); }
+void step_insert(PipeDev &p, cudaStream_t s) { launch_behind(k_insert_ordered, num_sms() * 4, 256, 0, s, p); }
 
 // Sweep (tracing/meeting.cpp:32-76, cuda/geometry.cu:595-736).
 
@@ -255,6 +256,7 @@ __device__ __forceinline__ void flush_emits(const PipeDev &p, const stc_meeting 
 
 // Slice `part` of `parts` sweeps slots [B * part / parts, B * (part + 1) / parts).
 __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(PipeDev p, uint32_t part, uint32_t parts) {
+  after_previous();
   if (fuse_halo(p)) return;
   const uint32_t t = p.st->step_t;
   __shared__ __align__(16) stc_meeting stage_all[SWEEP_WARPS][WARP_STAGE];
@@ -332,7 +334,7 @@ void step_sweep(PipeDev &p, cudaStream_t s) {
       (unsigned long long)num_sms() * SWEEP_BLOCKS_PER_SM * SWEEP_WAVES,
       p.B / (4 * SWEEP_WARPS * WARP_TILE) + 1);
   for (uint32_t part = 0; part < p.slices; part++)
-    STC_KL k_sweep<<<blocks, SWEEP_THREADS, 0, s>>>(p, part, p.slices);
+    launch_behind(k_sweep, blocks, SWEEP_THREADS, 0, s, p, part, p.slices);
 }
 
 }  // namespace stc

@@ -62,6 +62,7 @@ __device__ __forceinline__ long long word_pair(uint32_t lo, uint32_t hi) {
 // in double 0.77 ms; one load a level 0.60, from the cell's start in double
 // 0.71 (both bound by FP64, some 20 operations a point); this form 0.31.
 __global__ void __launch_bounds__(256) k_descend(PipeDev p) {
+  after_previous();
   uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x;
   if (pid >= p.N) return;
   double2 q;
@@ -198,6 +199,7 @@ __device__ __forceinline__ LeafGeo leaf_geo(const PipeDev &p, uint32_t g, uint32
 
 // A range of the member list for each leaf, and its geometry.
 __global__ void __launch_bounds__(256) k_leaf_alloc(PipeDev p) {
+  after_previous();
   __shared__ BlockTake s;
   const uint32_t ids = p.sd.high[1];
   for (uint32_t g0 = blockIdx.x * blockDim.x; g0 < ids; g0 += gridDim.x * blockDim.x) {
@@ -221,6 +223,7 @@ __global__ void __launch_bounds__(256) k_leaf_alloc(PipeDev p) {
 }
 
 __global__ void __launch_bounds__(256) k_leaf_scatter(PipeDev p) {
+  after_previous();
   const uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x;
   if (pid >= p.N) return;
   const uint32_t g = p.leaf_gid[pid];
@@ -330,6 +333,7 @@ __device__ const uint32_t *kept_members(const PipeDev &p, uint32_t base, uint32_
 // whatever the object count, 0.57 ms at 10M objects and 0.42 for the gather
 // before it; this form 8 us and 0.44 for both.)
 __global__ void __launch_bounds__(LEAF_SMALL / 2, 12) k_leaf_small(PipeDev p) {
+  after_previous();
   constexpr uint32_t T = LEAF_SMALL / 2;
   __shared__ uint32_t start[STRIPS_MAX + 2], hist[256], var[3], longest;
   __shared__ float sx[LEAF_SMALL], fx[LEAF_SMALL];  // offsets in (strip, arrival) and in final order
@@ -411,6 +415,7 @@ __global__ void __launch_bounds__(LEAF_SMALL / 2, 12) k_leaf_small(PipeDev p) {
 
 // Larger leaves: a block of 512 each, members in device memory.
 __global__ void __launch_bounds__(512) k_leaf_big(PipeDev p) {
+  after_previous();
   constexpr uint32_t T = 512;
   __shared__ uint32_t start[STRIPS_MAX + 2], hist[256], var[3], longest;
   __shared__ JobHead head;
@@ -699,6 +704,7 @@ __global__ void __launch_bounds__(TILE / 4, 4096 / TILE) k_border_count(PipeDev 
 
 // The units in the reference's order, and each unit's number within its leaf.
 __global__ void __launch_bounds__(256) k_border_fill(PipeDev p) {
+  after_previous();
   const uint32_t pid = blockIdx.x * blockDim.x + threadIdx.x;
   if (pid == 0 && p.st->border_units >= p.U_cap) stc_set_error(p.st, ERR_UNITS, (uint32_t)p.st->border_units);
   if (pid >= p.N) return;
@@ -724,6 +730,7 @@ __global__ void __launch_bounds__(256) k_border_fill(PipeDev p) {
 // 32 units against one chunk of refine_chunk positions of the leaf's members
 // (a unit's ranges hold at most all of them).
 __global__ void __launch_bounds__(256) k_border_alloc(PipeDev p) {
+  after_previous();
   __shared__ BlockTake s;
   __shared__ uint32_t split;
   const uint32_t lane = lane_id(), ids = p.sd.high[1];
@@ -764,19 +771,20 @@ __global__ void __launch_bounds__(256) k_border_alloc(PipeDev p) {
 }
 
 __global__ void __launch_bounds__(256) k_border_scatter(PipeDev p) {
+  after_previous();
   const unsigned long long n = p.st->border_units < p.U_cap ? p.st->border_units : 0ull;
   for (unsigned long long u = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; u < n;
        u += (unsigned long long)gridDim.x * blockDim.x)
     p.bu_sorted_pos[p.bu_start[p.bu_gid[u]] + p.bu_rank[u]] = (uint32_t)u;
 }
 
-void step_descend(PipeDev &p, cudaStream_t s) { STC_KL k_descend<<<nblk(p.N), 256, 0, s>>>(p); }
+void step_descend(PipeDev &p, cudaStream_t s) { launch_behind(k_descend, nblk(p.N), 256, 0, s, p); }
 
 void step_leaves(PipeDev &p, cudaStream_t s) {
-  STC_KL k_leaf_alloc<<<std::min<unsigned>(nblk(p.G), num_sms() * 4), 256, 0, s>>>(p);
-  STC_KL k_leaf_scatter<<<nblk(p.N), 256, 0, s>>>(p);
-  STC_KL k_leaf_small<<<num_sms() * 12, LEAF_SMALL / 2, 0, s>>>(p);
-  if (p.leaf_cap > LEAF_SMALL) STC_KL k_leaf_big<<<num_sms() * 2, 512, 0, s>>>(p);
+  launch_behind(k_leaf_alloc, std::min<unsigned>(nblk(p.G), num_sms() * 4), 256, 0, s, p);
+  launch_behind(k_leaf_scatter, nblk(p.N), 256, 0, s, p);
+  launch_behind(k_leaf_small, num_sms() * 12, LEAF_SMALL / 2, 0, s, p);
+  if (p.leaf_cap > LEAF_SMALL) launch_behind(k_leaf_big, num_sms() * 2, 512, 0, s, p);
 }
 
 void step_border(PipeDev &p, cudaStream_t s) {
@@ -784,9 +792,9 @@ void step_border(PipeDev &p, cudaStream_t s) {
   if (p.border_tile == 1024) STC_KL k_border_count<1024><<<tiles, 256, 0, s>>>(p);
   else STC_KL k_border_count<256><<<tiles, 64, 0, s>>>(p);
   scan_sums_u32(p.bsum, tiles, &p.st->border_units, s);
-  STC_KL k_border_fill<<<nblk(p.N), 256, 0, s>>>(p);
-  STC_KL k_border_alloc<<<std::min<unsigned>(nblk(p.G), num_sms() * 4), 256, 0, s>>>(p);
-  STC_KL k_border_scatter<<<std::min<unsigned>(nblk(p.N), num_sms() * 16), 256, 0, s>>>(p);
+  launch_behind(k_border_fill, nblk(p.N), 256, 0, s, p);
+  launch_behind(k_border_alloc, std::min<unsigned>(nblk(p.G), num_sms() * 4), 256, 0, s, p);
+  launch_behind(k_border_scatter, std::min<unsigned>(nblk(p.N), num_sms() * 16), 256, 0, s, p);
 }
 
 }  // namespace stc

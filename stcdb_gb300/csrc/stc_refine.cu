@@ -431,6 +431,7 @@ __device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows) {
 // per hit, two hits in flight per thread (both records and both home slots
 // are requested before either is used).
 __global__ void __launch_bounds__(256) k_hits(PipeDev p) {
+  after_previous();
   if (fuse_halo(p)) return;
   __shared__ Row rows_all[256 / 32][32];
   if (p.st->redo) {
@@ -521,7 +522,7 @@ void step_pairs(PipeDev &p, cudaStream_t s) {
 
 void step_hits(PipeDev &p, cudaStream_t s) {
   const unsigned most = std::max<unsigned>(p.nb, 4 * num_sms());
-  STC_KL k_hits<<<std::min<unsigned>(num_sms() * p.hits_bps, most), 256, 0, s>>>(p);
+  launch_behind(k_hits, std::min<unsigned>(num_sms() * p.hits_bps, most), 256, 0, s, p);
 }
 
 }  // namespace stc

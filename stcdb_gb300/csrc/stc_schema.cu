@@ -628,6 +628,7 @@ __device__ void replay_serial(const SchemaDev &sd, uint32_t *grid_count, const u
 // collects the flags of nodes [t * per, (t + 1) * per).
 __global__ void __launch_bounds__(1024) k_schema_phase2(SchemaDev sd, SchemaWork w, uint32_t *grid_count, uint32_t cap,
                                                         uint32_t delay, int serial_only, DevState *st) {
+  after_previous();
   __shared__ int warp_sum[32];
   const uint32_t tid = threadIdx.x, high = sd.high[0];
   const uint32_t per = ((high + 1023) / 1024 + 15) / 16 * 16;
@@ -659,6 +660,7 @@ __global__ void __launch_bounds__(1024) k_schema_phase2(SchemaDev sd, SchemaWork
 }
 
 __global__ void __launch_bounds__(256) k_schema_walk(SchemaDev sd) {
+  after_previous();
   const uint32_t high = sd.high[0];
   for (uint32_t i = blockIdx.x * blockDim.x + threadIdx.x; i < high; i += gridDim.x * blockDim.x) {
     const NodeMeta m = sd.meta[i];
@@ -691,6 +693,7 @@ __global__ void __launch_bounds__(256) k_schema_walk(SchemaDev sd) {
 // child: the descent compares each coordinate with the split points alone, so
 // every point between them takes it too.
 __global__ void __launch_bounds__(256) k_schema_start(SchemaDev sd) {
+  after_previous();
   const uint32_t i = blockIdx.x * blockDim.x + threadIdx.x, E = sd.start_edge;
   if (i >= E * E) return;
   const double cx = 1.0 / (double)sd.start_sx, cy = 1.0 / (double)sd.start_sy;
@@ -708,15 +711,15 @@ __global__ void __launch_bounds__(256) k_schema_start(SchemaDev sd) {
 }
 
 void schema_walk(SchemaDev sd, cudaStream_t s) {
-  STC_KL k_schema_walk<<<std::min<unsigned>(nblk(sd.S), num_sms() * 4), 256, 0, s>>>(sd);
-  STC_KL k_schema_start<<<nblk((size_t)sd.start_edge * sd.start_edge), 256, 0, s>>>(sd);
+  launch_behind(k_schema_walk, std::min<unsigned>(nblk(sd.S), num_sms() * 4), 256, 0, s, sd);
+  launch_behind(k_schema_start, nblk((size_t)sd.start_edge * sd.start_edge), 256, 0, s, sd);
 }
 
 void update_schema(SchemaDev sd, SchemaWork w, uint32_t *grid_count, double reach, uint32_t grid_capacity,
                    uint32_t delay, int serial_only, DevState *st, cudaStream_t s) {
   STC_KL k_schema_phase1<<<std::min<unsigned>(nblk(sd.S), num_sms() * 4), 256, 0, s>>>(
       sd, grid_count, reach, grid_capacity, delay, w.ev_flag, w.old_under);
-  STC_KL k_schema_phase2<<<1, 1024, 0, s>>>(sd, w, grid_count, grid_capacity, delay, serial_only, st);
+  launch_behind(k_schema_phase2, 1, 1024, 0, s, sd, w, grid_count, grid_capacity, delay, serial_only, st);
   schema_walk(sd, s);
 }
 

@@ -65,6 +65,7 @@ __device__ uint32_t block_excl_scan(uint32_t v, uint32_t *total) {
 }
 
 __global__ void k_scan_reduce(const uint32_t *in, size_t n, uint32_t *sums) {
+  after_previous();
   size_t base = (size_t)blockIdx.x * SCAN_TILE;
   uint32_t s = 0;
 #pragma unroll
@@ -78,6 +79,7 @@ __global__ void k_scan_reduce(const uint32_t *in, size_t n, uint32_t *sums) {
 }
 
 __global__ void k_scan_sums(uint32_t *sums, size_t nb, unsigned long long *total) {
+  after_previous();
   // one block of 1024 threads, each owns a contiguous chunk
   size_t per = (nb + blockDim.x - 1) / blockDim.x;
   size_t b0 = (size_t)threadIdx.x * per, b1 = b0 + per < nb ? b0 + per : nb;
@@ -94,6 +96,7 @@ __global__ void k_scan_sums(uint32_t *sums, size_t nb, unsigned long long *total
 }
 
 __global__ void k_scan_down(const uint32_t *in, uint32_t *out, size_t n, const uint32_t *sums) {
+  after_previous();
   size_t base = (size_t)blockIdx.x * SCAN_TILE + (size_t)threadIdx.x * SCAN_ITEMS;
   uint32_t v[SCAN_ITEMS];
   uint32_t s = 0;
@@ -119,6 +122,7 @@ __global__ void k_scan_down(const uint32_t *in, uint32_t *out, size_t n, const u
 static constexpr size_t SCAN_ONE = 16 * 1024;
 __global__ void __launch_bounds__(1024) k_scan_one(const uint32_t *in, uint32_t *out, uint32_t n,
                                                    unsigned long long *total) {
+  after_previous();
   constexpr int PER = SCAN_ONE / 1024;
   const uint32_t per = (n + 1023) / 1024, base = threadIdx.x * per;
   uint32_t v[PER];
@@ -147,17 +151,17 @@ void exclusive_scan_u32(const uint32_t *in, uint32_t *out, size_t n, unsigned lo
     return;
   }
   if (n <= SCAN_ONE) {
-    STC_KL k_scan_one<<<1, 1024, 0, s>>>(in, out, (uint32_t)n, total);
+    launch_behind(k_scan_one, 1, 1024, 0, s, in, out, (uint32_t)n, total);
     return;
   }
   size_t nb = (n + SCAN_TILE - 1) / SCAN_TILE;
-  STC_KL k_scan_reduce<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, n, tmp);
-  STC_KL k_scan_sums<<<1, 1024, 0, s>>>(tmp, nb, total);
-  STC_KL k_scan_down<<<(unsigned)nb, SCAN_THREADS, 0, s>>>(in, out, n, tmp);
+  launch_behind(k_scan_reduce, (unsigned)nb, SCAN_THREADS, 0, s, in, n, tmp);
+  launch_behind(k_scan_sums, 1, 1024, 0, s, tmp, nb, total);
+  launch_behind(k_scan_down, (unsigned)nb, SCAN_THREADS, 0, s, in, out, n, tmp);
 }
 
 void scan_sums_u32(uint32_t *sums, size_t nb, unsigned long long *total, cudaStream_t s) {
-  STC_KL k_scan_sums<<<1, 1024, 0, s>>>(sums, nb, total);
+  launch_behind(k_scan_sums, 1u, 1024u, 0, s, sums, nb, total);
 }
 
 // ---------------------------------------------------------------------------
@@ -176,6 +180,7 @@ size_t radix_hist_words(size_t n_max) { return 256 * ((n_max + RS_TILE - 1) / RS
 
 __global__ void k_rs_hist(const uint32_t *keys, const unsigned long long *n_dev, size_t n_max, int shift,
                           uint32_t dmask, uint32_t *hist, uint32_t nb) {
+  after_previous();
   __shared__ uint32_t h[256];
   h[threadIdx.x] = 0;
   __syncthreads();
@@ -248,6 +253,7 @@ __global__ void __launch_bounds__(RS_THREADS, 3) k_rs_scatter(const uint32_t *k_
                                                            uint32_t *k_out, uint32_t *v_out,
                                                            const unsigned long long *n_dev, size_t n_max, int shift,
                                                            uint32_t dmask, const uint32_t *hist, uint32_t nb) {
+  after_previous();
   __shared__ uint2 s_kv[RS_TILE];     // the tile in digit order
   __shared__ uint32_t base_off[256];  // output position of tile position i of digit d, less i
   // per warp and digit: counts, then the tile position of the warp's first item of the digit
@@ -336,9 +342,9 @@ void radix_sort_u32(const uint32_t *k_in, const uint32_t *v_in, uint32_t *k_out,
     // the last digit covers only the key bits that remain
     int left = bits - 8 * p;
     uint32_t dmask = left >= 8 ? 255u : (1u << left) - 1u;
-    STC_KL k_rs_hist<<<nb, RS_THREADS, 0, s>>>(ki, n_dev, n_max, 8 * p, dmask, hist, nb);
+    launch_behind(k_rs_hist, nb, RS_THREADS, 0, s, ki, n_dev, n_max, 8 * p, dmask, hist, nb);
     exclusive_scan_u32(hist, hist, (size_t)256 * nb, nullptr, scan_tmp, s);
-    STC_KL k_rs_scatter<<<nb, RS_THREADS, 0, s>>>(ki, vi, ko, vo, n_dev, n_max, 8 * p, dmask, hist, nb);
+    launch_behind(k_rs_scatter, nb, RS_THREADS, 0, s, ki, vi, ko, vo, n_dev, n_max, 8 * p, dmask, hist, nb);
     ki = ko;
     vi = vo;
   }

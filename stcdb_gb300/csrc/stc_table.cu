@@ -360,6 +360,7 @@ __device__ void tile_unpack(const PipeDev &p, Slot *slots, uint32_t tile, uint32
 // The largest bin and the largest (occupied slots + hits) of a tile, which
 // decide the step's path (fuse_halo).
 __global__ void __launch_bounds__(256) k_table_plan(PipeDev p) {
+  after_previous();
   uint32_t load = 0, most = 0;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb; j += gridDim.x * blockDim.x) {
     const uint32_t c = p.bin_cnt[j];
@@ -377,6 +378,7 @@ __global__ void __launch_bounds__(256) k_table_plan(PipeDev p) {
 // What is carried into each run: the halo tiles before it, worked through
 // with nothing carried into them. Writes nothing but the carry lists.
 __global__ void __launch_bounds__(TB_THREADS, TB_BLOCKS_PER_SM) k_table_halo(PipeDev p) {
+  after_previous();
   extern __shared__ __align__(128) unsigned char smem[];
   Tile &s = *(Tile *)smem;
   const uint32_t halo = fuse_halo(p), layout = p.st->packed;
@@ -421,6 +423,7 @@ __global__ void __launch_bounds__(TB_THREADS, TB_BLOCKS_PER_SM) k_table_halo(Pip
 // One block per run. Part `part` of `parts` works runs
 // [runs * part / parts, runs * (part + 1) / parts).
 __global__ void __launch_bounds__(TB_THREADS, TB_BLOCKS_PER_SM) k_table(PipeDev p, uint32_t part, uint32_t parts) {
+  after_previous();
   extern __shared__ __align__(128) unsigned char smem[];
   Tile &s = *(Tile *)smem;
   const uint32_t halo = fuse_halo(p), layout = p.st->packed;
@@ -643,15 +646,15 @@ void unpack_tiles(PipeDev &p, uint32_t layout, cudaStream_t s) {
 }
 
 void step_table_plan(PipeDev &p, cudaStream_t s) {
-  STC_KL k_table_plan<<<std::min<unsigned>((p.nb + 255) / 256, (unsigned)num_sms() * 2), 256, 0, s>>>(p);
-  STC_KL k_table_halo<<<p.runs, TB_THREADS, sizeof(Tile), s>>>(p);
+  launch_behind(k_table_plan, std::min<unsigned>((p.nb + 255) / 256, (unsigned)num_sms() * 2), 256, 0, s, p);
+  launch_behind(k_table_halo, p.runs, TB_THREADS, sizeof(Tile), s, p);
 }
 
 void step_table(PipeDev &p, cudaStream_t s) {
   for (uint32_t part = 0; part < p.slices; part++) {
     const uint32_t n = (uint32_t)((unsigned long long)p.runs * (part + 1) / p.slices -
                                   (unsigned long long)p.runs * part / p.slices);
-    if (n) STC_KL k_table<<<n, TB_THREADS, sizeof(Tile), s>>>(p, part, p.slices);
+    if (n) launch_behind(k_table, n, TB_THREADS, sizeof(Tile), s, p, part, p.slices);
   }
 }
 
