@@ -632,13 +632,16 @@ __device__ uint32_t border_lookup(const PipeDev &p, uint32_t pid, uint32_t lv, u
 #define BORDER_KEEP 4
 
 // Border units of the points of a block's TILE pids: their lookups packed
-// together, then each point's offset within the block. TILE / 4 threads.
-template <uint32_t TILE>
-__global__ void __launch_bounds__(TILE / 4, 4096 / TILE) k_border_count(PipeDev p) {
-  constexpr uint32_t T = TILE / 4;
+// together, then each point's offset within the block. T threads: a quarter of
+// TILE where that fills the GPU, TILE where all points have room for a thread
+// of their own at once (a lookup is a chain of dependent loads, and a dense
+// crowd's tile has two or three a thread: the wait for the border units of 20k objects in
+// hotspots 43 -> 25 us a step, of 60k 41 -> 14).
+template <uint32_t TILE, uint32_t T>
+__global__ void __launch_bounds__(T, 1024 / T) k_border_count(PipeDev p) {
   __shared__ __align__(16) uint32_t cnts[TILE];
   __shared__ uint16_t list[TILE];
-  __shared__ uint32_t nlist, warp_sum[T / 32];
+  __shared__ uint32_t nlist, warp_sum[TILE / 128];
   const uint32_t tid = threadIdx.x, lane = lane_id(), first = blockIdx.x * TILE;
   if (tid == 0) nlist = 0;
   __syncthreads();
@@ -677,7 +680,8 @@ __global__ void __launch_bounds__(TILE / 4, 4096 / TILE) k_border_count(PipeDev 
   }
   __syncthreads();
   // four consecutive points a thread
-  const uint4 c = ((const uint4 *)cnts)[tid];
+  uint4 c = make_uint4(0, 0, 0, 0);
+  if (tid < TILE / 4) c = ((const uint4 *)cnts)[tid];
   const uint32_t sum = c.x + c.y + c.z + c.w;
   uint32_t incl = sum;
 #pragma unroll
@@ -685,8 +689,9 @@ __global__ void __launch_bounds__(TILE / 4, 4096 / TILE) k_border_count(PipeDev 
     const uint32_t up = __shfl_up_sync(0xffffffffu, incl, d);
     if ((int)lane >= d) incl += up;
   }
-  if (lane == 31) warp_sum[tid >> 5] = incl;
+  if (lane == 31 && tid < TILE / 4) warp_sum[tid >> 5] = incl;
   __syncthreads();
+  if (tid >= TILE / 4) return;
   uint32_t before = incl - sum;
   for (uint32_t w = 0; w < (tid >> 5); w++) before += warp_sum[w];
   const uint32_t pid = first + 4 * tid;
@@ -699,7 +704,7 @@ __global__ void __launch_bounds__(TILE / 4, 4096 / TILE) k_border_count(PipeDev 
     }
     before += cc[k];
   }
-  if (tid == T - 1) p.bsum[blockIdx.x] = before;
+  if (tid == TILE / 4 - 1) p.bsum[blockIdx.x] = before;
 }
 
 // The units in the reference's order, and each unit's number within its leaf.
@@ -789,8 +794,9 @@ void step_leaves(PipeDev &p, cudaStream_t s) {
 
 void step_border(PipeDev &p, cudaStream_t s) {
   const unsigned tiles = nblk(p.N, p.border_tile);
-  if (p.border_tile == 1024) STC_KL k_border_count<1024><<<tiles, 256, 0, s>>>(p);
-  else STC_KL k_border_count<256><<<tiles, 64, 0, s>>>(p);
+  if (p.border_tile == 1024) STC_KL k_border_count<1024, 256><<<tiles, 256, 0, s>>>(p);
+  else if (p.N > num_sms() * 1024u) STC_KL k_border_count<256, 64><<<tiles, 64, 0, s>>>(p);
+  else STC_KL k_border_count<256, 256><<<tiles, 256, 0, s>>>(p);
   scan_sums_u32(p.bsum, tiles, &p.st->border_units, s);
   launch_behind(k_border_fill, nblk(p.N), 256, 0, s, p);
   launch_behind(k_border_alloc, std::min<unsigned>(nblk(p.G), num_sms() * 4), 256, 0, s, p);
