@@ -83,10 +83,6 @@ __device__ __forceinline__ unsigned long long key_fields(unsigned __int128 k, co
   return vm;
 }
 
-__device__ void decode_key(unsigned __int128 k, const stc_ctf &c, Key &o) {
-  exact_box(key_fields(k, c, o), c, o.box);
-}
-
 __device__ __forceinline__ bool time_ok(uint32_t start, uint32_t end, uint32_t t1, uint32_t t2) {
   return start < t2 && t1 < end;  // util/query_context.h:100-103
 }
@@ -134,6 +130,51 @@ __device__ __forceinline__ void oversize_key(const QBlock &b, unsigned long long
 
 // ---- object queries ----------------------------------------------------------
 
+// The reference's binary search for the first of `n` sorted oids equal to pid
+// (go on to the left of an equal one), -1 if there is none; oid_at(i) reads
+// one. By the whole warp, five levels a round: each lane reads one of the 31
+// positions that the next five comparisons can ask for, so the search takes a
+// fifth of the dependent loads and visits what the one-by-one search visits
+// (k_query_object with one thread searching: 68 us for 1.2k queries over four
+// blocks of 0.6M keys; now 23, without the boxes of counted contacts).
+template <typename Oid>
+__device__ __forceinline__ long long first_of(long long n, uint32_t pid, Oid oid_at) {
+  const uint32_t lane = lane_id();
+  long long low = 0, high = n - 1, find = -1;
+  // the bounds that node h of the comparisons' tree is asked with
+  auto bounds = [&](uint32_t h, long long &lo, long long &hi) {
+    lo = low;
+    hi = high;
+    for (int b = 30 - __clz((int)h); b >= 0 && lo <= hi; b--) {
+      const long long mid = lo + (hi - lo) / 2;
+      if ((h >> b) & 1u) lo = mid + 1;
+      else hi = mid - 1;
+    }
+  };
+  while (low <= high) {
+    long long lo = 1, hi = 0;
+    if (lane) bounds(lane, lo, hi);
+    const bool valid = lo <= hi;
+    const long long mid = lo + (hi - lo) / 2;
+    uint32_t oid = 0;
+    if (valid) oid = oid_at(mid);
+    const uint32_t there = __ballot_sync(0xffffffffu, valid);
+    const uint32_t right = __ballot_sync(0xffffffffu, valid && oid < pid);
+    const uint32_t equal = __ballot_sync(0xffffffffu, valid && oid == pid);
+    uint32_t h = 1, last = 0;
+    while (h < 32 && ((there >> h) & 1u)) {
+      if ((equal >> h) & 1u) last = h;
+      h = 2 * h + ((right >> h) & 1u);
+    }
+    const long long found = __shfl_sync(0xffffffffu, mid, last);
+    if (last) find = found;
+    bounds(h, lo, hi);
+    low = lo;
+    high = hi;
+  }
+  return find;
+}
+
 __global__ void __launch_bounds__(QOBJ_THREADS) k_query_object(const QBlock *qb, const stc_query *qs,
                                                               QueryRec *out, unsigned long long cap,
                                                               unsigned long long *count,
@@ -147,46 +188,28 @@ __global__ void __launch_bounds__(QOBJ_THREADS) k_query_object(const QBlock *qb,
   __shared__ unsigned long long s_lim, s_bad;
   __shared__ uint32_t s_ctf;
   const uint32_t pid = q.pid;
-  if (threadIdx.x == 0) {
-    s_find = -1;
-    s_lim = 0;
-    s_ctf = b.F;
-    uint16_t sid = b.sids[pid];
+  if (threadIdx.x < 32) {
+    long long find = -1;
+    unsigned long long lim = 0;
+    uint32_t ctf = b.F;
+    const uint16_t sid = b.sids[pid];
     if (sid == 1) {
       // oversize_buffer::search_buffer (tracing/step_merge.cpp:65-110)
-      long long low = 0, high = (long long)b.n_over - 1;
-      while (low <= high) {
-        long long mid = (low + high) / 2;
-        uint32_t p = b.orec[mid].x;
-        if (p == pid) { s_find = mid; high = mid - 1; }
-        else if (p > pid) high = mid - 1;
-        else low = mid + 1;
-      }
-      s_lim = b.n_over;
+      find = first_of((long long)b.n_over, pid, [&](long long i) { return b.orec[i].x; });
+      lim = b.n_over;
     } else if (sid >= 2 && (uint32_t)sid - 2 < b.F) {
       // CTF::binary_search (tracing/step_merge.cpp:496-521)
-      const uint32_t c = sid - 2;
-      const stc_ctf &t = b.ctfs[c];
+      ctf = sid - 2;
+      const stc_ctf &t = b.ctfs[ctf];
       const uint32_t kb = t.key_bit / 8u;
       const uint8_t *base = b.keys + t.key_offset;
-      uint32_t low = 0, high = t.kv_count - 1;
-      while (low <= high) {
-        unsigned long long mid = low + (unsigned long long)(high - low) / 2;
-        if (mid >= t.kv_count) break;
-        uint32_t oid = key_oid(load_key(base + mid * kb, kb), t);
-        if (oid == pid) {
-          s_find = (long long)mid;
-          if (mid == 0) break;
-          high = (uint32_t)mid - 1;
-        } else if (oid < pid) {
-          low = (uint32_t)mid + 1;
-        } else {
-          if (mid == 0) break;
-          high = (uint32_t)mid - 1;
-        }
-      }
-      s_lim = t.kv_count;
-      s_ctf = c;
+      find = first_of((long long)t.kv_count, pid, [&](long long i) { return key_oid(load_key(base + i * kb, kb), t); });
+      lim = t.kv_count;
+    }
+    if (threadIdx.x == 0) {
+      s_find = find;
+      s_lim = lim;
+      s_ctf = ctf;
     }
   }
   __syncthreads();
@@ -211,12 +234,14 @@ __global__ void __launch_bounds__(QOBJ_THREADS) k_query_object(const QBlock *qb,
       } else {
         const stc_ctf &t = b.ctfs[c];
         Key k;
-        decode_key(load_key(b.keys + t.key_offset + i * (t.key_bit / 8u), t.key_bit / 8u), t, k);
+        const unsigned long long vm =
+            key_fields(load_key(b.keys + t.key_offset + i * (t.key_bit / 8u), t.key_bit / 8u), t, k);
+        if (!count_only) exact_box(vm, t, k.box);  // hundreds of cycles of FP64 a warp
         match = k.oid == pid;
         target = k.target;
         end = k.end + t.end_time_min;
         start = end - k.duration;
-        box[0] = k.box[0]; box[1] = k.box[1]; box[2] = k.box[2]; box[3] = k.box[3];
+        if (!count_only) box[0] = k.box[0], box[1] = k.box[1], box[2] = k.box[2], box[3] = k.box[3];
       }
     }
     if (!match) atomicMin(&s_bad, i);
@@ -438,7 +463,7 @@ __global__ void k_set_one(unsigned long long *p, unsigned long long v) { *p = v;
 // over a crowd go to k_box_pieces, a warp a piece. (A warp a row, each
 // finding its pair by binary search and computing the pair's ranges in double,
 // took 2.35 ms for 2048 queries, 0.8k of them boxes, over four blocks of 0.6M
-// keys; now plan 59 us, rows 153, pieces 66.)
+// keys; now plan 59 us, rows 50, pieces 54.)
 
 constexpr uint32_t OV_CHUNK = 2048;       // oversize keys per work item
 constexpr uint32_t SEQ_BITMAP_CELLS = 1024;  // larger windows skip the per-thread bitmap test
@@ -532,7 +557,7 @@ __device__ __forceinline__ int level_rows(int j0, int j1, uint32_t g, uint32_t l
 // Most keys to decode, and most end offsets to compare, that one item keeps
 // (up to 32 rows of fewer than 32 or 256 each come on top), and the pieces that
 // the ranges of a fuller one are cut into.
-constexpr uint32_t ITEM_KEYS = 1024, PIECE_KEYS = 512, ITEM_ENDS = 8192, PIECE_ENDS = 4096;
+constexpr uint32_t ITEM_KEYS = 512, PIECE_KEYS = 256, ITEM_ENDS = 1024, PIECE_ENDS = 1024;
 constexpr size_t PIECE_CAP = 1 << 18;
 constexpr uint32_t PLAN_COUNT_ONLY = 1u, PLAN_ALL_ENDS = 2u;
 
@@ -782,7 +807,7 @@ __global__ void __launch_bounds__(QBOX_THREADS) k_box_rows(const QBlock *qb, con
       if (all_ends) mine += me2 - ma;
       // An item over a crowd goes to other warps: a few such held k_box_rows
       // for 1.78 ms with the SMs 28% active (2048 queries over four blocks of
-      // 0.6M keys).
+      // 0.6M keys), 0.15 ms when items kept up to 1024 keys and 8192 ends.
       const uint32_t scan = __reduce_add_sync(0xffffffffu, (ma - a) + (e - me2));
       const uint32_t ends = __reduce_add_sync(0xffffffffu, all_ends ? 0u : me2 - ma);
       if (scan > ITEM_KEYS) {
