@@ -630,19 +630,15 @@ def kernel_bytes(s, N, B, prev_live=None):
     """Algorithmic bytes per launch of the step's kernels.
     partition: 36 N (read positions, write leaf-ordered points, id map)
     refine:    16 N + 16 H + 32 per hit (its record, written)
-    sweep:     the table update and sweep: 32 B per hit record and per table
-               slot read, 32 B per slot it writes (each meeting extended or
-               started this step, each one not hit cleared) + 64 B per emitted
-               meeting. A meeting stays live only when hit, so the cleared
-               ones are the previous step's live meetings less this step's
-               extensions (hits - new); `prev_live` defaults to this step's
-               live count."""
+    sweep:     the table update and sweep: 32 B per hit record and per meeting
+               of the step before read, 32 B per meeting that goes on or
+               starts written, a bit per table slot read and written + 64 B
+               per emitted meeting; `prev_live` defaults to this step's live
+               count."""
     H, Q = s.border_units, s.hits
-    new = s.new_candidates
     prev = s.taken_buckets if prev_live is None else prev_live
-    cleared = max(prev - (Q - new), 0)
     return {"partition": 36.0 * N, "refine": 16.0 * N + 16.0 * H + 32.0 * Q,
-            "sweep": 32.0 * B + 32.0 * (Q + s.taken_buckets + cleared) + 64.0 * s.emitted}
+            "sweep": 32.0 * (Q + prev + s.taken_buckets) + B / 4.0 + 64.0 * s.emitted}
 
 
 FLUSH_STAGES = ("object_order", "key_sort", "ctf_limits", "encode", "store_and_index")

@@ -1178,6 +1178,10 @@ stc_status lsm_query_reserve(LsmHost &H, size_t nq, uint32_t F, int priority, st
     if (e == cudaSuccess && !Q.ev1) e = cudaEventCreate(&Q.ev1);
     if (e == cudaSuccess) e = query_buffers(H, Q, nq, F);
   }
+  // the pool's first use makes it, 3 ms that the first flush would take
+  void *first = nullptr;
+  if (e == cudaSuccess) e = pool_alloc(&first, 1 << 20, H.lanes[0].stream);
+  pool_free(first, H.lanes[0].stream);
   // load the query kernels now: with lazy module loading their first launch
   // would load them then, which waits for a step in flight
   cudaFuncAttributes fa;
