@@ -80,7 +80,7 @@ WORKLOADS = {
     # pair-test and 32 table-update blocks per SM: 15.12 -> 14.80 ms a step);
     # it does not change results
     "uniform-10M": dict(objects=10_000_000, hot=0, reach=10.0, min_meet=5, grid_capacity=200, amplify=2.0,
-                        buckets=1 << 28, kv_restriction=1 << 27, refine_bps=4, hits_bps=32),
+                        buckets=1 << 28, kv_restriction=1 << 27),
     "hotspot-1M": dict(objects=1_000_000, hot=1000, reach=10.0, min_meet=5, grid_capacity=200, amplify=8.0,
                        buckets=1 << 28, kv_restriction=1 << 27),
     # the hotspot model at larger object counts (live pairs grow with N^2)
@@ -621,9 +621,10 @@ def max_over_ranks(args, v):
 
 # DRAM bytes (read + write) of the table update and sweep (k_table) per
 # algorithmic byte, from an ncu capture on the 3M-object workload
-# (profiles/kernels_table_uniform-3M.md): 2.348 GB read and 0.296 GB written
-# for 2.636 GB of table slots, hit records and changed slots.
-TABLE_DRAM_PER_BYTE = (2.348 + 0.296) / 2.636
+# (profiles/kernels_table_uniform-3M.md): 0.409 GB read and 0.180 GB written
+# for 0.609 GB of hit records, meetings, slot marks and emitted meetings (L2
+# still holds some of the records).
+TABLE_DRAM_PER_BYTE = (0.409 + 0.180) / 0.609
 
 
 def kernel_bytes(s, N, B, prev_live=None):
@@ -995,8 +996,8 @@ def main():
                     "sigma_m": w.get("sigma_m", 300.0) if w["hot"] else None,
                     "reach_m": w["reach"], "min_meet_steps": w["min_meet"],
                     "leaf_capacity": w["grid_capacity"], "grid_amplify": w["amplify"],
-                    "launch_shape": {"refine_blocks_per_sm": w.get("refine_bps", 8),
-                                     "hits_blocks_per_sm": w.get("hits_bps", 16),
+                    "launch_shape": {"refine_blocks_per_sm": w.get("refine_bps", 0),  # 0: the library's choice
+                                     "hits_blocks_per_sm": w.get("hits_bps", 0),
                                      "refine_chunk": w.get("refine_chunk") or "by density (32, 64 or 256)"},
                     "meeting_buckets": make_cfg(w).resolved().num_meeting_buckets,
                     "memtable": (f"on, flush past {w['kv_restriction']} directed keys, 100 CTFs, "

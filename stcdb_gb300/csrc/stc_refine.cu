@@ -3,7 +3,7 @@
 // Work: every leaf's n kept members (the first leaf_cap in pid order,
 // tracing/filter.cpp:100-104) are ordered by horizontal strips at least
 // reach tall and, within small strips, by longitude (stc_partition.cu,
-// k_strip_order). The reference tests every own-leaf pair (pid < q,
+// k_leaf_small). The reference tests every own-leaf pair (pid < q,
 // tracing/refinement.cpp:30) and every (border unit, member) pair of the
 // leaf (tracing/filter.cpp:248-259); a pair more than a strip apart, or
 // farther apart in longitude than the leaf's window wx, is farther than
@@ -215,7 +215,7 @@ struct __align__(16) Row {
 };
 
 // One job: 32 rows of leaf g, each against its candidate ranges of members
-// in (strip, longitude) order (stc_partition.cu, k_strip_order). Rows are
+// in (strip, longitude) order (stc_partition.cu, k_leaf_small). Rows are
 // the leaf's own members (own = true; row i tests the members after it in
 // its strip up to its longitude window's end, and its window in the next
 // strip, so every pair of members within reach is tested once) or 32 border

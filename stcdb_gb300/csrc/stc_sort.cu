@@ -1,7 +1,7 @@
 // Device-wide exclusive scan and stable LSD radix sort (hand-written; no
 // CUB/thrust). The reference sorts with thrust::sort_by_key
-// (cuda/geometry.cu:1809-1907); here the partition step uses these kernels
-// to group object ids by quadtree leaf in pid order.
+// (cuda/geometry.cu:1809-1907); here the flush, the compaction and the query
+// index do with these kernels, and the border lookup with the scan's.
 #include <atomic>
 
 #include "stc_common.cuh"
