@@ -50,12 +50,13 @@ __device__ __forceinline__ unsigned long long tile_start(const PipeDev &p, uint3
 
 // Halo tiles the tiled table update (stc_table.cu) needs this step, or 0:
 // the step takes the general path (k_hits, k_insert_ordered, k_sweep).
-constexpr uint32_t MAX_HALO = 7;
+constexpr uint32_t MAX_HALO = 15;
+constexpr uint32_t MIN_TILES = 14;  // a smaller table is not worth tiles
 __device__ __forceinline__ uint32_t fuse_halo(const PipeDev &p) {
-  if (p.nb < 2 * MAX_HALO || p.st->hit_max > p.bin_cap) return 0;
+  if (p.nb < MIN_TILES || p.st->hit_max > p.bin_cap) return 0;
   const unsigned long long c = p.st->tile_load, T = p.B / p.nb;
   if (c >= TILE_LOAD) return 0;  // the carry lists hold TILE_LOAD hits
-  for (uint32_t h = 1; h <= MAX_HALO; h++)
+  for (uint32_t h = 1; h <= MAX_HALO && 2 * h <= p.nb; h++)
     if (c * (h + 1) < T * h) return h;
   return 0;
 }

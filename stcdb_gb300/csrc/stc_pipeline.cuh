@@ -160,7 +160,7 @@ void step_hits(PipeDev &p, cudaStream_t s);
 // step takes it and finds what is carried into each run of tiles.
 constexpr uint32_t TILE_SLOTS = 768;    // largest tile
 constexpr uint32_t OCC_WORDS = TILE_SLOTS / 32;
-constexpr uint32_t TILE_LOAD = 576;     // (occupied slots + hits) of a tile stay below this on the tiled path
+constexpr uint32_t TILE_LOAD = 704;     // (occupied slots + hits) of a tile stay below this on the tiled path
 cudaError_t table_prepare();
 void table_sizes(PipeDev &p);           // nb and runs of a table of p.B slots
 void count_tiles(PipeDev &p, cudaStream_t s);
