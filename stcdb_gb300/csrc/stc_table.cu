@@ -2,8 +2,8 @@
 // meetings and the expire/emit sweep in one pass over the meeting table.
 // Before and after, one GB300, per step: 10M uniform objects (2^28 slots,
 // 67.7M hits, 36.7M of them new) 8.4 ms of pair tests with the update beside
-// them and 2.7 of sweep -> 2.7 ms of pair tests and 2.5 of k_table;
-// hotspot-1M (34.7M hits) 4.0 + 1.9 -> 1.5 + 1.8 ms. Bound by instruction
+// them and 2.7 of sweep -> 2.0 ms of pair tests and 2.6 of k_table;
+// hotspot-1M (34.7M hits) 4.0 + 1.9 -> 1.15 + 1.6 ms. Bound by instruction
 // issue (60% of the slots in a tile's chain of short phases; DRAM at 30%).
 //
 // The pair tests leave the step's hits binned by table tile (TILE_SLOTS
