@@ -752,7 +752,7 @@ __global__ void __launch_bounds__(256) k_border_alloc(PipeDev p) {
     }
     // units, row blocks, jobs beyond one per row block; the block's leaves are
     // cut into chunks together, or not at all
-    const uint32_t v[3] = {m, rows, rows * (chunks - 1)};
+    const uint32_t v[3] = {m, rows, jobs_beyond(rows, chunks, p.jobs_extra)};
     unsigned long long at[3];
     block_take(v, at, s, [&](const uint32_t (&sum)[3]) {
       s.base[0] = sum[0] ? atomicAdd(&p.ctr[CTR_UNITS], (unsigned long long)sum[0]) : 0ull;

@@ -1,6 +1,7 @@
 // Device buffers of one pipeline context and the per-step launchers.
 #pragma once
 #include "stc_common.cuh"
+#include "stc_rules.cuh"
 #include "stc_schema.cuh"
 
 namespace stc {
