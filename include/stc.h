@@ -563,14 +563,26 @@ void stc_destroy(stc_ctx *ctx);
 
 /* Stable LSD radix sort of n (key, value) uint32 pairs on the low key_bits
  * bits of the key (1..32), on CUDA device `device`. All four pointers are
- * device memory; outputs must not alias inputs. Scratch (2n words plus
- * histograms) is allocated and freed inside the call; the call returns when
- * the sort is done. This is the sort the pipeline uses to group objects by
- * quadtree leaf in pid order; it replaces thrust::sort_by_key in the
+ * device memory; outputs must not alias inputs. The call returns when the
+ * sort is done. Its scratch (2n words plus histograms) comes from the
+ * library's memory pool of the device while it is at most 512 MB (about 63M
+ * pairs); that much may stay reserved in the pool for the next call. It is
+ * given back by stc_release_scratch, when a context of the device is
+ * destroyed, and when an allocation of the library would otherwise fail.
+ * Larger sorts allocate and free inside the call, which takes cudaMalloc's
+ * and cudaFree's time (0.6 ms and more). This is the sort of the flush, the
+ * compaction and the query index; it replaces thrust::sort_by_key in the
  * reference's flush (cuda/geometry.cu:1860-1907) for 32-bit keys. Errors:
  * stc_last_error(NULL). */
 stc_status stc_sort_pairs_u32(const uint32_t *keys, const uint32_t *values, uint32_t *keys_out,
                               uint32_t *values_out, size_t n, uint32_t key_bits, uint32_t device);
+
+/* Gives the memory that the library's pool of the device keeps between calls
+ * (at most 512 MB) back to the driver; without a context of the device it ends
+ * the pool as well, as the destruction of the last context does. A program
+ * that sorts without a context calls it when it needs the memory elsewhere or
+ * before cudaDeviceReset. Errors: stc_last_error(NULL). */
+stc_status stc_release_scratch(uint32_t device);
 
 /* Same sort and arguments as stc_sort_pairs_u32, for callers that cannot
  * have device memory allocated on their behalf: code that owns all device

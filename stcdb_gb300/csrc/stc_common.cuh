@@ -272,15 +272,18 @@ void iota_u32(uint32_t *out, size_t n, cudaStream_t s);
 // device, in stream order: cudaMalloc and cudaFree of a call's scratch cost
 // 0.3 ms each for 300 MB, and stop the device. The pool keeps at most
 // POOL_KEEP_BYTES of freed memory and gives it back when an allocation of the
-// library fails and when a context is destroyed (pool_trim). dev_malloc is
-// cudaMalloc with that second attempt. What the pool would not keep is taken
-// plainly: a pool maps new gigabytes at a quarter of cudaMalloc's rate (8 GB
-// of compaction scratch: 7.3 against 1.1 ms).
+// library fails, when a context of the device is destroyed and in
+// stc_release_scratch (pool_release); with the last context the pool goes too.
+// dev_malloc is cudaMalloc with a second attempt once the pool is empty. What
+// the pool would not keep is taken plainly: a pool maps new gigabytes at a
+// quarter of cudaMalloc's rate (8 GB of compaction scratch: 7.3 against 1.1 ms).
 constexpr unsigned long long POOL_KEEP_BYTES = 512ull << 20;
 constexpr size_t POOL_LARGEST_KEPT = 64u << 20;  // largest single array of a block that is kept for queries
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s);
 void pool_free(void *p, cudaStream_t s);
 void pool_trim();
+void pool_release();
+void pool_context(bool begins);  // a context of the current device begins or ends
 cudaError_t dev_malloc(void **p, size_t bytes);
 
 // Device scratch of one call on stream s, `total` bytes in all, freed when it

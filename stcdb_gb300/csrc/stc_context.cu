@@ -61,6 +61,7 @@ struct stc_ctx {
   std::string err;
   bool failed = false;
   bool stepped = false;
+  bool counted = false;          // among the device's contexts (pool_context)
   PipeDev p;
   DevState *st_host = nullptr;   // pinned mirror
   // pinned staging of drained meetings: copies from pinned memory are plain
@@ -190,6 +191,7 @@ static void destroy_all(stc_ctx *c) {
   lsm_release(c->lsmh);
   for (void *v : c->allocs) cudaFree(v);
   c->allocs.clear();
+  if (c->counted) pool_context(false);
   if (c->drain_stream) cudaStreamSynchronize(c->drain_stream);
   if (c->st_host) cudaFreeHost(c->st_host);
   if (c->t_pinned) cudaFreeHost(c->t_pinned);
@@ -234,7 +236,6 @@ extern "C" void stc_destroy(stc_ctx *c) {
   cudaGetDevice(&prev);
   cudaSetDevice(c->device);
   destroy_all(c);
-  pool_trim();
   cudaSetDevice(prev);
   delete c;
 }
@@ -324,6 +325,10 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   for (int i = 0; i < 4; i++) c->map[i] = mbr[i];
   memset(&c->stats, 0, sizeof(c->stats));
   cudaError_t e = cudaSetDevice(c->device);
+  if (e == cudaSuccess) {
+    pool_context(true);
+    c->counted = true;
+  }
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->stream, cudaStreamNonBlocking);
   // The side streams' short kernels go ahead of the main stream's waiting
   // blocks (behind the query lanes, which take the highest priority): beside

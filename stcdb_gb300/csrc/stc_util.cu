@@ -7,57 +7,110 @@
 namespace stc {
 void set_thread_error(const std::string &msg);
 
+// The pools of all devices. A pool is made by the first call that asks (where
+// that fails, this device's allocations are plain from then on) and destroyed
+// with the device's last context or by stc_release_scratch; memory still out
+// then goes back to the driver when it is freed. The lock is held over every
+// use of a pool's handle, so that none is used after that.
 static constexpr int POOL_DEVICES = 64;
+struct DevicePool {
+  cudaMemPool_t pool = nullptr;
+  bool none = false;      // could not be made
+  unsigned contexts = 0;  // of this device
+};
 static std::mutex g_pool_mutex;
-static cudaMemPool_t g_pool[POOL_DEVICES] = {};
+static DevicePool g_pools[POOL_DEVICES];
 
-// The current device's pool, made by the first call that asks; null without
-// one (allocations are then plain).
-static cudaMemPool_t device_pool(bool make) {
+// The current device's entry, with its pool made when `make`; null for a
+// device that has none. Called with the lock held.
+static DevicePool *device_pool(bool make) {
   int dev = 0;
   if (cudaGetDevice(&dev) != cudaSuccess || dev < 0 || dev >= POOL_DEVICES) return nullptr;
-  std::lock_guard<std::mutex> lock(g_pool_mutex);
-  if (!g_pool[dev] && make) {
+  DevicePool &d = g_pools[dev];
+  if (!d.pool && !d.none && make) {
     cudaMemPoolProps props = {};
     props.allocType = cudaMemAllocationTypePinned;
     props.location.type = cudaMemLocationTypeDevice;
     props.location.id = dev;
     unsigned long long keep = POOL_KEEP_BYTES;
-    cudaMemPool_t pool = nullptr;
-    if (cudaMemPoolCreate(&pool, &props) == cudaSuccess &&
-        cudaMemPoolSetAttribute(pool, cudaMemPoolAttrReleaseThreshold, &keep) == cudaSuccess)
-      g_pool[dev] = pool;
-    else
-      cudaGetLastError();
+    if (cudaMemPoolCreate(&d.pool, &props) != cudaSuccess) d.pool = nullptr;
+    if (d.pool && cudaMemPoolSetAttribute(d.pool, cudaMemPoolAttrReleaseThreshold, &keep) != cudaSuccess) {
+      cudaMemPoolDestroy(d.pool);
+      d.pool = nullptr;
+    }
+    d.none = !d.pool;
+    if (d.none) cudaGetLastError();
   }
-  return g_pool[dev];
+  return &d;
+}
+
+static void trim(DevicePool &d) {
+  if (d.pool) cudaMemPoolTrimTo(d.pool, 0);
+}
+
+// Gives back what the pool keeps; all of it where no context is left.
+static void release(DevicePool &d) {
+  trim(d);
+  if (d.contexts || !d.pool) return;
+  cudaMemPoolDestroy(d.pool);
+  d.pool = nullptr;
 }
 
 cudaError_t pool_alloc(void **p, size_t bytes, cudaStream_t s) {
   *p = nullptr;
-  cudaMemPool_t pool = device_pool(true);
-  if (!pool) return dev_malloc(p, bytes);
-  cudaError_t e = cudaMallocFromPoolAsync(p, bytes, pool, s);
-  if (e == cudaErrorMemoryAllocation) {
-    cudaGetLastError();
-    pool_trim();
-    e = cudaMallocFromPoolAsync(p, bytes, pool, s);
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    DevicePool *d = device_pool(true);
+    if (d && d->pool) {
+      cudaError_t e = cudaMallocFromPoolAsync(p, bytes, d->pool, s);
+      if (e == cudaErrorMemoryAllocation) {
+        cudaGetLastError();
+        trim(*d);
+        e = cudaMallocFromPoolAsync(p, bytes, d->pool, s);
+      }
+      if (e != cudaSuccess) {
+        cudaGetLastError();
+        *p = nullptr;
+      }
+      return e;
+    }
   }
-  if (e != cudaSuccess) {
-    cudaGetLastError();
-    *p = nullptr;
-  }
-  return e;
+  return dev_malloc(p, bytes);
 }
 
+// (memory of a pool that has been destroyed since goes by cudaFree)
 void pool_free(void *p, cudaStream_t s) {
   if (!p) return;
-  if (device_pool(false)) cudaFreeAsync(p, s);
+  bool pooled = false;
+  {
+    std::lock_guard<std::mutex> lock(g_pool_mutex);
+    DevicePool *d = device_pool(false);
+    pooled = d && d->pool;
+  }
+  if (pooled) cudaFreeAsync(p, s);
   else cudaFree(p);
 }
 
 void pool_trim() {
-  if (cudaMemPool_t pool = device_pool(false)) cudaMemPoolTrimTo(pool, 0);
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (DevicePool *d = device_pool(false)) trim(*d);
+}
+
+void pool_release() {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  if (DevicePool *d = device_pool(false)) release(*d);
+}
+
+void pool_context(bool begins) {
+  std::lock_guard<std::mutex> lock(g_pool_mutex);
+  DevicePool *d = device_pool(false);
+  if (!d) return;
+  if (begins) {
+    d->contexts++;
+  } else {
+    d->contexts--;
+    release(*d);
+  }
 }
 
 cudaError_t dev_malloc(void **p, size_t bytes) {
@@ -110,6 +163,16 @@ stc_status sort_args_ok(const uint32_t *keys, const uint32_t *values, uint32_t *
 }
 
 }  // namespace
+
+extern "C" stc_status stc_release_scratch(uint32_t device) {
+  const cudaError_t e = cudaSetDevice((int)device);
+  if (e != cudaSuccess) {
+    set_thread_error(std::string("stc_release_scratch: ") + cudaGetErrorString(e));
+    return STC_ERR_CUDA;
+  }
+  pool_release();
+  return STC_OK;
+}
 
 extern "C" stc_status stc_sort_pairs_u32(const uint32_t *keys, const uint32_t *values, uint32_t *keys_out,
                                          uint32_t *values_out, size_t n, uint32_t key_bits, uint32_t device) {
