@@ -105,9 +105,10 @@ typedef struct stc_config {
    * arrival). */
   uint32_t job_chunk;            /* refinement jobs (32 rows against their candidate ranges) a warp
                                     takes at a time, fewer when there are too few to go round;
-                                    0 = 8, or one at a time by demand where that is faster;
+                                    0 or 8 = 8, or one at a time by demand where that is faster;
                                     at most 64 */
-  uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 = 8 or 12, at most 32 */
+  uint32_t refine_blocks_per_sm; /* pair-test blocks launched per SM; 0 or 8 = 8, or 12 with short
+                                    tiles (refine_chunk); at most 32 */
   uint32_t hits_blocks_per_sm;   /* blocks per SM of the general table update (a step whose table tiles
                                     are too full for the tiled one); 0 = 16, at most 64 */
   uint32_t window_graphs;        /* stc_step_window replays each step from a captured CUDA graph:
@@ -235,7 +236,8 @@ typedef struct stc_tune_result {
  * grid_capacity, 2 * grid_capacity}; cfg's own grid_capacity is always tried
  * and gives base_step_ms), then job_chunk (2-32), refine_chunk (the tile
  * length: the automatic choice or 64-512), refine_blocks_per_sm and
- * hits_blocks_per_sm one after the other. The launch shape never changes
+ * hits_blocks_per_sm one after the other, from the built-in values on; a
+ * value is taken when it is more than 1% faster. The launch shape never changes
  * results; the leaf capacity is part of the reference's configuration (it
  * orders the reference's table inserts), so a run with the chosen capacity
  * matches the reference run with that capacity. */

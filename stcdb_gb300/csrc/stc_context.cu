@@ -407,11 +407,11 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   p.delay = k.schema_update_delay;
   p.mbr_filter = k.mbr_filter;
   p.slices = std::min<uint32_t>(std::max<uint32_t>(k.step_slices, 1u), MAX_SLICES);
-  p.job_chunk = k.job_chunk ? std::min<uint32_t>(k.job_chunk, 64u) : 8u;
+  p.job_chunk = job_chunk_of(k.job_chunk);
   p.job_share = 0;
   p.refine_chunk = k.refine_chunk ? k.refine_chunk : REFINE_CHUNK_DEFAULT;
-  p.refine_bps = k.refine_blocks_per_sm ? std::min<uint32_t>(k.refine_blocks_per_sm, 32u) : 0u;
-  p.hits_bps = k.hits_blocks_per_sm ? std::min<uint32_t>(k.hits_blocks_per_sm, 64u) : 16u;
+  p.refine_bps = refine_bps_of(k.refine_blocks_per_sm);
+  p.hits_bps = hits_bps_of(k.hits_blocks_per_sm);
 
   p.leaves_max = std::min(p.G, n);
   // refinement jobs: one per row block of 32 members or units, and room to
@@ -763,7 +763,7 @@ static void choose_refine_chunk(stc_ctx *c) {
   // by the last step's jobs; a quarter fewer before it changes back
   const unsigned long long jobs = c->st_host->jobs_total;
   const unsigned long long warps = (unsigned long long)num_sms() * refine_blocks(p) * (REFINE_THREADS / 32);
-  p.job_share = !c->cfg.job_chunk && job_shares(share0 ? jobs + jobs / 4 : jobs, warps, chunk);
+  p.job_share = jobs_may_share(c->cfg.job_chunk) && job_shares(share0 ? jobs + jobs / 4 : jobs, warps, chunk);
   if (chunk != chunk0 || p.job_share != share0) invalidate_graphs(c);  // the captured steps carry both
 }
 

@@ -131,7 +131,7 @@ inline size_t hit_records(uint32_t nb, uint32_t bin_cap) {
 // objects, half of them in hotspots, 0.46 -> 0.43 ms a step), else two.
 constexpr uint32_t REFINE_THREADS = 256;
 inline uint32_t refine_blocks(const PipeDev &p) {
-  return p.refine_bps ? p.refine_bps : p.refine_chunk <= REFINE_CHUNK_FEW ? 12u : 8u;
+  return p.refine_bps ? p.refine_bps : p.refine_chunk <= REFINE_CHUNK_FEW ? 12u : REFINE_BPS_BUILTIN;
 }
 
 // Whether warps take their jobs one by one from a common counter: `jobs` to

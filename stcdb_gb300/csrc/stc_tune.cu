@@ -9,6 +9,7 @@
 #include <vector>
 
 #include "stc.h"
+#include "stc_rules.cuh"
 
 namespace stc {
 void set_thread_error(const std::string &msg);
@@ -17,6 +18,10 @@ void set_thread_error(const std::string &msg);
 namespace {
 
 constexpr uint32_t TUNE_WARM = 2;  // steps before the timed ones
+// A launch shape replaces the one before it when its steps take at most this
+// part of the time: equal ones differ by up to 1% between runs, and some
+// fields do nothing for some workloads (the general table update's blocks).
+constexpr double TUNE_GAIN = 0.99;
 
 // Device ms of the timed steps of cfg over xy, or a negative value on error
 // (the message is left for stc_last_error(NULL)).
@@ -88,13 +93,14 @@ extern "C" stc_status stc_autotune(const stc_config *cfg, const double mbr[4], c
     }
   }
   if (best < 0) return STC_ERR_STATE;
-  // 2. launch shape, one field after the other (0 = the built-in default)
+  // 2. launch shape, one field after the other, from the built-in values (what
+  // 0 means: the settings timed so far)
   stc_config k = base;
   k.grid_capacity = r.config.grid_capacity;
-  k.job_chunk = cfg->job_chunk ? cfg->job_chunk : 8;  // 0 means about these built-in values
+  k.job_chunk = cfg->job_chunk ? cfg->job_chunk : stc::JOB_CHUNK_BUILTIN;
   k.refine_chunk = cfg->refine_chunk;  // 0: the per-step automatic choice, itself a candidate
-  k.refine_blocks_per_sm = cfg->refine_blocks_per_sm ? cfg->refine_blocks_per_sm : 8;
-  k.hits_blocks_per_sm = cfg->hits_blocks_per_sm ? cfg->hits_blocks_per_sm : 16;
+  k.refine_blocks_per_sm = cfg->refine_blocks_per_sm ? cfg->refine_blocks_per_sm : stc::REFINE_BPS_BUILTIN;
+  k.hits_blocks_per_sm = cfg->hits_blocks_per_sm ? cfg->hits_blocks_per_sm : stc::HITS_BPS_BUILTIN;
   const uint32_t job_chunks[] = {2, 4, 8, 16, 32}, refine_chunks[] = {64, 128, 256, 512},
                  refine_bps[] = {4, 8, 16}, hits_bps[] = {8, 16, 32};
   struct Field {
@@ -113,7 +119,7 @@ extern "C" stc_status stc_autotune(const stc_config *cfg, const double mbr[4], c
       c2.*(fd.f) = fd.vals[i];
       const double ms = run_candidate(c2, mbr, xy, n, steps);
       r.trials++;
-      if (ms >= 0 && ms < best) {
+      if (ms >= 0 && ms < best * TUNE_GAIN) {
         best = ms;
         keep = fd.vals[i];
       }

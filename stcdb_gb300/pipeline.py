@@ -233,8 +233,8 @@ class StcConfig:
     area_restriction: float = 0.0  # 0 = 100 (no cut)
     ctb_retain: int = 0       # flushed blocks kept for queries; 0 = 8
     step_slices: int = 0      # launches per long step kernel (query latency under ingest); 0 = 1
-    job_chunk: int = 0        # refinement launch shape (results do not depend on it); 0 = 8 or by demand
-    refine_blocks_per_sm: int = 0  # 0 = 8 or 12
+    job_chunk: int = 0        # refinement launch shape (results do not depend on it); 0 or 8 = 8 or by demand
+    refine_blocks_per_sm: int = 0  # 0 or 8 = 8 or 12
     hits_blocks_per_sm: int = 0    # 0 = 16
     window_graphs: int = 0    # step_window replays captured graphs: 0 = for short steps (automatic), 1 = always, 2 = never
     bitmap_edge: int = 0      # edge of a block's map bitmap (oversize buffer); 0 = 256

@@ -20,6 +20,17 @@ extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chun
   for (unsigned i = 0; i < n; i++) sum += jobs_beyond(rows[i], chunks[i], room);
   return sum;
 }
+extern "C" void shape_of(unsigned job_chunk, unsigned refine_bps, unsigned hits_bps, unsigned *out) {
+  out[0] = jobs_may_share(job_chunk);
+  out[1] = job_chunk_of(job_chunk);
+  out[2] = refine_bps_of(refine_bps);
+  out[3] = hits_bps_of(hits_bps);
+}
+extern "C" void builtin_shape(unsigned *out) {
+  out[0] = JOB_CHUNK_BUILTIN;
+  out[1] = REFINE_BPS_BUILTIN;
+  out[2] = HITS_BPS_BUILTIN;
+}
 """
 
 
@@ -53,3 +64,21 @@ def test_jobs_beyond_their_room_stay_beyond_it_in_32_bits(lib):
         got = f((ctypes.c_uint * n)(*rows), (ctypes.c_uint * n)(*chunks), len(rows), room)
         assert got == true if true <= room else got > room, (rows, chunks, room)
     assert wraps > 0
+
+
+def _shape(lib, *given):
+    out = (ctypes.c_uint * 4)()
+    lib.shape_of(*given, out)
+    return tuple(out)
+
+
+def test_the_built_in_launch_shape_is_the_automatic_one(lib):
+    """The autotuner names the built-in values where its first runs, which it
+    compares the later ones with, left them at 0: both run the same way."""
+    b = (ctypes.c_uint * 3)()
+    lib.builtin_shape(b)
+    auto = _shape(lib, 0, 0, 0)
+    assert _shape(lib, *b) == auto == (1, 8, 0, 16)
+    for chunk, bps, hits in [(1, 1, 1), (7, 4, 8), (9, 9, 32), (64, 32, 64)]:
+        assert _shape(lib, chunk, bps, hits) == (0, chunk, bps, hits)  # others as given
+    assert _shape(lib, 1000, 1000, 1000) == (0, 64, 32, 64)
