@@ -77,10 +77,14 @@ typedef struct stc_config {
   int32_t mbr_filter;            /* drop meetings whose MBR leaves the map box (cuda/geometry.cu:667-670) */
   uint64_t candidate_capacity;   /* new-meeting candidates per step; 0 = auto */
   uint64_t emit_capacity;        /* emitted meetings held between drains; 0 = auto */
-  uint64_t hit_capacity;         /* pairs buffered between refinement and table update, spread over
-                                    bins of one table tile (up to 768 slots) each; 0 = auto:
-                                    max(4M, 8 n) and a quarter more, grown after a step (or window)
-                                    that found a fuller bin */
+  uint64_t hit_capacity;         /* pairs (32 bytes each) buffered between refinement and table
+                                    update, in equal shares for the table's tiles of up to 768
+                                    slots: a step that finds more for one tile than its share
+                                    updates the table the slower, general way, so give a few times
+                                    the hits of a step. 0 = auto: max(4M, 8 n) and a quarter more,
+                                    at least 16 a tile, grown after a step (or window) that found
+                                    more for one tile, up to eight times that step's hits, or 48
+                                    records a tile, and 704 a tile */
   uint32_t device;               /* CUDA device ordinal */
   uint32_t flags;                /* STC_FLAG_* (0 for normal operation) */
   /* Memtable and flush into a contact tracing block (CTB) of CTFs, the

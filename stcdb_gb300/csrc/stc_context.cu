@@ -260,12 +260,6 @@ static stc_status read_state(stc_ctx *c, const char *where) {
   return STC_OK;
 }
 
-// Records per bin when `total` are spread over nb bins, times num / den, plus
-// `more` (at least 1; a run of bins stays below 2^32 records).
-static uint32_t bin_share(uint64_t total, uint32_t nb, uint32_t num = 1, uint32_t den = 1, uint32_t more = 0) {
-  return (uint32_t)std::min<uint64_t>(std::max<uint64_t>((total + nb - 1) / nb * num / den + more, 1), 1u << 24);
-}
-
 // Creates a context; builds the quadtree from xy0 unless xy0 is null (a
 // restore fills the schema from a checkpoint instead).
 static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const double *xy0, uint32_t n,
@@ -381,11 +375,8 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   p.cand_cap = cand_cap;
   p.C = next_pow2(2 * cand_cap);
   p.E = k.emit_capacity ? k.emit_capacity : std::max<uint64_t>(1u << 20, 4ULL * n);
-  // hits beyond a bin are applied inside the refinement instead; an automatic
-  // bin has room for a quarter more than its share
   table_sizes(p);
-  p.bin_cap = k.hit_capacity ? bin_share(k.hit_capacity, p.nb)
-                             : bin_share(std::max<uint64_t>(1u << 22, 8ULL * n), p.nb, 5, 4, 64);
+  p.bin_cap = k.hit_capacity ? bin_share(k.hit_capacity, p.nb) : bin_cap_auto(n, p.nb);
   p.U_cap = (uint64_t)k.refine_size * n - n;
   p.reach = k.reach_distance;
   p.reach_f = (float)k.reach_distance;
@@ -705,19 +696,24 @@ static void fill_stats(stc_ctx *c, uint32_t t, const float *phase, float step_ms
 // (cuda/geometry.cu:1752).
 static bool flush_due(const stc_ctx *c) { return c->lsm_on && c->st_host->kv_count > c->cfg.kv_restriction; }
 
-// With the automatic hit capacity (stc_config.hit_capacity 0) the bins grow to
-// the fullest bin seen: a hit beyond its bin is applied inside the pair tests,
-// which is correct but slow (random table accesses, and the general path for
-// that step). Called only with no step in flight; a failed allocation keeps
-// the old bins.
-static void grow_hits(stc_ctx *c, unsigned long long need) {
+// Records per bin after steps whose fullest bin had `fullest` hits and whose
+// largest step had `hits`. With the automatic hit capacity (stc_config.
+// hit_capacity 0) the bins grow, within the bounds of bin_cap_grown: a hit
+// beyond its bin costs the step the general path, and is applied inside the
+// pair tests, or, while the table's tiles are packed, by a second run of them.
+static uint32_t bins_wanted(const stc_ctx *c, unsigned long long fullest, unsigned long long hits) {
+  return c->cfg.hit_capacity ? c->p.bin_cap : bin_cap_grown(c->p.bin_cap, fullest, hits, c->p.nb);
+}
+
+// Gives the bins room for `cap` records each; false when there is no memory
+// for that, which keeps the old ones. Called only with no step in flight.
+static bool grow_hits(stc_ctx *c, uint32_t cap) {
   PipeDev &p = c->p;
-  if (c->cfg.hit_capacity || need <= p.bin_cap) return;
-  const uint32_t cap = bin_share(need, 1, 5, 4, 16);
+  if (cap <= p.bin_cap) return true;
   void *h = nullptr;
   if (dev_malloc(&h, hit_records(p.nb, cap) * sizeof(HitRec)) != cudaSuccess) {
     cudaGetLastError();
-    return;
+    return false;
   }
   for (void *&a : c->allocs)
     if (a == (void *)p.hits) {
@@ -727,6 +723,7 @@ static void grow_hits(stc_ctx *c, unsigned long long need) {
   p.hits = (HitRec *)h;
   p.bin_cap = cap;
   invalidate_graphs(c);  // the graphs hold the buffer by value
+  return true;
 }
 
 // Tile length of the refinement's jobs when stc_config.refine_chunk is 0.
@@ -785,7 +782,7 @@ static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copie
   float tot = 0;
   cudaEventElapsedTime(&tot, c->ev[PH_START], c->ev[PH_SCHEMA]);
   fill_stats(c, t, phase, tot, (uint32_t)(tl_launches - launches0));
-  grow_hits(c, c->st_host->hit_max);
+  grow_hits(c, bins_wanted(c, c->st_host->hit_max, c->st_host->hits));
   if (flush_due(c)) return flush_now(c, t);
   return STC_OK;
 }
@@ -1046,7 +1043,8 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
   const auto wall0 = std::chrono::steady_clock::now();
   double busy_ms = 0;  // device time of the window's steps
   size_t n = 0;
-  unsigned long long most_hits = 0;  // the window's fullest bin (the bins grow at its end)
+  unsigned long long fullest = 0, most_hits = 0;  // the window's fullest bin and largest step (the bins grow by them)
+  bool may_grow = true;                           // no attempt has failed
   unsigned long long dpos = 0;  // emit records [0, dpos) are on their way to out
   bool out_full = false;
   stc_status rs = STC_OK;
@@ -1078,7 +1076,10 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       ran = i + 1;
       busy_ms += c->stats.step_ms;
     }
-    if (rs == STC_OK) most_hits = std::max(most_hits, c->st_host->hit_max);
+    if (rs == STC_OK) {
+      fullest = std::max(fullest, c->st_host->hit_max);
+      most_hits = std::max(most_hits, c->st_host->hits);
+    }
     if (rs == STC_OK && out && !out_full) {
       const unsigned long long cnt = std::min<unsigned long long>(c->st_host->emit_count, p.E);
       const size_t k = (size_t)std::min<unsigned long long>(cnt - dpos, cap - n);
@@ -1126,7 +1127,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
           if (e != cudaSuccess) return cuda_fail(c, e, "stc_step_window drain");
           dpos = 0;
         }
-        grow_hits(c, most_hits);
+        may_grow = may_grow && grow_hits(c, bins_wanted(c, fullest, most_hits));
         hold = false;
         rs = issue_core(i + 1);
         if (rs == STC_OK && i + WIN_BUFS < steps) {
@@ -1146,9 +1147,9 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       // step i + 1 adds its meetings behind step i's; past half of the
       // emit buffer, step i + 2 waits until the buffer has been emptied
       if (out && c->st_host->emit_count > p.E / 2) hold = true;
-      // a step found more hits than a bin holds (the rest were applied
-      // inside its pair tests): grow the bins at the next step boundary
-      if (!c->cfg.hit_capacity && most_hits > p.bin_cap) hold = true;
+      // a step found more hits than a bin holds: grow the bins at the next
+      // step boundary
+      if (may_grow && bins_wanted(c, fullest, most_hits) > p.bin_cap) hold = true;
     }
   }
   cudaStreamSynchronize(c->copy_stream);
@@ -1157,7 +1158,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
     if (e != cudaSuccess) return cuda_fail(c, e, "stc_step_window drain");
   }
   cudaStreamSynchronize(s);
-  grow_hits(c, most_hits);
+  if (may_grow) grow_hits(c, bins_wanted(c, fullest, most_hits));
   c->stats.window_device_ms = (float)busy_ms;
   c->stats.window_input_wait_ms = (float)wait_ms;
   c->stats.window_copy_ms = (float)copy_ms;

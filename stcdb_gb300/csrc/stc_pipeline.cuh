@@ -112,13 +112,12 @@ struct PipeDev {
   stc_meeting *emit;                    // E
 };
 
-// Place of record i of bin j: bins are cut into chunks of HIT_CHUNK records, the
+// Place of record i of bin j: bins are cut into chunks of HIT_CHUNK (16) records, the
 // first chunks of all bins come first, then the second ones. The bins fill at
 // much the same pace, so the step writes to a few hundred MB at a time and not
 // to all of the buffer: scattered stores are bound by the reach of the address
 // translation (67.7M records into 349526 bins, with their counters: 36 G/s bin
 // after bin, 2.8 GB; 52 with chunks of 16; 80 if all went to 180 MB).
-constexpr uint32_t HIT_CHUNK = 16;
 __host__ __device__ __forceinline__ unsigned long long hit_place(const PipeDev &p, uint32_t j, uint32_t i) {
   return ((unsigned long long)(i / HIT_CHUNK) * p.nb + j) * HIT_CHUNK + i % HIT_CHUNK;
 }
@@ -159,9 +158,7 @@ void step_pairs(PipeDev &p, cudaStream_t s);
 void step_hits(PipeDev &p, cudaStream_t s);
 // stc_table.cu: the tiled table update and sweep. plan decides whether the
 // step takes it and finds what is carried into each run of tiles.
-constexpr uint32_t TILE_SLOTS = 768;    // largest tile
 constexpr uint32_t OCC_WORDS = TILE_SLOTS / 32;
-constexpr uint32_t TILE_LOAD = 704;     // (occupied slots + hits) of a tile stay below this on the tiled path
 cudaError_t table_prepare();
 void table_sizes(PipeDev &p);           // nb and runs of a table of p.B slots
 void count_tiles(PipeDev &p, cudaStream_t s);

@@ -17,6 +17,46 @@ __host__ __device__ __forceinline__ uint32_t jobs_beyond(uint32_t rows, uint32_t
   return (uint32_t)(n <= room ? n : room + 1);
 }
 
+// Tiles of the meeting table (stc_table.cu) and the bins of a step's hits.
+constexpr uint32_t TILE_SLOTS = 768;    // largest tile
+constexpr uint32_t TILE_LOAD = 704;     // (occupied slots + hits) of a tile stay below this on the tiled path
+constexpr uint32_t HIT_CHUNK = 16;      // records of a bin that lie together (hit_place)
+
+// Records per bin when `total` are spread over nb bins, rounded up (at least 1;
+// a run of bins stays below 2^32 records).
+inline uint32_t bin_share(uint64_t total, uint32_t nb) {
+  const uint64_t n = (total + nb - 1) / nb;
+  return (uint32_t)(n < 1 ? 1 : n > (1u << 24) ? 1u << 24 : n);
+}
+
+// Records per bin of an automatic hit buffer (stc_config.hit_capacity 0) for n
+// objects: room for 4M or 8 n hits, a quarter and two standard deviations of
+// an even spread more, in whole chunks. A table of many slots for few objects
+// has 16 records a tile, 2% of its slots' memory. (With 64 more a bin whatever
+// its share, 2^30 slots took 2.9 GB and 2^32 slots 11.5.)
+inline uint32_t bin_cap_auto(uint64_t n, uint32_t nb) {
+  const uint64_t share = bin_share(8 * n > (1u << 22) ? 8 * n : 1u << 22, nb);
+  uint64_t root = 0;
+  while ((root + 1) * (root + 1) <= share) root++;
+  const uint64_t cap = (share + share / 4 + 2 * root + 8 + HIT_CHUNK - 1) / HIT_CHUNK * HIT_CHUNK;
+  return (uint32_t)(cap > (1u << 24) ? 1u << 24 : cap);
+}
+
+// Records per bin after a step of `hits` hits whose fullest bin had `fullest`:
+// a quarter more than that, but no more than eight times the mean bin (or 48
+// records, a sixteenth of the slots' memory) and no more than the tiled path
+// can use. One crowd's bin must not size all the others: 1600 objects of
+// neighbouring ids fill one tile, and 2^28 slots then took 10.9 GB for it.
+inline uint32_t bin_cap_grown(uint32_t cap, uint64_t fullest, uint64_t hits, uint32_t nb) {
+  if (fullest <= cap) return cap;
+  uint64_t most = 8 * (uint64_t)bin_share(hits, nb);
+  if (most < 48) most = 48;
+  if (most > TILE_LOAD) most = TILE_LOAD;
+  uint64_t want = (fullest + fullest / 4 + 2 * HIT_CHUNK - 1) / HIT_CHUNK * HIT_CHUNK;
+  if (want > most) want = most / HIT_CHUNK * HIT_CHUNK;
+  return want > cap ? (uint32_t)want : cap;
+}
+
 // Launch shape of the refinement (stc_config.job_chunk, refine_blocks_per_sm).
 // The built-in value, given or not, leaves the choice to the library: jobs
 // taken by demand where that is faster (job_shares), more blocks where the

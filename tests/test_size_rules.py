@@ -20,6 +20,10 @@ extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chun
   for (unsigned i = 0; i < n; i++) sum += jobs_beyond(rows[i], chunks[i], room);
   return sum;
 }
+extern "C" unsigned cap_auto(unsigned long long n, unsigned nb) { return bin_cap_auto(n, nb); }
+extern "C" unsigned cap_grown(unsigned cap, unsigned long long fullest, unsigned long long hits, unsigned nb) {
+  return bin_cap_grown(cap, fullest, hits, nb);
+}
 extern "C" void shape_of(unsigned job_chunk, unsigned refine_bps, unsigned hits_bps, unsigned *out) {
   out[0] = jobs_may_share(job_chunk);
   out[1] = job_chunk_of(job_chunk);
@@ -82,3 +86,53 @@ def test_the_built_in_launch_shape_is_the_automatic_one(lib):
     for chunk, bps, hits in [(1, 1, 1), (7, 4, 8), (9, 9, 32), (64, 32, 64)]:
         assert _shape(lib, chunk, bps, hits) == (0, chunk, bps, hits)  # others as given
     assert _shape(lib, 1000, 1000, 1000) == (0, 64, 32, 64)
+
+
+REC = 32   # bytes of a hit record, and of a table slot
+TILE = 768
+
+
+def _caps(lib):
+    u, ll = ctypes.c_uint, ctypes.c_ulonglong
+    lib.cap_auto.restype = lib.cap_grown.restype = u
+    lib.cap_auto.argtypes = [ll, u]
+    lib.cap_grown.argtypes = [u, ll, ll, u]
+    return lib.cap_auto, lib.cap_grown
+
+
+def test_automatic_hit_bins_follow_the_objects_and_stay_small_beside_the_table(lib):
+    auto, _ = _caps(lib)
+    for log2 in (10, 16, 20, 24, 28, 30, 32, 33):
+        slots = 1 << log2
+        nb = (slots + TILE - 1) // TILE
+        for n in (1, 1000, 100_003, 300_000, 1_000_000, 10_000_000, 100_000_000):
+            cap = auto(n, nb)
+            room = max(1 << 22, 8 * n)
+            assert cap % 16 == 0 and cap >= 16
+            assert nb * cap >= room or cap == 1 << 24
+            # a quarter and two standard deviations more, 8 more and whole chunks a bin
+            assert nb * cap <= 1.25 * (room + nb) + 2 * (nb * (room + nb)) ** 0.5 + 24 * nb
+    # 300k objects in 2^28 slots had 0.89 GB of bins, 1M in 2^30 3.6 GB
+    assert auto(300_000, (1 << 28) // TILE + 1) * ((1 << 28) / TILE) * REC < 0.4e9
+    assert auto(1_000_000, (1 << 30) // TILE + 1) * ((1 << 30) / TILE) * REC < 1.5e9
+
+
+def test_hit_bins_grow_with_the_hits_not_with_one_crowd(lib):
+    _, grown = _caps(lib)
+    nb = (1 << 28) // TILE + 1
+    assert grown(80, 80, 10 ** 6, nb) == 80                     # nothing to grow for
+    assert grown(32, 781, 1_500_000, nb) == 48                  # one crowd of 1600 objects: 0.5 GB, not 10.9
+    assert grown(64, 781, 1_500_000, nb) == 64                  # never less
+    assert grown(64, 100, 35_000_000, nb) == 144  # an even crowd gets what it asks
+    assert grown(64, 5000, 350_000_000, nb) == 704              # what the tiled path can use
+    rng = random.Random(3)
+    for _ in range(2000):
+        nb = rng.randrange(1, 1 << 22)
+        cap = 16 * rng.randrange(1, 60)
+        hits = rng.randrange(1, 1 << rng.randrange(4, 36))
+        fullest = rng.randrange(1, max(hits, 2))
+        got = grown(cap, fullest, hits, nb)
+        assert cap <= got <= max(cap, 704)
+        assert got == cap or got * nb <= max(8 * hits + 8 * nb, 48 * nb)
+        if fullest > cap and fullest * 1.25 + 32 <= min(704, 8 * hits / nb):
+            assert got >= fullest * 1.25
