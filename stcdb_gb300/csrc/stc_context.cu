@@ -1677,9 +1677,15 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
     stc_destroy(c);
     return STC_ERR_CUDA;
   }
-  // the ids in use and on the free stacks are not searched for the highest
-  const uint32_t high[2] = {c->p.S, c->p.G};
-  e = cudaMemcpy(c->p.sd.high, high, sizeof(high), cudaMemcpyHostToDevice);
+  // up to where the step's schema kernels look (all 640,000 ids of a small
+  // context made its steps 0.196 ms instead of 0.157 at 20k objects)
+  std::vector<uint32_t> stack(std::max(c->p.S, c->p.G));
+  uint32_t high[2] = {0, 0};
+  e = cudaMemcpy(stack.data(), c->p.sd.schema_stack, (size_t)c->p.S * 4, cudaMemcpyDeviceToHost);
+  high[0] = ids_handed_out(stack.data(), h.st.schema_stack_index, c->p.S);
+  if (e == cudaSuccess) e = cudaMemcpy(stack.data(), c->p.sd.grids_stack, (size_t)c->p.G * 4, cudaMemcpyDeviceToHost);
+  high[1] = ids_handed_out(stack.data(), h.st.grids_stack_index, c->p.G);
+  if (e == cudaSuccess) e = cudaMemcpy(c->p.sd.high, high, sizeof(high), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);
     stc_destroy(c);

@@ -17,6 +17,15 @@ __host__ __device__ __forceinline__ uint32_t jobs_beyond(uint32_t rows, uint32_t
   return (uint32_t)(n <= room ? n : room + 1);
 }
 
+// Ids that a free stack of `size` entries (entry i holds id i until it is taken;
+// the entries below `index` are taken) ever handed out lie below this: behind
+// the last entry that holds another id than its own, everything is as it was.
+inline uint32_t ids_handed_out(const uint32_t *stack, uint32_t index, uint32_t size) {
+  uint32_t high = size;
+  while (high > index && stack[high - 1] == high - 1) high--;
+  return high;
+}
+
 // Tiles of the meeting table (stc_table.cu) and the bins of a step's hits.
 constexpr uint32_t TILE_SLOTS = 768;    // largest tile
 constexpr uint32_t TILE_LOAD = 704;     // (occupied slots + hits) of a tile stay below this on the tiled path

@@ -20,6 +20,9 @@ extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chun
   for (unsigned i = 0; i < n; i++) sum += jobs_beyond(rows[i], chunks[i], room);
   return sum;
 }
+extern "C" unsigned handed_out(const unsigned *stack, unsigned index, unsigned size) {
+  return ids_handed_out(stack, index, size);
+}
 extern "C" unsigned cap_auto(unsigned long long n, unsigned nb) { return bin_cap_auto(n, nb); }
 extern "C" unsigned cap_grown(unsigned cap, unsigned long long fullest, unsigned long long hits, unsigned nb) {
   return bin_cap_grown(cap, fullest, hits, nb);
@@ -136,3 +139,34 @@ def test_hit_bins_grow_with_the_hits_not_with_one_crowd(lib):
         assert got == cap or got * nb <= max(8 * hits + 8 * nb, 48 * nb)
         if fullest > cap and fullest * 1.25 + 32 <= min(704, 8 * hits / nb):
             assert got >= fullest * 1.25
+
+
+def test_ids_handed_out_are_found_from_the_free_stack(lib):
+    """Splits take four ids off the stack, merges put four back; the bound the
+    context itself keeps (the deepest the stack was ever taken to) is found
+    again from the stack, or a lower one that still covers every id in use
+    and every id that the stack hands out before its untouched end."""
+    f = lib.handed_out
+    f.restype = ctypes.c_uint
+    f.argtypes = [ctypes.c_void_p, ctypes.c_uint, ctypes.c_uint]
+    rng = random.Random(11)
+    for _ in range(200):
+        size = rng.choice([64, 400, 4000])
+        stack, index, used, deepest = list(range(size)), 1, [0], 1
+        groups = []
+        for _ in range(rng.randrange(0, 200)):
+            if index + 4 <= size and (not groups or rng.random() < 0.55):
+                groups.append(stack[index:index + 4])
+                index += 4
+                deepest = max(deepest, index)
+            elif groups:
+                for i in groups.pop(rng.randrange(len(groups))):
+                    index -= 1
+                    stack[index] = i
+        used = [0] + [i for g in groups for i in g]
+        high = f((ctypes.c_uint * size)(*stack), index, size)
+        assert index <= high <= deepest
+        assert max(used) < max(high, 1)
+        assert all(i < high for i in stack[index:high])
+        assert stack[high:] == list(range(high, size))
+    assert f((ctypes.c_uint * 8)(*range(8)), 8, 8) == 8 and f((ctypes.c_uint * 8)(*range(8)), 3, 8) == 3
