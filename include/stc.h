@@ -561,6 +561,13 @@ stc_status stc_restore(const char *path, uint32_t device, stc_ctx **out);
  * start between the slices, and runs whole steps otherwise. */
 stc_status stc_set_step_slices(stc_ctx *ctx, uint32_t slices);
 
+/* How the last step updated the meeting table: tile by tile, each run of
+ * tiles entered with what this many tiles before it carry on (1 to 15), or 0:
+ * the general way, one table access per hit and a pass over all slots (tiles
+ * too full, or more hits for one than its share of hit_capacity). Results do
+ * not depend on it. */
+uint32_t stc_table_halo(const stc_ctx *ctx);
+
 /* Last error message of ctx (or, when ctx is NULL, of the last failed
  * stc_create or context-free call on this thread). Never NULL. */
 const char *stc_last_error(const stc_ctx *ctx);

@@ -95,7 +95,7 @@ struct DevState {
   unsigned long long tests, exact_tests, hits, ambiguous;
   unsigned long long taken;
   unsigned long long step_emitted;
-  unsigned long long da_iters;
+  unsigned long long halo;            // halo tiles of the step's tiled table update; 0: general path
   uint32_t splits, merges, events, overflow_objects;
   uint32_t build_nodes, build_leaves, build_active, build_level;
   uint32_t work_next;                 // generic persistent-kernel work counter

@@ -1712,6 +1712,8 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
   return STC_OK;
 }
 
+extern "C" uint32_t stc_table_halo(const stc_ctx *c) { return c && c->stepped ? (uint32_t)c->st_host->halo : 0; }
+
 extern "C" stc_status stc_get_config(const stc_ctx *c, stc_config *cfg) {
   if (!c || !cfg) return STC_ERR_INVALID_ARG;
   *cfg = c->cfg;

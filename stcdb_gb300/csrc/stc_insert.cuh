@@ -48,17 +48,11 @@ __device__ __forceinline__ unsigned long long tile_start(const PipeDev &p, uint3
   return q;
 }
 
-// Halo tiles the tiled table update (stc_table.cu) needs this step, or 0:
-// the step takes the general path (k_hits, k_insert_ordered, k_sweep).
-constexpr uint32_t MAX_HALO = 15;
-constexpr uint32_t MIN_TILES = 14;  // a smaller table is not worth tiles
+// Halo tiles of the step's tiled table update (stc_table.cu), or 0: the step
+// takes the general path.
 __device__ __forceinline__ uint32_t fuse_halo(const PipeDev &p) {
-  if (p.nb < MIN_TILES || p.st->hit_max > p.bin_cap) return 0;
-  const unsigned long long c = p.st->tile_load, T = p.B / p.nb;
-  if (c >= TILE_LOAD) return 0;  // the carry lists hold TILE_LOAD hits
-  for (uint32_t h = 1; h <= MAX_HALO && 2 * h <= p.nb; h++)
-    if (c * (h + 1) < T * h) return h;
-  return 0;
+  if (p.st->hit_max > p.bin_cap) return 0;
+  return halo_tiles(p.st->tile_load, p.nb, p.B / p.nb);
 }
 
 // (key, claim) pair of a slot in one 16-byte load at L2 (claims change during

@@ -62,7 +62,6 @@ __global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t
   st->tests = st->exact_tests = st->hits = st->ambiguous = 0;
   st->taken = 0;
   st->step_emitted = 0;
-  st->da_iters = 0;
   st->splits = st->merges = st->events = 0;
   st->overflow_objects = 0;
 }
@@ -103,10 +102,12 @@ void init_tables(PipeDev &p, cudaStream_t s) {
 // priority once all instances are merged.
 __global__ void k_insert_ordered(PipeDev p) {
   after_previous();
-  const bool fused = fuse_halo(p) != 0;
-  if (blockIdx.x == 0 && threadIdx.x == 0)  // what the tiled update, or the general path, leaves
-    p.st->packed = !fused ? TABLE_SLOTS : p.st->packed == TABLE_FRONT ? TABLE_BACK : TABLE_FRONT;
-  if (fused) return;
+  const uint32_t halo = fuse_halo(p);
+  if (blockIdx.x == 0 && threadIdx.x == 0) {  // what the tiled update, or the general path, leaves
+    p.st->halo = halo;
+    p.st->packed = !halo ? TABLE_SLOTS : p.st->packed == TABLE_FRONT ? TABLE_BACK : TABLE_FRONT;
+  }
+  if (halo) return;
   const uint32_t t = p.st->step_t;
   // counted and marked again by the sweep
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb * OCC_WORDS; j += gridDim.x * blockDim.x) {

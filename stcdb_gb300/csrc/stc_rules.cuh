@@ -31,6 +31,20 @@ constexpr uint32_t TILE_SLOTS = 768;    // largest tile
 constexpr uint32_t TILE_LOAD = 704;     // (occupied slots + hits) of a tile stay below this on the tiled path
 constexpr uint32_t HIT_CHUNK = 16;      // records of a bin that lie together (hit_place)
 
+// Halo tiles the tiled table update needs for a step whose fullest tile has
+// `load` occupied slots and hits, in a table of nb tiles of `slots` slots or
+// one more; 0: the step takes the general path (k_hits, k_insert_ordered,
+// k_sweep). Why that many, see stc_table.cu.
+constexpr uint32_t MAX_HALO = 15;
+constexpr uint32_t MIN_TILES = 14;  // a smaller table is not worth tiles
+__host__ __device__ __forceinline__ uint32_t halo_tiles(unsigned long long load, uint32_t nb,
+                                                        unsigned long long slots) {
+  if (nb < MIN_TILES || load >= TILE_LOAD) return 0;  // the carry lists hold TILE_LOAD hits
+  for (uint32_t h = 1; h <= MAX_HALO && 2 * h <= nb; h++)
+    if (load * (h + 1) < slots * h) return h;
+  return 0;
+}
+
 // Records per bin when `total` are spread over nb bins, rounded up (at least 1;
 // a run of bins stays below 2^32 records).
 inline uint32_t bin_share(uint64_t total, uint32_t nb) {

@@ -349,6 +349,8 @@ def _lib():
         lib.stc_query_box.argtypes = [ctypes.c_void_p, ctypes.c_void_p, ctypes.c_uint32, ctypes.c_uint32,
                                       ctypes.c_void_p, ctypes.c_size_t, ctypes.POINTER(ctypes.c_size_t)]
         lib.stc_query_box.restype = ctypes.c_int
+        lib.stc_table_halo.argtypes = [ctypes.c_void_p]
+        lib.stc_table_halo.restype = ctypes.c_uint32
         lib._stc_typed = True
     return lib
 
@@ -403,6 +405,10 @@ class Pipeline:
         s = StcStats()
         self._check(self._lib.stc_get_stats(self._h, ctypes.byref(s)))
         return s
+
+    def table_halo(self) -> int:
+        """Halo tiles of the last step's tiled table update; 0: the general one."""
+        return int(self._lib.stc_table_halo(self._h))
 
     def drain_some(self, out: np.ndarray) -> np.ndarray:
         """Up to len(out) pending meetings (stc_drain_meetings) into `out`, a
