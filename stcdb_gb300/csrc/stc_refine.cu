@@ -413,13 +413,14 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
 }
 
 // The pair tests of a step whose bins overflowed while the table's tiles were
-// packed, once more, by the whole grid.
-__device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows) {
+// packed, once more: part `part` of `parts` of the jobs, by the whole grid.
+__device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows, uint32_t part, uint32_t parts) {
   const uint32_t t = p.st->step_t;
   const unsigned long long warp = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5;
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
+  const unsigned long long J = p.st->jobs_total, J1 = J * (part + 1) / parts;
   Counters ct = {0, 0, 0, 0};  // counted the first time
-  for (unsigned long long job = warp; job < p.st->jobs_total; job += nwarps) {
+  for (unsigned long long job = J * part / parts + warp; job < J1; job += nwarps) {
     if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
     const uint4 w = p.jobs[job];
     for (uint32_t c = 0; c < w.w; c++)
@@ -433,22 +434,24 @@ __device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows) {
 // claims, and more registers, for redo_pairs, leave fewer warps: 371M hits in a
 // table of 2^30 slots, two thirds of its slots and hits a tile, 85 ms with a
 // warp a bin and 80 registers, 63 this way.
+// Part `part` of `parts` takes that part of the bins.
 constexpr uint32_t HITS_LANE = 8;
-__global__ void __launch_bounds__(256, 5) k_hits(PipeDev p) {
+__global__ void __launch_bounds__(256, 5) k_hits(PipeDev p, uint32_t part, uint32_t parts) {
   after_previous();
   if (fuse_halo(p)) return;
   __shared__ Row rows_all[256 / 32][32];
   if (p.st->redo) {
-    redo_pairs(p, rows_all[threadIdx.x >> 5]);
+    redo_pairs(p, rows_all[threadIdx.x >> 5], part, parts);
     return;
   }
   const uint32_t t = p.st->step_t;
   const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
-  const uint32_t parts = (min((uint32_t)p.st->hit_max, p.bin_cap) + HITS_LANE - 1) / HITS_LANE;  // of the fullest bin
+  const uint32_t turns = (min((uint32_t)p.st->hit_max, p.bin_cap) + HITS_LANE - 1) / HITS_LANE;  // of the fullest bin
   const unsigned long long groups = (p.nb + 31u) / 32u;
-  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < groups * parts;
+  const unsigned long long g0 = groups * part / parts, g1 = groups * (part + 1) / parts;
+  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (g1 - g0) * turns;
        w += warps) {
-    const uint32_t bin = (uint32_t)(w / parts) * 32u + lane_id(), i0 = (uint32_t)(w % parts) * HITS_LANE;
+    const uint32_t bin = (uint32_t)(g0 + w / turns) * 32u + lane_id(), i0 = (uint32_t)(w % turns) * HITS_LANE;
     if (bin >= p.nb) continue;
     const uint32_t n = min(min(p.bin_cnt[bin], p.bin_cap), i0 + HITS_LANE);
     for (uint32_t i = i0; i < n; i += 2) {
@@ -529,7 +532,8 @@ void step_pairs(PipeDev &p, cudaStream_t s) {
 
 void step_hits(PipeDev &p, cudaStream_t s) {
   const unsigned most = std::max<unsigned>(p.nb, 4 * num_sms());
-  launch_behind(k_hits, std::min<unsigned>(num_sms() * p.hits_bps, most), 256, 0, s, p);
+  for (uint32_t part = 0; part < p.slices; part++)
+    launch_behind(k_hits, std::min<unsigned>(num_sms() * p.hits_bps, most), 256, 0, s, p, part, p.slices);
 }
 
 }  // namespace stc
