@@ -82,6 +82,8 @@ struct __align__(16) U128 {
 // packed in slot order at the front or the back of the tile, the slots being
 // the marks of PipeDev::occ (stc_table.cu).
 enum TableLayout : uint32_t { TABLE_SLOTS = 0, TABLE_FRONT = 1, TABLE_BACK = 2 };
+constexpr unsigned long long HALO_TOLD = ~0ull;  // the step was told to take the general path
+constexpr uint32_t TOLD_STALE = 1u << 31;  // tile_live and occ are not the table's: the step before did not count
 
 // Small device-resident control block.
 struct DevState {
@@ -95,14 +97,16 @@ struct DevState {
   unsigned long long tests, exact_tests, hits, ambiguous;
   unsigned long long taken;
   unsigned long long step_emitted;
-  unsigned long long halo;            // halo tiles of the step's tiled table update; 0: general path
-  uint32_t splits, merges, events, overflow_objects;
+  unsigned long long halo;            // halo tiles of the step's tiled table update; 0: general path; HALO_TOLD
+  uint32_t splits, merges;
+  uint32_t told;                      // steps told to be general in a row (PathChoice); TOLD_STALE
+  uint32_t overflow_objects;
   uint32_t build_nodes, build_leaves, build_active, build_level;
   uint32_t work_next;                 // generic persistent-kernel work counter
   uint32_t step_t;                    // time of the step in flight (set at its start)
   uint32_t packed;                    // layout of the meeting table's tiles (TableLayout)
   uint32_t redo;                      // a bin overflowed while the tiles were packed (stc_refine.cu, bin_hit)
-  unsigned long long border_points;   // points whose lookup starts above their leaf
+  unsigned long long hit_count;       // places taken in the hit buffer by a step told to be general
   unsigned long long fast_claims;     // new meetings started this step (claims finalised by the sweep)
   unsigned long long hit_max;         // most hits of a table tile this step
   uint32_t schema_path;               // 1 parallel replay, 2 serial (cascade), 0 serial (other)

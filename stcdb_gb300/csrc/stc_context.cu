@@ -55,8 +55,12 @@ struct stc_ctx {
   int device = 0;
   cudaStream_t stream = nullptr;
   cudaStream_t side = nullptr;   // border units, beside the leaf order
+  cudaStream_t hits = nullptr;   // the table update of general steps, beside the pair tests
   cudaStream_t side2 = nullptr;  // the schema update, beside the table update and sweep
   cudaEvent_t fork_ev = nullptr, join_ev = nullptr, fork2_ev = nullptr, join2_ev = nullptr;
+  cudaEvent_t part_ev = nullptr, hits_ev = nullptr;  // general steps: a part's hits are there; all are applied
+  PathChoice path;               // of the steps to come
+  bool no_growth = false;        // the hit bins could not grow
   cudaEvent_t ev[PH_COUNT] = {};
   std::string err;
   bool failed = false;
@@ -223,9 +227,12 @@ static void destroy_all(stc_ctx *c) {
     if (c->ev[i]) cudaEventDestroy(c->ev[i]);
   if (c->fork_ev) cudaEventDestroy(c->fork_ev);
   if (c->fork2_ev) cudaEventDestroy(c->fork2_ev);
+  if (c->part_ev) cudaEventDestroy(c->part_ev);
+  if (c->hits_ev) cudaEventDestroy(c->hits_ev);
   if (c->join2_ev) cudaEventDestroy(c->join2_ev);
   if (c->join_ev) cudaEventDestroy(c->join_ev);
   if (c->side) cudaStreamDestroy(c->side);
+  if (c->hits) cudaStreamDestroy(c->hits);
   if (c->side2) cudaStreamDestroy(c->side2);
   if (c->stream) cudaStreamDestroy(c->stream);
 }
@@ -332,11 +339,15 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   if (e == cudaSuccess) e = cudaDeviceGetStreamPriorityRange(&least_prio, &greatest_prio);
   const int side_prio = std::min(least_prio, greatest_prio + 1);
   if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->side, cudaStreamNonBlocking, side_prio);
+  // (not ahead of the pair tests: they would wait for each part's update)
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->hits, cudaStreamNonBlocking);
   if (e == cudaSuccess) e = cudaStreamCreateWithPriority(&c->side2, cudaStreamNonBlocking, side_prio);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->fork2_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->join2_ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->part_ev, cudaEventDisableTiming);
+  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->hits_ev, cudaEventDisableTiming);
   for (int i = 0; i < PH_COUNT && e == cudaSuccess; i++) e = cudaEventCreate(&c->ev[i]);
   if (e == cudaSuccess) e = cudaMallocHost(&c->st_host, sizeof(DevState));
   if (e == cudaSuccess) e = cudaMallocHost(&c->t_pinned, WIN_BUFS * sizeof(uint32_t));
@@ -447,7 +458,7 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
             dalloc(c, &p.bu_gid, p.U_cap) && dalloc(c, &p.bu_pid, p.U_cap) && dalloc(c, &p.bu_rank, p.U_cap) &&
             dalloc(c, &p.bu_sorted_pos, p.U_cap) && dalloc(c, &p.bu_cnt, p.G) && dalloc(c, &p.bu_start, p.G) &&
             dalloc(c, &p.slots, p.B) &&
-            dalloc(c, &p.hits, hit_records(p.nb, p.bin_cap)) && dalloc(c, &p.bin_cnt, p.nb) &&
+            dalloc(c, &p.hits, hit_records(p.nb, p.bin_cap)) && dalloc(c, &p.bin_cnt, p.nb) && dalloc(c, &p.hit_bounds, MAX_SLICES + 1) &&
             dalloc(c, &p.tile_live, p.nb) && dalloc(c, &p.occ, (size_t)p.nb * OCC_WORDS) && dalloc(c, &p.carry, (size_t)p.runs * TILE_LOAD) &&
             dalloc(c, &p.carry_cnt, p.runs) && dalloc(c, &p.cset, p.C) &&
             dalloc(c, &p.cand_list, p.cand_cap) && dalloc(c, &p.emit, p.E);
@@ -602,8 +613,23 @@ static void issue_step(stc_ctx *c, bool events, bool append, const uint32_t *two
   if (events) cudaEventRecord(c->ev[PH_PART], s);
   cudaStreamWaitEvent(s, c->join2_ev, 0);
   if (events) cudaEventRecord(c->ev[PH_BORDER], s);
-  step_pairs(p, s);
-  if (events) cudaEventRecord(c->ev[PH_REFINE], s);
+  if (p.general) {
+    // the pair tests in parts; each part's hits are applied to the table on
+    // another stream while the next part's pairs are tested (new meetings
+    // take their slots by priority, so concurrent updates are safe)
+    step_table_slots(p, s);
+    const uint32_t parts = std::max(p.slices, GENERAL_PARTS);
+    for (uint32_t part = 0; part < parts; part++) {
+      step_pairs_part(p, part, parts, s);
+      cudaEventRecord(c->part_ev, s);
+      cudaStreamWaitEvent(c->hits, c->part_ev, 0);
+      step_hits_part(p, part, c->hits);
+    }
+    cudaEventRecord(c->hits_ev, c->hits);
+  } else {
+    step_pairs(p, s);
+    if (events) cudaEventRecord(c->ev[PH_REFINE], s);
+  }
   // The schema update reads this step's leaf counts and rewrites quadtree
   // nodes, which only the pair tests read: once they are done it runs on a
   // third stream while the table update, sweep and memtable append run (none
@@ -617,13 +643,19 @@ static void issue_step(stc_ctx *c, bool events, bool append, const uint32_t *two
                   (c->cfg.flags & STC_FLAG_SERIAL_SCHEMA) != 0, p.st, c->side2);
     cudaEventRecord(c->join_ev, c->side2);
   }
+  if (p.general) {
+    cudaStreamWaitEvent(s, c->hits_ev, 0);
+    if (events) cudaEventRecord(c->ev[PH_REFINE], s);
+  }
   step_table_plan(p, s);
   if (events) cudaEventRecord(c->ev[PH_INSERT], s);
   if (c->gate_ev) cudaEventRecord(c->gate_ev, s);
-  step_table(p, s);
-  // the general path, for a step the tiled one cannot take (decided on the
-  // device; otherwise these return at once)
-  step_hits(p, s);
+  if (!p.general) {
+    step_table(p, s);
+    // the general path, for a step the tiled one cannot take (decided on the
+    // device; otherwise these return at once)
+    step_hits(p, s);
+  }
   step_insert(p, s);
   step_sweep(p, s);
   if (events) cudaEventRecord(c->ev[PH_SWEEP], s);
@@ -662,6 +694,30 @@ static stc_status capture_step(stc_ctx *c, int b) {
   return STC_OK;
 }
 
+// Records a bin that the step in c->st_host would have wanted: those of its
+// fullest bin, or, in sequence, its hits spread over the buffer.
+static unsigned long long bin_need(const stc_ctx *c) {
+  const DevState &st = *c->st_host;
+  return st.halo == HALO_TOLD ? bin_share(st.hit_count, c->p.nb) : st.hit_max;
+}
+
+// Records per bin after steps whose fullest bin had `fullest` hits and whose
+// largest step had `hits`. With the automatic hit capacity (stc_config.
+// hit_capacity 0) the bins grow, within the bounds of bin_cap_grown: a hit
+// beyond its bin costs the step the general path, and is applied inside the
+// pair tests, or, while the table's tiles are packed, by a second run of them.
+static uint32_t bins_wanted(const stc_ctx *c, unsigned long long fullest, unsigned long long hits) {
+  return c->cfg.hit_capacity || c->no_growth ? c->p.bin_cap : bin_cap_grown(c->p.bin_cap, fullest, hits, c->p.nb);
+}
+
+// Chooses the path of the steps to come by the step in c->st_host.
+static void choose_path(stc_ctx *c) {
+  const DevState &st = *c->st_host;
+  const bool told = st.halo == HALO_TOLD;
+  const unsigned long long fullest = !told ? st.hit_max : st.tile_load == LOAD_UNKNOWN ? 0 : st.tile_load + st.tile_load / 16;
+  c->path.step_done(told, st.tile_load, fullest, bins_wanted(c, fullest, st.hits), c->p.nb, c->p.B / c->p.nb);
+}
+
 // Counters of the step whose state is in c->st_host.
 static void fill_stats(stc_ctx *c, uint32_t t, const float *phase, float step_ms, uint32_t launches) {
   const DevState &h = *c->st_host;
@@ -690,30 +746,23 @@ static void fill_stats(stc_ctx *c, uint32_t t, const float *phase, float step_ms
   o.memtable_keys = h.kv_count;
   c->stepped = true;
   c->last_t = t;
+  choose_path(c);
 }
 
 // The reference flushes once a step leaves more keys than kv_restriction
 // (cuda/geometry.cu:1752).
 static bool flush_due(const stc_ctx *c) { return c->lsm_on && c->st_host->kv_count > c->cfg.kv_restriction; }
 
-// Records per bin after steps whose fullest bin had `fullest` hits and whose
-// largest step had `hits`. With the automatic hit capacity (stc_config.
-// hit_capacity 0) the bins grow, within the bounds of bin_cap_grown: a hit
-// beyond its bin costs the step the general path, and is applied inside the
-// pair tests, or, while the table's tiles are packed, by a second run of them.
-static uint32_t bins_wanted(const stc_ctx *c, unsigned long long fullest, unsigned long long hits) {
-  return c->cfg.hit_capacity ? c->p.bin_cap : bin_cap_grown(c->p.bin_cap, fullest, hits, c->p.nb);
-}
-
-// Gives the bins room for `cap` records each; false when there is no memory
-// for that, which keeps the old ones. Called only with no step in flight.
-static bool grow_hits(stc_ctx *c, uint32_t cap) {
+// Gives the bins room for `cap` records each; where there is no memory for
+// that they keep their size from then on. Called only with no step in flight.
+static void grow_hits(stc_ctx *c, uint32_t cap) {
   PipeDev &p = c->p;
-  if (cap <= p.bin_cap) return true;
+  if (cap <= p.bin_cap) return;
   void *h = nullptr;
   if (dev_malloc(&h, hit_records(p.nb, cap) * sizeof(HitRec)) != cudaSuccess) {
     cudaGetLastError();
-    return false;
+    c->no_growth = true;
+    return;
   }
   for (void *&a : c->allocs)
     if (a == (void *)p.hits) {
@@ -723,7 +772,6 @@ static bool grow_hits(stc_ctx *c, uint32_t cap) {
   p.hits = (HitRec *)h;
   p.bin_cap = cap;
   invalidate_graphs(c);  // the graphs hold the buffer by value
-  return true;
 }
 
 // Tile length of the refinement's jobs when stc_config.refine_chunk is 0.
@@ -755,13 +803,15 @@ static void choose_refine_chunk(stc_ctx *c) {
     else
       chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * units ? REFINE_CHUNK_DENSE : REFINE_CHUNK_DEFAULT;
   }
-  const uint32_t chunk0 = p.refine_chunk, share0 = p.job_share;
+  const uint32_t chunk0 = p.refine_chunk, share0 = p.job_share, general0 = p.general;
   p.refine_chunk = chunk;
+  p.general = c->path.general;
   // by the last step's jobs; a quarter fewer before it changes back
   const unsigned long long jobs = c->st_host->jobs_total;
   const unsigned long long warps = (unsigned long long)num_sms() * refine_blocks(p) * (REFINE_THREADS / 32);
   p.job_share = jobs_may_share(c->cfg.job_chunk) && job_shares(share0 ? jobs + jobs / 4 : jobs, warps, chunk);
-  if (chunk != chunk0 || p.job_share != share0) invalidate_graphs(c);  // the captured steps carry both
+  if (chunk != chunk0 || p.job_share != share0 || p.general != general0)
+    invalidate_graphs(c);  // the captured steps carry all three
 }
 
 static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copied) {
@@ -782,7 +832,7 @@ static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copie
   float tot = 0;
   cudaEventElapsedTime(&tot, c->ev[PH_START], c->ev[PH_SCHEMA]);
   fill_stats(c, t, phase, tot, (uint32_t)(tl_launches - launches0));
-  grow_hits(c, bins_wanted(c, c->st_host->hit_max, c->st_host->hits));
+  grow_hits(c, bins_wanted(c, bin_need(c), c->st_host->hits));
   if (flush_due(c)) return flush_now(c, t);
   return STC_OK;
 }
@@ -1044,7 +1094,6 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
   double busy_ms = 0;  // device time of the window's steps
   size_t n = 0;
   unsigned long long fullest = 0, most_hits = 0;  // the window's fullest bin and largest step (the bins grow by them)
-  bool may_grow = true;                           // no attempt has failed
   unsigned long long dpos = 0;  // emit records [0, dpos) are on their way to out
   bool out_full = false;
   stc_status rs = STC_OK;
@@ -1077,7 +1126,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       busy_ms += c->stats.step_ms;
     }
     if (rs == STC_OK) {
-      fullest = std::max(fullest, c->st_host->hit_max);
+      fullest = std::max(fullest, bin_need(c));
       most_hits = std::max(most_hits, c->st_host->hits);
     }
     if (rs == STC_OK && out && !out_full) {
@@ -1127,7 +1176,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
           if (e != cudaSuccess) return cuda_fail(c, e, "stc_step_window drain");
           dpos = 0;
         }
-        may_grow = may_grow && grow_hits(c, bins_wanted(c, fullest, most_hits));
+        grow_hits(c, bins_wanted(c, fullest, most_hits));
         hold = false;
         rs = issue_core(i + 1);
         if (rs == STC_OK && i + WIN_BUFS < steps) {
@@ -1149,7 +1198,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
       if (out && c->st_host->emit_count > p.E / 2) hold = true;
       // a step found more hits than a bin holds: grow the bins at the next
       // step boundary
-      if (may_grow && bins_wanted(c, fullest, most_hits) > p.bin_cap) hold = true;
+      if (bins_wanted(c, fullest, most_hits) > p.bin_cap) hold = true;
     }
   }
   cudaStreamSynchronize(c->copy_stream);
@@ -1158,7 +1207,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
     if (e != cudaSuccess) return cuda_fail(c, e, "stc_step_window drain");
   }
   cudaStreamSynchronize(s);
-  if (may_grow) grow_hits(c, bins_wanted(c, fullest, most_hits));
+  grow_hits(c, bins_wanted(c, fullest, most_hits));
   c->stats.window_device_ms = (float)busy_ms;
   c->stats.window_input_wait_ms = (float)wait_ms;
   c->stats.window_copy_ms = (float)copy_ms;
@@ -1671,6 +1720,7 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
   cudaFreeHost(stage);
   if (!bad.empty()) return bail(STC_ERR_INVALID_ARG, bad);
   fclose(f);
+  h.st.told = 0;  // its tiles are counted again below
   e = cudaMemcpy(c->p.st, &h.st, sizeof(DevState), cudaMemcpyHostToDevice);
   if (e != cudaSuccess) {
     g_create_error = std::string("stc_restore: ") + cudaGetErrorString(e);
@@ -1712,7 +1762,7 @@ extern "C" stc_status stc_restore(const char *path, uint32_t device, stc_ctx **o
   return STC_OK;
 }
 
-extern "C" uint32_t stc_table_halo(const stc_ctx *c) { return c && c->stepped ? (uint32_t)c->st_host->halo : 0; }
+extern "C" uint32_t stc_table_halo(const stc_ctx *c) { return c && c->stepped && c->st_host->halo != HALO_TOLD ? (uint32_t)c->st_host->halo : 0; }
 
 extern "C" stc_status stc_get_config(const stc_ctx *c, stc_config *cfg) {
   if (!c || !cfg) return STC_ERR_INVALID_ARG;

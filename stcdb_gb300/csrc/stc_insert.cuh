@@ -51,7 +51,7 @@ __device__ __forceinline__ unsigned long long tile_start(const PipeDev &p, uint3
 // Halo tiles of the step's tiled table update (stc_table.cu), or 0: the step
 // takes the general path.
 __device__ __forceinline__ uint32_t fuse_halo(const PipeDev &p) {
-  if (p.st->hit_max > p.bin_cap) return 0;
+  if (p.general || p.st->hit_max > p.bin_cap) return 0;
   return halo_tiles(p.st->tile_load, p.nb, p.B / p.nb);
 }
 

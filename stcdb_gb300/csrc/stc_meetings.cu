@@ -46,6 +46,7 @@ __global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t
   if (first < CTR_COUNT) p.ctr[first] = 0;
   if (first) return;
   DevState *st = p.st;
+  const uint32_t told = st->told & ~TOLD_STALE;
   const uint32_t t = *(const volatile uint32_t *)t_pinned;
   st->same_t = t == st->step_t;
   st->step_t = t;
@@ -53,7 +54,7 @@ __global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t
   st->error = 0;
   st->error_info = 0;
   st->border_units = 0;
-  st->border_points = 0;
+  st->hit_count = 0;
   st->fast_claims = 0;
   st->hit_max = 0;
   st->jobs_total = 0;
@@ -62,7 +63,8 @@ __global__ void __launch_bounds__(256) k_step_begin(PipeDev p, const uint32_t *t
   st->tests = st->exact_tests = st->hits = st->ambiguous = 0;
   st->taken = 0;
   st->step_emitted = 0;
-  st->splits = st->merges = st->events = 0;
+  st->splits = st->merges = 0;
+  st->told = (p.general ? told + 1 : 0) | (told % COUNT_EVERY ? TOLD_STALE : 0);
   st->overflow_objects = 0;
 }
 
@@ -98,21 +100,27 @@ void init_tables(PipeDev &p, cudaStream_t s) {
   STC_KL k_init_cands<<<num_sms() * 8, 256, 0, s>>>(p.cset, p.C);
 }
 
+// Whether this general step leaves its tiles' counts and marks.
+__device__ __forceinline__ bool counts_tiles(const PipeDev &p) {
+  return !p.general || (p.st->told & ~TOLD_STALE) % COUNT_EVERY == 0;
+}
+
 // Candidates that may occur twice in a step: walk with their minimum
 // priority once all instances are merged.
 __global__ void k_insert_ordered(PipeDev p) {
   after_previous();
   const uint32_t halo = fuse_halo(p);
   if (blockIdx.x == 0 && threadIdx.x == 0) {  // what the tiled update, or the general path, leaves
-    p.st->halo = halo;
+    p.st->halo = p.general ? HALO_TOLD : halo;
     p.st->packed = !halo ? TABLE_SLOTS : p.st->packed == TABLE_FRONT ? TABLE_BACK : TABLE_FRONT;
   }
   if (halo) return;
   const uint32_t t = p.st->step_t;
-  // counted and marked again by the sweep
-  for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb * OCC_WORDS; j += gridDim.x * blockDim.x) {
-    p.occ[j] = 0;
-    if (j < p.nb) p.tile_live[j] = 0;
+  if (counts_tiles(p)) {  // counted and marked again by the sweep
+    for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb * OCC_WORDS; j += gridDim.x * blockDim.x) {
+      p.occ[j] = 0;
+      if (j < p.nb) p.tile_live[j] = 0;
+    }
   }
   const unsigned long long nc = p.st->cand_count < p.cand_cap ? p.st->cand_count : p.cand_cap;
   for (unsigned long long c = (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; c < nc;
@@ -256,9 +264,11 @@ __device__ __forceinline__ void flush_emits(const PipeDev &p, const stc_meeting 
 }
 
 // Slice `part` of `parts` sweeps slots [B * part / parts, B * (part + 1) / parts).
+// COUNTS: and counts and marks the tiles' live slots (counts_tiles).
+template <bool COUNTS>
 __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(PipeDev p, uint32_t part, uint32_t parts) {
   after_previous();
-  if (fuse_halo(p)) return;
+  if (fuse_halo(p) || counts_tiles(p) != COUNTS) return;
   const uint32_t t = p.st->step_t;
   __shared__ __align__(16) stc_meeting stage_all[SWEEP_WARPS][WARP_STAGE];
   const uint32_t lane = lane_id(), warp = threadIdx.x >> 5;
@@ -286,7 +296,7 @@ __global__ void __launch_bounds__(SWEEP_THREADS, SWEEP_BLOCKS_PER_SM) k_sweep(Pi
     for (uint32_t u = 0; u < SWEEP_UNROLL; u++) {
       const unsigned long long before = active;
       bool emit = idx[u] < B && sweep_slot(p, t, idx[u], sl[u], cp[u], active, fresh);
-      count_live(p, idx[u], active != before);
+      if (COUNTS) count_live(p, idx[u], active != before);
       uint32_t ball = __ballot_sync(0xffffffffu, emit);
       if (emit) {
         stc_meeting m;
@@ -334,8 +344,10 @@ void step_sweep(PipeDev &p, cudaStream_t s) {
   const unsigned blocks = (unsigned)std::min<unsigned long long>(
       (unsigned long long)num_sms() * SWEEP_BLOCKS_PER_SM * SWEEP_WAVES,
       p.B / (4 * SWEEP_WARPS * WARP_TILE) + 1);
-  for (uint32_t part = 0; part < p.slices; part++)
-    launch_behind(k_sweep, blocks, SWEEP_THREADS, 0, s, p, part, p.slices);
+  for (uint32_t part = 0; part < p.slices; part++) {
+    launch_behind(k_sweep<true>, blocks, SWEEP_THREADS, 0, s, p, part, p.slices);
+    if (p.general) launch_behind(k_sweep<false>, blocks, SWEEP_THREADS, 0, s, p, part, p.slices);
+  }
 }
 
 }  // namespace stc

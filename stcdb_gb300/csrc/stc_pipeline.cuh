@@ -50,6 +50,7 @@ struct PipeDev {
   int mbr_filter;
   uint32_t slices;                 // launches per long step kernel (stc_config.step_slices)
   uint32_t job_chunk;              // refinement jobs a warp takes at a time (stc_config.job_chunk)
+  uint32_t general;                // 1: this step takes the general path, whatever its tiles (PathChoice)
   uint32_t job_share;              // 1: or one at a time from a common counter (job_shares)
   uint32_t refine_chunk;               // candidate positions per refinement job (a multiple of 32)
   uint32_t refine_bps, hits_bps;   // blocks per SM of the pair tests (0: step_pairs chooses) and of the table update
@@ -100,6 +101,7 @@ struct PipeDev {
   // min(bin_cnt[j], bin_cap) records, at hit_place; a hit its bin has no room
   // for is applied inside the pair tests
   HitRec *hits;                         // hit_records(nb, bin_cap)
+  unsigned long long *hit_bounds;       // [MAX_SLICES + 1]: end of each part's hits (general steps)
   uint32_t nb, bin_cap;                 // tiles of the table, records per bin
   unsigned long long nb_magic;          // ceil(2^64 / nb)
   uint32_t *bin_cnt;                    // nb
@@ -121,7 +123,7 @@ struct PipeDev {
 __host__ __device__ __forceinline__ unsigned long long hit_place(const PipeDev &p, uint32_t j, uint32_t i) {
   return ((unsigned long long)(i / HIT_CHUNK) * p.nb + j) * HIT_CHUNK + i % HIT_CHUNK;
 }
-inline size_t hit_records(uint32_t nb, uint32_t bin_cap) {
+__host__ __device__ __forceinline__ size_t hit_records(uint32_t nb, uint32_t bin_cap) {
   return (size_t)nb * ((bin_cap + HIT_CHUNK - 1) / HIT_CHUNK * HIT_CHUNK);
 }
 
@@ -156,6 +158,12 @@ void step_border(PipeDev &p, cudaStream_t s);
 // path's table update of them (nothing when the tiled path took the step)
 void step_pairs(PipeDev &p, cudaStream_t s);
 void step_hits(PipeDev &p, cudaStream_t s);
+// of a step told to be general: part `part` of `parts` of the pair tests, whose
+// hits go to the buffer in sequence, and the table update of them, which may
+// run beside the next part
+constexpr uint32_t GENERAL_PARTS = 4;  // or more, for step_slices
+void step_pairs_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s);
+void step_hits_part(PipeDev &p, uint32_t part, cudaStream_t s);
 // stc_table.cu: the tiled table update and sweep. plan decides whether the
 // step takes it and finds what is carried into each run of tiles.
 constexpr uint32_t OCC_WORDS = TILE_SLOTS / 32;
@@ -163,6 +171,7 @@ cudaError_t table_prepare();
 void table_sizes(PipeDev &p);           // nb and runs of a table of p.B slots
 void count_tiles(PipeDev &p, cudaStream_t s);
 void unpack_tiles(PipeDev &p, uint32_t layout, cudaStream_t s);  // every meeting into its slot
+void step_table_slots(PipeDev &p, cudaStream_t s);  // the same if the tiles are packed
 void step_table_plan(PipeDev &p, cudaStream_t s);
 void step_table(PipeDev &p, cudaStream_t s);
 // stc_meetings.cu: the general path's insert and sweep

@@ -37,8 +37,9 @@
 // Hits (tracing/refinement.cpp:34-55) go to the bin of the table tile their
 // home slot key % B lies in, with their position in the reference's
 // sequential processing order: unit rank << order_shift | pid. stc_table.cu
-// applies them; the general path here (k_hits) does so for a step whose tiles
-// are too full: a key found before the first empty slot is extended in place
+// applies them; the general path here does so for a step whose tiles are too
+// full (k_hits) and for the steps told so beforehand, whose hits are not binned
+// (k_hits_part): a key found before the first empty slot is extended in place
 // (end = t, MBR), every other key walks on for a slot by priority.
 #include <algorithm>
 
@@ -162,6 +163,46 @@ __device__ __forceinline__ void bin_hit(const PipeDev &p, const HitRec &h, uint3
   else p.st->redo = 1;
 }
 
+// Steps told to be general (PathChoice) leave their hits in sequence instead: a
+// warp takes HIT_WINDOW places of the buffer at a time, more the more it has
+// taken (508M hits in windows of 64, 256, up to 1024: 102, 94, 94 ms a step, by
+// the shared counter), and the rest of its last ones stay empty (a = STC_NONE).
+// Random to the table, but the update of one part runs beside the tests of the
+// next, and a crowd's long walks are spread over all warps. Stress model, ms a
+// step with bins and k_hits behind all pair tests, and this way: 1M objects at
+// 0.47 meetings a slot 104, 90; 200k at 0.35 3.68, 3.73, at 0.5 5.2, 5.3, at 0.6
+// 80, 40.
+constexpr uint32_t HIT_WINDOW = 64, HIT_WINDOW_MOST = 1024;
+struct HitWindow {
+  unsigned long long next, end;  // the same for the whole warp
+  uint32_t taken;                // places so far
+};
+__device__ __forceinline__ void window_rest(const PipeDev &p, const HitWindow &w) {
+  const unsigned long long room = hit_records(p.nb, p.bin_cap);
+  for (unsigned long long i = w.next + lane_id(); i < w.end; i += 32)
+    if (i < room) p.hits[i].a = STC_NONE;
+}
+// The round's hits (one a lane with has set); the ones the buffer has no room
+// for are applied here. Called by the whole warp.
+__device__ __forceinline__ void append_round(const PipeDev &p, const HitRec &h, bool has, uint32_t t, HitWindow &w) {
+  const uint32_t hm = __ballot_sync(0xffffffffu, has), cnt = __popc(hm);
+  if (w.end - w.next < cnt) {
+    window_rest(p, w);
+    const uint32_t size = min(max(w.taken / 4, HIT_WINDOW), HIT_WINDOW_MOST);
+    unsigned long long base = 0;
+    if (lane_id() == 0) base = atomicAdd(&p.st->hit_count, (unsigned long long)size);
+    w.next = __shfl_sync(0xffffffffu, base, 0);
+    w.end = w.next + size;
+    w.taken += size;
+  }
+  if (has) {
+    const unsigned long long pos = w.next + __popc(hm & ((1u << lane_id()) - 1u));
+    if (pos < hit_records(p.nb, p.bin_cap)) store_hit(&p.hits[pos], h);
+    else process_hit(p, h, t);
+  }
+  w.next += cnt;
+}
+
 __device__ __forceinline__ HitRec load_hit(const HitRec *r) {
   // streamed once: evict-first loads keep L2 for the table and positions
   const ulonglong2 v = __ldcs((const ulonglong2 *)r);
@@ -230,11 +271,13 @@ struct __align__(16) Row {
 // records' stores 2.85, or 2.4 in chunks (hit_place): bound by the rate of
 // scattered stores over that many pages (52 G/s measured). A row per lane and a shared-memory queue
 // of records before it: 3.0 ms for the tests with sequential records.
-// REDO: every hit is applied to the table at once, nothing is binned; the
+// HITS_APPLY: every hit is applied to the table at once, nothing is binned; the
 // schema is not read, which its update may be rewriting.
-template <bool REDO>
+enum HitsGo { HITS_BIN, HITS_APPLY, HITS_APPEND };
+template <HitsGo GO>
 __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblock, uint32_t chunk, uint32_t t,
-                         Counters &ct, Row *rows) {
+                         Counters &ct, Row *rows, HitWindow &window) {
+  constexpr bool REDO = GO == HITS_APPLY;
   const uint32_t lane = lane_id();
   const LeafGeo *lg = &p.lgeo[g];
   const uint32_t base = lg->base, n = lg->n;
@@ -286,7 +329,7 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
       const int c = (int)fminf(fmaxf(floorf(y * lg->inv), -4.0f), (float)H + 4.0f);
       const uint16_t *ss = p.sstart + (size_t)g * STRIP_STRIDE;
       const float4 *sp = p.spts + base;
-      auto window = [&](int sidx, uint32_t &a, uint32_t &len) {
+      auto candidates = [&](int sidx, uint32_t &a, uint32_t &len) {
         if (sidx < 0 || sidx >= H) return;
         const uint32_t st = ss[sidx], en = ss[sidx + 1];
         uint32_t lo = st, hi = en;
@@ -297,9 +340,9 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
         a = lo;
         len = hi - lo;
       };
-      window(c - 1, sa0, sl0);
-      window(c, sa1, sl1);
-      window(c + 1, sa2, sl2);
+      candidates(c - 1, sa0, sl0);
+      candidates(c, sa1, sl1);
+      candidates(c + 1, sa2, sl2);
     }
   }
   // this job's chunk: positions [chunk * refine_chunk, (chunk + 1) *
@@ -352,62 +395,70 @@ __device__ void run_rows(const PipeDev &p, uint32_t g, bool own, uint32_t rowblo
     const uint32_t starts = __reduce_or_sync(0xffffffffu, len != 0 && off - f0 < 32u ? 1u << (off - f0) : 0u);
     const uint32_t ri = before + __popc(starts & (0xffffffffu >> (31u - lane))) - 1u;
     before += __popc(starts);
-    if (f0 + lane >= total) continue;
-    const Row *w = &rows[ri];
-    const float4 rp = *(const float4 *)w;
-    const float4 r1 = *((const float4 *)w + 1);
-    const uint4 r2 = *((const uint4 *)w + 2);
-    const uint32_t k = f0 + lane - __float_as_uint(r1.z);
-    const uint32_t e0 = r2.x >> 16, e1 = r2.y >> 16;
-    const uint32_t j = base + (k < e0 ? (r2.x & 0xFFFFu) + k : k < e1 ? (r2.y & 0xFFFFu) + k - e0 : r2.z + k - e1);
-    const float4 c = __ldg(&p.spts[j]);
-    const float2 fc = __ldg(&p.sfxy[j]);
-    const uint32_t pid1 = __float_as_uint(rp.w), pid2 = __float_as_uint(c.w);
-    const bool less = pid1 < pid2;
-    // the reference measures from the unit's point: an own pair from its
-    // lower pid (tracing/refinement.cpp:30), a border pair from the unit
-    const bool swap = own && !less;
-    const float dx = (rp.x - c.x) * (swap ? c.z : rp.z);
-    const float dy = (rp.y - c.y) * STC_SLAT_F;
-    const float d2 = dx * dx + dy * dy;
-    ct.tests++;
-    bool hit = d2 <= lo2;
-    if (!hit && d2 < hi2) {
-      ct.exact++;
-      hit = swap ? exact_within(p, pid2, pid1, ct.amb) : exact_within(p, pid1, pid2, ct.amb);
-    }
-    if (!hit) continue;
-    ct.hits++;
-    HitRec h;
-    h.a = less ? pid1 : pid2;
-    h.b = less ? pid2 : pid1;
-    const float2 f1 = make_float2(r1.x, r1.y), fa = less ? f1 : fc, fb = less ? fc : f1;
-    h.lo_x = fminf(fa.x, fb.x);
-    h.lo_y = fminf(fa.y, fb.y);
-    h.hi_x = fmaxf(fa.x, fb.x);
-    h.hi_y = fmaxf(fa.y, fb.y);
-    if (own) {
-      // the pair is found by the lower pid's own unit (rank = its pid) at
-      // the higher pid's place in the pid-ordered member list
-      h.order = ((unsigned long long)h.a << p.order_shift) | h.b;
-    } else {
-      // border units follow the N own units
-      h.order = (((unsigned long long)p.N + __float_as_uint(r1.w)) << p.order_shift) | pid2;
-      // the member has a unit targeting the row's leaf only if it lies below
-      // that leaf, or left of it and below its top (the border lookup's
-      // rule); rounding to float keeps the order, so the test on floats
-      // passes every such member, and the three dependent loads of its units
-      // are left to the few that pass
-      const float4 r3 = *((const float4 *)w + 3);
-      if (REDO || fc.y <= r3.y || (fc.y <= r3.z && fc.x <= r3.x)) {
-        const uint32_t cnb = p.bcount[pid2];
-        const uint32_t coff = cnb ? p.boff[pid2] : 0u;
-        for (uint32_t u2 = 0; u2 < cnb; u2++)
-          if (p.bu_gid[coff + u2] == r2.w) h.order |= DUP_BIT;
+    // this lane's test; its record if it is a hit
+    auto test = [&](HitRec &h) {
+      const Row *w = &rows[ri];
+      const float4 rp = *(const float4 *)w;
+      const float4 r1 = *((const float4 *)w + 1);
+      const uint4 r2 = *((const uint4 *)w + 2);
+      const uint32_t k = f0 + lane - __float_as_uint(r1.z);
+      const uint32_t e0 = r2.x >> 16, e1 = r2.y >> 16;
+      const uint32_t j = base + (k < e0 ? (r2.x & 0xFFFFu) + k : k < e1 ? (r2.y & 0xFFFFu) + k - e0 : r2.z + k - e1);
+      const float4 c = __ldg(&p.spts[j]);
+      const float2 fc = __ldg(&p.sfxy[j]);
+      const uint32_t pid1 = __float_as_uint(rp.w), pid2 = __float_as_uint(c.w);
+      const bool less = pid1 < pid2;
+      // the reference measures from the unit's point: an own pair from its
+      // lower pid (tracing/refinement.cpp:30), a border pair from the unit
+      const bool swap = own && !less;
+      const float dx = (rp.x - c.x) * (swap ? c.z : rp.z);
+      const float dy = (rp.y - c.y) * STC_SLAT_F;
+      const float d2 = dx * dx + dy * dy;
+      ct.tests++;
+      bool hit = d2 <= lo2;
+      if (!hit && d2 < hi2) {
+        ct.exact++;
+        hit = swap ? exact_within(p, pid2, pid1, ct.amb) : exact_within(p, pid1, pid2, ct.amb);
       }
+      if (!hit) return false;
+      ct.hits++;
+      h.a = less ? pid1 : pid2;
+      h.b = less ? pid2 : pid1;
+      const float2 f1 = make_float2(r1.x, r1.y), fa = less ? f1 : fc, fb = less ? fc : f1;
+      h.lo_x = fminf(fa.x, fb.x);
+      h.lo_y = fminf(fa.y, fb.y);
+      h.hi_x = fmaxf(fa.x, fb.x);
+      h.hi_y = fmaxf(fa.y, fb.y);
+      if (own) {
+        // the pair is found by the lower pid's own unit (rank = its pid) at
+        // the higher pid's place in the pid-ordered member list
+        h.order = ((unsigned long long)h.a << p.order_shift) | h.b;
+      } else {
+        // border units follow the N own units
+        h.order = (((unsigned long long)p.N + __float_as_uint(r1.w)) << p.order_shift) | pid2;
+        // the member has a unit targeting the row's leaf only if it lies below
+        // that leaf, or left of it and below its top (the border lookup's
+        // rule); rounding to float keeps the order, so the test on floats
+        // passes every such member, and the three dependent loads of its units
+        // are left to the few that pass
+        const float4 r3 = *((const float4 *)w + 3);
+        if (REDO || fc.y <= r3.y || (fc.y <= r3.z && fc.x <= r3.x)) {
+          const uint32_t cnb = p.bcount[pid2];
+          const uint32_t coff = cnb ? p.boff[pid2] : 0u;
+          for (uint32_t u2 = 0; u2 < cnb; u2++)
+            if (p.bu_gid[coff + u2] == r2.w) h.order |= DUP_BIT;
+        }
+      }
+      return true;
+    };
+    HitRec h;
+    if (GO == HITS_APPEND) {
+      const bool has = f0 + lane < total && test(h);
+      append_round(p, h, has, t, window);
+    } else if (f0 + lane < total && test(h)) {
+      if (REDO) process_hit(p, h, t);
+      else bin_hit(p, h, t);
     }
-    if (REDO) process_hit(p, h, t);
-    else bin_hit(p, h, t);
   }
   __syncwarp();
 }
@@ -420,11 +471,12 @@ __device__ __noinline__ void redo_pairs(const PipeDev &p, Row *rows, uint32_t pa
   const unsigned long long nwarps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const unsigned long long J = p.st->jobs_total, J1 = J * (part + 1) / parts;
   Counters ct = {0, 0, 0, 0};  // counted the first time
+  HitWindow none = {0, 0, 0};
   for (unsigned long long job = J * part / parts + warp; job < J1; job += nwarps) {
     if (__shfl_sync(0xffffffffu, (int)stc_failed(p.st), 0)) break;
     const uint4 w = p.jobs[job];
     for (uint32_t c = 0; c < w.w; c++)
-      run_rows<true>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
+      run_rows<HITS_APPLY>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows, none);
   }
 }
 
@@ -475,7 +527,8 @@ __global__ void __launch_bounds__(256, 5) k_hits(PipeDev p, uint32_t part, uint3
 // (job_share): a warp takes its next job from a common counter instead, and a
 // quarter more than its share at most, so that blocks still end, and let query
 // batches in, during the kernel.
-template <bool SHARE>
+// APPEND: the hits in sequence (append_round).
+template <bool SHARE, bool APPEND>
 __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint32_t part, uint32_t parts) {
   __shared__ Row rows_all[REFINE_THREADS / 32][32];
   Row *rows = rows_all[threadIdx.x >> 5];
@@ -488,6 +541,7 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
   const unsigned long long jc = SHARE || !each ? 1ull : each >= p.job_chunk ? p.job_chunk : each;
   const unsigned long long quota = each + each / 4 + 2;
   Counters ct = {0, 0, 0, 0};
+  HitWindow window = {0, 0, 0};
   unsigned long long taken = 0;
   for (unsigned long long j0 = J0 + warp * jc; j0 < J1;) {
     // one lane reads the flag so that the whole warp leaves together
@@ -501,10 +555,12 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
     for (unsigned long long job = j0; job < j1; job++) {
       const uint4 w = p.jobs[job];
       for (uint32_t c = 0; c < w.w; c++)
-        run_rows<false>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows);
+        run_rows<APPEND ? HITS_APPEND : HITS_BIN>(p, w.x, (w.y & JOB_OWN) != 0, w.y & ~JOB_OWN, w.z + c, t, ct, rows,
+                                                  window);
     }
     j0 = SHARE ? __shfl_sync(0xffffffffu, next, 0) : next;
   }
+  if (APPEND) window_rest(p, window);
   // reduce counters per warp (64-bit sums)
   unsigned long long tests = ct.tests, exact = ct.exact, hits = ct.hits, amb = ct.amb;
 #pragma unroll
@@ -525,9 +581,60 @@ __global__ void __launch_bounds__(REFINE_THREADS, 4) k_refine_a(PipeDev p, uint3
 void step_pairs(PipeDev &p, cudaStream_t s) {
   for (uint32_t part = 0; part < p.slices; part++) {
     const unsigned blocks = num_sms() * refine_blocks(p);
-    if (p.job_share) STC_KL k_refine_a<true><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
-    else STC_KL k_refine_a<false><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
+    if (p.job_share) STC_KL k_refine_a<true, false><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
+    else STC_KL k_refine_a<false, false><<<blocks, REFINE_THREADS, 0, s>>>(p, part, p.slices);
   }
+}
+
+// hit_bounds[part + 1] = the end of the hits after part `part` (parts run in
+// stream order).
+__global__ void k_hit_mark(PipeDev p, uint32_t part) {
+  const unsigned long long n = p.st->hit_count, room = hit_records(p.nb, p.bin_cap);
+  p.hit_bounds[part + 1] = n < room ? n : room;
+  if (part == 0) p.hit_bounds[0] = 0;
+}
+
+// The table update of part `part`'s hits, one thread per hit, two in flight:
+// both records and both home slots are requested before either is used.
+__global__ void __launch_bounds__(256) k_hits_part(PipeDev p, uint32_t part) {
+  const uint32_t t = p.st->step_t;
+  const unsigned long long first = p.hit_bounds[part], end = p.hit_bounds[part + 1];
+  const unsigned long long stride = (unsigned long long)gridDim.x * blockDim.x;
+  for (unsigned long long i = first + (unsigned long long)blockIdx.x * blockDim.x + threadIdx.x; i < end;
+       i += 2 * stride) {
+    const HitRec h0 = load_hit(&p.hits[i]);
+    HitRec h1;
+    h1.a = STC_NONE;
+    if (i + stride < end) h1 = load_hit(&p.hits[i + stride]);
+    const bool v0 = h0.a != STC_NONE, v1 = h1.a != STC_NONE;
+    const unsigned long long k0 = v0 ? stc_cantor(h0.a, h0.b) : 0, k1 = v1 ? stc_cantor(h1.a, h1.b) : 0;
+    const unsigned long long s0 = fast_mod(k0, p.B, p.B_magic), s1 = fast_mod(k1, p.B, p.B_magic);
+    U128 kv0 = {0, 0}, kv1 = {0, 0};
+    float4 m0 = make_float4(0.f, 0.f, 0.f, 0.f), m1 = m0;
+    if (v0) {
+      kv0 = load_slot_pair(&p.slots[s0]);
+      m0 = __ldcg((const float4 *)&p.slots[s0].lo_x);
+    }
+    if (v1) {
+      kv1 = load_slot_pair(&p.slots[s1]);
+      m1 = __ldcg((const float4 *)&p.slots[s1].lo_x);
+    }
+    if (v0) process_hit_at(p, h0, k0, t, s0, kv0, m0);
+    if (v1) process_hit_at(p, h1, k1, t, s1, kv1, m1);
+  }
+}
+
+void step_pairs_part(PipeDev &p, uint32_t part, uint32_t parts, cudaStream_t s) {
+  const unsigned blocks = num_sms() * refine_blocks(p);
+  if (p.job_share) STC_KL k_refine_a<true, true><<<blocks, REFINE_THREADS, 0, s>>>(p, part, parts);
+  else STC_KL k_refine_a<false, true><<<blocks, REFINE_THREADS, 0, s>>>(p, part, parts);
+  STC_KL k_hit_mark<<<1, 1, 0, s>>>(p, part);
+}
+
+// (twice the blocks of k_hits: few hits a thread, so that the pair tests' blocks
+// find room beside them; 16, 32 blocks an SM: 94.2, 89.7 ms a step)
+void step_hits_part(PipeDev &p, uint32_t part, cudaStream_t s) {
+  STC_KL k_hits_part<<<num_sms() * 2 * p.hits_bps, 256, 0, s>>>(p, part);
 }
 
 void step_hits(PipeDev &p, cudaStream_t s) {

@@ -562,7 +562,6 @@ __device__ __forceinline__ bool replay_block(const SchemaDev &sd, const uint32_t
   if (tid == 0) {
     st->splits = (uint32_t)((int)nev + total) / 2;
     st->merges = (uint32_t)((int)nev - total) / 2;
-    st->events = nev;
   }
   return true;
 }
@@ -621,7 +620,6 @@ __device__ void replay_serial(const SchemaDev &sd, uint32_t *grid_count, const u
   }
   st->splits = splits;
   st->merges = merges;
-  st->events = nev;
 }
 
 // The flagged nodes in index order, then their replay. One block: thread t

@@ -45,7 +45,8 @@
 // the halo run on its own and the keys behind it end up in the same slots.
 // The rule is checked on the device before anything is written (fuse_halo);
 // a step that fails it (a loaded table, or more hits in a bin than it holds)
-// takes the general path: k_hits, k_insert_ordered and k_sweep.
+// takes the general path: k_hits, k_insert_ordered and k_sweep. The steps after
+// it are told to beforehand until the tiles would do again (PathChoice).
 //
 // Claims by priority in shared memory are the deferred acceptance of
 // stc_insert.cuh: an empty slot's start word names the hit claiming it (its
@@ -358,14 +359,20 @@ __device__ void tile_unpack(const PipeDev &p, Slot *slots, uint32_t tile, uint32
 }  // namespace
 
 // The largest bin and the largest (occupied slots + hits) of a tile, which
-// decide the step's path (fuse_halo).
+// decide the step's path (fuse_halo). A step told to be general has no bins:
+// the load is the meetings of the step before (PathChoice), if it counted them.
 __global__ void __launch_bounds__(256) k_table_plan(PipeDev p) {
   after_previous();
+  const uint32_t told = p.st->told;
   uint32_t load = 0, most = 0;
   for (uint32_t j = blockIdx.x * blockDim.x + threadIdx.x; j < p.nb; j += gridDim.x * blockDim.x) {
     const uint32_t c = p.bin_cnt[j];
     most = max(most, c);
     load = max(load, c + p.tile_live[j]);
+  }
+  if (told & TOLD_STALE) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) atomicMax(&p.st->tile_load, (unsigned long long)LOAD_UNKNOWN);
+    load = 0;
   }
   load = __reduce_max_sync(0xffffffffu, load);
   most = __reduce_max_sync(0xffffffffu, most);
@@ -645,9 +652,22 @@ void unpack_tiles(PipeDev &p, uint32_t layout, cudaStream_t s) {
   STC_KL k_table_unpack<<<num_sms() * 8, TB_THREADS, 0, s>>>(p, layout);
 }
 
+__global__ void __launch_bounds__(TB_THREADS) k_table_slots(PipeDev p) {
+  __shared__ Slot slots[TILE_SLOTS];
+  const uint32_t layout = p.st->packed;
+  if (layout == TABLE_SLOTS) return;
+  for (uint32_t tile = blockIdx.x; tile < p.nb; tile += gridDim.x) tile_unpack(p, slots, tile, layout);
+}
+__global__ void k_layout_slots(DevState *st) { st->packed = TABLE_SLOTS; }
+
+void step_table_slots(PipeDev &p, cudaStream_t s) {
+  STC_KL k_table_slots<<<num_sms() * 8, TB_THREADS, 0, s>>>(p);
+  STC_KL k_layout_slots<<<1, 1, 0, s>>>(p.st);
+}
+
 void step_table_plan(PipeDev &p, cudaStream_t s) {
   launch_behind(k_table_plan, std::min<unsigned>((p.nb + 255) / 256, (unsigned)num_sms() * 2), 256, 0, s, p);
-  launch_behind(k_table_halo, p.runs, TB_THREADS, sizeof(Tile), s, p);
+  if (!p.general) launch_behind(k_table_halo, p.runs, TB_THREADS, sizeof(Tile), s, p);
 }
 
 void step_table(PipeDev &p, cudaStream_t s) {

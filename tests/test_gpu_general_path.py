@@ -1,12 +1,16 @@
-"""The general path of the table update: its kernels are cut into step_slices
+"""The general path of the table update (csrc/stc_refine.cu): a step that the
+tiles cannot take, and the steps after it, which are told beforehand, leave
+their hits in sequence and update the table beside the pair tests. Against the
+oracle and against each other: on loaded tables, with bins that overflow, in
+plain steps, windows and replayed graphs. Its kernels are cut into step_slices
 launches as the tiled path's are."""
 import numpy as np
 import pytest
 
-from stcdb_gb300.pipeline import Pipeline, StcConfig
+from stcdb_gb300.pipeline import MEETING_DTYPE, Pipeline, StcConfig
 from stcdb_gb300.tracegen import hotspot_grid
 
-from parity import trace_and_box
+from parity import as_tuples, describe_diff, run_pair, trace_and_box
 
 pytestmark = pytest.mark.gpu
 
@@ -46,9 +50,60 @@ def _steps(trace, cfg):
 @pytest.mark.parametrize("per_bin", [1, 40])
 def test_slices_cut_every_long_kernel(trace, slices, per_bin):
     """Pair tests, tiled update, general update and sweep: one launch each, or
-    one a slice."""
+    one a slice. A step told to be general has four parts of pair tests, of
+    their ends' marks and of the update at least, and two forms of the sweep."""
     want, whole, halos = _steps(trace, _config(hit_capacity=391 * per_bin))
     assert 0 in halos
     got, cut, _ = _steps(trace, _config(hit_capacity=391 * per_bin, step_slices=slices))
     assert got == want
-    assert [c - w for c, w in zip(cut, whole)] == [4 * (slices - 1)] * STEPS
+    more = [c - w for c, w in zip(cut, whole)]
+    assert more[0] == 4 * (slices - 1)
+    assert set(more) <= {4 * (slices - 1), 3 * (max(slices, 4) - 4) + 2 * (slices - 1)}
+
+
+@pytest.mark.parametrize("load", [0.3, 0.5, 0.58])
+def test_loaded_table_equals_the_oracle(trace, load):
+    """The crowd at up to `load` live meetings a slot: some steps in tiles, the
+    others general, told and not."""
+    tr, mbr = trace
+    cfg = _config(num_meeting_buckets=1 << 20)
+    live = max(r[3] for r in _steps(trace, cfg)[0])
+    cfg = _config(num_meeting_buckets=int(live / load) | 1)
+    halos, emitted = _steps(trace, cfg)[2], 0
+    for t, g, o, gs, os_ in run_pair(cfg, tr, mbr):
+        assert gs.hits == os_.hits
+        assert np.array_equal(g, o), f"step {t}: " + describe_diff(g, o)
+        emitted += len(o)
+    assert emitted > 0 and (0 in halos or load < 0.5)
+
+
+def _window(trace, cfg, sizes):
+    tr, mbr = trace
+    rows, t = [], 0
+    with Pipeline(cfg, mbr, tr[0]) as p:
+        for n in sizes:
+            m = p.step_window(np.ascontiguousarray(tr[t:t + n]), t, out=np.empty(1 << 20, MEETING_DTYPE))
+            t += n
+            rows.append(np.ascontiguousarray(m).copy())
+            last = p.stats()
+        return np.concatenate(rows), last.hits, last.taken_buckets
+
+
+# records a bin: none to speak of, too few in the crowd's tiles (overflows
+# while the tiles are packed: the pair tests again), room for all
+@pytest.mark.parametrize("graphs", [1, 2])
+@pytest.mark.parametrize("more", [dict(hit_capacity=1), dict(hit_capacity=391 * 40), dict(hit_capacity=391 * 90),
+                                  dict(load=0.5), dict(load=0.5, step_slices=5), {}])
+def test_windows_and_graphs_take_the_same_paths(trace, graphs, more):
+    tr, mbr = trace
+    more = dict(more)
+    if "load" in more:
+        live = max(r[3] for r in _steps(trace, _config(num_meeting_buckets=1 << 20))[0])
+        more["num_meeting_buckets"] = int(live / more.pop("load")) | 1
+    plain, _, halos = _steps(trace, _config(**more))
+    assert ("num_meeting_buckets" not in more and more != dict(hit_capacity=1)) or 0 in halos
+    want = np.concatenate([np.frombuffer(r[0], MEETING_DTYPE) for r in plain])
+    for sizes in ([STEPS], [1, 4, 2, 3]):
+        got, hits, taken = _window(trace, _config(window_graphs=graphs, **more), sizes)
+        assert (hits, taken) == (plain[-1][1], plain[-1][3])
+        assert np.array_equal(as_tuples(got), as_tuples(want))

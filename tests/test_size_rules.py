@@ -20,6 +20,18 @@ extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chun
   for (unsigned i = 0; i < n; i++) sum += jobs_beyond(rows[i], chunks[i], room);
   return sum;
 }
+extern "C" void paths(unsigned steps, const unsigned *load, const unsigned *fullest, const unsigned *live, unsigned cap,
+                      unsigned nb, unsigned *told) {
+  PathChoice c;
+  unsigned row = 0;  // told steps in a row; one in COUNT_EVERY counts its tiles for the next
+  for (unsigned i = 0; i < steps; i++) {
+    told[i] = c.general;
+    const bool known = row % COUNT_EVERY == 0;
+    row = c.general ? row + 1 : 0;
+    if (c.general) c.step_done(true, known ? live[i] : LOAD_UNKNOWN, live[i], cap, nb, TILE_SLOTS);
+    else c.step_done(false, known ? load[i] : LOAD_UNKNOWN, fullest[i], cap, nb, TILE_SLOTS);
+  }
+}
 extern "C" unsigned handed_out(const unsigned *stack, unsigned index, unsigned size) {
   return ids_handed_out(stack, index, size);
 }
@@ -170,3 +182,33 @@ def test_ids_handed_out_are_found_from_the_free_stack(lib):
         assert all(i < high for i in stack[index:high])
         assert stack[high:] == list(range(high, size))
     assert f((ctypes.c_uint * 8)(*range(8)), 8, 8) == 8 and f((ctypes.c_uint * 8)(*range(8)), 3, 8) == 3
+
+
+def _told(lib, load, fullest, live, cap=704, nb=1000):
+    n = len(load)
+    arr = [(ctypes.c_uint * n)(*v) for v in (load, fullest, live)]
+    out = (ctypes.c_uint * n)()
+    lib.paths(n, *arr, cap, nb, out)
+    return list(out)
+
+
+def test_steps_are_told_to_be_general_while_the_tiles_would_not_do(lib):
+    # a table that fills up and empties again: tiles, general from the step
+    # after the first that failed; the ninth of those knows the tiles, in the
+    # fullest of which 320 meetings and a hit for each and a sixteenth are 680
+    live = [100, 200, 300, 340, 360] + [400] * 8 + [320] * 4
+    assert _told(lib, [2 * v for v in live], live, live) == [0] * 5 + [1] * 9 + [0] * 3
+    live = [100, 200, 300, 340, 360] + [400] * 8 + [340] * 4 + [300] * 8
+    assert _told(lib, [2 * v for v in live], live, live) == [0] * 5 + [1] * 17 + [0] * 3
+    # steps stay in tiles whenever they fit
+    assert _told(lib, [10] * 20, [5] * 20, [5] * 20) == [0] * 20
+    # overflowing bins that may not grow
+    assert _told(lib, [10] * 30, [50] * 30, [50] * 30, cap=40) == [0] + [1] * 29
+    # a table of a few tiles has no tiled path to choose
+    assert _told(lib, [900] * 6, [50] * 6, [50] * 6, nb=13) == [0] * 6
+    # a guess that keeps failing (few meetings a tile, more hits than fit): the
+    # first try after a told step finds nothing counted, the next one fails
+    told = _told(lib, [800] * 700, [10] * 700, [100] * 700)
+    tries = [i for i, v in enumerate(told) if not v]
+    gaps = [b - a - 1 for a, b in zip(tries, tries[1:]) if b - a > 1]
+    assert gaps == sorted(gaps) and gaps[0] >= 2 and gaps[-1] >= 64 and len(gaps) < 20
