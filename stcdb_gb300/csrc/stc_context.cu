@@ -714,8 +714,8 @@ static uint32_t bins_wanted(const stc_ctx *c, unsigned long long fullest, unsign
 static void choose_path(stc_ctx *c) {
   const DevState &st = *c->st_host;
   const bool told = st.halo == HALO_TOLD;
-  const unsigned long long fullest = !told ? st.hit_max : st.tile_load == LOAD_UNKNOWN ? 0 : st.tile_load + st.tile_load / 16;
-  c->path.step_done(told, st.tile_load, fullest, bins_wanted(c, fullest, st.hits), c->p.nb, c->p.B / c->p.nb);
+  const unsigned long long fullest = !told ? st.hit_max : st.tile_load == LOAD_UNKNOWN ? 0 : st.tile_load;
+  c->path.step_done(told, st.tile_load, fullest, bins_wanted(c, fullest, st.hits), c->p.nb, c->p.B);
 }
 
 // Counters of the step whose state is in c->st_host.
@@ -746,7 +746,6 @@ static void fill_stats(stc_ctx *c, uint32_t t, const float *phase, float step_ms
   o.memtable_keys = h.kv_count;
   c->stepped = true;
   c->last_t = t;
-  choose_path(c);
 }
 
 // The reference flushes once a step leaves more keys than kv_restriction
@@ -832,6 +831,7 @@ static stc_status run_step(stc_ctx *c, const double2 *xy, uint32_t t, bool copie
   float tot = 0;
   cudaEventElapsedTime(&tot, c->ev[PH_START], c->ev[PH_SCHEMA]);
   fill_stats(c, t, phase, tot, (uint32_t)(tl_launches - launches0));
+  choose_path(c);
   grow_hits(c, bins_wanted(c, bin_need(c), c->st_host->hits));
   if (flush_due(c)) return flush_now(c, t);
   return STC_OK;
@@ -1087,6 +1087,7 @@ extern "C" stc_status stc_step_window(stc_ctx *c, const double *xy, int on_devic
     cudaGetLastError();
     float phase[8] = {0, 0, 0, 0, 0, 0, 0, app};
     fill_stats(c, t0 + i, phase, core + app, (uint32_t)launches[b]);
+    choose_path(c);
     return STC_OK;
   };
 

@@ -168,10 +168,8 @@ __device__ __forceinline__ void bin_hit(const PipeDev &p, const HitRec &h, uint3
 // taken (508M hits in windows of 64, 256, up to 1024: 102, 94, 94 ms a step, by
 // the shared counter), and the rest of its last ones stay empty (a = STC_NONE).
 // Random to the table, but the update of one part runs beside the tests of the
-// next, and a crowd's long walks are spread over all warps. Stress model, ms a
-// step with bins and k_hits behind all pair tests, and this way: 1M objects at
-// 0.47 meetings a slot 104, 90; 200k at 0.35 3.68, 3.73, at 0.5 5.2, 5.3, at 0.6
-// 80, 40.
+// next, and a crowd's long walks are spread over all warps (figures at
+// PathChoice).
 constexpr uint32_t HIT_WINDOW = 64, HIT_WINDOW_MOST = 1024;
 struct HitWindow {
   unsigned long long next, end;  // the same for the whole warp
@@ -497,13 +495,13 @@ __global__ void __launch_bounds__(256, 5) k_hits(PipeDev p, uint32_t part, uint3
     return;
   }
   const uint32_t t = p.st->step_t;
-  const unsigned long long warps = ((unsigned long long)gridDim.x * blockDim.x) >> 5;
   const uint32_t turns = (min((uint32_t)p.st->hit_max, p.bin_cap) + HITS_LANE - 1) / HITS_LANE;  // of the fullest bin
-  const unsigned long long groups = (p.nb + 31u) / 32u;
-  const unsigned long long g0 = groups * part / parts, g1 = groups * (part + 1) / parts;
-  for (unsigned long long w = ((unsigned long long)blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < (g1 - g0) * turns;
-       w += warps) {
-    const uint32_t bin = (uint32_t)(g0 + w / turns) * 32u + lane_id(), i0 = (uint32_t)(w % turns) * HITS_LANE;
+  const uint32_t groups = (p.nb + 31u) / 32u;
+  const uint32_t g0 = (uint32_t)((unsigned long long)groups * part / parts);
+  // (a 256th of the records that the buffer has room for, about)
+  const uint32_t total = ((uint32_t)((unsigned long long)groups * (part + 1) / parts) - g0) * turns;
+  for (uint32_t w = (blockIdx.x * blockDim.x + threadIdx.x) >> 5; w < total; w += (gridDim.x * blockDim.x) >> 5) {
+    const uint32_t bin = (g0 + w / turns) * 32u + lane_id(), i0 = w % turns * HITS_LANE;
     if (bin >= p.nb) continue;
     const uint32_t n = min(min(p.bin_cnt[bin], p.bin_cap), i0 + HITS_LANE);
     for (uint32_t i = i0; i < n; i += 2) {

@@ -45,33 +45,46 @@ __host__ __device__ __forceinline__ uint32_t halo_tiles(unsigned long long load,
   return 0;
 }
 
-// Whether the next step is told beforehand to take the general path (its pair
-// tests then leave the hits in sequence, and the table update runs beside
-// them), from each step's counters. A step that the tiles could not take says
-// yes. After that, the fullest tile of the step before says whether the tiles
-// would do again: its meetings, and a hit for each. That guess can be wrong
-// (hits of one tile whose meetings lie in the next), so a wrong one is followed
-// by twice as many general steps as the last, up to 64.
+// What general steps do, and whether the next step is told beforehand to be one,
+// from each step's counters. A step that the tiles cannot take finds its hits in
+// bins and updates the table bin by bin (k_hits). A step told to be general
+// leaves them in sequence, and its table update runs beside the pair tests
+// (k_hits_part), which also spreads a crowded table's long walks: general steps
+// of the stress model by bins and told, ms, at 0.35 to 0.59 meetings a slot: 200k
+// objects (1.3 to 2.1 GB of slots) 4.4 and 3.9, 5.2 and 5.0, 34 and 18; 700k (19
+// GB) 55 and 47; 1M (34 GB) 107 and 88; 1.4M (69 GB) 165 and 134. A larger table
+// is out of reach of the address translation, and the bins' locality counts for
+// more: at 137 GB 1.9M objects 274 and 390, the hotspot model at 10M 340 and 460.
+// So a step that the tiles could not take tells the next ones, in tables of up
+// to TOLD_MOST_SLOTS (103 GB).
+// Told steps cannot see whether the tiles would do again. The fullest tile of
+// the step before is the guess: its meetings, and a hit for each, less a
+// sixteenth, since the tile with most meetings is seldom the one with most
+// hits. It can be wrong (hits of one tile whose meetings lie in the next): a
+// wrong one is followed by twice as many told steps as the last, up to 64.
 // Told steps count their tiles' meetings one time in COUNT_EVERY: the marks
 // cost the sweep of 507M meetings 4.7 of 14.4 ms.
+constexpr uint64_t TOLD_MOST_SLOTS = 3ull << 30;
 constexpr uint64_t LOAD_UNKNOWN = ~0ull;  // the step before did not count
 constexpr uint32_t COUNT_EVERY = 8;
 struct PathChoice {
-  bool general = false;
+  bool general = false;  // tell the next step
   uint32_t wait = 0, next_wait = 2;
-  // told: the step was told to. load: meetings and hits of its fullest tile
-  // (told: meetings of the step before). fullest: hits of its fullest bin (told:
-  // not used). cap: records a bin may have.
+  // One step, in the order of their issue. told: it was told to. load: meetings
+  // and hits of its fullest tile (told: meetings of the step before). fullest:
+  // hits of its fullest bin (told: not used). cap: records a bin may have.
+  // slots: of the table.
   void step_done(bool told, uint64_t load, uint64_t fullest, uint32_t cap, uint32_t nb, uint64_t slots) {
-    if (nb < MIN_TILES) return;
+    if (nb < MIN_TILES || slots > TOLD_MOST_SLOTS) return;
     if (told) {
       if (wait) wait--;
-      if (!wait && load != LOAD_UNKNOWN && load + load / 16 <= cap && halo_tiles(2 * load + load / 8, nb, slots))
-        general = false;
+      if (wait || load == LOAD_UNKNOWN) return;
+      const uint64_t guess = load - load / 16;
+      if (guess <= cap && halo_tiles(2 * guess, nb, slots / nb)) general = false;
       return;
     }
-    if (load == LOAD_UNKNOWN) return;  // it has counted, the next one shows
-    general = fullest > cap || !halo_tiles(load, nb, slots);
+    if (load == LOAD_UNKNOWN) return;  // a told one before it did not count; the next one shows
+    general = fullest > cap || !halo_tiles(load, nb, slots / nb);
     if (!general) {
       next_wait = 2;
       return;

@@ -1,6 +1,6 @@
 """The general path of the table update (csrc/stc_refine.cu): a step that the
-tiles cannot take, and the steps after it, which are told beforehand, leave
-their hits in sequence and update the table beside the pair tests. Against the
+tiles cannot take goes by its bins; steps after it may be told beforehand to
+leave their hits in sequence and update the table beside the pair tests. Against the
 oracle and against each other: on loaded tables, with bins that overflow, in
 plain steps, windows and replayed graphs. Its kernels are cut into step_slices
 launches as the tiled path's are."""
@@ -56,9 +56,11 @@ def test_slices_cut_every_long_kernel(trace, slices, per_bin):
     assert 0 in halos
     got, cut, _ = _steps(trace, _config(hit_capacity=391 * per_bin, step_slices=slices))
     assert got == want
-    more = [c - w for c, w in zip(cut, whole)]
-    assert more[0] == 4 * (slices - 1)
-    assert set(more) <= {4 * (slices - 1), 3 * (max(slices, 4) - 4) + 2 * (slices - 1)}
+    told = whole[0] - 5 + 16  # for the five kernels of one launch each: 2 + 4 * 3 + 2 launches
+    assert set(whole) <= {whole[0], told}
+    bins_cut, told_cut = whole[0] + 4 * (slices - 1), told + 3 * (max(slices, 4) - 4) + 2 * (slices - 1)
+    assert cut[0] == bins_cut and set(cut) <= {bins_cut, told_cut}
+    assert per_bin > 1 or cut[1:] == [told_cut] * (STEPS - 1)  # every step is general
 
 
 @pytest.mark.parametrize("load", [0.3, 0.5, 0.58])

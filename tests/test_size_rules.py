@@ -13,6 +13,7 @@ SHIM = r"""
 #define __host__
 #define __device__
 #define __forceinline__ inline
+#include <vector>
 #include "stc_rules.cuh"
 using namespace stc;
 extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chunks, unsigned n, unsigned long long room) {
@@ -21,15 +22,21 @@ extern "C" unsigned block_jobs_beyond(const unsigned *rows, const unsigned *chun
   return sum;
 }
 extern "C" void paths(unsigned steps, const unsigned *load, const unsigned *fullest, const unsigned *live, unsigned cap,
-                      unsigned nb, unsigned *told) {
+                      unsigned nb, unsigned lag, unsigned *told) {
   PathChoice c;
   unsigned row = 0;  // told steps in a row; one in COUNT_EVERY counts its tiles for the next
-  for (unsigned i = 0; i < steps; i++) {
-    told[i] = c.general;
-    const bool known = row % COUNT_EVERY == 0;
-    row = c.general ? row + 1 : 0;
-    if (c.general) c.step_done(true, known ? live[i] : LOAD_UNKNOWN, live[i], cap, nb, TILE_SLOTS);
-    else c.step_done(false, known ? load[i] : LOAD_UNKNOWN, fullest[i], cap, nb, TILE_SLOTS);
+  std::vector<bool> known;
+  for (unsigned i = 0; i < steps + lag; i++) {
+    if (i < steps) {
+      told[i] = c.general;
+      known.push_back(row % COUNT_EVERY == 0);
+      row = c.general ? row + 1 : 0;
+    }
+    if (i < lag) continue;
+    const unsigned j = i - lag;  // the state that is taken after step i was issued
+    const unsigned long long slots = (unsigned long long)nb * TILE_SLOTS;
+    if (told[j]) c.step_done(true, known[j] ? live[j] : LOAD_UNKNOWN, live[j], cap, nb, slots);
+    else c.step_done(false, known[j] ? load[j] : LOAD_UNKNOWN, fullest[j], cap, nb, slots);
   }
 }
 extern "C" unsigned handed_out(const unsigned *stack, unsigned index, unsigned size) {
@@ -184,31 +191,34 @@ def test_ids_handed_out_are_found_from_the_free_stack(lib):
     assert f((ctypes.c_uint * 8)(*range(8)), 8, 8) == 8 and f((ctypes.c_uint * 8)(*range(8)), 3, 8) == 3
 
 
-def _told(lib, load, fullest, live, cap=704, nb=1000):
+def _told(lib, load, fullest, live, cap=704, nb=1000, lag=0):
     n = len(load)
     arr = [(ctypes.c_uint * n)(*v) for v in (load, fullest, live)]
     out = (ctypes.c_uint * n)()
-    lib.paths(n, *arr, cap, nb, out)
+    lib.paths(n, *arr, cap, nb, lag, out)
     return list(out)
 
 
-def test_steps_are_told_to_be_general_while_the_tiles_would_not_do(lib):
-    # a table that fills up and empties again: tiles, general from the step
-    # after the first that failed; the ninth of those knows the tiles, in the
-    # fullest of which 320 meetings and a hit for each and a sixteenth are 680
-    live = [100, 200, 300, 340, 360] + [400] * 8 + [320] * 4
-    assert _told(lib, [2 * v for v in live], live, live) == [0] * 5 + [1] * 9 + [0] * 3
-    live = [100, 200, 300, 340, 360] + [400] * 8 + [340] * 4 + [300] * 8
-    assert _told(lib, [2 * v for v in live], live, live) == [0] * 5 + [1] * 17 + [0] * 3
-    # steps stay in tiles whenever they fit
-    assert _told(lib, [10] * 20, [5] * 20, [5] * 20) == [0] * 20
-    # overflowing bins that may not grow
-    assert _told(lib, [10] * 30, [50] * 30, [50] * 30, cap=40) == [0] + [1] * 29
-    # a table of a few tiles has no tiled path to choose
-    assert _told(lib, [900] * 6, [50] * 6, [50] * 6, nb=13) == [0] * 6
-    # a guess that keeps failing (few meetings a tile, more hits than fit): the
-    # first try after a told step finds nothing counted, the next one fails
-    told = _told(lib, [800] * 700, [10] * 700, [100] * 700)
-    tries = [i for i, v in enumerate(told) if not v]
-    gaps = [b - a - 1 for a, b in zip(tries, tries[1:]) if b - a > 1]
-    assert gaps == sorted(gaps) and gaps[0] >= 2 and gaps[-1] >= 64 and len(gaps) < 20
+@pytest.mark.parametrize("lag", [0, 1, 2])
+def test_steps_are_told_to_be_general_while_the_tiles_would_not_do(lib, lag):
+    n = 600
+    fits, full = ([300] * n, [150] * n, [150] * n), ([800] * n, [400] * n, [400] * n)
+    assert _told(lib, *fits, lag=lag) == [0] * n
+    for cap, nb in [(704, 1000), (40, 1000)]:  # too full tiles, or bins that may not grow
+        assert _told(lib, *full, cap=cap, nb=nb, lag=lag) == [0] * (1 + lag) + [1] * (n - 1 - lag)
+    assert sum(_told(lib, *fits, cap=140, lag=lag)) > 0.8 * n  # tried again, 141 of 140 guessed
+    assert _told(lib, *full, nb=13, lag=lag) == [0] * n        # no tiles to choose
+    assert _told(lib, *full, nb=4194304, lag=lag)[-1] == 1     # 3 * 2^30 slots
+    assert _told(lib, *full, nb=4194305, lag=lag) == [0] * n
+
+
+@pytest.mark.parametrize("lag", [0, 1, 2])
+def test_told_steps_go_back_to_tiles_when_they_would_do(lib, lag):
+    """A table that fills up and empties again, and a guess that keeps failing."""
+    live = [200] * 50 + [400] * 100 + [340] * 400
+    told = _told(lib, [2 * v for v in live], live, live, lag=lag)
+    assert sum(told[:50]) == 0 and sum(told[50:150]) >= 99 - lag and sum(told[165:]) == 0
+    # few meetings a tile, more hits than fit: tried again ever more seldom
+    n = 3000
+    told = _told(lib, [800] * n, [10] * n, [100] * n, lag=lag)
+    assert sum(told[:100]) > 50 and sum(told[500:]) > 0.9 * (n - 500)
