@@ -109,3 +109,32 @@ def test_windows_and_graphs_take_the_same_paths(trace, graphs, more):
         got, hits, taken = _window(trace, _config(window_graphs=graphs, **more), sizes)
         assert (hits, taken) == (plain[-1][1], plain[-1][3])
         assert np.array_equal(as_tuples(got), as_tuples(want))
+
+
+# records a bin of 391 tiles: none to speak of (general from the second step on),
+# some overflow while the tiles are packed, so that the pair tests run again
+@pytest.mark.parametrize("per_bin", [1, 8, 40, 90])
+@pytest.mark.parametrize("graphs", [0, 1])
+def test_overflowing_bins_equal_the_oracle(trace, per_bin, graphs):
+    """Against a run with room for every hit, and the oracle: plain steps, and
+    a window of replayed graphs."""
+    import oracle
+    tr, mbr = trace
+    cfg = _config(hit_capacity=391 * per_bin, window_graphs=graphs)
+    ref = oracle.Oracle(cfg, mbr, tr[0])
+    try:
+        want = [as_tuples(ref.step(tr[t], t)) for t in range(STEPS)]
+    finally:
+        ref.close()
+    assert sum(len(w) for w in want) > 0
+    if graphs:
+        got, _, _ = _window(trace, cfg, [3, STEPS - 3])
+        assert np.array_equal(as_tuples(got), as_tuples(np.concatenate(want)))
+        return
+    rows, _, halos = _steps(trace, cfg)
+    room, _, tiled = _steps(trace, _config())
+    assert 0 in halos and 0 not in tiled
+    assert rows == room
+    for t in range(STEPS):
+        got = as_tuples(np.frombuffer(rows[t][0], MEETING_DTYPE))
+        assert np.array_equal(got, want[t]), f"step {t}: " + describe_diff(got, want[t])
