@@ -1,4 +1,5 @@
-"""Benchmark of the GB300 co-occurrence pipeline (one JSON line on rank 0).
+"""Benchmark of the GB300 co-occurrence pipeline: one JSON line on stdout of
+rank 0 (short_line), and all figures in another on stderr.
 
 A step is one time step of the hot path over all objects: partition, border
 lookup, refinement, meeting-table insert, expire/emit sweep and quadtree
@@ -76,9 +77,6 @@ METRIC = "pos-updates/s at 10M objs (bit-exact meetings); query p50/p99 under in
 UNIT = "pos-updates/s"
 
 WORKLOADS = {
-    # launch shape chosen by stc_autotune on 8 steps of this workload (4
-    # pair-test and 32 table-update blocks per SM: 15.12 -> 14.80 ms a step);
-    # it does not change results
     "uniform-10M": dict(objects=10_000_000, hot=0, reach=10.0, min_meet=5, grid_capacity=200, amplify=2.0,
                         buckets=1 << 28, kv_restriction=1 << 27),
     "hotspot-1M": dict(objects=1_000_000, hot=1000, reach=10.0, min_meet=5, grid_capacity=200, amplify=8.0,
@@ -960,6 +958,34 @@ def cpu_baseline(w, warmup, steps, threads, sample_note):
             "sample": sample_note.format(steps=steps, first=warmup, last=warmup + steps - 1, seconds=round(dt, 2))}
 
 
+def short_line(full):
+    """The line for stdout: what the metric, its configuration and its checks
+    need, in under 1450 characters, since a reader may keep only the end of an
+    output. The full line, with the phases, the flush, the compaction, the
+    batched windows and the queries in detail, goes to stderr."""
+    def cut(d, *names):
+        return {k: d[k] for k in names if k in d} if d else None
+
+    def num(v):
+        return float(f"{v:.6g}") if isinstance(v, float) else v
+
+    def trim(v):
+        return {k: trim(x) for k, x in v.items()} if isinstance(v, dict) else num(v)
+
+    line = cut(full, "metric", "value", "unit", "n_gpus", "steps", "warmup", "ms_per_step", "higher_is_better",
+               "scaling", "vs_baseline", "dtype", "data")
+    line["config"] = cut(full["config"], "workload", "objects", "street_grid", "hotspots", "reach_m", "min_meet_steps",
+                         "leaf_capacity", "meeting_buckets", "memtable", "l2", "parallelism")
+    line["e2e"] = cut(full["e2e"], "value", "unit", "h2d_bytes_per_step", "d2h_bytes_per_step")
+    line["gpu_launches"] = full["gpu_launches"]
+    line["clocks"] = cut(full["clocks"], "sm_mhz", "sm_max_mhz", "reasons")
+    line["bit_exact"] = full["bit_exact"]
+    line["queries_under_ingest"] = trim(cut(full["queries_under_ingest"], "p50_ms", "p99_ms", "qps",
+                                            "ingest_pos_updates_per_s"))
+    line["roofline"] = trim(cut(full["roofline"], "kernel", "achieved", "peak", "unit", "frac"))
+    return line
+
+
 def main():
     ap = argparse.ArgumentParser()
     ap.add_argument("--gpus", type=int, default=1)
@@ -998,7 +1024,7 @@ def main():
                     "leaf_capacity": w["grid_capacity"], "grid_amplify": w["amplify"],
                     "launch_shape": {"refine_blocks_per_sm": w.get("refine_bps", 0),  # 0: the library's choice
                                      "hits_blocks_per_sm": w.get("hits_bps", 0),
-                                     "refine_chunk": w.get("refine_chunk") or "by density (32, 64 or 256)"},
+                                     "refine_chunk": w.get("refine_chunk") or "by density (16 to 256)"},
                     "meeting_buckets": make_cfg(w).resolved().num_meeting_buckets,
                     "memtable": (f"on, flush past {w['kv_restriction']} directed keys, 100 CTFs, "
                                  f"{w.get('bitmap_edge', 256)}x{w.get('bitmap_edge', 256)} map bitmaps"
@@ -1081,17 +1107,8 @@ def main():
         "clocks": r["clocks"],
         "cpu_baseline": base,
     }
-    # the figures a reader of the line's tail needs, repeated last
-    q = r["queries"] or {}
-    line["summary"] = {"value": value, "e2e": e2e, "bit_exact": line["bit_exact"],
-                       "query_p50_ms": q.get("p50_ms"), "query_p99_ms": q.get("p99_ms"),
-                       "query_max_ms": q.get("max_ms"), "queries_per_s": q.get("qps"),
-                       "ingest_pos_updates_per_s_while_serving": q.get("ingest_pos_updates_per_s"),
-                       "ingest_pos_updates_per_s_while_serving_hbm_input":
-                           (r["queries_hbm"] or {}).get("ingest_pos_updates_per_s"),
-                       "query_p99_ms_hbm_input": (r["queries_hbm"] or {}).get("p99_ms"),
-                       "roofline_frac": line["roofline"]["frac"]}
-    print(json.dumps(line), flush=True)
+    print(json.dumps(line), file=sys.stderr, flush=True)
+    print(json.dumps(short_line(line)), flush=True)
 
 
 if __name__ == "__main__":
