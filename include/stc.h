@@ -128,9 +128,10 @@ typedef struct stc_config {
   uint32_t refine_chunk;         /* refinement tile length: a job tests 32 rows against this many
                                     positions of their candidate windows (launch shape, results do
                                     not depend on it); a multiple of 32 from 32 to 4096; 0 =
-                                    automatic, per step: 32 when there are too few rows to fill the
-                                    GPU several times over, 64 when the step before tested more than
-                                    16 candidates per checking unit (dense leaves), else 256 */
+                                    automatic, per step: 32 (16 with few tests in all) when there are
+                                    too few rows to fill the GPU several times over, 64 when the
+                                    step before tested more than 16 candidates per checking unit
+                                    (dense leaves), else 256 */
 } stc_config;
 
 /* Replay quadtree splits/merges on one device thread only (tests compare it

@@ -63,7 +63,8 @@ struct NodeMeta {
 };
 
 // One pair within reach found by the refinement, waiting to be applied to
-// the meeting table: the pair (a < b; a = STC_NONE marks an unused record),
+// the meeting table: the pair (a < b; a = STC_NONE marks an unused place of a
+// step that leaves its hits in sequence),
 // its priority and its MBR contribution, the box of the two objects' float
 // positions of the step (lo = fminf(a's, b's), hi = fmaxf(a's, b's)).
 // The key cantor(a, b) is rebuilt when applied. Carrying the box saves the
@@ -109,7 +110,7 @@ struct DevState {
   unsigned long long hit_count;       // places taken in the hit buffer by a step told to be general
   unsigned long long fast_claims;     // new meetings started this step (claims finalised by the sweep)
   unsigned long long hit_max;         // most hits of a table tile this step
-  uint32_t schema_path;               // 1 parallel replay, 2 serial (cascade), 0 serial (other)
+  uint32_t schema_path;               // 1 parallel replay; by one thread: 2 (a cascade, or many events), 0 (asked to)
   uint32_t same_t;                    // the step's time is the last step's
   // memtable (stc_lsm.cu)
   unsigned long long kv_count;        // directed keys in the memtable

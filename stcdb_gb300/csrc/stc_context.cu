@@ -86,7 +86,6 @@ struct stc_ctx {
   cudaEvent_t wev[2][4] = {};                     // start of the core, start and end of the append,
                                                   // core's start once its positions are in
   cudaStream_t drain_stream = nullptr;            // meetings of a window go out here beside the next step
-  cudaEvent_t drained_ev = nullptr;
   // the step's core captured as a CUDA graph, replayed by stc_step_window;
   // it holds the pipeline's arguments by value, so anything that changes
   // them (a flush, the slice count, a larger hit buffer) invalidates it; one
@@ -205,7 +204,6 @@ static void destroy_all(stc_ctx *c) {
     for (cudaEvent_t ev : c->wev[i])
       if (ev) cudaEventDestroy(ev);
   }
-  if (c->drained_ev) cudaEventDestroy(c->drained_ev);
   if (c->drain_stream) cudaStreamDestroy(c->drain_stream);
   for (int i = 0; i < WIN_BUFS; i++) {
     if (c->graph[i]) cudaGraphExecDestroy(c->graph[i]);
@@ -358,7 +356,6 @@ static stc_status create_ctx(const stc_config *cfg, const double mbr[4], const d
   }
   for (int i = 0; i < WIN_BUFS && e == cudaSuccess; i++) e = cudaEventCreate(&c->core_ev[i]);
   if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&c->drain_stream, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaEventCreateWithFlags(&c->drained_ev, cudaEventDisableTiming);
   if (e == cudaSuccess) e = table_prepare();
   for (int i = 0; i < 2 && e == cudaSuccess; i++) {
     e = cudaMallocHost(&c->drain_stage[i], DRAIN_CHUNK);
@@ -775,8 +772,8 @@ static void grow_hits(stc_ctx *c, uint32_t cap) {
 
 // Tile length of the refinement's jobs when stc_config.refine_chunk is 0.
 // With fewer than FEW_ROW_BLOCKS row blocks of 32 checking units a warp, the
-// pair tests end with a few warps in the longest jobs, so the tiles are as
-// short as they go (32: hotspot window of 300k objects, 10k row blocks, 0.68
+// pair tests end with a few warps in the longest jobs, so the tiles are
+// short (32: hotspot window of 300k objects, 10k row blocks, 0.68
 // ms of pair tests and table update with 256, 0.47 with 64, 0.39 with 32; at
 // 24k row blocks all lengths are within 2%), half that where some
 // units have several tests (four on average) but all tests fewer than FEW_TESTS, seven
@@ -798,7 +795,7 @@ static void choose_refine_chunk(stc_ctx *c) {
     const DevState &st = *c->st_host;  // the last step's counters
     const unsigned long long units = (unsigned long long)p.N + st.border_units;
     if (units / 32 < FEW_ROW_BLOCKS * 32 * (unsigned long long)num_sms())
-      chunk = st.tests > 4 * units && st.tests < FEW_TESTS ? REFINE_CHUNK_FEW / 2 : REFINE_CHUNK_FEW;
+      chunk = st.tests > 4 * units && st.tests < FEW_TESTS ? REFINE_CHUNK_FEWEST : REFINE_CHUNK_FEW;
     else
       chunk = st.tests > SHORT_TILE_TESTS_PER_UNIT * units ? REFINE_CHUNK_DENSE : REFINE_CHUNK_DEFAULT;
   }

@@ -30,7 +30,8 @@ enum { CTR_MEMBERS = 0, CTR_SMALL, CTR_BIG, CTR_EXTRA, CTR_UNITS, CTR_POOL, CTR_
 // ranges are cut into chunks of this many, so that the n^2 / 2 pair tests of
 // a dense leaf spread over many warps.
 constexpr uint32_t REFINE_CHUNK_DEFAULT = 256;  // tile length before the first step's density is known
-constexpr uint32_t REFINE_CHUNK_DENSE = 64, REFINE_CHUNK_FEW = 32;  // of dense leaves, of few rows (choose_refine_chunk)
+// of dense leaves, of few rows, of few rows with few tests (choose_refine_chunk)
+constexpr uint32_t REFINE_CHUNK_DENSE = 64, REFINE_CHUNK_FEW = 32, REFINE_CHUNK_FEWEST = 16;
 
 struct PipeDev {
   // sizes
@@ -52,7 +53,7 @@ struct PipeDev {
   uint32_t job_chunk;              // refinement jobs a warp takes at a time (stc_config.job_chunk)
   uint32_t general;                // 1: this step takes the general path, whatever its tiles (PathChoice)
   uint32_t job_share;              // 1: or one at a time from a common counter (job_shares)
-  uint32_t refine_chunk;               // candidate positions per refinement job (a multiple of 32)
+  uint32_t refine_chunk;               // candidate positions per refinement job (16 or a multiple of 32)
   uint32_t refine_bps, hits_bps;   // blocks per SM of the pair tests (0: step_pairs chooses) and of the table update
   // state
   DevState *st;

@@ -56,7 +56,6 @@ struct SchemaWork {
   NodeMeta *bmeta;
   uint32_t *bcount, *bsub_nodes, *bsub_leaves, *bpre, *bleafbase;
   uint32_t *node_of;      // N
-  uint32_t *level_start;  // host mirror kept in SchemaBuilder
   // update temporaries
   uint8_t *ev_flag;       // S, padded with zeros to a multiple of 16 (0 none, 1 split, 2 merge)
   uint32_t *ev_list;      // S

@@ -69,7 +69,7 @@ constexpr uint32_t TB_RECS = 256;       // hits whose pair and order are held in
 constexpr uint32_t TB_STAGE = 48;       // emitted meetings staged per block
 constexpr uint32_t TB_DUPS = 64;        // hits of possible double pairs listed per tile
 
-// 26 KB, eight blocks an SM: a tile is a chain of short phases of a hundred or
+// 27.5 KB, eight blocks an SM with no byte to spare: a tile is a chain of short phases of a hundred or
 // two items each, so many blocks of few warps keep the SM busy. It holds what
 // the phases look up at random, the keys and each hit's pair and order; boxes
 // and start times stay in global memory (L2 by then) until the write-back
