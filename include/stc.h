@@ -175,7 +175,8 @@ typedef struct stc_stats {
   uint32_t ambiguous_tests;      /* distance decisions within a few ulp of reach, where
                                     the last bit of sin() could matter */
   float step_ms;                 /* device time of the step */
-  float phase_ms[8];             /* partition, border+jobs, refine (pair tests), insert (plan of the table
+  float phase_ms[8];             /* partition, border+jobs, refine (pair tests, and the table update where
+                                    general steps follow each other), insert (plan of the table
                                     update: what is carried into its runs), sweep (table update, expiry and
                                     emission), schema, copy-in, memtable append */
   uint64_t memtable_keys;        /* directed keys in the memtable after the step (and any flush) */
